@@ -7,6 +7,7 @@
 #include <torch/csrc/distributed/c10d/ProcessGroup.hpp>
 #include <torch/csrc/distributed/c10d/symm_mem/SymmetricMemory.hpp>
 
+#include <algorithm>
 #include <cstring>
 #include <sstream>
 
@@ -109,6 +110,9 @@ Group::Group(std::string group_name, int64_t rank, int64_t world, int64_t device
 
 Group::~Group()
 {
+    if (order_event_) {
+        cudaEventDestroy(order_event_);
+    }
     // Windows may still be the target of a kernel in flight on some stream; wait for the device
     // before the allocations go back. No collective here: a destructor is no place for one.
     if (alive_ && on_cuda() && (!windows_.empty() || lend_calls_ > 0)) {
@@ -129,6 +133,24 @@ void Group::check_alive() const
 const Plan& Group::plan(at::IntArrayRef sizes, at::IntArrayRef strides, at::ScalarType dtype, int64_t mode,
                         const Splits& seq, const Splits& heads)
 {
+    const std::lock_guard<std::mutex> lock(plan_mutex_);
+    const bool plain = !seq.has_value() && !heads.has_value() && sizes.size() == 4 && (strides.empty() || strides.size() == 4);
+    if (plain && last_plan_.plan && last_plan_.mode == mode && last_plan_.dtype == dtype
+        && std::equal(sizes.begin(), sizes.end(), last_plan_.sizes) && last_plan_.strided == !strides.empty()
+        && (strides.empty() || std::equal(strides.begin(), strides.end(), last_plan_.strides))) {
+        return *last_plan_.plan;
+    }
+    auto remember = [&](const Plan& found) -> const Plan& {
+        if (plain) {
+            last_plan_.mode    = mode;
+            last_plan_.dtype   = dtype;
+            last_plan_.strided = !strides.empty();
+            std::copy(sizes.begin(), sizes.end(), last_plan_.sizes);
+            std::copy(strides.begin(), strides.end(), last_plan_.strides);
+            last_plan_.plan = &found;  // map nodes do not move; clear() below forgets it
+        }
+        return found;
+    };
     std::vector<int64_t> key;
     key.reserve(16 + 2 * world_);
     key.push_back(mode);
@@ -147,7 +169,7 @@ const Plan& Group::plan(at::IntArrayRef sizes, at::IntArrayRef strides, at::Scal
     }
     auto it = plans_.find(key);
     if (it != plans_.end()) {
-        return it->second;
+        return remember(it->second);
     }
     const Geometry       g    = geometry_for(sizes, dtype, mode, world_, rank_, seq, heads);
     const int64_t        elem = static_cast<int64_t>(c10::elementSize(dtype));
@@ -167,9 +189,10 @@ const Plan& Group::plan(at::IntArrayRef sizes, at::IntArrayRef strides, at::Scal
                 "this call moves no data: every rank's shard is empty. Check the shape and the splits -- a "
                 "sequence or head axis of 0 on ALL ranks has nothing to exchange");
     if (plans_.size() >= kPlanCacheCap) {
+        last_plan_.plan = nullptr;
         plans_.clear();
     }
-    return plans_.emplace(std::move(key), std::move(p)).first->second;
+    return remember(plans_.emplace(std::move(key), std::move(p)).first->second);
 }
 
 Window Group::allocate(int64_t bytes)
@@ -480,6 +503,16 @@ void Group::barrier(Role role, void* stream)
     TORCH_CHECK(rc == FU_OK, "fast_ulysses_b200: ", fu_last_error());
 }
 
+void Group::order_streams(void* from, void* to)
+{
+    const std::lock_guard<std::mutex> lock(order_mutex_);
+    if (!order_event_) {
+        cuda_ok(cudaEventCreateWithFlags(&order_event_, cudaEventDisableTiming), "cudaEventCreateWithFlags");
+    }
+    cuda_ok(cudaEventRecord(order_event_, static_cast<cudaStream_t>(from)), "cudaEventRecord");
+    cuda_ok(cudaStreamWaitEvent(static_cast<cudaStream_t>(to), order_event_, 0), "cudaStreamWaitEvent");
+}
+
 void Group::run_cpu(const Plan& plan, const at::Tensor& x, at::Tensor& out)
 {
     // The same routes, executed as: pack each peer's share densely, one all_to_all over the
@@ -565,7 +598,7 @@ void Group::check()
                     ". The result of that call is not valid.");
     };
     for (auto& kv : windows_) {
-        probe(kv.second, kv.first == 0 ? "sync" : "async");
+        probe(kv.second, kv.first == 0 ? "sync" : kv.first == 1 ? "async" : "fp8");
     }
     for (auto& w : lent_) {
         probe(w, "lent");
@@ -627,6 +660,7 @@ void Group::destroy()
         const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_index_));
         cudaDeviceSynchronize();
     }
+    last_plan_.plan = nullptr;
     plans_.clear();
     windows_.clear();
     pool_.clear();

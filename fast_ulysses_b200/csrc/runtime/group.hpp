@@ -11,12 +11,14 @@
 // pool (the kernel reads the caller's tensor directly); the handshake state is a FuCtrl block at
 // the tail of each window rather than a slice of torch's signal pad.
 #include <ATen/ATen.h>
+#include <cuda_runtime_api.h>
 #include <torch/custom_class.h>
 
 #include <array>
 #include <atomic>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <optional>
 #include <string>
 #include <vector>
@@ -31,6 +33,7 @@ using Splits = std::optional<std::vector<int64_t>>;
 enum class Role : int64_t {
     kSync  = 0,  // all_to_all_4d on the caller's stream
     kAsync = 1,  // all_to_all_4d_async on the comm stream; unordered against kSync, hence separate
+    kFp8   = 2,  // the block-scaled fp8 exchange: payload and scale planes, another layout
 };
 
 struct Window {
@@ -109,6 +112,8 @@ public:
     void launch(const Plan& plan, const void* src, int64_t src_bytes, const Window& w, void* out, int64_t out_bytes,
                 void* stream, int extra_flags, int pool_slot = 0, bool pool_possible = false);
     void barrier(Role role, void* stream);
+    // Work queued on `to` from now on waits for what has been queued on `from` so far.
+    void order_streams(void* from, void* to);
 
     // CPU/gloo execution of the same plan.
     void run_cpu(const Plan& plan, const at::Tensor& x, at::Tensor& out);
@@ -140,7 +145,21 @@ private:
     int         ctas_       = 0;
     int64_t     allocations_ = 0;
 
+    // The event behind order_streams(), made once. A wait takes the state of the record before it, so
+    // the pair is what must not be interleaved by two threads.
+    std::mutex  order_mutex_;
+    cudaEvent_t order_event_ = nullptr;
+
+    std::mutex                           plan_mutex_;  // autograd's thread and the caller's may both ask
     std::map<std::vector<int64_t>, Plan> plans_;
+    // The call before this one: a loop over layers asks for the same plan again and again.
+    struct LastPlan {
+        int64_t        mode = -1;
+        at::ScalarType dtype = at::kByte;
+        bool           strided = false;
+        int64_t        sizes[4] = {}, strides[4] = {};
+        const Plan*    plan = nullptr;
+    } last_plan_;
     std::map<int64_t, Window>            windows_;  // by role
     std::array<Window, kLentSlots>       lent_;
     uint64_t                             lend_calls_ = 0;
