@@ -29,7 +29,7 @@ import torch.distributed as dist
 import fast_ulysses_b200 as fu
 from fast_ulysses_b200.models.attention import HEAD_DIM, UlyssesSelfAttention
 from fast_ulysses_b200.ops import attention as fa
-from fast_ulysses_b200.ops import gemm, outproj, qkv
+from fast_ulysses_b200.ops import gemm, qkv
 
 
 def peaks() -> tuple[float, float]:
@@ -60,11 +60,9 @@ def main() -> None:
     x = torch.randn(m, hidden, device="cuda").bfloat16()
     dy = torch.randn(m, hidden, device="cuda").bfloat16()
     y_save = torch.empty(m, 2 * heads * HEAD_DIM, dtype=torch.bfloat16, device="cuda")
-    gather = torch.empty(m, heads * HEAD_DIM, dtype=torch.bfloat16, device="cuda")
-    out = torch.empty(m, hidden, dtype=torch.bfloat16, device="cuda")
     dyqkv = torch.empty(m, 3 * heads * HEAD_DIM, dtype=torch.bfloat16, device="cuda")
     dgq, dgk = torch.zeros(HEAD_DIM, device="cuda"), torch.zeros(HEAD_DIM, device="cuda")
-    gq, gk = mod._f32("gamma_q", mod.gamma_q), mod._f32("gamma_k", mod.gamma_k)
+    native = mod._native
     flush = torch.empty(256 << 20, dtype=torch.uint8, device="cuda")
     (tflops, hbm), link = peaks(), args.link_gbs
     remote = (world - 1) / world  # share of a rank's rows or heads that lives on other ranks
@@ -100,27 +98,24 @@ def main() -> None:
 
     row_bytes = heads * HEAD_DIM * 2
     # fused QKV projection + RMSNorm + RoPE + scatter: 3 x (m, hidden) of results leave for the head owners
-    ms = timed(lambda: mod._launch_scatter(x, mod.w_qkv, mod.qkv_win, 3, 2, mod.gamma_q, mod.gamma_k, y_save))
+    ms = timed(lambda: native.scatter_qkv(x, mod.w_qkv, mod.rope, mod.gamma_q, mod.gamma_k, y_save))
     report("qkv_rope_scatter", ms, 2.0 * m * 3 * heads * HEAD_DIM * hidden, 3 * m * row_bytes * remote)
     # attention on this rank's heads over the whole sequence (no collective; for the block's budget)
     ms = timed(lambda: fa.fmha_fwd(mod.q_view, mod.k_view, mod.v_view, out=mod.o_view))
     report("fmha_fwd", ms, 4.0 * args.tokens * args.tokens * HEAD_DIM * n_local, 0.0)
     _, lse = fa.fmha_fwd(mod.q_view, mod.k_view, mod.v_view, out=mod.o_view)
     # pull + output projection: the attention output of this rank's tokens comes from the head owners
-    ready = mod._ready_flags(m)
-    ms = timed(lambda: outproj.pull_outproj_raw(mod.w_o, out, gather, ready, s_local=m, seq_off=mod.seq_off,
-                                                s_total=mod.s_total, head_splits=mod.head_splits, rank=mod.rank,
-                                                peer_o=mod.o_buf.base, ctrl=mod.o_buf.ctrl, o_bytes=mod._region))
+    ms = timed(lambda: native.pull_outproj(mod.w_o))
     report("pull_outproj", ms, 2.0 * m * hidden * heads * HEAD_DIM, m * row_bytes * remote)
     # backward: d(attention output) scattered from the dgrad GEMM's epilogue
-    ms = timed(lambda: mod._launch_scatter(dy, mod.w_o, mod.do_win, 1, 0, None, None, None, w_kn=True))
+    ms = timed(lambda: native.scatter_dout(dy, mod.w_o))
     report("dout_scatter", ms, 2.0 * m * hidden * heads * HEAD_DIM, m * row_bytes * remote)
     ms = timed(lambda: fa.fmha_bwd(mod.q_view, mod.k_view, mod.v_view, mod.o_view, lse, mod.do_view,
                                    out=(mod.dq_view, mod.dk_view, mod.dv_view)))
     report("fmha_bwd", ms, 10.0 * args.tokens * args.tokens * HEAD_DIM * n_local, 0.0)
     # dq, dk, dv pulled home with RoPE and RMSNorm undone on the way (memory-bound: no FLOPs to speak of)
     R = mod._region
-    ms = timed(lambda: qkv.pull_qkv_grads_raw(dyqkv, y_save, mod.rope, gq, gk, dgq, dgk, heads=heads, s_local=m,
+    ms = timed(lambda: qkv.pull_qkv_grads_raw(dyqkv, y_save, mod.rope, mod.gamma_q, mod.gamma_k, dgq, dgk, heads=heads, s_local=m,
                                               seq_off=mod.seq_off, s_total=mod.s_total, head_splits=mod.head_splits,
                                               rank=mod.rank, peer_dq=mod.dqkv_buf.base,
                                               peer_dk=[p + R for p in mod.dqkv_buf.base],

@@ -139,8 +139,8 @@ __global__ void __launch_bounds__(256) layernorm_fwd_kernel(const __nv_bfloat16*
 }
 
 __global__ void __launch_bounds__(256) layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
-                                                            const float* stats, __nv_bfloat16* dx, int64_t rows,
-                                                            int64_t cols, int64_t ld)
+                                                            const float* stats, const __nv_bfloat16* add,
+                                                            __nv_bfloat16* dx, int64_t rows, int64_t cols, int64_t ld)
 {
     const int     lane = threadIdx.x & 31;
     const int64_t row  = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -173,16 +173,109 @@ __global__ void __launch_bounds__(256) layernorm_bwd_kernel(const __nv_bfloat16*
     for (int64_t c = lane * 8; c < cols; c += 256) {
         const uint4           xv = *reinterpret_cast<const uint4*>(xr + c);
         const uint4           gv = *reinterpret_cast<const uint4*>(gr + c);
+        uint4                 av = make_uint4(0u, 0u, 0u, 0u);
+        if (add) {
+            av = *reinterpret_cast<const uint4*>(add + row * ld + c);
+        }
+        const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&av);
         const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xv);
         const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&gv);
         uint32_t              o[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
             const float2 xf = __bfloat1622float2(xh[j]), gf = __bfloat1622float2(gh[j]);
-            o[j] = fu::ptx::pack_bf16x2(rstd * (gf.x - mg - (xf.x - mean) * rstd * mgx),
-                                        rstd * (gf.y - mg - (xf.y - mean) * rstd * mgx));
+            float2       d  = make_float2(rstd * (gf.x - mg - (xf.x - mean) * rstd * mgx),
+                                          rstd * (gf.y - mg - (xf.y - mean) * rstd * mgx));
+            if (add) {
+                const float2 af = __bfloat1622float2(ah[j]);
+                d.x += af.x;
+                d.y += af.y;
+            }
+            o[j] = fu::ptx::pack_bf16x2(d.x, d.y);
         }
         *reinterpret_cast<uint4*>(dr + c) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+}
+
+// ---- column sums (bias gradients) --------------------------------------------------------------------------
+// A cluster of eight CTAs owns 64 columns and splits the rows; a warp reads four rows of 128 bytes per
+// instruction. The CTAs' sums meet in the first one's shared memory, so there is no scratch buffer, no
+// atomic and no second launch, and the order of the additions is fixed. Bound by HBM.
+constexpr int kSumCluster = 8;
+constexpr int kSumCols    = 64;
+constexpr int kSumThreads = 256;
+
+template <bool kVec>
+__global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThreads)
+    colsum_kernel(const __nv_bfloat16* x, __nv_bfloat16* out, int64_t rows, int64_t cols, int64_t ld)
+{
+    constexpr int kGroups = kSumThreads / 8;  // rows a CTA reads at once; eight lanes of 8 columns each per row
+    constexpr int kAhead  = 4;
+    __shared__ float part[kGroups][kSumCols + 4];
+    __shared__ float total[kSumCluster][kSumCols];
+    // the first CTA's shared memory is written by the others: they say here that they have started
+    // and wait for that just before they write
+    asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory");
+    const int     rank = static_cast<int>(fu::ptx::cluster_ctarank());
+    const int     cg   = threadIdx.x & 7, rg = threadIdx.x >> 3;
+    const int64_t c0   = static_cast<int64_t>(blockIdx.y) * kSumCols + cg * 8;
+    float         acc[8] = {};
+    const int64_t step = static_cast<int64_t>(kSumCluster) * kGroups;
+    for (int64_t r0 = rank * kGroups + rg; r0 < rows; r0 += step * kAhead) {
+        uint4 v[kAhead];
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const int64_t r = r0 + u * step;
+            v[u]            = make_uint4(0u, 0u, 0u, 0u);
+            if (r < rows) {
+                if (kVec && c0 + 8 <= cols) {
+                    v[u] = fu::ptx::ld_nc_v4(x + r * ld + c0);
+                }
+                else {
+                    __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&v[u]);
+                    for (int k = 0; k < 8; ++k) {
+                        if (c0 + k < cols) {
+                            e[k] = x[r * ld + c0 + k];
+                        }
+                    }
+                }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v[u]);
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const float2 f = __bfloat1622float2(h[k]);
+                acc[2 * k] += f.x;
+                acc[2 * k + 1] += f.y;
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        part[rg][cg * 8 + k] = acc[k];
+    }
+    __syncthreads();
+    asm volatile("barrier.cluster.wait;" ::: "memory");
+    if (threadIdx.x < kSumCols) {
+        float s = 0.f;
+#pragma unroll 8
+        for (int g = 0; g < kGroups; ++g) {
+            s += part[g][threadIdx.x];
+        }
+        const uint32_t to = fu::ptx::cluster_addr(&total[rank][threadIdx.x], 0);
+        asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(to), "f"(s) : "memory");
+    }
+    fu::ptx::cluster_sync();
+    const int64_t col = static_cast<int64_t>(blockIdx.y) * kSumCols + threadIdx.x;
+    if (rank == 0 && threadIdx.x < kSumCols && col < cols) {
+        float s = 0.f;
+#pragma unroll
+        for (int g = 0; g < kSumCluster; ++g) {
+            s += total[g][threadIdx.x];
+        }
+        out[col] = __float2bfloat16(s);
     }
 }
 
@@ -474,17 +567,38 @@ extern "C" int fu_layernorm_fwd(const void* x, void* y, float* stats, int64_t ro
     return FU_OK;
 }
 
-extern "C" int fu_layernorm_bwd(const void* dy, const void* x, const float* stats, void* dx, int64_t rows, int64_t cols,
-                                int64_t ld, void* stream)
+extern "C" int fu_layernorm_bwd_add(const void* dy, const void* x, const float* stats, const void* add, void* dx, int64_t rows,
+                                    int64_t cols, int64_t ld, void* stream)
 {
     if (!dy || !x || !stats || !dx || rows <= 0 || cols <= 0 || (cols % 8) || (ld % 8)
-        || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)) & 15u)) {
+        || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)
+             | reinterpret_cast<uintptr_t>(add)) & 15u)) {
         return fu::fail(FU_E_ARG, "fu_layernorm_bwd: needs 16-byte aligned rows of a multiple of 8 columns");
     }
     const unsigned blocks = static_cast<unsigned>((rows + 7) / 8);
     layernorm_bwd_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
         static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
-        static_cast<__nv_bfloat16*>(dx), rows, cols, ld);
+        static_cast<const __nv_bfloat16*>(add), static_cast<__nv_bfloat16*>(dx), rows, cols, ld);
+    FU_CUDA_OK(cudaGetLastError());
+    return FU_OK;
+}
+
+extern "C" int fu_layernorm_bwd(const void* dy, const void* x, const float* stats, void* dx, int64_t rows, int64_t cols,
+                                int64_t ld, void* stream)
+{
+    return fu_layernorm_bwd_add(dy, x, stats, nullptr, dx, rows, cols, ld, stream);
+}
+
+extern "C" int fu_colsum_bf16(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, void* stream)
+{
+    if (!x || !out || rows <= 0 || cols <= 0) {
+        return fu::fail(FU_E_ARG, "fu_colsum_bf16: null or empty operand");
+    }
+    const bool     vec    = (ld % 8) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+    const dim3     grid(kSumCluster, static_cast<unsigned>((cols + kSumCols - 1) / kSumCols));
+    auto           kernel = vec ? colsum_kernel<true> : colsum_kernel<false>;
+    kernel<<<grid, kSumThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(x),
+                                                                        static_cast<__nv_bfloat16*>(out), rows, cols, ld);
     FU_CUDA_OK(cudaGetLastError());
     return FU_OK;
 }

@@ -142,13 +142,14 @@ enum {
     FU_GEMM_B_KN = 2,
     FU_GEMM_PAIR = 4,    // run on CTA pairs (256 x 256 tiles, tcgen05 cta_group::2) whatever the default is
     FU_GEMM_SINGLE = 8,  // run on single CTAs (128 x 256 tiles) whatever the default is
+    FU_GEMM_BIAS_BF16 = 16,  // `bias` points to bf16 values
 };
 typedef struct FuGemmArgs {
     const void*  a;
     const void*  b;
     void*        c;
     int64_t      m, n, k, lda, ldb, ldc;
-    const float* bias;
+    const void*  bias;      // (n) fp32, or bf16 with FU_GEMM_BIAS_BF16; nullable
     const void*  residual;
     int32_t      act;
     int32_t      ctas;
@@ -253,11 +254,13 @@ FU_API int fu_pull_qkv_grads_check(const FuPullGradsArgs* args);  // the argumen
 // gathered from its owners: A[m, head*128 + x] = O_owner(head)[batch, seq_off + s, local head, x].
 // Every rank's O buffer has layout (b, s_total, head_splits[p], 128) bf16. `gather` is local scratch
 // of m x (heads*128) bf16 and `ready` of ceil(m/128)*world uint32 (zeroed by the launcher).
+// FuPullArgs::flags: `bias` points to bf16 values.
+#define FU_PULL_BIAS_BF16 1024
 typedef struct FuPullArgs {
     const void*  w;
     void*        c;
     int64_t      m, n, ldw, ldc;
-    const float* bias;
+    const void*  bias;      // (n) fp32, or bf16 with FU_PULL_BIAS_BF16; nullable
     const void*  residual;
     int64_t      s_local, seq_off, s_total;
     int32_t      rank, world;
@@ -266,7 +269,7 @@ typedef struct FuPullArgs {
     FuCtrl*      peer_ctrl[FU_MAX_WORLD];
     void*        gather;
     uint32_t*    ready;
-    int32_t      flags;
+    int32_t      flags;    // FU_A2A_NO_HANDSHAKE, FU_A2A_MUTE, FU_PULL_BIAS_BF16
     uint32_t     timeout_ms;
     int32_t      ctas;
     int32_t      pad_;
@@ -346,8 +349,14 @@ FU_API int fu_fmha_bwd_noalloc(const FuFmhaArgs* args, void* stream);
 FU_API int fu_layernorm_fwd(const void* x, void* y, float* stats, int64_t rows, int64_t cols, int64_t ldx, int64_t ldy,
                             float eps, void* stream);
 // dx = rstd * (dy - mean(dy) - xhat * mean(dy * xhat)), xhat recomputed from x and the saved statistics.
+// `add` (nullable, laid out like dx) is added before the one rounding to bf16: the gradient that reached x
+// past the norm, through a residual connection.
 FU_API int fu_layernorm_bwd(const void* dy, const void* x, const float* stats, void* dx, int64_t rows, int64_t cols,
                             int64_t ld, void* stream);
+FU_API int fu_layernorm_bwd_add(const void* dy, const void* x, const float* stats, const void* add, void* dx, int64_t rows,
+                                int64_t cols, int64_t ld, void* stream);
+// out[c] = bf16(sum over rows of x[r, c]), x bf16 with leading dimension ld, summed in fp32 in a fixed order.
+FU_API int fu_colsum_bf16(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, void* stream);
 
 // ---- block-scaled fp8 payloads ----------------------------------------------------------------------
 // `blocks` runs of 128 bf16 values <-> `blocks` packed rows of 144 bytes (128 e4m3 + fp32 scale + pad).
@@ -371,6 +380,9 @@ typedef struct FuA2AFp8Args {
     uint32_t    timeout_ms;
     FuRoute     routes[FU_MAX_WORLD];
 } FuA2AFp8Args;
+// `rows` rows of 128 bf16 values, each rounded to block-scaled e4m3 and back: what the exchange does to
+// every row, and all of it for a group of one rank. 32-byte aligned operands.
+FU_API int fu_fp8_round_trip(const void* src, void* dst, int64_t rows, void* stream);
 FU_API int fu_a2a4d_fp8(const FuA2AFp8Args* args, void* stream);
 FU_API int fu_a2a4d_fp8_check(const FuA2AFp8Args* args);  // the argument checks alone; no CUDA call
 

@@ -26,9 +26,9 @@ using namespace fu::gemm;
 struct PlainEpi {
     __nv_bfloat16*       c;
     const __nv_bfloat16* residual;
-    const float*         bias;
+    const void*          bias;
     int64_t              ldc;
-    int                  M, N, act;
+    int                  M, N, act, bias_bf16;
     const __nv_bfloat16* aux;    // act 3: where the tanh-form GELU's derivative is evaluated
     __nv_bfloat16*       c_pre;  // optional second output: the value before the activation
 
@@ -76,7 +76,8 @@ struct PlainEpi {
 #pragma unroll
                 for (int j = 0; j < 32; ++j) {
                     if (col0 + j < N) {
-                        v[j] += bias[col0 + j];
+                        v[j] += bias_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[col0 + j])
+                                          : static_cast<const float*>(bias)[col0 + j];
                     }
                 }
             }
@@ -644,6 +645,7 @@ extern "C" int fu_gemm_bf16(const FuGemmArgs* g, void* stream)
     a.epi.c        = static_cast<__nv_bfloat16*>(g->c);
     a.epi.residual = static_cast<const __nv_bfloat16*>(g->residual);
     a.epi.bias     = g->bias;
+    a.epi.bias_bf16 = (g->flags & FU_GEMM_BIAS_BF16) ? 1 : 0;
     a.epi.ldc      = g->ldc;
     a.epi.M        = a.core.M;
     a.epi.N        = a.core.N;
@@ -904,6 +906,7 @@ extern "C" int fu_pull_outproj(const FuPullArgs* q, void* stream_v)
     a.epi.c            = static_cast<__nv_bfloat16*>(q->c);
     a.epi.residual     = static_cast<const __nv_bfloat16*>(q->residual);
     a.epi.bias         = q->bias;
+    a.epi.bias_bf16    = (q->flags & FU_PULL_BIAS_BF16) ? 1 : 0;
     a.epi.ldc          = q->ldc;
     a.epi.M            = a.core.M;
     a.epi.N            = a.core.N;

@@ -12,11 +12,13 @@
 #include <cuda_runtime.h>
 #include <torch/autograd.h>
 #include <torch/extension.h>
+#include <torch/csrc/utils/pybind.h>
 #include <torch/library.h>
 
 #include "../runtime/group.hpp"
 #include "../runtime/nvlink.hpp"
 #include "../runtime/work.hpp"
+#include "fused.hpp"
 
 namespace py = pybind11;
 
@@ -293,12 +295,13 @@ void all_to_all_4d_out_meta(const GroupPtr& group, const at::Tensor& input, int6
 // ---- async (comm-stream) op ---------------------------------------------------------------------------
 // Runs with the comm stream current. The kernel reads the caller's tensor directly: the comm
 // stream waits for the caller's stream to have produced it, and the caching allocator is told that
-// the comm stream uses the block, so there is no staging copy.
+// the comm stream uses the block, so there is no staging copy. With `hold_caller` the caller's stream
+// also waits for the kernel, so that whatever it does to the input next comes after the last read.
 namespace {
 
 at::Tensor run_async(Group& g, const at::Tensor& input, int64_t mode, const Splits& seq, const Splits& heads,
                      const std::optional<at::Tensor>& out, int64_t caller_stream_id, int64_t caller_device_index,
-                     bool lend)
+                     bool lend, bool hold_caller = false)
 {
     g.check_alive();
     require_backend(g, input, "input");
@@ -326,13 +329,14 @@ at::Tensor run_async(Group& g, const at::Tensor& input, int64_t mode, const Spli
         // Allocated while the caller's stream was current; the comm stream writes it.
         c10::cuda::CUDACachingAllocator::recordStream(p.output.storage().data_ptr(), comm);
     }
-    cudaEvent_t ready = nullptr;
-    cuda_ok(cudaEventCreateWithFlags(&ready, cudaEventDisableTiming), "cudaEventCreateWithFlags");
-    cuda_ok(cudaEventRecord(ready, caller.stream()), "cudaEventRecord");
-    cuda_ok(cudaStreamWaitEvent(comm.stream(), ready, 0), "cudaStreamWaitEvent");
-    cuda_ok(cudaEventDestroy(ready), "cudaEventDestroy");
-    c10::cuda::CUDACachingAllocator::recordStream(p.x.storage().data_ptr(), comm);
+    g.order_streams(caller.stream(), comm.stream());
+    if (!hold_caller) {
+        c10::cuda::CUDACachingAllocator::recordStream(p.x.storage().data_ptr(), comm);
+    }
     run_prepared(g, p, comm.stream(), FU_A2A_MINOR_SHARE | (g.async_copy_engine() ? FU_A2A_COPY_ENGINE : 0));
+    if (hold_caller) {
+        g.order_streams(comm.stream(), caller.stream());
+    }
     return p.output;
 }
 
@@ -486,6 +490,50 @@ at::Tensor all_to_all_4d_autograd(const GroupPtr& group, const at::Tensor& input
     return primal_out;
 }
 
+// ---- the calls of the Python class without torch.ops' argument parsing ---------------------------------
+// Parsing a torch.ops call whose first argument is a TorchScript object costs several microseconds,
+// as much as a small exchange takes on the device. These entries take the group as a pybind object
+// and go through the same dispatcher entry points (autograd, FakeTensor, vmap refusal included);
+// the GIL is dropped as torch.ops drops it, because a call may have to allocate collectively.
+at::Tensor direct_all_to_all_4d(const GroupRef& ref, const at::Tensor& input, int64_t mode, const Splits& seq,
+                                const Splits& heads)
+{
+    static auto op =
+        c10::Dispatcher::singleton().findSchemaOrThrow("fast_ulysses_b200::all_to_all_4d", "").typed<A2ASig>();
+    return op.call(ref.group, input, mode, seq, heads);
+}
+
+void direct_all_to_all_4d_out(const GroupRef& ref, const at::Tensor& input, int64_t mode, const Splits& seq,
+                              const Splits& heads, at::Tensor out)
+{
+    using Sig      = void(const GroupPtr&, const at::Tensor&, int64_t, const Splits&, const Splits&, at::Tensor);
+    static auto op = c10::Dispatcher::singleton().findSchemaOrThrow("fast_ulysses_b200::all_to_all_4d_out", "").typed<Sig>();
+    op.call(ref.group, input, mode, seq, heads, out);
+}
+
+// The whole asynchronous call: the exchange on the comm stream, its completion event bound to the
+// result in torch's work registry, and the allocator told about both streams. Returns the result
+// and whether a registry exists.
+std::pair<at::Tensor, bool> direct_async(const GroupRef& ref, const at::Tensor& input, int64_t mode, const Splits& seq,
+                                         const Splits& heads, const std::optional<at::Tensor>& out, bool lend,
+                                         int64_t comm_stream_id, bool hold_caller)
+{
+    const at::AutoDispatchBelowADInplaceOrView below;
+    const c10::Device                 dev = input.device();
+    const c10::cuda::CUDAGuard        guard(dev);
+    const c10::cuda::CUDAStream       caller = at::cuda::getCurrentCUDAStream(dev.index());
+    const c10::cuda::CUDAStream       comm(c10::Stream(c10::Stream::UNSAFE, dev, comm_stream_id));
+    at::Tensor                        y;
+    {
+        const c10::cuda::CUDAStreamGuard on_comm(comm);
+        y = run_async(*ref.group, input, mode, seq, heads, out, caller.id(), caller.device_index(), lend, hold_caller);
+    }
+    const bool registered = register_stream_completion(y, reinterpret_cast<int64_t>(comm.stream()));
+    c10::cuda::CUDACachingAllocator::recordStream(y.storage().data_ptr(), comm);
+    c10::cuda::CUDACachingAllocator::recordStream(y.storage().data_ptr(), caller);
+    return {y, registered};
+}
+
 // ---- plan debug ----------------------------------------------------------------------------------------------
 // The plan as tensors, so that a CPU test can replay it over plain byte arrays for any rank.
 std::tuple<std::vector<int64_t>, int64_t, at::Tensor, at::Tensor, at::Tensor> a2a_plan_debug(
@@ -609,6 +657,13 @@ TORCH_LIBRARY(fast_ulysses_b200, m)
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m)
 {
     m.def("register_stream_completion", &fu::register_stream_completion);
+    py::class_<fu::GroupRef>(m, "GroupRef").def(py::init([](const torch::jit::Object& handle) {
+        return fu::GroupRef{c10::IValue(handle._ivalue()).toCustomClass<fu::Group>()};
+    }));
+    m.def("all_to_all_4d", torch::wrap_pybind_function_no_gil(&fu::direct_all_to_all_4d));
+    m.def("all_to_all_4d_out", torch::wrap_pybind_function_no_gil(&fu::direct_all_to_all_4d_out));
+    m.def("all_to_all_4d_async", torch::wrap_pybind_function_no_gil(&fu::direct_async));
+    fu::bind_fused(m);
     m.def("nvlink_matrix", [](const std::vector<int64_t>& devices) -> py::object {
         const auto matrix = fu::nvlink_matrix(devices);
         if (!matrix.has_value()) {

@@ -15,7 +15,7 @@ import torch.nn as nn
 import torch.nn.functional as F
 
 from ..ops.gemm import feed_forward
-from ..ops.norm import layer_norm
+from ..ops.norm import layer_norm_fork
 from .attention import UlyssesSelfAttention, reference_attention
 
 
@@ -31,8 +31,11 @@ class DiTBlock(nn.Module):
         self.b2 = nn.Parameter(torch.zeros(hidden, device=dev).bfloat16())
 
     def forward(self, x):
-        x = self.attn(layer_norm(x), residual=x)  # x + Attn(LN(x)): the add is the out-projection's epilogue
-        return feed_forward(layer_norm(x), self.w1, self.b1, self.w2, self.b2, residual=x)
+        # each add is an epilogue (of the out-projection, of the second feed-forward GEMM), and the two
+        # gradients that meet at a norm's input are joined in the norm's backward
+        h, x = layer_norm_fork(x)
+        h, x = layer_norm_fork(self.attn(h, residual=x))
+        return feed_forward(h, self.w1, self.b1, self.w2, self.b2, residual=x)
 
 
 class DiTStack(nn.Module):

@@ -1,4 +1,5 @@
-"""Flash attention on the tcgen05 tensor cores (csrc/kernels/fmha_fwd_sm100.cu, fmha_bwd_sm100.cu).
+"""Flash attention on the tcgen05 tensor cores (csrc/kernels/fmha_fwd_sm100.cu, fmha_bwd_sm100.cu;
+argument handling and autograd in csrc/ops/fused.cc).
 
 Tensors use the ``(batch, seq, heads, 128)`` layout of the all-to-all windows; any view whose last
 axis is contiguous and whose other strides are multiples of 8 elements is read in place.
@@ -6,12 +7,11 @@ axis is contiguous and whose other strides are multiples of 8 elements is read i
 
 from __future__ import annotations
 
-import ctypes as C
 import math
 
 import torch
 
-from . import _ckernels as ck
+from .. import _C
 from .gemm import error_word
 
 
@@ -21,6 +21,7 @@ def _strides(t: torch.Tensor):
 
 
 def _fill(a, q, k, v, o):
+    """Operands, shape and strides of a ``_ckernels.FuFmhaArgs`` for a caller of the C symbols themselves."""
     b, sq, h, _ = q.shape
     a.q, a.k, a.v, a.o = q.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr()
     a.batch, a.heads, a.seq_q, a.seq_kv, a.head_dim = b, h, sq, k.shape[1], 128
@@ -39,22 +40,8 @@ def fmha_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: float 
     every 16 exponential pairs are computed on the FMA pipe instead of the special-function unit.
     ``trace`` (int64[256] on the device) selects the instrumented build of the kernel: CTA 0 stores the
     SM clock of 32 pipeline events for kv steps 64..71 of its first item."""
-    b, sq, h, d = q.shape
-    assert k.shape == v.shape and k.shape[0] == b and k.shape[2] == h and d == 128
-    o = out if out is not None else torch.empty(b, sq, h, d, dtype=torch.bfloat16, device=q.device)
-    lse = torch.empty(b, h, sq, dtype=torch.float32, device=q.device)
-    a = ck.FuFmhaArgs()
-    _fill(a, q, k, v, o)
-    a.lse = lse.data_ptr()
-    a.scale = scale if scale is not None else 1.0 / math.sqrt(d)
-    a.ctas = ctas
-    if poly is not None:
-        a.flags = 0x1000 | ((poly & 15) << 8)  # FU_FMHA_POLY(poly)
-    if trace is not None:
-        assert trace.dtype == torch.int64 and trace.numel() >= 256 and trace.is_cuda
-        a.trace = trace.data_ptr()
-    ck.check(ck.lib().fu_fmha_fwd(C.byref(a), ck.stream_ptr()))
-    return o, lse
+    flags = 0 if poly is None else 0x1000 | ((poly & 15) << 8)  # FU_FMHA_POLY(poly)
+    return _C.fmha_fwd(q, k, v, scale, out, ctas, flags, trace)
 
 
 def attention_reference(q, k, v, scale=None):
@@ -74,53 +61,9 @@ def fmha_bwd(q, k, v, o, lse, d_o, *, scale: float | None = None, ctas: int = 0,
     bit-reproducible, dQ to rounding); ``deterministic=True`` runs two passes without atomics
     (dK/dV with the K/V block stationary, then dQ with the query rows stationary) at about 1.5x
     the time."""
-    b, sq, h, d = q.shape
-    if d_o.stride() != o.stride():
-        d_o = d_o.contiguous()
-        o = o.contiguous()
-    if out is not None:
-        dq, dk, dv = out  # dense (b, s, h, 128) tensors provided by the caller
-        assert dq.is_contiguous() and dk.is_contiguous() and dv.is_contiguous()
-    else:
-        dq = torch.empty(b, sq, h, d, dtype=torch.bfloat16, device=q.device)
-        dk = torch.empty(b, k.shape[1], h, d, dtype=torch.bfloat16, device=q.device)
-        dv = torch.empty_like(dk)
-    # the launcher addresses dq/dk/dv with the strides of q/k/v: hand it dense q/k/v views
-    qc, kc, vc = (t if t.is_contiguous() else t.contiguous() for t in (q, k, v))
-    sq_pad = (sq + 127) // 128 * 128
-    stats = torch.empty(2 * b * h * sq_pad, dtype=torch.float32, device=q.device)
-    dq_acc = None if deterministic else torch.empty(b, sq, h, d, dtype=torch.float32, device=q.device)
-    a = ck.FuFmhaArgs()
-    _fill(a, qc, kc, vc, o)
-    a.lse = lse.data_ptr()
-    a.scale = scale if scale is not None else 1.0 / math.sqrt(d)
-    a.ctas = ctas
-    a.d_o, a.dq, a.dk, a.dv = d_o.data_ptr(), dq.data_ptr(), dk.data_ptr(), dv.data_ptr()
-    a.delta = stats.data_ptr()
-    if dq_acc is not None:
-        a.dq_acc = dq_acc.data_ptr()
-    a.flags = 1 if deterministic else 0
-    if trace is not None:  # int64[128] on the device: SM clock of 16 pipeline events for 8 blocks of CTA 0
-        a.trace = trace.data_ptr()
-    ck.check(ck.lib().fu_fmha_bwd(C.byref(a), ck.stream_ptr()))
-    return dq, dk, dv
-
-
-class _Attention(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, q, k, v, scale):
-        o, lse = fmha_fwd(q, k, v, scale=scale)
-        ctx.save_for_backward(q, k, v, o, lse)
-        ctx.scale = scale
-        return o
-
-    @staticmethod
-    def backward(ctx, d_o):
-        q, k, v, o, lse = ctx.saved_tensors
-        dq, dk, dv = fmha_bwd(q, k, v, o, lse, d_o.contiguous() if not d_o.is_contiguous() else d_o, scale=ctx.scale)
-        return dq, dk, dv, None
+    return _C.fmha_bwd(q, k, v, o, lse, d_o, scale, ctas, None if out is None else list(out), deterministic, trace)
 
 
 def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: float | None = None) -> torch.Tensor:
     """Differentiable non-causal attention on (b, s, h, 128) bf16 tensors (tcgen05 fwd and bwd)."""
-    return _Attention.apply(q, k, v, scale)
+    return _C.attention(q, k, v, scale)

@@ -21,6 +21,14 @@ import torch.distributed as dist
 from .. import _C  # noqa: F401  (registers torch.ops.fast_ulysses_b200)
 
 _OPS = torch.ops.fast_ulysses_b200
+_is_compiling = torch.compiler.is_compiling
+_torch_function_mode = torch._C._is_torch_function_mode_enabled
+
+
+def _direct(x) -> bool:
+    """Whether a call may skip torch.ops' argument parsing (csrc/ops/bindings.cc: GroupRef). A tensor
+    subclass, a TorchFunctionMode or a tracing compiler has to see the torch.ops call itself."""
+    return type(x) is torch.Tensor and not _is_compiling() and not _torch_function_mode()
 
 
 class CompletedHandle:
@@ -97,6 +105,7 @@ class UlyssesGroup:
 
         index = int(device.index) if device.type == "cuda" else -1
         self._handle = torch.classes.fast_ulysses_b200.UlyssesGroup(name, int(self.rank), int(self.world_size), index)
+        self._ref = _C.GroupRef(self._handle)  # the same group for the direct calls of the binding
         self._handle.set_timeout_ms(int(timeout_ms))
         self._comm_stream = None
         if device.type == "cuda":
@@ -105,7 +114,6 @@ class UlyssesGroup:
             _, greatest = torch.cuda.Stream.priority_range()
             self._comm_stream = torch.cuda.Stream(device=device, priority=greatest)
         self._destroyed = False
-        self._fp8_window: dict = {}
 
     # ------------------------------------------------------------------------------------------
     def _require_nvlink(self) -> None:
@@ -151,6 +159,8 @@ class UlyssesGroup:
         copy-out into an ordinary allocation.
         """
         if out is None:
+            if _direct(x):
+                return _C.all_to_all_4d(self._ref, x, mode, seq_splits, head_splits)
             return _OPS.all_to_all_4d(self._handle, x, mode, seq_splits, head_splits)
         if torch.is_grad_enabled() and x.requires_grad:
             raise RuntimeError(
@@ -158,7 +168,10 @@ class UlyssesGroup:
                 "own and has no backward, so the gradient would be dropped without an error. Drop out=, "
                 "or run under torch.no_grad()."
             )
-        _OPS.all_to_all_4d_out(self._handle, x, mode, seq_splits, head_splits, out)
+        if _direct(x) and _direct(out):
+            _C.all_to_all_4d_out(self._ref, x, mode, seq_splits, head_splits, out)
+        else:
+            _OPS.all_to_all_4d_out(self._handle, x, mode, seq_splits, head_splits, out)
         return out
 
     def all_to_all_4d_async(
@@ -202,7 +215,16 @@ class UlyssesGroup:
 
         from torch.distributed._functional_collectives import AsyncCollectiveTensor
 
-        if stage:
+        # A group of one rank moves the tensor once, on this device: copying it aside first would be
+        # the same work over again, so the caller's stream waits for that one move instead.
+        hold_caller = stage and self.world_size == 1
+        if stage and not hold_caller:
+            x = x.clone()
+        if _direct(x) and (out is None or _direct(out)):
+            y, registered = _C.all_to_all_4d_async(self._ref, x, mode, seq_splits, head_splits, out, lend,
+                                                   self._comm_stream.stream_id, hold_caller)
+            return AsyncCollectiveTensor(y) if registered else CompletedHandle(y)
+        if hold_caller:
             x = x.clone()
         caller = torch.cuda.current_stream(self.device)
         with torch.cuda.stream(self._comm_stream):
@@ -289,7 +311,6 @@ class UlyssesGroup:
         if self.pg is not None and self.world_size > 1:
             dist.barrier(group=self.pg)
         self._handle.destroy()
-        self._fp8_window = {}  # the fp8 exchange's cached symmetric window (ops/fp8.py) goes with the group
         self._destroyed = True
 
     def __del__(self) -> None:
