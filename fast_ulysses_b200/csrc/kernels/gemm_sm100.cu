@@ -16,6 +16,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <mutex>
 
 namespace {
 
@@ -23,155 +24,164 @@ using namespace fu;
 using namespace fu::gemm;
 
 // ---- plain epilogue --------------------------------------------------------------------------------
+// GELU(x) = x * sigmoid(2u), u = sqrt(2/pi) (x + 0.044715 x^3), written with one exponential and one
+// reciprocal: 1 + tanh(u) = 2 sigmoid(2u), without tanhf's branches and without the cancellation of
+// 1 + tanh for negative x. The approximations' relative error (about 1e-6) is far below the bf16 result's.
+__device__ __forceinline__ float sigmoid2(float u)
+{
+    return __fdividef(1.0f, 1.0f + __expf(-2.0f * u));
+}
+__device__ __forceinline__ float gelu_tanh(float x)
+{
+    return x * sigmoid2(0.7978845608028654f * x * (1.0f + 0.044715f * x * x));
+}
+__device__ __forceinline__ float gelu_erf(float x)
+{
+    return 0.5f * x * (1.0f + erff(x * 0.7071067811865476f));
+}
+__device__ __forceinline__ float gelu_tanh_grad(float x)
+{
+    const float x2 = x * x;
+    const float s  = sigmoid2(0.7978845608028654f * x * (1.0f + 0.044715f * x2));
+    return s + x * s * (1.0f - s) * 1.5957691216057308f * (1.0f + 0.134145f * x2);
+}
+
+// ACT: 0 none, 1 GELU (tanh form), 2 GELU (erf form), 3 the tanh form's derivative at aux.
+template <int ACT>
 struct PlainEpi {
+    static constexpr bool kPeers = false;
     __nv_bfloat16*       c;
     const __nv_bfloat16* residual;
     const void*          bias;
     int64_t              ldc;
-    int                  M, N, act, bias_bf16;
+    int                  M, N, bias_bf16;
     const __nv_bfloat16* aux;    // act 3: where the tanh-form GELU's derivative is evaluated
     __nv_bfloat16*       c_pre;  // optional second output: the value before the activation
 
     __device__ void open(int) {}
     __device__ void close(int) {}
 
-    __device__ __forceinline__ static float gelu_tanh(float x)
+    __device__ __forceinline__ static void pack_row(const float (&v)[64], uint8_t* stage, int lane)
     {
-        const float u = 0.7978845608028654f * (x + 0.044715f * x * x * x);
-        return 0.5f * x * (1.0f + tanhf(u));
-    }
-    __device__ __forceinline__ static float gelu_erf(float x)
-    {
-        return 0.5f * x * (1.0f + erff(x * 0.7071067811865476f));
-    }
-    __device__ __forceinline__ static float gelu_tanh_grad(float x)
-    {
-        const float x2 = x * x;
-        const float th = tanhf(0.7978845608028654f * (x + 0.044715f * x * x2));
-        return 0.5f * (1.0f + th) + 0.5f * x * (1.0f - th * th) * 0.7978845608028654f * (1.0f + 0.134145f * x2);
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            *stage_unit(stage, lane, g) = make_uint4(pack_bf16(v[8 * g], v[8 * g + 1]), pack_bf16(v[8 * g + 2], v[8 * g + 3]),
+                                                     pack_bf16(v[8 * g + 4], v[8 * g + 5]), pack_bf16(v[8 * g + 6], v[8 * g + 7]));
+        }
     }
 
-    __device__ void tile(uint32_t tmem_acc, int mt, int nt, int quarter, int lane)
+    template <int H>
+    __device__ __forceinline__ void half(const uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage) const
     {
-        const int  row    = mt * BM + quarter * 32 + lane;
-        const bool row_ok = row < M;
-#pragma unroll 1
-        for (int chunk = 0; chunk < BN / 32; ++chunk) {
-            const int col0 = nt * BN + chunk * 32;
-            if (col0 >= N) {
-                break;  // warp-uniform
-            }
-            uint32_t r[32];
-            ptx::tmem_ld_32x32(tmem_acc + chunk * 32, r);
-            ptx::tmem_ld_wait();
-            if (!row_ok) {
-                continue;
-            }
-            float v[32];
+        float v[64];
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
-                v[j] = __uint_as_float(r[j]);
-            }
-            if (bias) {
+        for (int j = 0; j < 64; ++j) {
+            v[j] = __uint_as_float(r[H * 64 + j]);
+        }
+        if (bias) {
+            if (col0 + 64 <= N && !bias_bf16) {
+                const float4* b = reinterpret_cast<const float4*>(static_cast<const float*>(bias) + col0);
 #pragma unroll
-                for (int j = 0; j < 32; ++j) {
+                for (int j = 0; j < 16; ++j) {
+                    const float4 f = __ldg(b + j);
+                    v[4 * j] += f.x, v[4 * j + 1] += f.y, v[4 * j + 2] += f.z, v[4 * j + 3] += f.w;
+                }
+            }
+            else if (col0 + 64 <= N) {
+                const uint4* b = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(bias) + col0);
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    const uint4           q = __ldg(b + j);
+                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+                    for (int k = 0; k < 4; ++k) {
+                        const float2 f = __bfloat1622float2(h[k]);
+                        v[8 * j + 2 * k] += f.x, v[8 * j + 2 * k + 1] += f.y;
+                    }
+                }
+            }
+            else {
+#pragma unroll
+                for (int j = 0; j < 64; ++j) {
                     if (col0 + j < N) {
                         v[j] += bias_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[col0 + j])
                                           : static_cast<const float*>(bias)[col0 + j];
                     }
                 }
             }
-            if (c_pre) {  // the pre-activation, for the backward (whole 8-column groups only: N % 8 == 0 is checked)
-                uint4* pre = reinterpret_cast<uint4*>(c_pre + static_cast<int64_t>(row) * ldc + col0);
+        }
+        if (c_pre) {
+            pack_row(v, stage, lane);
+            stage_out(stage, c_pre, ldc, row0, col0, M, N, lane);
+        }
+        if (ACT == 1 || ACT == 2) {
 #pragma unroll
-                for (int g8 = 0; g8 < 4; ++g8) {
-                    if (col0 + g8 * 8 + 8 <= N) {
-                        pre[g8] = make_uint4(pack_bf16(v[g8 * 8 + 0], v[g8 * 8 + 1]), pack_bf16(v[g8 * 8 + 2], v[g8 * 8 + 3]),
-                                             pack_bf16(v[g8 * 8 + 4], v[g8 * 8 + 5]), pack_bf16(v[g8 * 8 + 6], v[g8 * 8 + 7]));
-                    }
+            for (int j = 0; j < 64; ++j) {
+                v[j] = ACT == 1 ? gelu_tanh(v[j]) : gelu_erf(v[j]);
+            }
+        }
+        if (ACT == 3) {
+            stage_in(stage, aux, ldc, row0, col0, M, N, lane);
+#pragma unroll
+            for (int g = 0; g < 8; ++g) {
+                const uint4           q = *stage_unit(stage, lane, g);
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const float2 f = __bfloat1622float2(h[k]);
+                    v[8 * g + 2 * k] *= gelu_tanh_grad(f.x);
+                    v[8 * g + 2 * k + 1] *= gelu_tanh_grad(f.y);
                 }
             }
-            if (act == 3) {
-                const __nv_bfloat16* at = aux + static_cast<int64_t>(row) * ldc + col0;
+        }
+        if (residual) {
+            stage_in(stage, residual, ldc, row0, col0, M, N, lane);
 #pragma unroll
-                for (int g8 = 0; g8 < 4; ++g8) {
-                    if (col0 + g8 * 8 + 8 <= N) {
-                        const uint4           av = *reinterpret_cast<const uint4*>(at + g8 * 8);
-                        const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&av);
+            for (int g = 0; g < 8; ++g) {
+                const uint4           q = *stage_unit(stage, lane, g);
+                const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float2 f = __bfloat1622float2(ap[j]);
-                            v[g8 * 8 + 2 * j] *= gelu_tanh_grad(f.x);
-                            v[g8 * 8 + 2 * j + 1] *= gelu_tanh_grad(f.y);
-                        }
-                    }
+                for (int k = 0; k < 4; ++k) {
+                    const float2 f = __bfloat1622float2(h[k]);
+                    v[8 * g + 2 * k] += f.x;
+                    v[8 * g + 2 * k + 1] += f.y;
                 }
             }
-            if (act == 1) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    v[j] = gelu_tanh(v[j]);
-                }
-            }
-            else if (act == 2) {
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    v[j] = gelu_erf(v[j]);
-                }
-            }
-            __nv_bfloat16*       dst = c + static_cast<int64_t>(row) * ldc + col0;
-            const __nv_bfloat16* res = residual ? residual + static_cast<int64_t>(row) * ldc + col0 : nullptr;
-#pragma unroll
-            for (int g8 = 0; g8 < 4; ++g8) {
-                if (col0 + g8 * 8 + 8 <= N) {
-                    if (res) {
-                        const uint4 rv = *reinterpret_cast<const uint4*>(res + g8 * 8);
-                        const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&rv);
-#pragma unroll
-                        for (int j = 0; j < 4; ++j) {
-                            const float2 f = __bfloat1622float2(rp[j]);
-                            v[g8 * 8 + 2 * j] += f.x;
-                            v[g8 * 8 + 2 * j + 1] += f.y;
-                        }
-                    }
-                    uint4 o;
-                    o.x = pack_bf16(v[g8 * 8 + 0], v[g8 * 8 + 1]);
-                    o.y = pack_bf16(v[g8 * 8 + 2], v[g8 * 8 + 3]);
-                    o.z = pack_bf16(v[g8 * 8 + 4], v[g8 * 8 + 5]);
-                    o.w = pack_bf16(v[g8 * 8 + 6], v[g8 * 8 + 7]);
-                    *reinterpret_cast<uint4*>(dst + g8 * 8) = o;
-                }
-                else {
-                    for (int j = 0; j < 8; ++j) {
-                        if (col0 + g8 * 8 + j < N) {
-                            float x = v[g8 * 8 + j];
-                            if (res) {
-                                x += __bfloat162float(res[g8 * 8 + j]);
-                            }
-                            dst[g8 * 8 + j] = __float2bfloat16(x);
-                        }
-                    }
-                }
-            }
+        }
+        pack_row(v, stage, lane);
+        stage_out(stage, c, ldc, row0, col0, M, N, lane);
+    }
+
+    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage) const
+    {
+        if (row0 >= M || col0 >= N) {
+            return;  // warp-uniform
+        }
+        half<0>(r, row0, col0, lane, stage);
+        if (col0 + 64 < N) {
+            half<1>(r, row0, col0 + 64, lane, stage);
         }
     }
 };
 
+template <int ACT>
 struct PlainArgs {
-    Core     core;
-    PlainEpi epi;
+    WideCore      core;
+    PlainEpi<ACT> epi;
 };
 
-__global__ void __launch_bounds__(THREADS, 1) gemm_plain_kernel(const __grid_constant__ PlainArgs a)
+template <int MB, int NB, int ACT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WIDE_THREADS, 1) gemm_wide_kernel(const __grid_constant__ PlainArgs<ACT> a)
 {
-    PlainEpi epi = a.epi;
-    run(a.core, epi);
+    PlainEpi<ACT> epi = a.epi;
+    run_wide<MB, NB>(a.core, epi);
 }
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS, 1) gemm_pair_kernel(const __grid_constant__ PlainArgs a)
+template <int ACT>
+__global__ void __launch_bounds__(SMALL_THREADS, 1) gemm_small_kernel(const __grid_constant__ PlainArgs<ACT> a)
 {
-    PlainEpi epi = a.epi;
-    run_pair(a.core, epi);
+    PlainEpi<ACT> epi = a.epi;
+    run_small(a.core, epi);
 }
 
 // ---- fused QKV epilogue: RMSNorm + 3D RoPE + scatter ---------------------------------------------------
@@ -197,25 +207,28 @@ struct QkvParams {
 };
 
 // The functor keeps a reference to the parameters (they stay in the kernel's constant bank) and
-// only its own mutable state in registers.
+// only its own mutable state in registers. A unit is one head of 32 tokens: a thread has the whole
+// 128-value row in registers, so the sum of squares needs no second read of the accumulator.
+template <int EPI_THREADS>
 struct QkvEpi {
+    static constexpr bool kPeers = true;
     const QkvParams& p;
     uint64_t         base_epoch;
 
     __device__ explicit QkvEpi(const QkvParams& params) : p(params), base_epoch(0) {}
 
-    __device__ void open(int epi_warp)
+    __device__ void open(int epi_tid)
     {
         const Peers& peers     = p.peers;
         const int    handshake = p.handshake;
         base_epoch = *reinterpret_cast<volatile uint64_t*>(&peers.own->epoch);
-        if (handshake && epi_warp == 0) {
+        if (handshake && epi_tid < 32) {
             if (blockIdx.x == 0) {
                 hs_announce(peers, base_epoch + 1);
             }
             hs_await(peers, base_epoch + 1, FU_ST_OPEN_TIMEOUT);
         }
-        epi_barrier();  // no epilogue thread stores to a peer before the owners said "go"
+        epi_barrier(EPI_THREADS);  // no epilogue thread stores to a peer before the owners said "go"
     }
 
     __device__ void close(int epi_tid)
@@ -224,11 +237,11 @@ struct QkvEpi {
         const Peers& peers     = p.peers;
         const int    handshake = p.handshake;
         ptx::fence_sys();
-        epi_barrier();
+        epi_barrier(EPI_THREADS);
         if (epi_tid == 0) {
             ticket = atomicAdd(&peers.own->arrive[0], 1u);
         }
-        epi_barrier();
+        epi_barrier(EPI_THREADS);
         if (ticket == gridDim.x - 1 && epi_tid < 32) {
             if (handshake) {
                 ptx::fence_sys();
@@ -243,130 +256,123 @@ struct QkvEpi {
         }
     }
 
-    __device__ void tile(uint32_t tmem_acc, int mt, int nt, int quarter, int lane)
+    // 64 columns of a head: rotate (NORMED), round, and store each row's 128 bytes to its owner. The
+    // staging buffer makes every store instruction write whole 128-byte lines: written straight from
+    // the accumulator layout (a lane is a row) each would scatter 32 separate 16-byte pieces, which
+    // NVLink carries at a fraction of its rate.
+    template <int H, bool NORMED>
+    __device__ __forceinline__ void half(const uint32_t (&r)[128], float scale, const float* gamma, const float2* cs,
+                                         unsigned long long my_dst, int lane, uint8_t* stage) const
     {
-        const int     M = p.M, heads = p.heads;
-        const int64_t s_local = p.s_local, s_total = p.s_total, seq_off = p.seq_off;
-        const float   eps = p.eps;
-        const int     row    = mt * BM + quarter * 32 + lane;
-        const bool    row_ok = row < M;
-        const int64_t batch  = row / s_local;
-        const int64_t s      = row - batch * s_local;
-#pragma unroll 1
-        for (int hh = 0; hh < BN / HEAD_DIM; ++hh) {
-            const int head_global = nt * (BN / HEAD_DIM) + hh;
-            const int type        = head_global / heads;  // 0 q, 1 k, 2 v
-            if (type >= p.n_types) {
-                break;
-            }
-            const bool normed = type < p.n_normed;
-            const int      head  = head_global - type * heads;
-            const int      peer  = p.owner[head];
-            const int64_t  hp    = p.heads_of[peer];
-            uint8_t*       dst   = p.win[type][peer]
-                           + (((batch * s_total + seq_off + s) * hp + p.local[head]) * HEAD_DIM) * 2;
-            const uint32_t tcol  = tmem_acc + hh * HEAD_DIM;
-            float          scale = 1.0f;
-            if (normed) {
-                float ss = 0.0f;
-#pragma unroll 1
-                for (int chunk = 0; chunk < 4; ++chunk) {
-                    uint32_t r[32];
-                    ptx::tmem_ld_32x32(tcol + chunk * 32, r);
-                    ptx::tmem_ld_wait();
 #pragma unroll
-                    for (int j = 0; j < 32; ++j) {
-                        const float x = __uint_as_float(r[j]);
-                        ss += x * x;
-                    }
-                }
-                scale = rsqrtf(ss * (1.0f / HEAD_DIM) + eps);
-            }
-            const float*  gamma = type == 0 ? p.gamma_q : p.gamma_k;
-            const float2* cs    = p.rope + (row_ok ? s : 0) * (HEAD_DIM / 2);
-            // The finished head rows (256 bytes each) go through a per-warp staging buffer so that
-            // every store instruction to the owner's window writes whole rows: lanes 0-15 one row,
-            // lanes 16-31 the next. Written straight from the accumulator layout (a lane is a row)
-            // each instruction would scatter 32 separate 16-byte pieces, which NVLink carries at a
-            // fraction of its rate. 16-byte units are XOR-swizzled by the row so that neither the
-            // row-wise writes nor the row-wide reads conflict on shared-memory banks.
-            uint8_t* stage = stage_of(quarter);
-#pragma unroll 1
-            for (int chunk = 0; chunk < 4; ++chunk) {
-                uint32_t r[32];
-                ptx::tmem_ld_32x32(tcol + chunk * 32, r);
-                ptx::tmem_ld_wait();
-                uint32_t o[16];
-                if (normed) {
-                    if (p.y_save && row_ok) {
-                        uint4* ys = reinterpret_cast<uint4*>(p.y_save + static_cast<int64_t>(row) * p.ld_y
-                                                             + head_global * HEAD_DIM + chunk * 32);
+        for (int g = 0; g < 8; ++g) {
+            uint32_t o[4];
+            if (NORMED) {
+                const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + H * 64 + g * 8));
+                const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma + H * 64 + g * 8 + 4));
+                const float  gm[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
+                const float4 t0 = __ldg(reinterpret_cast<const float4*>(cs + H * 32 + g * 4));
+                const float4 t1 = __ldg(reinterpret_cast<const float4*>(cs + H * 32 + g * 4 + 2));
+                const float  cc[4] = {t0.x, t0.z, t1.x, t1.z}, sn[4] = {t0.y, t0.w, t1.y, t1.w};
 #pragma unroll
-                        for (int q4 = 0; q4 < 4; ++q4) {
-                            ys[q4] = make_uint4(pack_bf16(__uint_as_float(r[8 * q4]), __uint_as_float(r[8 * q4 + 1])),
-                                                pack_bf16(__uint_as_float(r[8 * q4 + 2]), __uint_as_float(r[8 * q4 + 3])),
-                                                pack_bf16(__uint_as_float(r[8 * q4 + 4]), __uint_as_float(r[8 * q4 + 5])),
-                                                pack_bf16(__uint_as_float(r[8 * q4 + 6]), __uint_as_float(r[8 * q4 + 7])));
-                        }
-                    }
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        const int    c0 = chunk * 32 + 2 * i;
-                        const float  x0 = __uint_as_float(r[2 * i]) * scale * gamma[c0];
-                        const float  x1 = __uint_as_float(r[2 * i + 1]) * scale * gamma[c0 + 1];
-                        const float2 t  = cs[chunk * 16 + i];
-                        o[i]            = pack_bf16(x0 * t.x - x1 * t.y, x0 * t.y + x1 * t.x);
-                    }
-                }
-                else {
-#pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        o[i] = pack_bf16(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-                    }
-                }
-#pragma unroll
-                for (int q4 = 0; q4 < 4; ++q4) {
-                    const int unit = (chunk * 4 + q4) ^ (lane & 15);
-                    *reinterpret_cast<uint4*>(stage + lane * 256 + unit * 16) =
-                        make_uint4(o[4 * q4], o[4 * q4 + 1], o[4 * q4 + 2], o[4 * q4 + 3]);
+                for (int k = 0; k < 4; ++k) {
+                    const float x0 = __uint_as_float(r[H * 64 + g * 8 + 2 * k]) * scale * gm[2 * k];
+                    const float x1 = __uint_as_float(r[H * 64 + g * 8 + 2 * k + 1]) * scale * gm[2 * k + 1];
+                    o[k]           = pack_bf16(x0 * cc[k] - x1 * sn[k], x0 * sn[k] + x1 * cc[k]);
                 }
             }
-            __syncwarp();
-            const unsigned long long my_dst = row_ok ? reinterpret_cast<unsigned long long>(dst) : 0ull;
-            const int                unit   = lane & 15;
-#pragma unroll 4
-            for (int i = 0; i < 16; ++i) {
-                const int                r_src = 2 * i + (lane >> 4);
-                const unsigned long long to    = __shfl_sync(0xffffffffu, my_dst, r_src);
-                const uint4 v = *reinterpret_cast<const uint4*>(stage + r_src * 256 + ((unit ^ (r_src & 15)) * 16));
-                if (to) {
-                    ptx::st_v4(reinterpret_cast<uint4*>(to) + unit, v);
+            else {
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    o[k] = pack_bf16(__uint_as_float(r[H * 64 + g * 8 + 2 * k]), __uint_as_float(r[H * 64 + g * 8 + 2 * k + 1]));
                 }
             }
-            __syncwarp();  // the buffer is refilled by the next head
+            *stage_unit(stage, lane, g) = make_uint4(o[0], o[1], o[2], o[3]);
         }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int                from = i * 4 + (lane >> 3);
+            const unsigned long long to   = __shfl_sync(0xffffffffu, my_dst, from);
+            const uint4              v    = *stage_unit(stage, from, lane & 7);
+            if (to) {
+                ptx::st_v4(reinterpret_cast<uint4*>(to) + H * 8 + (lane & 7), v);
+            }
+        }
+        __syncwarp();  // the buffer may be refilled
     }
 
-    // 8 KiB of staging per epilogue warp, behind the operand ring in dynamic shared memory.
-    static constexpr int kStageBytesPerWarp = 32 * HEAD_DIM * 2;
-    static constexpr int kExtraSmem         = 4 * kStageBytesPerWarp;
-    __device__ static uint8_t* stage_of(int quarter)
+    template <int H>
+    __device__ __forceinline__ void save(const uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage) const
     {
-        extern __shared__ uint8_t smem_raw[];
-        const uint32_t base = (ptx::smem_addr(smem_raw) + 1023u) & ~1023u;
-        return smem_raw + (base - ptx::smem_addr(smem_raw)) + STAGES * STAGE_BYTES + quarter * kStageBytesPerWarp;
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            uint32_t o[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                o[k] = pack_bf16(__uint_as_float(r[H * 64 + g * 8 + 2 * k]), __uint_as_float(r[H * 64 + g * 8 + 2 * k + 1]));
+            }
+            *stage_unit(stage, lane, g) = make_uint4(o[0], o[1], o[2], o[3]);
+        }
+        stage_out(stage, p.y_save, p.ld_y, row0, col0 + H * 64, p.M, 0x7fffffff, lane);
+    }
+
+    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage) const
+    {
+        const int head_global = col0 / HEAD_DIM;
+        const int type        = head_global / p.heads;  // 0 q, 1 k, 2 v
+        if (row0 >= p.M || type >= p.n_types) {
+            return;  // warp-uniform
+        }
+        const int     row    = row0 + lane;
+        const bool    row_ok = row < p.M;
+        const int64_t batch  = row / p.s_local;
+        const int64_t s      = row - batch * p.s_local;
+        const int     head   = head_global - type * p.heads;
+        const int     peer   = p.owner[head];
+        const int64_t hp     = p.heads_of[peer];
+        uint8_t*      dst    = p.win[type][peer] + (((batch * p.s_total + p.seq_off + s) * hp + p.local[head]) * HEAD_DIM) * 2;
+        const unsigned long long my_dst = row_ok ? reinterpret_cast<unsigned long long>(dst) : 0ull;
+        if (type < p.n_normed) {
+            float ss4[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int j = 0; j < HEAD_DIM; ++j) {
+                const float x = __uint_as_float(r[j]);
+                ss4[j & 3] += x * x;
+            }
+            const float   scale = rsqrtf(((ss4[0] + ss4[1]) + (ss4[2] + ss4[3])) * (1.0f / HEAD_DIM) + p.eps);
+            const float*  gamma = type == 0 ? p.gamma_q : p.gamma_k;
+            const float2* cs    = p.rope + (row_ok ? s : 0) * (HEAD_DIM / 2);
+            if (p.y_save) {
+                save<0>(r, row0, col0, lane, stage);
+                save<1>(r, row0, col0, lane, stage);
+            }
+            half<0, true>(r, scale, gamma, cs, my_dst, lane, stage);
+            half<1, true>(r, scale, gamma, cs, my_dst, lane, stage);
+        }
+        else {
+            half<0, false>(r, 1.0f, nullptr, nullptr, my_dst, lane, stage);
+            half<1, false>(r, 1.0f, nullptr, nullptr, my_dst, lane, stage);
+        }
     }
 };
 
 struct QkvArgs {
-    Core      core;
+    WideCore  core;
     QkvParams epi;
 };
 
-__global__ void __launch_bounds__(THREADS, 1) qkv_rope_scatter_kernel(const __grid_constant__ QkvArgs a)
+template <int MB, int NB>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WIDE_THREADS, 1) qkv_wide_kernel(const __grid_constant__ QkvArgs a)
 {
-    QkvEpi epi(a.epi);
-    run(a.core, epi);
+    QkvEpi<32 * WIDE_EPI_WARPS> epi(a.epi);
+    run_wide<MB, NB>(a.core, epi);
+}
+
+__global__ void __launch_bounds__(SMALL_THREADS, 1) qkv_small_kernel(const __grid_constant__ QkvArgs a)
+{
+    QkvEpi<32 * SMALL_EPI_WARPS> epi(a.epi);
+    run_small(a.core, epi);
 }
 
 // ---- fused mode-1 path: pull attention output from peers, feed the output projection -----------------
@@ -500,24 +506,103 @@ struct PullAux {
     }
 };
 
+// The projection's epilogue: bias and residual. A lane is a row.
+struct PullEpi {
+    __nv_bfloat16*       c;
+    const __nv_bfloat16* residual;
+    const void*          bias;
+    int64_t              ldc;
+    int                  M, N, bias_bf16;
+
+    __device__ void open(int) {}
+    __device__ void close(int) {}
+
+    __device__ void tile(uint32_t tmem_acc, int mt, int nt, int quarter, int lane)
+    {
+        const int  row    = mt * BM + quarter * 32 + lane;
+        const bool row_ok = row < M;
+#pragma unroll 1
+        for (int chunk = 0; chunk < BN / 32; ++chunk) {
+            const int col0 = nt * BN + chunk * 32;
+            if (col0 >= N) {
+                break;  // warp-uniform
+            }
+            uint32_t r[32];
+            ptx::tmem_ld_32x32(tmem_acc + chunk * 32, r);
+            ptx::tmem_ld_wait();
+            if (!row_ok) {
+                continue;
+            }
+            __nv_bfloat16*       dst = c + static_cast<int64_t>(row) * ldc + col0;
+            const __nv_bfloat16* res = residual ? residual + static_cast<int64_t>(row) * ldc + col0 : nullptr;
+#pragma unroll
+            for (int g8 = 0; g8 < 4; ++g8) {
+                float v[8];
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    v[j] = __uint_as_float(r[g8 * 8 + j]);
+                    if (bias && col0 + g8 * 8 + j < N) {
+                        v[j] += bias_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[col0 + g8 * 8 + j])
+                                          : static_cast<const float*>(bias)[col0 + g8 * 8 + j];
+                    }
+                }
+                if (col0 + g8 * 8 + 8 <= N) {
+                    if (res) {
+                        const uint4 rv = *reinterpret_cast<const uint4*>(res + g8 * 8);
+                        const __nv_bfloat162* rp = reinterpret_cast<const __nv_bfloat162*>(&rv);
+#pragma unroll
+                        for (int j = 0; j < 4; ++j) {
+                            const float2 f = __bfloat1622float2(rp[j]);
+                            v[2 * j] += f.x;
+                            v[2 * j + 1] += f.y;
+                        }
+                    }
+                    *reinterpret_cast<uint4*>(dst + g8 * 8) =
+                        make_uint4(pack_bf16(v[0], v[1]), pack_bf16(v[2], v[3]), pack_bf16(v[4], v[5]), pack_bf16(v[6], v[7]));
+                }
+                else {
+                    for (int j = 0; j < 8; ++j) {
+                        if (col0 + g8 * 8 + j < N) {
+                            dst[g8 * 8 + j] = __float2bfloat16(v[j] + (res ? __bfloat162float(res[g8 * 8 + j]) : 0.0f));
+                        }
+                    }
+                }
+            }
+        }
+    }
+};
+
 struct PullArgs {
     Core       core;
-    PlainEpi   epi;
+    PullEpi    epi;
     PullParams pull;
 };
 
 __global__ void __launch_bounds__(THREADS + 128, 1) pull_outproj_kernel(const __grid_constant__ PullArgs a)
 {
-    PlainEpi epi = a.epi;
+    PullEpi epi = a.epi;
     run(a.core, epi, PullSrc(a.pull), PullAux(a.pull));
+}
+
+int device_sms()
+{
+    static int cached[64] = {};
+    int        dev        = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        return 148;
+    }
+    if (cached[dev] == 0) {
+        int sms = 0;
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+        cached[dev] = sms;
+    }
+    return cached[dev];
 }
 
 int launch_grid(int ctas, int tiles)
 {
-    int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    int g = ctas > 0 ? std::min(ctas, sms) : sms;
+    const int sms = device_sms();
+    const int g   = ctas > 0 ? std::min(ctas, sms) : sms;
     return std::max(1, std::min(g, tiles));
 }
 
@@ -530,11 +615,13 @@ int set_smem(K kernel, int bytes = SMEM_BYTES)
         int         dev;
         const void* fn;
     };
-    static Done done[256];
-    static int  n_done = 0;
-    int         dev    = 0;
+    static std::mutex lock;
+    static Done       done[256];
+    static int        n_done = 0;
+    int               dev    = 0;
     FU_CUDA_OK(cudaGetDevice(&dev));
-    const void* fn = reinterpret_cast<const void*>(kernel);
+    const void*                       fn = reinterpret_cast<const void*>(kernel);
+    const std::lock_guard<std::mutex> guard(lock);
     for (int i = 0; i < n_done; ++i) {
         if (done[i].dev == dev && done[i].fn == fn) {
             return FU_OK;
@@ -547,8 +634,8 @@ int set_smem(K kernel, int bytes = SMEM_BYTES)
     return FU_OK;
 }
 
-// How many CTA pairs of the pair kernel the device holds at once (GPCs with an odd number of SMs
-// leave one SM without a partner). Asked once per device.
+// How many CTA pairs of the wide kernels the device holds at once (GPCs with an odd number of SMs
+// leave one SM without a partner). Asked once per device; all of them have the same shape.
 int pair_capacity()
 {
     static int cached[64] = {};
@@ -557,10 +644,11 @@ int pair_capacity()
         return 0;
     }
     if (cached[dev] == 0) {
+        auto               kernel = gemm_wide_kernel<1, 2, 0>;
         cudaLaunchConfig_t cfg{};
         cfg.gridDim          = dim3(2, 1, 1);
-        cfg.blockDim         = dim3(THREADS, 1, 1);
-        cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
+        cfg.blockDim         = dim3(WIDE_THREADS, 1, 1);
+        cfg.dynamicSmemBytes = WIDE_SMEM_BYTES;
         cudaLaunchAttribute attr{};
         attr.id               = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = 2;
@@ -569,19 +657,18 @@ int pair_capacity()
         cfg.attrs             = &attr;
         cfg.numAttrs          = 1;
         int n                 = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel, &cfg) != cudaSuccess || n < 1) {
+        if (set_smem(kernel, WIDE_SMEM_BYTES) != FU_OK || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess
+            || n < 1) {
             (void)cudaGetLastError();
             // the kernel carries its cluster shape itself; ask again without naming it
             cfg.attrs    = nullptr;
             cfg.numAttrs = 0;
             n            = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, gemm_pair_kernel, &cfg) != cudaSuccess || n < 1) {
+            if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
                 (void)cudaGetLastError();
                 // Pairs do not wait for one another, so a grid larger than what is resident at once
                 // is merely scheduled in turns: assume every SM finds a partner.
-                int sms = 0;
-                cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-                n = sms / 2;
+                n = device_sms() / 2;
             }
         }
         cached[dev] = n > 0 ? n : -1;
@@ -589,23 +676,61 @@ int pair_capacity()
     return cached[dev] > 0 ? cached[dev] : 0;
 }
 
-int fill_core(Core& core, const void* a, const void* b, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb,
-              uint32_t* err, int flags = 0)
+// Which core and tile a problem gets, from its size alone: the one whose estimated time is lowest. The
+// estimate is a start-and-end time plus, per wave of CTAs, a time per 64-wide K-block, both measured
+// (us, SM clock 1.9 GHz, problems of 64 - 2048 rows and 256 - 5120 columns and K):
+//   128 x 128 tiles on single CTAs   5 + 0.225 per K-block and wave of 148
+//   256 x 256 blocks on pairs        8 + 0.305 per K-block and block of each wave of 74 (a whole tile is two
+//                                    blocks; a block by itself takes 1.05)
+// Of the two wide orientations, which move the same bytes, the one with the fuller last wave wins; when at
+// most half as many tiles as pairs are left over, those are split into blocks.
+enum class Shape { kSmall, kTall, kBroad };  // 128 x 128; 512 x 256; 256 x 512
+struct Choice {
+    Shape shape;
+    int   tiles_m, tiles_n, full, items;
+};
+
+Choice wide_choice(int64_t m, int64_t n, Shape shape, int pairs)
+{
+    const int64_t tm    = shape == Shape::kTall ? (m + 511) / 512 : (m + 255) / 256;
+    const int64_t tn    = shape == Shape::kTall ? (n + 255) / 256 : (n + 511) / 512;
+    const int64_t tiles = tm * tn, left = tiles % pairs;
+    const int64_t full = 2 * left <= pairs ? tiles - left : tiles;
+    return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(full), static_cast<int>(full + 2 * (tiles - full))};
+}
+
+double wide_cost(const Choice& c, int pairs)
+{
+    return 2.0 * ((c.full + pairs - 1) / pairs) + 1.05 * ((c.items - c.full + pairs - 1) / pairs);
+}
+
+Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int flags)
+{
+    const int64_t t128 = ((m + 127) / 128) * ((n + 127) / 128);
+    const Choice  small{Shape::kSmall, static_cast<int>((m + 127) / 128), static_cast<int>((n + 127) / 128), 0,
+                       static_cast<int>(t128)};
+    if (flags & FU_GEMM_SINGLE) {
+        return small;
+    }
+    const Choice tall = wide_choice(m, n, Shape::kTall, pairs), broad = wide_choice(m, n, Shape::kBroad, pairs);
+    const Choice wide = wide_cost(tall, pairs) < wide_cost(broad, pairs) ? tall : broad;
+    if (flags & FU_GEMM_PAIR) {
+        return wide;
+    }
+    const double kb = static_cast<double>((k + BK - 1) / BK);
+    return 5.0 + 0.225 * kb * ((t128 + sms - 1) / sms) < 8.0 + 0.305 * kb * wide_cost(wide, pairs) ? small : wide;
+}
+
+int fill_core(Core& core, const void* a, const void* b, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb, uint32_t* err)
 {
     if (m <= 0 || n <= 0 || k <= 0) {
         return fu::fail(FU_E_ARG, "gemm: empty problem (m=%lld n=%lld k=%lld)", (long long)m, (long long)n, (long long)k);
     }
-    // K itself may be anything (TMA zero-fills the part of a box that lies past it); what TMA needs
-    // is a 16-byte row pitch, which make_map_2d checks on lda and ldb.
-    core.a_mn = (flags & FU_GEMM_A_KM) ? 1 : 0;
-    core.b_mn = (flags & FU_GEMM_B_KN) ? 1 : 0;
-    int rc = core.a_mn ? make_map_2d(&core.map_a, a, 2, k, m, lda, 64, 64) : make_map_2d(&core.map_a, a, 2, m, k, lda, BM, BK);
+    int rc = make_map_2d(&core.map_a, a, 2, m, k, lda, BM, BK);
     if (rc != FU_OK) {
         return rc;
     }
-    // a CTA pair splits B's rows of a tile between its two CTAs
-    const int b_rows = (flags & FU_GEMM_PAIR) ? BN / 2 : BN;
-    rc = core.b_mn ? make_map_2d(&core.map_b, b, 2, k, n, ldb, 64, 64) : make_map_2d(&core.map_b, b, 2, n, k, ldb, b_rows, BK);
+    rc = make_map_2d(&core.map_b, b, 2, n, k, ldb, BN, BK);
     if (rc != FU_OK) {
         return rc;
     }
@@ -618,9 +743,104 @@ int fill_core(Core& core, const void* a, const void* b, int64_t m, int64_t n, in
     return FU_OK;
 }
 
+int fill_wide(WideCore& core, const Choice& c, const void* a, const void* b, int64_t m, int64_t n, int64_t k, int64_t lda,
+              int64_t ldb, uint32_t* err, int flags)
+{
+    // K itself may be anything (TMA zero-fills the part of a box that lies past it); what TMA needs
+    // is a 16-byte row pitch, which make_map_2d checks on lda and ldb. Every box is 128 rows of one
+    // operand (or a 64 x 64 block of one stored with the contraction along its rows).
+    core.a_mn = (flags & FU_GEMM_A_KM) ? 1 : 0;
+    core.b_mn = (flags & FU_GEMM_B_KN) ? 1 : 0;
+    int rc = core.a_mn ? make_map_2d(&core.map_a, a, 2, k, m, lda, 64, 64) : make_map_2d(&core.map_a, a, 2, m, k, lda, 128, BK);
+    if (rc != FU_OK) {
+        return rc;
+    }
+    rc = core.b_mn ? make_map_2d(&core.map_b, b, 2, k, n, ldb, 64, 64) : make_map_2d(&core.map_b, b, 2, n, k, ldb, 128, BK);
+    if (rc != FU_OK) {
+        return rc;
+    }
+    core.M       = static_cast<int>(m);
+    core.N       = static_cast<int>(n);
+    core.K       = static_cast<int>(k);
+    core.tiles_m = c.tiles_m;
+    core.tiles_n = c.tiles_n;
+    core.full    = c.full;
+    core.items   = c.items;
+    core.err     = err;
+    return FU_OK;
+}
+
+int check_extents(int64_t m, int64_t n, int64_t k)
+{
+    if (m <= 0 || n <= 0 || k <= 0 || m > 0x7fffff00 || n > 0x7fffff00 || k > 0x7fffff00) {
+        return fu::fail(FU_E_ARG, "gemm: empty problem or one too large (m=%lld n=%lld k=%lld)", (long long)m, (long long)n,
+                        (long long)k);
+    }
+    return FU_OK;
+}
+
+// How many pairs a launch may use (`ctas` > 0 limits it), or 0 with the error set.
+int pairs_for(int ctas)
+{
+    const int pairs = pair_capacity();
+    if (pairs < 1) {
+        fu::fail(FU_E_CUDA, "this device cannot hold a cluster of two CTAs of the pair kernels");
+        return 0;
+    }
+    return ctas > 0 ? std::max(1, std::min(pairs, ctas / 2)) : pairs;
+}
+
+template <class Kernel, class Args>
+int launch_pairs(Kernel kernel, const Args& a, int pairs, cudaStream_t stream)
+{
+    const int rc = set_smem(kernel, WIDE_SMEM_BYTES);
+    if (rc != FU_OK) {
+        return rc;
+    }
+    kernel<<<2 * std::max(1, std::min(pairs, a.core.items)), WIDE_THREADS, WIDE_SMEM_BYTES, stream>>>(a);
+    FU_CUDA_OK(cudaGetLastError());
+    return FU_OK;
+}
+
+template <class Kernel, class Args>
+int launch_small(Kernel kernel, const Args& a, int ctas, cudaStream_t stream)
+{
+    const int rc = set_smem(kernel, SMALL_SMEM_BYTES);
+    if (rc != FU_OK) {
+        return rc;
+    }
+    kernel<<<launch_grid(ctas, a.core.items), SMALL_THREADS, SMALL_SMEM_BYTES, stream>>>(a);
+    FU_CUDA_OK(cudaGetLastError());
+    return FU_OK;
+}
+
+template <int ACT>
+int launch_plain(const FuGemmArgs* g, const Choice& c, int pairs, int flags, cudaStream_t stream)
+{
+    PlainArgs<ACT> a{};
+    const int      rc = fill_wide(a.core, c, g->a, g->b, g->m, g->n, g->k, g->lda, g->ldb, g->err, flags);
+    if (rc != FU_OK) {
+        return rc;
+    }
+    a.epi.c         = static_cast<__nv_bfloat16*>(g->c);
+    a.epi.residual  = static_cast<const __nv_bfloat16*>(g->residual);
+    a.epi.bias      = g->bias;
+    a.epi.bias_bf16 = (flags & FU_GEMM_BIAS_BF16) ? 1 : 0;
+    a.epi.ldc       = g->ldc;
+    a.epi.M         = a.core.M;
+    a.epi.N         = a.core.N;
+    a.epi.aux       = static_cast<const __nv_bfloat16*>(g->aux);
+    a.epi.c_pre     = static_cast<__nv_bfloat16*>(g->c_pre);
+    switch (c.shape) {
+    case Shape::kTall: return launch_pairs(gemm_wide_kernel<2, 1, ACT>, a, pairs, stream);
+    case Shape::kBroad: return launch_pairs(gemm_wide_kernel<1, 2, ACT>, a, pairs, stream);
+    default: return launch_small(gemm_small_kernel<ACT>, a, g->ctas, stream);
+    }
+}
+
 }  // namespace
 
-extern "C" int fu_gemm_bf16(const FuGemmArgs* g, void* stream)
+extern "C" int fu_gemm_bf16(const FuGemmArgs* g, void* stream_v)
 {
     if (!g || !g->a || !g->b || !g->c) {
         return fu::fail(FU_E_ARG, "fu_gemm_bf16: null operand");
@@ -629,29 +849,6 @@ extern "C" int fu_gemm_bf16(const FuGemmArgs* g, void* stream)
         || (g->residual && (reinterpret_cast<uintptr_t>(g->residual) & 15u))) {
         return fu::fail(FU_E_ARG, "fu_gemm_bf16: C (and the residual) need 16-byte aligned rows");
     }
-    // CTA pairs are chosen per call (FU_GEMM_PAIR / FU_GEMM_SINGLE) or, for calls that say nothing,
-    // by the environment variable FU_GEMM_PAIR (read once).
-    static const bool pair_default = [] {
-        const char* e = std::getenv("FU_GEMM_PAIR");
-        return e && e[0] == '1';
-    }();
-    const bool pair  = (g->flags & FU_GEMM_PAIR) || (pair_default && !(g->flags & FU_GEMM_SINGLE));
-    const int  flags = pair ? (g->flags | FU_GEMM_PAIR) : (g->flags & ~FU_GEMM_PAIR);
-    PlainArgs a{};
-    int       rc = fill_core(a.core, g->a, g->b, g->m, g->n, g->k, g->lda, g->ldb, g->err, flags);
-    if (rc != FU_OK) {
-        return rc;
-    }
-    a.epi.c        = static_cast<__nv_bfloat16*>(g->c);
-    a.epi.residual = static_cast<const __nv_bfloat16*>(g->residual);
-    a.epi.bias     = g->bias;
-    a.epi.bias_bf16 = (g->flags & FU_GEMM_BIAS_BF16) ? 1 : 0;
-    a.epi.ldc      = g->ldc;
-    a.epi.M        = a.core.M;
-    a.epi.N        = a.core.N;
-    a.epi.act      = g->act;
-    a.epi.aux      = static_cast<const __nv_bfloat16*>(g->aux);
-    a.epi.c_pre    = static_cast<__nv_bfloat16*>(g->c_pre);
     if (g->act < 0 || g->act > 3 || (g->act == 3 && !g->aux)) {
         return fu::fail(FU_E_ARG, "fu_gemm_bf16: act=%d (0..3; 3 needs aux)", g->act);
     }
@@ -659,30 +856,31 @@ extern "C" int fu_gemm_bf16(const FuGemmArgs* g, void* stream)
                                  || (reinterpret_cast<uintptr_t>(g->c_pre) & 15u))) {
         return fu::fail(FU_E_ARG, "fu_gemm_bf16: aux / c_pre need n %% 8 == 0 and 16-byte aligned rows");
     }
-    if (pair) {
-        rc = set_smem(gemm_pair_kernel, PAIR_SMEM_BYTES);
-        if (rc != FU_OK) {
-            return rc;
-        }
-        const int pairs = pair_capacity();
-        if (pairs < 1) {
-            return fu::fail(FU_E_CUDA, "fu_gemm_bf16: this device cannot hold a cluster of two CTAs of the pair kernel");
-        }
-        const int tiles = ((a.core.tiles_m + 1) / 2) * a.core.tiles_n;
-        int       want  = g->ctas > 0 ? std::max(1, g->ctas / 2) : pairs;
-        want            = std::max(1, std::min(std::min(want, pairs), tiles));
-        gemm_pair_kernel<<<2 * want, THREADS, PAIR_SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(a);
-        FU_CUDA_OK(cudaGetLastError());
-        return FU_OK;
-    }
-    rc             = set_smem(gemm_plain_kernel);
+    int rc = check_extents(g->m, g->n, g->k);
     if (rc != FU_OK) {
         return rc;
     }
-    const int grid = launch_grid(g->ctas, a.core.tiles_m * a.core.tiles_n);
-    gemm_plain_kernel<<<grid, THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(a);
-    FU_CUDA_OK(cudaGetLastError());
-    return FU_OK;
+    // The shape is chosen by size unless the call (FU_GEMM_PAIR / FU_GEMM_SINGLE) or, for calls that say
+    // nothing, the environment variable FU_GEMM_PAIR (read once) asks for pairs.
+    static const bool pair_default = [] {
+        const char* e = std::getenv("FU_GEMM_PAIR");
+        return e && e[0] == '1';
+    }();
+    const int pairs = pairs_for(g->ctas);
+    if (pairs < 1) {
+        return FU_E_CUDA;
+    }
+    const bool   forced = pair_default && !(g->flags & FU_GEMM_SINGLE);
+    const int    flags  = forced ? (g->flags | FU_GEMM_PAIR) : g->flags;
+    const int    sms    = g->ctas > 0 ? std::min(g->ctas, device_sms()) : device_sms();
+    const Choice c      = choose_shape(g->m, g->n, g->k, pairs, sms, flags);
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    switch (g->act) {
+    case 0: return launch_plain<0>(g, c, pairs, flags, stream);
+    case 1: return launch_plain<1>(g, c, pairs, flags, stream);
+    case 2: return launch_plain<2>(g, c, pairs, flags, stream);
+    default: return launch_plain<3>(g, c, pairs, flags, stream);
+    }
 }
 
 extern "C" int fu_qkv_rope_scatter_check(const FuQkvArgs* q)
@@ -738,7 +936,7 @@ extern "C" int fu_qkv_rope_scatter_check(const FuQkvArgs* q)
     return FU_OK;
 }
 
-extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream)
+extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream_v)
 {
     int rc = fu_qkv_rope_scatter_check(q);
     if (rc != FU_OK) {
@@ -746,9 +944,20 @@ extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream)
     }
     const int n_types  = q->n_types > 0 ? q->n_types : 3;
     const int n_normed = q->n_types > 0 ? q->n_normed : 2;
-    QkvArgs a{};
-    rc = fill_core(a.core, q->x, q->w, q->m, static_cast<int64_t>(n_types) * q->heads * HEAD_DIM, q->k, q->ldx, q->ldw,
-                   q->err, (q->flags & FU_QKV_W_KN) ? FU_GEMM_B_KN : 0);
+    QkvArgs       a{};
+    const int64_t n = static_cast<int64_t>(n_types) * q->heads * HEAD_DIM;
+    rc              = check_extents(q->m, n, q->k);
+    if (rc != FU_OK) {
+        return rc;
+    }
+    const int pairs = pairs_for(q->ctas);
+    if (pairs < 1) {
+        return FU_E_CUDA;
+    }
+    const int    sms   = q->ctas > 0 ? std::min(q->ctas, device_sms()) : device_sms();
+    const int    flags = (q->flags & FU_QKV_W_KN) ? FU_GEMM_B_KN : 0;
+    const Choice c     = choose_shape(q->m, n, q->k, pairs, sms, flags);
+    rc = fill_wide(a.core, c, q->x, q->w, q->m, n, q->k, q->ldx, q->ldw, q->err, flags);
     if (rc != FU_OK) {
         return rc;
     }
@@ -799,14 +1008,12 @@ extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream)
     if (q->y_save && ((q->ld_y % 8) || (reinterpret_cast<uintptr_t>(q->y_save) & 15u))) {
         return fu::fail(FU_E_ARG, "fu_qkv_rope_scatter: y_save needs 16-byte aligned rows");
     }
-    rc                 = set_smem(qkv_rope_scatter_kernel, SMEM_BYTES + QkvEpi::kExtraSmem);
-    if (rc != FU_OK) {
-        return rc;
+    cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+    switch (c.shape) {
+    case Shape::kTall: return launch_pairs(qkv_wide_kernel<2, 1>, a, pairs, stream);
+    case Shape::kBroad: return launch_pairs(qkv_wide_kernel<1, 2>, a, pairs, stream);
+    default: return launch_small(qkv_small_kernel, a, q->ctas, stream);
     }
-    const int grid = launch_grid(q->ctas, a.core.tiles_m * a.core.tiles_n);
-    qkv_rope_scatter_kernel<<<grid, THREADS, SMEM_BYTES + QkvEpi::kExtraSmem, static_cast<cudaStream_t>(stream)>>>(a);
-    FU_CUDA_OK(cudaGetLastError());
-    return FU_OK;
 }
 
 extern "C" int fu_pull_outproj_check(const FuPullArgs* q)
@@ -910,7 +1117,6 @@ extern "C" int fu_pull_outproj(const FuPullArgs* q, void* stream_v)
     a.epi.ldc          = q->ldc;
     a.epi.M            = a.core.M;
     a.epi.N            = a.core.N;
-    a.epi.act          = 0;
     rc                 = set_smem(pull_outproj_kernel);
     if (rc != FU_OK) {
         return rc;

@@ -1,20 +1,18 @@
 #pragma once
-// A persistent, warp-specialised bf16 GEMM for sm_100a: D[M,N] = A[M,K] * B[N,K]^T with fp32
+// Persistent, warp-specialised bf16 GEMM cores for sm_100a: D[M,N] = A[M,K] * B[N,K]^T with fp32
 // accumulation in tensor memory. Either operand may instead be given with the contraction along
 // its rows (A stored K x M, B stored K x N, "MN-major"): the weight gradient of a linear layer
 // contracts over the tokens and reads dY and X as they lie in memory, without a transposed copy.
 //
-//   warp 0      TMA producer: A and B tiles (128B-swizzled, K-major) into a 4-stage shared-memory ring
-//   warp 1      MMA issuer:   one elected thread issues tcgen05.mma 128x256x16, accumulators in TMEM
-//   warps 2..5  epilogue:     tcgen05.ld the accumulator (each warp owns a 32-lane quarter) and apply
-//                             the epilogue functor; double-buffered accumulators (2 x 256 TMEM
-//                             columns) let the epilogue of tile i overlap the main loop of tile i+1
+//   run_wide    two 256 x 256 blocks per pair of CTAs: everything large enough to occupy the device
+//   run_small   128 x 128 tiles on single CTAs: everything else
+//   run         128 x 256 tiles on single CTAs, A gathered from the peers by extra warps while the GEMM runs
 //
-// One CTA per SM, tiles visited in bands of 16 M-tiles so that a wave of CTAs shares A and B tiles
-// through L2. No TMA load is multicast; every CTA fetches its own tiles.
-//
-// The epilogue is a template parameter: a functor called by the four epilogue warps with the
-// accumulator buffer of a finished tile. Kernels that write peers' memory from the epilogue run
+// In each, warp 0 is the TMA producer (128B-swizzled operand tiles into a ring of shared-memory
+// stages), warp 1 issues tcgen05.mma, and the other warps are the epilogue: they read the accumulator
+// from tensor memory (each warp may touch one 32-lane quarter) and apply the epilogue functor. Tiles are
+// visited in bands of M-tiles so that a wave of CTAs shares operand tiles through L2. No TMA load is
+// multicast; every CTA fetches its own tiles. Kernels that write peers' memory from the epilogue run
 // their handshake through `Epi::open` / `Epi::close`.
 #include <cuda.h>
 #include <cuda_bf16.h>
@@ -51,7 +49,6 @@ struct Core {
     CUtensorMap map_b;
     int         M, N, K;
     int         tiles_m, tiles_n;
-    int         a_mn, b_mn;  // operand stored K x M (K x N): tiles are fetched as 64 x 64 blocks
     uint32_t*   err;
 };
 
@@ -72,24 +69,16 @@ __device__ __forceinline__ void flag_error(const Core& c, uint32_t code)
     }
 }
 
-// Optional policies. `Src::ready(mt, kb)` runs in the producer thread before the loads of K-block
+// `Src::ready(mt, kb)` runs in the producer thread before the loads of K-block
 // `kb` of M-tile `mt` are issued and may wait (bounded) for that part of A to exist; it returns
 // false to give up. `Aux::run(aux_warp, lane)` is executed by `Aux::kWarps` extra warps (warps 6..)
 // alongside the GEMM, e.g. to pull A from peers' memory into the buffer the GEMM reads.
-struct NoSrc {
-    __device__ __forceinline__ bool ready(int, int) const { return true; }
-};
-struct NoAux {
-    static constexpr int kWarps = 0;
-    __device__ __forceinline__ void run(int, int) const {}
-};
-
 // Epi requirements:
 //   __device__ void open(int epi_warp)                       once, before the first tile
 //   __device__ void tile(uint32_t tmem_acc, int mt, int nt, int quarter, int lane)
 //   __device__ void close(int epi_tid)                       once, after the last tile (all 128 threads)
-template <class Epi, class Src = NoSrc, class Aux = NoAux>
-__device__ __forceinline__ void run(const Core& core, Epi& epi, Src src = Src{}, Aux aux = Aux{})
+template <class Epi, class Src, class Aux>
+__device__ __forceinline__ void run(const Core& core, Epi& epi, Src src, Aux aux)
 {
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t       full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2];
@@ -97,7 +86,7 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src = Src{},
 
     const uint32_t base = (ptx::smem_addr(smem_raw) + 1023u) & ~1023u;
     uint8_t*       ring = smem_raw + (base - ptx::smem_addr(smem_raw));
-    const int      warp = threadIdx.x >> 5;
+    const int      warp = static_cast<int>(ptx::uniform(threadIdx.x >> 5));
     const int      lane = threadIdx.x & 31;
     const int      total_tiles = core.tiles_m * core.tiles_n;
     const int      kblocks     = (core.K + BK - 1) / BK;
@@ -122,7 +111,7 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src = Src{},
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem_base = tmem_holder;
+    const uint32_t tmem_base = ptx::uniform(tmem_holder);
 
     if (warp == 0) {
         if (lane == 0) {
@@ -142,67 +131,51 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src = Src{},
                     uint8_t* sa = ring + s * STAGE_BYTES;
                     uint8_t* sb = sa + A_BYTES;
                     ptx::mbar_expect_tx(&full[s], STAGE_BYTES);
-                    if (!core.a_mn) {
-                        ptx::tma_load_2d(sa, &core.map_a, kb * BK, mt * BM, &full[s]);
-                    }
-                    else {  // 64 (k) x 64 (m) blocks of 8 KiB, one per 64 columns of the tile
-                        for (int j = 0; j < BM / 64; ++j) {
-                            ptx::tma_load_2d(sa + j * 8192, &core.map_a, mt * BM + j * 64, kb * BK, &full[s]);
-                        }
-                    }
-                    if (!core.b_mn) {
-                        ptx::tma_load_2d(sb, &core.map_b, kb * BK, nt * BN, &full[s]);
-                    }
-                    else {
-                        for (int j = 0; j < BN / 64; ++j) {
-                            ptx::tma_load_2d(sb + j * 8192, &core.map_b, nt * BN + j * 64, kb * BK, &full[s]);
-                        }
-                    }
+                    ptx::tma_load_2d(sa, &core.map_a, kb * BK, mt * BM, &full[s]);
+                    ptx::tma_load_2d(sb, &core.map_b, kb * BK, nt * BN, &full[s]);
                 }
             }
         }
         __syncwarp();
     }
     else if (warp == 1) {
-        if (lane == 0) {
-            const uint32_t idesc = ptx::make_idesc(1, 1, BM, BN, core.a_mn ? 1 : 0, core.b_mn ? 1 : 0);
-            // K-major: 16 bf16 along K are 32 bytes inside the swizzle atom (+2 in the descriptor's
-            // 16-byte units). MN-major: 16 rows of K are 2048 bytes (+128), 64-column blocks 8 KiB apart.
-            const uint32_t a_lbo = core.a_mn ? 8192u : 16u, a_step = core.a_mn ? 128u : 2u;
-            const uint32_t b_lbo = core.b_mn ? 8192u : 16u, b_step = core.b_mn ? 128u : 2u;
-            uint32_t       it    = 0;
-            uint32_t           tcount = 0;
-            bool               ok    = true;
-            for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tcount) {
-                const uint32_t acc = tcount & 1u;
-                if (!ptx::mbar_wait(&tmem_empty[acc], ((tcount >> 1) & 1u) ^ 1u)) {
-                    flag_error(core, ERR_MMA_WAIT_TMEM);
-                    ok = false;
+        const uint32_t  leader = ptx::elect_one();
+        const uint32_t  idesc  = ptx::make_idesc(1, 1, BM, BN, 0, 0);
+        const ptx::Desc a_desc(ptx::smem_desc_sw128(base, 16u, 1024)), b_desc(ptx::smem_desc_sw128(base + A_BYTES, 16u, 1024));
+        const uint32_t  full_b = ptx::smem_addr(full), empty_b = ptx::smem_addr(empty);
+        const uint32_t  tfull_b = ptx::smem_addr(tmem_full), tempty_b = ptx::smem_addr(tmem_empty);
+        uint32_t        stage = 0, phase = 0, tcount = 0;
+        uint32_t        gave_up = ERR_NONE;
+        for (int t = blockIdx.x; t < total_tiles && !gave_up; t += gridDim.x, ++tcount) {
+            const uint32_t acc = tcount & 1u;
+            if (!ptx::mbar_wait_warp(tempty_b + acc * 8, ((tcount >> 1) & 1u) ^ 1u)) {
+                gave_up = ERR_MMA_WAIT_TMEM;
+                break;
+            }
+            ptx::tc_fence_after();
+            for (int kb = 0; kb < kblocks; ++kb) {
+                if (!ptx::mbar_wait_warp(full_b + stage * 8, phase)) {
+                    gave_up = ERR_MMA_WAIT_FULL;
                     break;
                 }
                 ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * BN;
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % STAGES;
-                    if (!ptx::mbar_wait(&full[s], (it / STAGES) & 1u)) {
-                        flag_error(core, ERR_MMA_WAIT_FULL);
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after();
-                    const uint32_t sa     = base + s * STAGE_BYTES;
-                    const uint64_t a_desc = ptx::smem_desc_sw128(sa, a_lbo, 1024);
-                    const uint64_t b_desc = ptx::smem_desc_sw128(sa + A_BYTES, b_lbo, 1024);
+                const ptx::Desc a = a_desc.at(stage * STAGE_BYTES), b = b_desc.at(stage * STAGE_BYTES);
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k) {
-                        ptx::mma_f16_ss(d_tmem, a_desc + a_step * k, b_desc + b_step * k, idesc, (kb | k) != 0);
-                    }
-                    ptx::mma_commit(&empty[s]);
+                for (int k = 0; k < BK / UMMA_K; ++k) {
+                    ptx::mma_f16_ss_if<1>(tmem_base + acc * BN, a.at(32 * k), b.at(32 * k), idesc, static_cast<uint32_t>(kb | k), leader);
                 }
-                if (ok) {
-                    ptx::mma_commit(&tmem_full[acc]);
+                ptx::mma_commit_if<1>(empty_b + stage * 8, leader);
+                if (++stage == STAGES) {
+                    stage = 0;
+                    phase ^= 1u;
                 }
             }
+            if (!gave_up) {
+                ptx::mma_commit_if<1>(tfull_b + acc * 8, leader);
+            }
+        }
+        if (gave_up) {
+            flag_error(core, gave_up);
         }
         __syncwarp();
     }
@@ -242,58 +215,136 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src = Src{},
     }
 }
 
-// ---- the same GEMM on CTA pairs ---------------------------------------------------------------------
-// Two CTAs of a cluster share a 256 x 256 output tile: each loads its own 128 rows of A and its own
-// 128 rows of B per K-block (32 KiB per stage instead of 48, so six stages fit), the even CTA
-// issues tcgen05.mma.cta_group::2 (M = 256) over both CTAs' shared memory, and each CTA's 128
-// accumulator lanes hold its own rows of the tile. Per 256 x 256 of output the pair moves 64 KiB
-// per K-block from L2 into shared memory where two single CTAs move 96: operand delivery is what
-// bounds the single-CTA kernel. Operand loads are ordinary per-CTA TMA loads; what crosses between
-// the CTAs are completion signals only (the loads' byte counts land on the even CTA's mbarrier,
-// the MMA's completion is signalled to both CTAs, the odd CTA's epilogue frees the accumulator
-// with a remote arrival).
-constexpr int PAIR_STAGES      = 6;
-constexpr int PAIR_B_BYTES     = (BN / 2) * BK * 2;
-constexpr int PAIR_STAGE_BYTES = A_BYTES + PAIR_B_BYTES;
-constexpr int PAIR_SMEM_BYTES  = PAIR_STAGES * PAIR_STAGE_BYTES + 1024;
-constexpr int PAIR_BAND        = 8;  // 256-row tiles per rasterisation band
+// ---- work units of the cores below --------------------------------------------------------------------
+// Both cores hand their epilogue 32 rows x 128 columns at a time ("a unit": one warp, one row per
+// thread, the whole row of 128 fp32 in registers) and give the accumulator back to the MMA thread as
+// soon as the registers are loaded, before any arithmetic or store. Epi requirements:
+//   static constexpr bool kPeers          whether open() / close() run (kernels that touch peers)
+//   void open(int epi_tid), close(int epi_tid)          all epilogue threads, once before / after the tiles
+//   void unit(uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage)
+// `stage` is 4 KiB of shared memory of this warp's own (32 rows x 128 bytes).
+constexpr int UNIT_STAGE_BYTES = 32 * 128;
 
-__device__ __forceinline__ void pair_tile_coords(const Core& c, int tiles_m2, int t, int& mt2, int& nt)
+__device__ __forceinline__ void load_unit(uint32_t taddr, uint32_t (&r)[128])
 {
-    const int band_tiles = PAIR_BAND * c.tiles_n;
-    const int band       = t / band_tiles;
-    const int r          = t - band * band_tiles;
-    const int rows       = min(PAIR_BAND, tiles_m2 - band * PAIR_BAND);
-    nt                   = r / rows;
-    mt2                  = band * PAIR_BAND + (r - nt * rows);
+#pragma unroll
+    for (int ch = 0; ch < 4; ++ch) {
+        ptx::tmem_ld_32x32(taddr + ch * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[ch * 32]));
+    }
+    ptx::tmem_ld_wait();
 }
 
-// `core.map_b` must have been built with a box of BN / 2 rows. Launch with cluster dimension 2.
-template <class Epi>
-__device__ __forceinline__ void run_pair(const Core& core, Epi& epi)
+// ---- the GEMM on CTA pairs, two accumulator blocks per pair ---------------------------------------------
+// A pair of CTAs (one cluster, tcgen05.mma.cta_group::2) owns MB x NB blocks of 256 x 256 outputs,
+// MB * NB = 2: 512 x 256 or 256 x 512. Per 64-wide K-block a CTA loads its own 128 rows of A per block
+// row and its own 128 rows of B per block column (48 KiB; four stages), and the even CTA's thread issues
+// 2 x 4 MMAs of 256 x 256 x 16 over both CTAs' shared memory. All 512 tensor-memory columns hold
+// accumulators.
+//
+// Why two blocks: shared memory moves 128 bytes a clock per SM. An MMA of 256 x 256 x 16 takes 128
+// clocks and reads 4 KiB of A and 4 KiB of B from each SM (64 B/clk); with one block per pair TMA has to
+// write 32 KiB per 512 clocks beside it (64 B/clk), all the bandwidth there is, with two blocks 48 KiB
+// per 1024 (48 B/clk).
+//
+// Measured at 8192 cubed with operands of zeros (no power limit; SM clock 1965 MHz): 0.548 ms, 0.84 of the
+// tensor pipe's rate (cuBLAS 0.523). The same kernel with its MMAs issued by one lane on its own took
+// 0.753: see ptx.cuh, elect_one(). Random operands, back to back for seconds (1000 W power cap): 1330 -
+// 1390 TFLOP/s on the feed-forward shapes, 9450 x 13824 x 5120 and its relatives (cuBLAS 1320 - 1430; the
+// 128 x 256 single-CTA tiles before this kernel 1120 - 1200).
+//
+// There is no second accumulator buffer, so the blocks' order hides the epilogue instead: the first
+// kStages K-blocks of a tile are multiplied into block 0 and then into block 1, and so are the last
+// ones. Block 0 is finished (and read out) four stages before block 1, and the next tile can start in
+// block 0 while block 1 is still being read out.
+constexpr int WIDE_STAGES      = 4;
+constexpr int WIDE_BLOCK_BYTES = 128 * BK * 2;  // 128 rows of one operand, one K-block
+constexpr int WIDE_STAGE_BYTES = 3 * WIDE_BLOCK_BYTES;
+constexpr int WIDE_EPI_WARPS   = 8;
+constexpr int WIDE_FIRST_EPI   = 4;  // warps 2 and 3 idle: they fill the first warpgroup, whose registers go to the others
+constexpr int WIDE_THREADS     = 32 * (WIDE_FIRST_EPI + WIDE_EPI_WARPS);
+constexpr int WIDE_REGS_LIGHT  = 88;   // 128 x 88 + 256 x 208 = the 384 x 168 of the launch
+constexpr int WIDE_REGS_EPI    = 208;  // a unit's 128 values, a row of loads in flight, addresses
+constexpr int WIDE_SMEM_BYTES  = WIDE_STAGES * WIDE_STAGE_BYTES + WIDE_EPI_WARPS * UNIT_STAGE_BYTES + 1024;
+constexpr int WIDE_BAND_ROWS   = 4096;  // rows per rasterisation band: a wave of 74 tiles is roughly square
+
+// Tiles are visited in bands of `band` M-tiles so that a wave of CTAs shares operand tiles through L2.
+__device__ __forceinline__ void pair_tile_coords(int tiles_m, int tiles_n, int band_rows, int t, int& mt, int& nt)
 {
+    const int band_tiles = band_rows * tiles_n;
+    const int band       = t / band_tiles;
+    const int r          = t - band * band_tiles;
+    const int rows       = min(band_rows, tiles_m - band * band_rows);
+    nt                   = r / rows;
+    mt                   = band * band_rows + (r - nt * rows);
+}
+
+// The schedule: `full` whole tiles, then the remaining tiles block by block (two items each), which the
+// host asks for when half as many items as pairs are left, so that the last wave is half as long.
+struct WideCore {
+    CUtensorMap map_a, map_b;
+    int         M, N, K;
+    int         tiles_m, tiles_n;  // of MB * 256 x NB * 256
+    int         full, items;
+    int         a_mn, b_mn;
+    uint32_t*   err;
+};
+
+__device__ __forceinline__ void flag_error(uint32_t* err, uint32_t code)
+{
+    if (err) {
+        atomicCAS(err, 0u, code);
+    }
+}
+
+template <int MB, int NB>
+struct WideItem {
+    int m0, n0, u0, u1;
+    __device__ __forceinline__ WideItem(const WideCore& c, int item)
+    {
+        const bool whole = item < c.full;
+        const int  rest  = item - c.full;
+        int        mt, nt;
+        pair_tile_coords(c.tiles_m, c.tiles_n, WIDE_BAND_ROWS / (MB * 256), whole ? item : c.full + (rest >> 1), mt, nt);
+        m0 = mt * MB * 256;
+        n0 = nt * NB * 256;
+        u0 = whole ? 0 : (rest & 1);
+        u1 = whole ? 2 : u0 + 1;
+        // a block that lies outside the result altogether is not computed
+        if (u1 == 2 && (MB == 2 ? m0 + 256 >= c.M : n0 + 256 >= c.N)) {
+            u1 = 1;
+        }
+        if (u0 == 1 && (MB == 2 ? m0 + 256 >= c.M : n0 + 256 >= c.N)) {
+            u1 = u0;  // empty
+        }
+    }
+    __device__ __forceinline__ int row(int u) const { return m0 + (MB == 2 ? u * 256 : 0); }
+    __device__ __forceinline__ int col(int u) const { return n0 + (NB == 2 ? u * 256 : 0); }
+};
+
+template <int MB, int NB, class Epi>
+__device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
+{
+    static_assert(MB * NB == 2, "two blocks of 256 x 256");
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t       full[PAIR_STAGES], empty[PAIR_STAGES], tmem_full[2], tmem_empty[2];
+    __shared__ uint64_t       full[WIDE_STAGES], empty[WIDE_STAGES], tmem_full[2], tmem_empty[2];
     __shared__ uint32_t       tmem_holder;
 
     const uint32_t base = (ptx::smem_addr(smem_raw) + 1023u) & ~1023u;
     uint8_t*       ring = smem_raw + (base - ptx::smem_addr(smem_raw));
-    const int      warp = threadIdx.x >> 5;
+    const int      warp = static_cast<int>(ptx::uniform(threadIdx.x >> 5));
     const int      lane = threadIdx.x & 31;
-    const uint32_t half = ptx::cluster_ctarank();  // 0: issues the MMAs; 1: the other half of the tile
+    const int      half = static_cast<int>(ptx::uniform(ptx::cluster_ctarank()));  // 0: issues the MMAs; 1: the other rows
     const int      pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-    const int      tiles_m2    = (core.tiles_m + 1) / 2;
-    const int      total_tiles = tiles_m2 * core.tiles_n;
-    const int      kblocks     = (core.K + BK - 1) / BK;
+    const int      kblocks = (core.K + BK - 1) / BK;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < PAIR_STAGES; ++s) {
+        for (int s = 0; s < WIDE_STAGES; ++s) {
             ptx::mbar_init(&full[s], 1);
             ptx::mbar_init(&empty[s], 1);
         }
-        for (int a = 0; a < 2; ++a) {
-            ptx::mbar_init(&tmem_full[a], 1);
-            ptx::mbar_init(&tmem_empty[a], 8);  // four epilogue warps in each CTA
+        for (int u = 0; u < 2; ++u) {
+            ptx::mbar_init(&tmem_full[u], 1);
+            ptx::mbar_init(&tmem_empty[u], 2 * WIDE_EPI_WARPS);  // the epilogue warps of both CTAs
         }
         ptx::mbar_fence_init();
         ptx::tma_prefetch_desc(&core.map_a);
@@ -307,117 +358,199 @@ __device__ __forceinline__ void run_pair(const Core& core, Epi& epi)
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem_base = tmem_holder;
+    const uint32_t tmem_base = ptx::uniform(tmem_holder);
 
+    if (warp < WIDE_FIRST_EPI) {
+    ptx::setmaxnreg_dec<WIDE_REGS_LIGHT>();
+    const uint32_t leader = ptx::elect_one();
+    const uint32_t full_b = ptx::smem_addr(full), empty_b = ptx::smem_addr(empty);
     if (warp == 0) {
-        if (lane == 0) {
-            uint32_t it = 0;
-            bool     ok = true;
-            for (int t = pair; t < total_tiles && ok; t += npairs) {
-                int mt2, nt;
-                pair_tile_coords(core, tiles_m2, t, mt2, nt);
-                const int m0 = (mt2 * 2 + static_cast<int>(half)) * BM;
-                const int n0 = nt * BN + static_cast<int>(half) * (BN / 2);
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int      s      = it % PAIR_STAGES;
-                    const uint32_t parity = ((it / PAIR_STAGES) & 1u) ^ 1u;
-                    if (!ptx::mbar_wait(&empty[s], parity)) {
-                        flag_error(core, ERR_PRODUCER_WAIT);
-                        ok = false;
-                        break;
+        uint32_t stage = 0, phase = 1;
+        bool     ok    = true;
+        for (int w = pair; w < core.items && ok; w += npairs) {
+            const WideItem<MB, NB> item(core, w);
+            if (item.u0 == item.u1) {
+                continue;
+            }
+            const uint32_t blocks = (MB == 2 ? item.u1 - item.u0 : 1) + (NB == 2 ? item.u1 - item.u0 : 1);
+            for (int kb = 0; kb < kblocks; ++kb) {
+                if (!ptx::mbar_wait_warp(empty_b + stage * 8, phase)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t sa = base + stage * WIDE_STAGE_BYTES, sb = sa + MB * WIDE_BLOCK_BYTES, bar = full_b + stage * 8;
+                if (half == 0) {
+                    ptx::mbar_expect_tx_if(bar, 2 * blocks * WIDE_BLOCK_BYTES, leader);  // both CTAs' bytes
+                }
+#pragma unroll
+                for (int u = 0; u < MB; ++u) {
+                    if (MB == 2 && (u < item.u0 || u >= item.u1)) {
+                        continue;
                     }
-                    uint8_t* sa = ring + s * PAIR_STAGE_BYTES;
-                    uint8_t* sb = sa + A_BYTES;
-                    if (half == 0) {
-                        ptx::mbar_expect_tx(&full[s], 2 * PAIR_STAGE_BYTES);  // both CTAs' bytes
-                    }
+                    const int      m  = item.m0 + u * 256 + half * 128;
+                    const uint32_t to = sa + u * WIDE_BLOCK_BYTES;
                     if (!core.a_mn) {
-                        ptx::tma_load_2d_pair(sa, &core.map_a, kb * BK, m0, &full[s]);
+                        ptx::tma_load_2d_pair_if(to, &core.map_a, kb * BK, m, bar, leader);
                     }
-                    else {
-                        for (int j = 0; j < BM / 64; ++j) {
-                            ptx::tma_load_2d_pair(sa + j * 8192, &core.map_a, m0 + j * 64, kb * BK, &full[s]);
-                        }
-                    }
-                    if (!core.b_mn) {
-                        ptx::tma_load_2d_pair(sb, &core.map_b, kb * BK, n0, &full[s]);
-                    }
-                    else {
-                        for (int j = 0; j < BN / 128; ++j) {
-                            ptx::tma_load_2d_pair(sb + j * 8192, &core.map_b, n0 + j * 64, kb * BK, &full[s]);
-                        }
+                    else {  // 64 (k) x 64 (m) blocks of 8 KiB
+                        ptx::tma_load_2d_pair_if(to, &core.map_a, m, kb * BK, bar, leader);
+                        ptx::tma_load_2d_pair_if(to + 8192, &core.map_a, m + 64, kb * BK, bar, leader);
                     }
                 }
+#pragma unroll
+                for (int u = 0; u < NB; ++u) {
+                    if (NB == 2 && (u < item.u0 || u >= item.u1)) {
+                        continue;
+                    }
+                    const int      n  = item.n0 + u * 256 + half * 128;
+                    const uint32_t to = sb + u * WIDE_BLOCK_BYTES;
+                    if (!core.b_mn) {
+                        ptx::tma_load_2d_pair_if(to, &core.map_b, kb * BK, n, bar, leader);
+                    }
+                    else {
+                        ptx::tma_load_2d_pair_if(to, &core.map_b, n, kb * BK, bar, leader);
+                        ptx::tma_load_2d_pair_if(to + 8192, &core.map_b, n + 64, kb * BK, bar, leader);
+                    }
+                }
+                if (++stage == WIDE_STAGES) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
             }
+        }
+        if (!ok) {
+            flag_error(core.err, ERR_PRODUCER_WAIT);
         }
         __syncwarp();
     }
     else if (warp == 1) {
-        if (lane == 0 && half == 0) {
-            const uint32_t idesc = ptx::make_idesc(1, 1, 2 * BM, BN, core.a_mn ? 1 : 0, core.b_mn ? 1 : 0);
-            const uint32_t a_lbo = core.a_mn ? 8192u : 16u, a_step = core.a_mn ? 128u : 2u;
-            const uint32_t b_lbo = core.b_mn ? 8192u : 16u, b_step = core.b_mn ? 128u : 2u;
-            uint32_t       it    = 0;
-            uint32_t       tcount = 0;
-            bool           ok    = true;
-            for (int t = pair; t < total_tiles && ok; t += npairs, ++tcount) {
-                const uint32_t acc = tcount & 1u;
-                if (!ptx::mbar_wait_cluster(&tmem_empty[acc], ((tcount >> 1) & 1u) ^ 1u)) {
-                    flag_error(core, ERR_MMA_WAIT_TMEM);
-                    ok = false;
-                    break;
-                }
-                ptx::tc_fence_after();
-                const uint32_t d_tmem = tmem_base + acc * BN;
-                for (int kb = 0; kb < kblocks; ++kb, ++it) {
-                    const int s = it % PAIR_STAGES;
-                    if (!ptx::mbar_wait(&full[s], (it / PAIR_STAGES) & 1u)) {
-                        flag_error(core, ERR_MMA_WAIT_FULL);
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after();
-                    const uint32_t sa     = base + s * PAIR_STAGE_BYTES;
-                    const uint64_t a_desc = ptx::smem_desc_sw128(sa, a_lbo, 1024);
-                    const uint64_t b_desc = ptx::smem_desc_sw128(sa + A_BYTES, b_lbo, 1024);
+        if (half == 0) {
+            const uint32_t  idesc = ptx::make_idesc(1, 1, 256, 256, core.a_mn ? 1 : 0, core.b_mn ? 1 : 0);
+            // K-major: 16 bf16 along K are 32 bytes inside the swizzle atom. MN-major: 16 rows of K are
+            // 2048 bytes, 64-column blocks 8 KiB apart.
+            const uint32_t  a_step = core.a_mn ? 2048u : 32u, b_step = core.b_mn ? 2048u : 32u;
+            const ptx::Desc a_desc(ptx::smem_desc_sw128(base, core.a_mn ? 8192u : 16u, 1024));
+            const ptx::Desc b_desc(ptx::smem_desc_sw128(base + MB * WIDE_BLOCK_BYTES, core.b_mn ? 8192u : 16u, 1024));
+            const uint32_t  tfull_b = ptx::smem_addr(tmem_full), tempty_b = ptx::smem_addr(tmem_empty);
+            uint32_t        stage = 0, phase = 0, uses0 = 0, uses1 = 0;
+            uint32_t        gave_up = ERR_NONE;
+            auto issue = [&](int u, uint32_t s, uint32_t accumulate) {  // one K-block into block u
+                const ptx::Desc a = a_desc.at(s * WIDE_STAGE_BYTES + (MB == 2 ? u * WIDE_BLOCK_BYTES : 0));
+                const ptx::Desc b = b_desc.at(s * WIDE_STAGE_BYTES + (NB == 2 ? u * WIDE_BLOCK_BYTES : 0));
 #pragma unroll
-                    for (int k = 0; k < BK / UMMA_K; ++k) {
-                        ptx::mma_f16_ss_pair(d_tmem, a_desc + a_step * k, b_desc + b_step * k, idesc, (kb | k) != 0);
+                for (int k = 0; k < BK / UMMA_K; ++k) {
+                    ptx::mma_f16_ss_if<2>(tmem_base + u * 256, a.at(a_step * k), b.at(b_step * k), idesc, accumulate | k, leader);
+                }
+            };
+            auto advance = [](uint32_t& s, uint32_t& ph) {
+                if (++s == WIDE_STAGES) {
+                    s = 0;
+                    ph ^= 1u;
+                }
+            };
+            for (int w = pair; w < core.items && !gave_up; w += npairs) {
+                const WideItem<MB, NB> item(core, w);
+                if (item.u0 == item.u1) {
+                    continue;
+                }
+                for (int kb = 0; kb < kblocks && !gave_up;) {
+                    const int left = kblocks - kb;
+                    if (kb > 0 && left > WIDE_STAGES && item.u1 - item.u0 == 2) {
+                        // the middle of a whole tile: both blocks, one K-block after another
+                        const int n = left - WIDE_STAGES;
+                        for (int i = 0; i < n; ++i) {
+                            if (!ptx::mbar_wait_warp(full_b + stage * 8, phase)) {
+                                gave_up = ERR_MMA_WAIT_FULL;
+                                break;
+                            }
+                            ptx::tc_fence_after();
+                            issue(0, stage, 1u);
+                            issue(1, stage, 1u);
+                            ptx::mma_commit_if<2>(empty_b + stage * 8, leader);
+                            advance(stage, phase);
+                        }
+                        kb += n;
+                        continue;
                     }
-                    ptx::mma_commit_pair(&empty[s]);
+                    // the first K-blocks of a tile, its last ones, or any of a single block
+                    const int run = min(left, WIDE_STAGES);
+                    uint32_t  s = stage, ph = phase;
+                    for (int u = item.u0; u < item.u1 && !gave_up; ++u) {
+                        if (kb == 0) {
+                            uint32_t& uses = u == 0 ? uses0 : uses1;
+                            if (!ptx::mbar_wait_warp_cluster(tempty_b + u * 8, (uses & 1u) ^ 1u)) {
+                                gave_up = ERR_MMA_WAIT_TMEM;
+                                break;
+                            }
+                            ++uses;
+                            ptx::tc_fence_after();
+                        }
+                        s  = stage;
+                        ph = phase;
+                        for (int i = 0; i < run; ++i) {
+                            if (u == item.u0) {
+                                if (!ptx::mbar_wait_warp(full_b + s * 8, ph)) {
+                                    gave_up = ERR_MMA_WAIT_FULL;
+                                    break;
+                                }
+                                ptx::tc_fence_after();
+                            }
+                            issue(u, s, static_cast<uint32_t>(kb | i));
+                            if (u + 1 == item.u1) {
+                                ptx::mma_commit_if<2>(empty_b + s * 8, leader);
+                            }
+                            advance(s, ph);
+                        }
+                        if (!gave_up && run == left) {
+                            ptx::mma_commit_if<2>(tfull_b + u * 8, leader);
+                        }
+                    }
+                    stage = s;
+                    phase = ph;
+                    kb += run;
                 }
-                if (ok) {
-                    ptx::mma_commit_pair(&tmem_full[acc]);
-                }
+            }
+            if (gave_up) {
+                flag_error(core.err, gave_up);
             }
         }
         __syncwarp();
     }
+    }
     else {
-        const int epi_warp = warp - 2;
-        const int quarter  = warp & 3;
-        epi.open(epi_warp);
-        uint32_t tcount = 0;
-        bool     ok     = true;
-        for (int t = pair; t < total_tiles && ok; t += npairs, ++tcount) {
-            const uint32_t acc = tcount & 1u;
-            if (!ptx::mbar_wait(&tmem_full[acc], (tcount >> 1) & 1u)) {
-                flag_error(core, ERR_EPI_WAIT);
-                ok = false;
-                break;
-            }
-            ptx::tc_fence_after();
-            int mt2, nt;
-            pair_tile_coords(core, tiles_m2, t, mt2, nt);
-            epi.tile(tmem_base + acc * BN + (static_cast<uint32_t>(quarter * 32) << 16), mt2 * 2 + static_cast<int>(half), nt,
-                     quarter, lane);
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) {
-                ptx::mbar_arrive_cluster(ptx::cluster_addr(&tmem_empty[acc], 0));
+        ptx::setmaxnreg_inc<WIDE_REGS_EPI>();
+        const int epi_warp = warp - WIDE_FIRST_EPI;
+        const int quarter  = warp & 3;        // the TMEM lane quarter this warp may access
+        const int cg       = epi_warp >> 2;   // which 128 of a block's 256 columns
+        uint8_t*  stage    = ring + WIDE_STAGES * WIDE_STAGE_BYTES + epi_warp * UNIT_STAGE_BYTES;
+        if (Epi::kPeers) {
+            epi.open(threadIdx.x - 32 * WIDE_FIRST_EPI);
+        }
+        uint32_t uses[2] = {0, 0};
+        bool     ok      = true;
+        for (int w = pair; w < core.items && ok; w += npairs) {
+            const WideItem<MB, NB> item(core, w);
+            for (int u = item.u0; u < item.u1; ++u) {
+                if (!ptx::mbar_wait(&tmem_full[u], uses[u] & 1u)) {
+                    flag_error(core.err, ERR_EPI_WAIT);
+                    ok = false;
+                    break;
+                }
+                ++uses[u];
+                ptx::tc_fence_after();
+                uint32_t r[128];
+                load_unit(tmem_base + u * 256 + cg * 128 + (static_cast<uint32_t>(quarter * 32) << 16), r);
+                ptx::tc_fence_before();
+                __syncwarp();
+                if (lane == 0) {
+                    ptx::mbar_arrive_cluster(ptx::cluster_addr(&tmem_empty[u], 0));
+                }
+                epi.unit(r, item.row(u) + half * 128 + quarter * 32, item.col(u) + cg * 128, lane, stage);
             }
         }
-        epi.close(threadIdx.x - 64);
+        if (Epi::kPeers) {
+            epi.close(threadIdx.x - 32 * WIDE_FIRST_EPI);
+        }
     }
 
     // Neither CTA may free its tensor memory, or leave, while the other can still signal it or
@@ -429,15 +562,251 @@ __device__ __forceinline__ void run_pair(const Core& core, Epi& epi)
     }
 }
 
+// ---- the GEMM on single CTAs, 128 x 128 tiles -------------------------------------------------------------
+// For problems with too few 256 x 256 blocks to occupy the device: four times as many tiles, a short
+// epilogue, and nothing shared between SMs. Bound by shared memory (its MMAs read 128 B/clk by
+// themselves) at about half the tensor pipe's rate, which a problem of this size does not reach anyway.
+// The two halves of the tensor memory in use alternate between tiles.
+constexpr int SMALL_STAGES      = 6;
+constexpr int SMALL_STAGE_BYTES = 2 * WIDE_BLOCK_BYTES;
+constexpr int SMALL_EPI_WARPS   = 4;
+constexpr int SMALL_THREADS     = 32 * (2 + SMALL_EPI_WARPS);
+constexpr int SMALL_SMEM_BYTES  = SMALL_STAGES * SMALL_STAGE_BYTES + SMALL_EPI_WARPS * UNIT_STAGE_BYTES + 1024;
+
+template <class Epi>
+__device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
+{
+    extern __shared__ uint8_t smem_raw[];
+    __shared__ uint64_t       full[SMALL_STAGES], empty[SMALL_STAGES], tmem_full[2], tmem_empty[2];
+    __shared__ uint32_t       tmem_holder;
+
+    const uint32_t base = (ptx::smem_addr(smem_raw) + 1023u) & ~1023u;
+    uint8_t*       ring = smem_raw + (base - ptx::smem_addr(smem_raw));
+    const int      warp = static_cast<int>(ptx::uniform(threadIdx.x >> 5));
+    const int      lane = threadIdx.x & 31;
+    const int      tiles   = core.tiles_m * core.tiles_n;  // of 128 x 128 here
+    const int      kblocks = (core.K + BK - 1) / BK;
+
+    if (warp == 0 && lane == 0) {
+        ptx::tma_prefetch_desc(&core.map_a);
+        ptx::tma_prefetch_desc(&core.map_b);
+        for (int s = 0; s < SMALL_STAGES; ++s) {
+            ptx::mbar_init(&full[s], 1);
+            ptx::mbar_init(&empty[s], 1);
+        }
+        for (int a = 0; a < 2; ++a) {
+            ptx::mbar_init(&tmem_full[a], 1);
+            ptx::mbar_init(&tmem_empty[a], SMALL_EPI_WARPS);
+        }
+        ptx::mbar_fence_init();
+    }
+    if (warp == 1) {
+        ptx::tmem_alloc<256>(&tmem_holder);
+        ptx::tmem_relinquish();
+    }
+    ptx::tc_fence_before();
+    __syncthreads();
+    ptx::tc_fence_after();
+    const uint32_t tmem_base = ptx::uniform(tmem_holder);
+    const uint32_t leader = ptx::elect_one();
+    const uint32_t full_b = ptx::smem_addr(full), empty_b = ptx::smem_addr(empty);
+
+    if (warp == 0) {
+        uint32_t stage = 0, phase = 1;
+        bool     ok    = true;
+        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+            int mt, nt;
+            pair_tile_coords(core.tiles_m, core.tiles_n, 16, t, mt, nt);
+            for (int kb = 0; kb < kblocks; ++kb) {
+                if (!ptx::mbar_wait_warp(empty_b + stage * 8, phase)) {
+                    ok = false;
+                    break;
+                }
+                const uint32_t sa = base + stage * SMALL_STAGE_BYTES, sb = sa + WIDE_BLOCK_BYTES, bar = full_b + stage * 8;
+                ptx::mbar_expect_tx_if(bar, SMALL_STAGE_BYTES, leader);
+                if (!core.a_mn) {
+                    ptx::tma_load_2d_if(sa, &core.map_a, kb * BK, mt * 128, bar, leader);
+                }
+                else {
+                    ptx::tma_load_2d_if(sa, &core.map_a, mt * 128, kb * BK, bar, leader);
+                    ptx::tma_load_2d_if(sa + 8192, &core.map_a, mt * 128 + 64, kb * BK, bar, leader);
+                }
+                if (!core.b_mn) {
+                    ptx::tma_load_2d_if(sb, &core.map_b, kb * BK, nt * 128, bar, leader);
+                }
+                else {
+                    ptx::tma_load_2d_if(sb, &core.map_b, nt * 128, kb * BK, bar, leader);
+                    ptx::tma_load_2d_if(sb + 8192, &core.map_b, nt * 128 + 64, kb * BK, bar, leader);
+                }
+                if (++stage == SMALL_STAGES) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+        }
+        if (!ok) {
+            flag_error(core.err, ERR_PRODUCER_WAIT);
+        }
+        __syncwarp();
+    }
+    else if (warp == 1) {
+        const uint32_t  idesc  = ptx::make_idesc(1, 1, 128, 128, core.a_mn ? 1 : 0, core.b_mn ? 1 : 0);
+        const uint32_t  a_step = core.a_mn ? 2048u : 32u, b_step = core.b_mn ? 2048u : 32u;
+        const ptx::Desc a_desc(ptx::smem_desc_sw128(base, core.a_mn ? 8192u : 16u, 1024));
+        const ptx::Desc b_desc(ptx::smem_desc_sw128(base + WIDE_BLOCK_BYTES, core.b_mn ? 8192u : 16u, 1024));
+        const uint32_t  tfull_b = ptx::smem_addr(tmem_full), tempty_b = ptx::smem_addr(tmem_empty);
+        uint32_t        stage = 0, phase = 0, tcount = 0;
+        uint32_t        gave_up = ERR_NONE;
+        for (int t = blockIdx.x; t < tiles && !gave_up; t += gridDim.x, ++tcount) {
+            const uint32_t acc = tcount & 1u;
+            if (!ptx::mbar_wait_warp(tempty_b + acc * 8, ((tcount >> 1) & 1u) ^ 1u)) {
+                gave_up = ERR_MMA_WAIT_TMEM;
+                break;
+            }
+            ptx::tc_fence_after();
+            for (int kb = 0; kb < kblocks; ++kb) {
+                if (!ptx::mbar_wait_warp(full_b + stage * 8, phase)) {
+                    gave_up = ERR_MMA_WAIT_FULL;
+                    break;
+                }
+                ptx::tc_fence_after();
+                const ptx::Desc a = a_desc.at(stage * SMALL_STAGE_BYTES), b = b_desc.at(stage * SMALL_STAGE_BYTES);
+#pragma unroll
+                for (int k = 0; k < BK / UMMA_K; ++k) {
+                    ptx::mma_f16_ss_if<1>(tmem_base + acc * 128, a.at(a_step * k), b.at(b_step * k), idesc,
+                                          static_cast<uint32_t>(kb | k), leader);
+                }
+                ptx::mma_commit_if<1>(empty_b + stage * 8, leader);
+                if (++stage == SMALL_STAGES) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+            if (!gave_up) {
+                ptx::mma_commit_if<1>(tfull_b + acc * 8, leader);
+            }
+        }
+        if (gave_up) {
+            flag_error(core.err, gave_up);
+        }
+        __syncwarp();
+    }
+    else {
+        const int epi_warp = warp - 2;
+        const int quarter  = warp & 3;
+        uint8_t*  stage    = ring + SMALL_STAGES * SMALL_STAGE_BYTES + epi_warp * UNIT_STAGE_BYTES;
+        if (Epi::kPeers) {
+            epi.open(threadIdx.x - 64);
+        }
+        uint32_t tcount = 0;
+        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++tcount) {
+            const uint32_t acc = tcount & 1u;
+            if (!ptx::mbar_wait(&tmem_full[acc], (tcount >> 1) & 1u)) {
+                flag_error(core.err, ERR_EPI_WAIT);
+                break;
+            }
+            ptx::tc_fence_after();
+            int mt, nt;
+            pair_tile_coords(core.tiles_m, core.tiles_n, 16, t, mt, nt);
+            uint32_t r[128];
+            load_unit(tmem_base + acc * 128 + (static_cast<uint32_t>(quarter * 32) << 16), r);
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) {
+                ptx::mbar_arrive(&tmem_empty[acc]);
+            }
+            epi.unit(r, mt * 128 + quarter * 32, nt * 128, lane, stage);
+        }
+        if (Epi::kPeers) {
+            epi.close(threadIdx.x - 64);
+        }
+    }
+
+    ptx::tc_fence_before();
+    __syncthreads();
+    if (warp == 1) {
+        ptx::tmem_dealloc<256>(tmem_base);
+    }
+}
+
+// ---- a unit's 64-column halves through the staging buffer ----------------------------------------------------
+// A thread holds a row, so its global accesses would be 32 scattered pieces per instruction. They go
+// through the warp's staging buffer instead: eight lanes move the 128 bytes of one row, four rows per
+// instruction. 16-byte units are XOR-swizzled by the row: neither side has bank conflicts.
+__device__ __forceinline__ uint4* stage_unit(uint8_t* stage, int row, int unit)
+{
+    return reinterpret_cast<uint4*>(stage + row * 128 + ((unit ^ (row & 7)) << 4));
+}
+
+// 32 rows x 64 columns of a bf16 matrix into the staging buffer; what lies outside reads as zero.
+__device__ __forceinline__ void stage_in(uint8_t* stage, const __nv_bfloat16* src, int64_t ld, int row0, int col0, int M, int N,
+                                         int lane)
+{
+    const int unit = lane & 7, col = col0 + unit * 8;
+    uint4     v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int row = row0 + i * 4 + (lane >> 3);
+        v[i]          = make_uint4(0u, 0u, 0u, 0u);
+        if (row < M) {
+            const __nv_bfloat16* p = src + static_cast<int64_t>(row) * ld + col;
+            if (col + 8 <= N) {
+                v[i] = *reinterpret_cast<const uint4*>(p);
+            }
+            else if (col < N) {
+                __nv_bfloat16 e[8] = {};
+                for (int j = 0; j < N - col; ++j) {
+                    e[j] = p[j];
+                }
+                v[i] = *reinterpret_cast<const uint4*>(e);
+            }
+        }
+    }
+    __syncwarp();  // the buffer's previous contents have been read
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        *stage_unit(stage, i * 4 + (lane >> 3), unit) = v[i];
+    }
+    __syncwarp();
+}
+
+// The rows of the staging buffer to a bf16 matrix. The caller's threads have each written their row.
+__device__ __forceinline__ void stage_out(uint8_t* stage, __nv_bfloat16* dst, int64_t ld, int row0, int col0, int M, int N,
+                                          int lane)
+{
+    const int unit = lane & 7, col = col0 + unit * 8;
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int   r   = i * 4 + (lane >> 3);
+        const int   row = row0 + r;
+        const uint4 v   = *stage_unit(stage, r, unit);
+        if (row < M) {
+            __nv_bfloat16* p = dst + static_cast<int64_t>(row) * ld + col;
+            if (col + 8 <= N) {
+                *reinterpret_cast<uint4*>(p) = v;
+            }
+            else if (col < N) {
+                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
+                for (int j = 0; j < N - col; ++j) {
+                    p[j] = e[j];
+                }
+            }
+        }
+    }
+    __syncwarp();  // the buffer may be refilled
+}
+
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
 {
     __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
     return *reinterpret_cast<uint32_t*>(&v);
 }
 
-__device__ __forceinline__ void epi_barrier()
+// All `threads` epilogue threads of a CTA.
+__device__ __forceinline__ void epi_barrier(int threads)
 {
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
 }  // namespace gemm

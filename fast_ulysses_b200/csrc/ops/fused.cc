@@ -760,6 +760,15 @@ struct SpAttention : public torch::CustomClassHolder {
         const int64_t m = batch * s_local, hidden = w.size(0);
         expect(w.dim() == 2 && w.size(1) == heads * kHeadDim && w.stride(1) == 1 && w.scalar_type() == at::kBFloat16,
                "attention block: output weight ", w.sizes());
+        if (world == 1) {
+            // Nothing to pull: this rank's attention output is the operand as it lies in its buffer (which
+            // stays this forward's until the next forward, like q, k and v).
+            GemmExtra e;
+            e.bias         = bias_ready(bias);
+            e.residual     = residual;
+            const Tensor a = o.view({m, heads * kHeadDim});
+            return {gemm(a, w, e), a};
+        }
         Tensor        gather = empty_bf16({m, heads * kHeadDim}, w), out = empty_bf16({m, hidden}, w);
         const int64_t flags = (m + 127) / 128 * world;
         if (!ready.defined() || ready.numel() < flags) {
