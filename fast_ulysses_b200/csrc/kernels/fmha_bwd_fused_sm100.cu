@@ -87,7 +87,7 @@ __device__ __forceinline__ void flag(const Params& p, uint32_t code)
 
 __device__ __forceinline__ void stamp(const Params& p, uint32_t it, int ev)
 {
-    if (p.trace && blockIdx.x == 0 && it >= 64u && it < 72u) {
+    if (p.trace && blockIdx.x == 0 && (threadIdx.x & 31u) == 0u && it >= 64u && it < 72u) {
         p.trace[(it - 64u) * 16 + ev] = clock64();
     }
 }
@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_bwd_fused_kernel(const __grid
     extern __shared__ __align__(1024) uint8_t sm[];
     const uint32_t base = ptx::smem_addr(sm);
     Bars&          bar  = *reinterpret_cast<Bars*>(sm + OFF_BARS);
-    const int      warp = threadIdx.x >> 5;
+    const int      warp = static_cast<int>(ptx::uniform(threadIdx.x >> 5));
     const int      lane = threadIdx.x & 31;
     if (base & 1023u) {
         if (threadIdx.x == 0) {
@@ -180,163 +180,161 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_bwd_fused_kernel(const __grid
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem = bar.tmem_holder;
+    const uint32_t tmem = ptx::uniform(bar.tmem_holder);
     const int      n_q  = p.n_q;
 
+    // The first two roles are run by the whole warp, see ptx.cuh: elect_one().
+    const uint32_t leader = ptx::elect_one();
+    auto           b_of   = [](uint64_t& x) { return ptx::smem_addr(&x); };
     if (warp == 0) {
         // ---------------------------------------------------------------- producer
-        if (lane == 0) {
-            uint32_t it = 0, wc = 0;
-            bool     ok = true;
-            for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
-                const int jb = w % p.kv_blocks;
-                const int h  = (w / p.kv_blocks) % p.H;
-                const int b  = w / (p.kv_blocks * p.H);
-                if (!ptx::mbar_wait(&bar.kv_empty, (wc & 1u) ^ 1u)) {
-                    flag(p, ERR_LOAD);
+        uint32_t s = 0, ph = 1, wc = 0;
+        bool     ok = true;
+        for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
+            const int jb = w % p.kv_blocks;
+            const int h  = (w / p.kv_blocks) % p.H;
+            const int b  = w / (p.kv_blocks * p.H);
+            if (!ptx::mbar_wait_warp(b_of(bar.kv_empty), (wc & 1u) ^ 1u)) {
+                ok = false;
+                break;
+            }
+            ptx::mbar_expect_tx_if(b_of(bar.kv_full), 2 * TILE_BYTES, leader);
+            for (int half = 0; half < 2; ++half) {
+                ptx::tma_load_4d_if(base + OFF_K + half * HALF_BYTES, &p.map_k, half * 64, jb * BLK, h, b, b_of(bar.kv_full), leader);
+                ptx::tma_load_4d_if(base + OFF_V + half * HALF_BYTES, &p.map_v, half * 64, jb * BLK, h, b, b_of(bar.kv_full), leader);
+            }
+            const float* lse2  = p.lse2 + (static_cast<int64_t>(b) * p.H + h) * p.Sq_pad;
+            const float* delta = p.delta + (static_cast<int64_t>(b) * p.H + h) * p.Sq_pad;
+            int          i     = first_block(p, jb);
+            for (int i0 = 0; i0 < n_q; ++i0) {
+                const uint32_t ss = base + OFF_STATS + s * 1024, qf = b_of(bar.q_full[0]) + s * 8, df = b_of(bar.do_full[0]) + s * 8;
+                // one release per stage (after dK of the block that used it): the statistics of
+                // a stage are read by the element-wise warps until then
+                if (!ptx::mbar_wait_warp(b_of(bar.empty[0]) + s * 8, ph)) {
+                    ok = false;
                     break;
                 }
-                ptx::mbar_expect_tx(&bar.kv_full, 2 * TILE_BYTES);
+                ptx::mbar_expect_tx_if(qf, TILE_BYTES + 512, leader);
                 for (int half = 0; half < 2; ++half) {
-                    ptx::tma_load_4d(sm + OFF_K + half * HALF_BYTES, &p.map_k, half * 64, jb * BLK, h, b, &bar.kv_full);
-                    ptx::tma_load_4d(sm + OFF_V + half * HALF_BYTES, &p.map_v, half * 64, jb * BLK, h, b, &bar.kv_full);
+                    ptx::tma_load_4d_if(base + OFF_Q + s * TILE_BYTES + half * HALF_BYTES, &p.map_q, half * 64, i * BLK, h, b, qf,
+                                        leader);
                 }
-                const float* lse2  = p.lse2 + (static_cast<int64_t>(b) * p.H + h) * p.Sq_pad;
-                const float* delta = p.delta + (static_cast<int64_t>(b) * p.H + h) * p.Sq_pad;
-                const int    first = first_block(p, jb);
-                for (int i0 = 0; i0 < n_q; ++i0, ++it) {
-                    const int      i  = i0 + first < n_q ? i0 + first : i0 + first - n_q;
-                    const int      s  = it % STAGES;
-                    const uint32_t ph = ((it / STAGES) & 1u) ^ 1u;
-                    uint8_t*       ss = sm + OFF_STATS + s * 1024;
-                    // one release per stage (after dK of the block that used it): the statistics of
-                    // a stage are read by the element-wise warps until then
-                    if (!ptx::mbar_wait(&bar.empty[s], ph)) {
-                        flag(p, ERR_LOAD);
-                        ok = false;
-                        break;
-                    }
-                    ptx::mbar_expect_tx(&bar.q_full[s], TILE_BYTES + 512);
-                    for (int half = 0; half < 2; ++half) {
-                        ptx::tma_load_4d(sm + OFF_Q + s * TILE_BYTES + half * HALF_BYTES, &p.map_q, half * 64, i * BLK, h,
-                                         b, &bar.q_full[s]);
-                    }
-                    ptx::bulk_g2s(ss, lse2 + i * BLK, 512, &bar.q_full[s]);
-                    ptx::mbar_expect_tx(&bar.do_full[s], TILE_BYTES + 512);
-                    for (int half = 0; half < 2; ++half) {
-                        ptx::tma_load_4d(sm + OFF_DO + s * TILE_BYTES + half * HALF_BYTES, &p.map_do, half * 64, i * BLK,
-                                         h, b, &bar.do_full[s]);
-                    }
-                    ptx::bulk_g2s(ss + 512, delta + i * BLK, 512, &bar.do_full[s]);
+                ptx::bulk_g2s_if(ss, lse2 + i * BLK, 512, qf, leader);
+                ptx::mbar_expect_tx_if(df, TILE_BYTES + 512, leader);
+                for (int half = 0; half < 2; ++half) {
+                    ptx::tma_load_4d_if(base + OFF_DO + s * TILE_BYTES + half * HALF_BYTES, &p.map_do, half * 64, i * BLK, h, b, df,
+                                        leader);
+                }
+                ptx::bulk_g2s_if(ss + 512, delta + i * BLK, 512, df, leader);
+                i = i + 1 < n_q ? i + 1 : 0;
+                if (++s == STAGES) {
+                    s = 0;
+                    ph ^= 1u;
                 }
             }
+        }
+        if (!ok) {
+            flag(p, ERR_LOAD);
         }
         __syncwarp();
     }
     else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc_kk = ptx::make_idesc(1, 1, BLK, BLK, 0, 0);  // A, B K-major
-            constexpr uint32_t idesc_tn = ptx::make_idesc(1, 1, BLK, D, 0, 1);    // A from TMEM, B MN-major
-            constexpr uint32_t idesc_nn = ptx::make_idesc(1, 1, D, BLK, 1, 1);    // A, B MN-major
-            // one descriptor per operand and role, built once; every MMA below only steps it
-            const uint64_t k_kmaj  = ptx::smem_desc_sw128(base + OFF_K, 16, 1024);
-            const uint64_t v_kmaj  = ptx::smem_desc_sw128(base + OFF_V, 16, 1024);
-            const uint64_t q_kmaj  = ptx::smem_desc_sw128(base + OFF_Q, 16, 1024);
-            const uint64_t do_kmaj = ptx::smem_desc_sw128(base + OFF_DO, 16, 1024);
-            const uint64_t k_mn    = ptx::smem_desc_sw128(base + OFF_K, HALF_BYTES, 1024);
-            const uint64_t q_mn    = ptx::smem_desc_sw128(base + OFF_Q, HALF_BYTES, 1024);
-            const uint64_t do_mn   = ptx::smem_desc_sw128(base + OFF_DO, HALF_BYTES, 1024);
-            const uint64_t ds_mn   = ptx::smem_desc_sw128(base + OFF_DS, HALF_BYTES, 1024);
-            uint32_t           it = 0, wc = 0;
-            bool               ok = true;
-            auto issue_s = [&](int stage) {  // S^T = K Q^T
-                const uint64_t qd = ptx::desc_advance(q_kmaj, stage * TILE_BYTES);
+        constexpr uint32_t idesc_kk = ptx::make_idesc(1, 1, BLK, BLK, 0, 0);  // A, B K-major
+        constexpr uint32_t idesc_tn = ptx::make_idesc(1, 1, BLK, D, 0, 1);    // A from TMEM, B MN-major
+        constexpr uint32_t idesc_nn = ptx::make_idesc(1, 1, D, BLK, 1, 1);    // A, B MN-major
+        // one descriptor per operand and role, built once; every MMA below only steps it
+        const ptx::Desc k_kmaj(ptx::smem_desc_sw128(base + OFF_K, 16, 1024));
+        const ptx::Desc v_kmaj(ptx::smem_desc_sw128(base + OFF_V, 16, 1024));
+        const ptx::Desc q_kmaj(ptx::smem_desc_sw128(base + OFF_Q, 16, 1024));
+        const ptx::Desc do_kmaj(ptx::smem_desc_sw128(base + OFF_DO, 16, 1024));
+        const ptx::Desc k_mn(ptx::smem_desc_sw128(base + OFF_K, HALF_BYTES, 1024));
+        const ptx::Desc q_mn(ptx::smem_desc_sw128(base + OFF_Q, HALF_BYTES, 1024));
+        const ptx::Desc do_mn(ptx::smem_desc_sw128(base + OFF_DO, HALF_BYTES, 1024));
+        const ptx::Desc ds_mn(ptx::smem_desc_sw128(base + OFF_DS, HALF_BYTES, 1024));
+        uint32_t        it = 0, wc = 0, s = 0, ph = 0;
+        bool            ok = true;
+        auto issue_s = [&](uint32_t stage) {  // S^T = K Q^T
+            const ptx::Desc qd = q_kmaj.at(stage * TILE_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t off = (kk >> 2) * HALF_BYTES + (kk & 3) * 32;
-                    ptx::mma_f16_ss(tmem, ptx::desc_advance(k_kmaj, off), ptx::desc_advance(qd, off), idesc_kk, kk != 0);
-                }
-                ptx::mma_commit(&bar.s_full);
-            };
-            for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
-                if (!ptx::mbar_wait(&bar.kv_full, wc & 1u) || !ptx::mbar_wait(&bar.q_full[it % STAGES], (it / STAGES) & 1u)) {
-                    flag(p, ERR_MMA);
+            for (int kk = 0; kk < D / 16; ++kk) {
+                const uint32_t off = (kk >> 2) * HALF_BYTES + (kk & 3) * 32;
+                ptx::mma_f16_ss_if<1>(tmem, k_kmaj.at(off), qd.at(off), idesc_kk, kk, leader);
+            }
+            ptx::mma_commit_if<1>(b_of(bar.s_full), leader);
+        };
+        for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
+            if (!ptx::mbar_wait_warp(b_of(bar.kv_full), wc & 1u) || !ptx::mbar_wait_warp(b_of(bar.q_full[0]) + s * 8, ph)) {
+                ok = false;
+                break;
+            }
+            ptx::tc_fence_after();
+            issue_s(s);
+            for (int i = 0; i < n_q; ++i, ++it) {
+                const ptx::Desc o_k = do_kmaj.at(s * TILE_BYTES), o_m = do_mn.at(s * TILE_BYTES), q_m = q_mn.at(s * TILE_BYTES);
+                const uint32_t  next = s + 1 == STAGES ? 0 : s + 1, next_ph = next == 0 ? ph ^ 1u : ph;
+                // the previous block's dQ^T must have left the columns dP^T is written to
+                if (!ptx::mbar_wait_warp(b_of(bar.do_full[0]) + s * 8, ph) || !ptx::mbar_wait_warp(b_of(bar.dq_free), (it & 1u) ^ 1u)) {
+                    ok = false;
                     break;
                 }
                 ptx::tc_fence_after();
-                issue_s(it % STAGES);
-                for (int i = 0; i < n_q; ++i, ++it) {
-                    const int      s  = it % STAGES;
-                    const uint32_t ph = (it / STAGES) & 1u;
-                    const uint64_t o_k = ptx::desc_advance(do_kmaj, s * TILE_BYTES);
-                    const uint64_t o_m = ptx::desc_advance(do_mn, s * TILE_BYTES);
-                    const uint64_t q_m = ptx::desc_advance(q_mn, s * TILE_BYTES);
-                    // the previous block's dQ^T must have left the columns dP^T is written to
-                    if (!ptx::mbar_wait(&bar.do_full[s], ph) || !ptx::mbar_wait(&bar.dq_free, (it & 1u) ^ 1u)) {
-                        flag(p, ERR_MMA);
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after();
-                    stamp(p, it, 1);
+                stamp(p, it, 1);
 #pragma unroll
-                    for (int kk = 0; kk < D / 16; ++kk) {  // dP^T = V dO^T
-                        const uint32_t off = (kk >> 2) * HALF_BYTES + (kk & 3) * 32;
-                        ptx::mma_f16_ss(tmem + 128, ptx::desc_advance(v_kmaj, off), ptx::desc_advance(o_k, off), idesc_kk,
-                                        kk != 0);
-                    }
-                    ptx::mma_commit(&bar.dp_full);
-                    if (!ptx::mbar_wait(&bar.p_ready, it & 1u)
-                        || (i == 0 && !ptx::mbar_wait(&bar.acc_free, (wc & 1u) ^ 1u))) {
-                        flag(p, ERR_MMA);
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after();
-                    stamp(p, it, 0);
-#pragma unroll
-                    for (int kk = 0; kk < BLK / 16; ++kk) {  // dV += P^T dO   (contraction over q)
-                        ptx::mma_f16_ts(tmem + 256, tmem + (kk >> 2) * 64 + (kk & 3) * 8, ptx::desc_advance(o_m, kk * 2048),
-                                        idesc_tn, i != 0 || kk != 0);
-                    }
-                    if (i + 1 < n_q) {
-                        const uint32_t n = it + 1;
-                        if (!ptx::mbar_wait(&bar.q_full[n % STAGES], (n / STAGES) & 1u)) {
-                            flag(p, ERR_MMA);
-                            ok = false;
-                            break;
-                        }
-                        ptx::tc_fence_after();
-                        issue_s(n % STAGES);
-                    }
-                    stamp(p, it, 2);
-                    if (!ptx::mbar_wait(&bar.ds_ready, it & 1u)) {
-                        flag(p, ERR_MMA);
-                        ok = false;
-                        break;
-                    }
-                    ptx::tc_fence_after();
-                    stamp(p, it, 3);
-#pragma unroll
-                    for (int kk = 0; kk < BLK / 16; ++kk) {  // dK += dS^T Q
-                        ptx::mma_f16_ts(tmem + 384, tmem + 128 + (kk >> 2) * 64 + (kk & 3) * 8,
-                                        ptx::desc_advance(q_m, kk * 2048), idesc_tn, i != 0 || kk != 0);
-                    }
-                    ptx::mma_commit(&bar.empty[s]);
-#pragma unroll
-                    for (int kk = 0; kk < BLK / 16; ++kk) {  // dQ^T = K^T dS^T   (contraction over kv)
-                        ptx::mma_f16_ss(tmem + 128, ptx::desc_advance(k_mn, kk * 2048), ptx::desc_advance(ds_mn, kk * 2048),
-                                        idesc_nn, kk != 0);
-                    }
-                    ptx::mma_commit(&bar.dq_full);
-                    stamp(p, it, 4);
+                for (int kk = 0; kk < D / 16; ++kk) {  // dP^T = V dO^T
+                    const uint32_t off = (kk >> 2) * HALF_BYTES + (kk & 3) * 32;
+                    ptx::mma_f16_ss_if<1>(tmem + 128, v_kmaj.at(off), o_k.at(off), idesc_kk, kk, leader);
                 }
-                if (ok) {
-                    ptx::mma_commit(&bar.acc_full);
-                    ptx::mma_commit(&bar.kv_empty);
+                ptx::mma_commit_if<1>(b_of(bar.dp_full), leader);
+                if (!ptx::mbar_wait_warp(b_of(bar.p_ready), it & 1u)
+                    || (i == 0 && !ptx::mbar_wait_warp(b_of(bar.acc_free), (wc & 1u) ^ 1u))) {
+                    ok = false;
+                    break;
                 }
+                ptx::tc_fence_after();
+                stamp(p, it, 0);
+#pragma unroll
+                for (int kk = 0; kk < BLK / 16; ++kk) {  // dV += P^T dO   (contraction over q)
+                    ptx::mma_f16_ts_if(tmem + 256, tmem + (kk >> 2) * 64 + (kk & 3) * 8, o_m.at(kk * 2048), idesc_tn,
+                                       static_cast<uint32_t>(i | kk), leader);
+                }
+                if (i + 1 < n_q) {
+                    if (!ptx::mbar_wait_warp(b_of(bar.q_full[0]) + next * 8, next_ph)) {
+                        ok = false;
+                        break;
+                    }
+                    ptx::tc_fence_after();
+                    issue_s(next);
+                }
+                stamp(p, it, 2);
+                if (!ptx::mbar_wait_warp(b_of(bar.ds_ready), it & 1u)) {
+                    ok = false;
+                    break;
+                }
+                ptx::tc_fence_after();
+                stamp(p, it, 3);
+#pragma unroll
+                for (int kk = 0; kk < BLK / 16; ++kk) {  // dK += dS^T Q
+                    ptx::mma_f16_ts_if(tmem + 384, tmem + 128 + (kk >> 2) * 64 + (kk & 3) * 8, q_m.at(kk * 2048), idesc_tn,
+                                       static_cast<uint32_t>(i | kk), leader);
+                }
+                ptx::mma_commit_if<1>(b_of(bar.empty[0]) + s * 8, leader);
+#pragma unroll
+                for (int kk = 0; kk < BLK / 16; ++kk) {  // dQ^T = K^T dS^T   (contraction over kv)
+                    ptx::mma_f16_ss_if<1>(tmem + 128, k_mn.at(kk * 2048), ds_mn.at(kk * 2048), idesc_nn, kk, leader);
+                }
+                ptx::mma_commit_if<1>(b_of(bar.dq_full), leader);
+                stamp(p, it, 4);
+                s  = next;
+                ph = next_ph;
             }
+            if (ok) {
+                ptx::mma_commit_if<1>(b_of(bar.acc_full), leader);
+                ptx::mma_commit_if<1>(b_of(bar.kv_empty), leader);
+            }
+        }
+        if (!ok) {
+            flag(p, ERR_MMA);
         }
         __syncwarp();
     }

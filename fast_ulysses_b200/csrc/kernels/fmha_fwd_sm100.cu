@@ -134,16 +134,12 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
     __shared__ uint32_t       tmem_holder;
 
     const uint32_t base = (ptx::smem_addr(smem_raw) + 1023u) & ~1023u;
-    uint8_t*       sm   = smem_raw + (base - ptx::smem_addr(smem_raw));
     // layout: Q0 | Q1 | K[0] | K[1] | V[0] | V[1]
     const uint32_t sq_addr = base;
     const uint32_t sk_addr = base + QT * TILE_BYTES;
     const uint32_t sv_addr = sk_addr + KV_STAGES * TILE_BYTES;
-    uint8_t*       sq      = sm;
-    uint8_t*       sk      = sm + QT * TILE_BYTES;
-    uint8_t*       sv      = sk + KV_STAGES * TILE_BYTES;
 
-    const int warp = threadIdx.x >> 5;
+    const int warp = static_cast<int>(ptx::uniform(threadIdx.x >> 5));
     const int lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
@@ -174,172 +170,158 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
     ptx::tc_fence_before();
     __syncthreads();
     ptx::tc_fence_after();
-    const uint32_t tmem = tmem_holder;
+    const uint32_t tmem = ptx::uniform(tmem_holder);
     const int      n_kv = p.n_kv;
 
     if (warp < 4) {
     ptx::setmaxnreg_dec<REGS_SMALL>();
+    // Both roles are run by the whole warp, see ptx.cuh: elect_one().
+    const uint32_t leader = ptx::elect_one();
+    auto           b_of   = [](uint64_t& x) { return ptx::smem_addr(&x); };
     if (warp == 0) {
         // ---------------------------------------------------------------- producer
-        if (lane == 0) {
-            uint32_t it = 0, wc = 0;
-            bool     ok = true;
-            for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
-                const int qb = w % p.q_blocks;
-                const int h  = (w / p.q_blocks) % p.H;
-                const int b  = w / (p.q_blocks * p.H);
-                if (!ptx::mbar_wait(&bar.q_empty, (wc & 1u) ^ 1u)) {
-                    flag(p, ERR_LOAD);
-                    break;
-                }
-                ptx::mbar_expect_tx(&bar.q_full, QT * TILE_BYTES);
-                for (int t = 0; t < QT; ++t) {
-                    for (int half = 0; half < 2; ++half) {
-                        ptx::tma_load_4d(sq + t * TILE_BYTES + half * HALF_BYTES, &p.map_q, half * 64,
-                                         qb * (QT * BM) + t * BM, h, b, &bar.q_full);
-                    }
-                }
-                for (int j = 0; j < n_kv; ++j, ++it) {
-                    const int      s      = it % KV_STAGES;
-                    const uint32_t parity = ((it / KV_STAGES) & 1u) ^ 1u;
-                    if (!ptx::mbar_wait(&bar.k_empty[s], parity)) {
-                        flag(p, ERR_LOAD);
-                        ok = false;
-                        break;
-                    }
-                    ptx::mbar_expect_tx(&bar.k_full[s], TILE_BYTES);
-                    for (int half = 0; half < 2; ++half) {
-                        ptx::tma_load_4d(sk + s * TILE_BYTES + half * HALF_BYTES, &p.map_k, half * 64, j * BN, h, b,
-                                         &bar.k_full[s]);
-                    }
-                    if (!ptx::mbar_wait(&bar.v_empty[s], parity)) {
-                        flag(p, ERR_LOAD);
-                        ok = false;
-                        break;
-                    }
-                    ptx::mbar_expect_tx(&bar.v_full[s], TILE_BYTES);
-                    for (int half = 0; half < 2; ++half) {
-                        ptx::tma_load_4d(sv + s * TILE_BYTES + half * HALF_BYTES, &p.map_v, half * 64, j * BN, h, b,
-                                         &bar.v_full[s]);
-                    }
+        uint32_t stage = 0, phase = 1, wc = 0;
+        bool     ok = true;
+        for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
+            const int qb = w % p.q_blocks;
+            const int h  = (w / p.q_blocks) % p.H;
+            const int b  = w / (p.q_blocks * p.H);
+            if (!ptx::mbar_wait_warp(b_of(bar.q_empty), (wc & 1u) ^ 1u)) {
+                ok = false;
+                break;
+            }
+            ptx::mbar_expect_tx_if(b_of(bar.q_full), QT * TILE_BYTES, leader);
+            for (int t = 0; t < QT; ++t) {
+                for (int half = 0; half < 2; ++half) {
+                    ptx::tma_load_4d_if(sq_addr + t * TILE_BYTES + half * HALF_BYTES, &p.map_q, half * 64,
+                                        qb * (QT * BM) + t * BM, h, b, b_of(bar.q_full), leader);
                 }
             }
+            for (int j = 0; j < n_kv; ++j) {
+                const uint32_t kf = b_of(bar.k_full[0]) + stage * 8, vf = b_of(bar.v_full[0]) + stage * 8;
+                if (!ptx::mbar_wait_warp(b_of(bar.k_empty[0]) + stage * 8, phase)) {
+                    ok = false;
+                    break;
+                }
+                ptx::mbar_expect_tx_if(kf, TILE_BYTES, leader);
+                for (int half = 0; half < 2; ++half) {
+                    ptx::tma_load_4d_if(sk_addr + stage * TILE_BYTES + half * HALF_BYTES, &p.map_k, half * 64, j * BN, h, b, kf,
+                                        leader);
+                }
+                if (!ptx::mbar_wait_warp(b_of(bar.v_empty[0]) + stage * 8, phase)) {
+                    ok = false;
+                    break;
+                }
+                ptx::mbar_expect_tx_if(vf, TILE_BYTES, leader);
+                for (int half = 0; half < 2; ++half) {
+                    ptx::tma_load_4d_if(sv_addr + stage * TILE_BYTES + half * HALF_BYTES, &p.map_v, half * 64, j * BN, h, b, vf,
+                                        leader);
+                }
+                if (++stage == KV_STAGES) {
+                    stage = 0;
+                    phase ^= 1u;
+                }
+            }
+        }
+        if (!ok) {
+            flag(p, ERR_LOAD);
         }
         __syncwarp();
     }
     else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        if (lane == 0) {
-            constexpr uint32_t idesc_qk = ptx::make_idesc(1, 1, BM, BN, 0, 0);  // both K-major
-            constexpr uint32_t idesc_pv = ptx::make_idesc(1, 1, BM, D, 0, 1);   // V is MN-major
-            uint32_t           it = 0, wc = 0;
-            uint32_t           pcount[QT] = {0, 0};
-            bool               ok = true;
+        constexpr uint32_t idesc_qk = ptx::make_idesc(1, 1, BM, BN, 0, 0);  // both K-major
+        constexpr uint32_t idesc_pv = ptx::make_idesc(1, 1, BM, D, 0, 1);   // V is MN-major
+        // one descriptor per operand, built once; every MMA below only steps it
+        const ptx::Desc desc_q(ptx::smem_desc_sw128(sq_addr, 16, 1024));
+        const ptx::Desc desc_k(ptx::smem_desc_sw128(sk_addr, 16, 1024));
+        const ptx::Desc desc_v(ptx::smem_desc_sw128(sv_addr, HALF_BYTES, 1024));
+        uint32_t        stage = 0, phase = 0, it = 0, wc = 0;
+        bool            ok = true;
 
-            // one descriptor per operand, built once; every MMA below only steps it
-            const uint64_t desc_q = ptx::smem_desc_sw128(sq_addr, 16, 1024);
-            const uint64_t desc_k = ptx::smem_desc_sw128(sk_addr, 16, 1024);
-            const uint64_t desc_v = ptx::smem_desc_sw128(sv_addr, HALF_BYTES, 1024);
-
-            auto issue_qk = [&](int t, int stage) {
-                const uint64_t qa = ptx::desc_advance(desc_q, t * TILE_BYTES);
-                const uint64_t ka = ptx::desc_advance(desc_k, stage * TILE_BYTES);
+        auto issue_qk = [&](int t, uint32_t st) {
+            const ptx::Desc qa = desc_q.at(t * TILE_BYTES), ka = desc_k.at(st * TILE_BYTES);
 #pragma unroll
-                for (int kk = 0; kk < D / 16; ++kk) {
-                    const uint32_t off = (kk >> 2) * HALF_BYTES + (kk & 3) * 32;
-                    ptx::mma_f16_ss(tmem + t * 128, ptx::desc_advance(qa, off), ptx::desc_advance(ka, off), idesc_qk,
-                                    kk != 0);
-                }
-                ptx::mma_commit(&bar.s_full[t]);
-            };
-            // One half (64 kv rows) of P_t V: the softmax hands P over in two halves so that the
-            // first half's products run under the second half's exponentials.
-            auto issue_pv = [&](int t, int stage, int half, bool accumulate) {
-                // 16 kv rows = 2048 bytes further down; the two 64-wide halves of d are HALF_BYTES
-                // apart (leading byte offset), 8-row groups 1024 bytes apart
-                const uint64_t va = ptx::desc_advance(desc_v, stage * TILE_BYTES);
+            for (int kk = 0; kk < D / 16; ++kk) {
+                const uint32_t off = (kk >> 2) * HALF_BYTES + (kk & 3) * 32;
+                ptx::mma_f16_ss_if<1>(tmem + t * 128, qa.at(off), ka.at(off), idesc_qk, kk, leader);
+            }
+            ptx::mma_commit_if<1>(b_of(bar.s_full[0]) + t * 8, leader);
+        };
+        // One half (64 kv rows) of P_t V: the softmax hands P over in two halves so that the
+        // first half's products run under the second half's exponentials.
+        auto issue_pv = [&](int t, uint32_t st, int half, uint32_t accumulate) {
+            // 16 kv rows = 2048 bytes further down; the two 64-wide halves of d are HALF_BYTES
+            // apart (leading byte offset), 8-row groups 1024 bytes apart
+            const ptx::Desc va = desc_v.at(st * TILE_BYTES);
 #pragma unroll
-                for (int k4 = 0; k4 < BN / 32; ++k4) {
-                    const int kk = half * (BN / 32) + k4;
-                    ptx::mma_f16_ts(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, ptx::desc_advance(va, kk * 2048),
-                                    idesc_pv, accumulate || kk != 0);
-                }
-            };
+            for (int k4 = 0; k4 < BN / 32; ++k4) {
+                const int kk = half * (BN / 32) + k4;
+                ptx::mma_f16_ts_if(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, va.at(kk * 2048), idesc_pv,
+                                   accumulate | static_cast<uint32_t>(kk), leader);
+            }
+        };
 
-            for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
-                if (!ptx::mbar_wait(&bar.q_full, wc & 1u)) {
-                    flag(p, ERR_MMA);
+        for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
+            // prologue: S for both query tiles of kv step 0
+            if (!ptx::mbar_wait_warp(b_of(bar.q_full), wc & 1u)
+                || !ptx::mbar_wait_warp(b_of(bar.k_full[0]) + stage * 8, phase)) {
+                ok = false;
+                break;
+            }
+            ptx::tc_fence_after();
+            issue_qk(0, stage);
+            issue_qk(1, stage);
+            ptx::mma_commit_if<1>(b_of(bar.k_empty[0]) + stage * 8, leader);
+            for (int j = 0; j < n_kv && ok; ++j, ++it) {
+                const uint32_t next = stage + 1 == KV_STAGES ? 0 : stage + 1, next_phase = next == 0 ? phase ^ 1u : phase;
+                const bool     more = j + 1 < n_kv;
+                if (!ptx::mbar_wait_warp(b_of(bar.v_full[0]) + stage * 8, phase)
+                    || (more && !ptx::mbar_wait_warp(b_of(bar.k_full[0]) + next * 8, next_phase))) {
+                    ok = false;
                     break;
                 }
-                // prologue: S for both query tiles of kv step 0
-                {
-                    const int s = it % KV_STAGES;
-                    if (!ptx::mbar_wait(&bar.k_full[s], (it / KV_STAGES) & 1u)) {
-                        flag(p, ERR_MMA);
+#pragma unroll
+                for (int t = 0; t < QT; ++t) {
+                    stamp<TRACE>(p, it, 20 + t * 6 + 0);
+                    if (!ptx::mbar_wait_warp(b_of(bar.p_lo[t]), it & 1u)
+                        || (j == 0 && !ptx::mbar_wait_warp(b_of(bar.o_free[t]), (wc & 1u) ^ 1u))) {
+                        ok = false;
                         break;
                     }
+                    stamp<TRACE>(p, it, 20 + t * 6 + 1);
                     ptx::tc_fence_after();
-                    issue_qk(0, s);
-                    issue_qk(1, s);
-                    ptx::mma_commit(&bar.k_empty[s]);
-                }
-                for (int j = 0; j < n_kv && ok; ++j, ++it) {
-                    const int  s    = it % KV_STAGES;
-                    const int  sn   = (it + 1) % KV_STAGES;
-                    const bool more = j + 1 < n_kv;
-                    if (!ptx::mbar_wait(&bar.v_full[s], (it / KV_STAGES) & 1u)) {
-                        flag(p, ERR_MMA);
+                    issue_pv(t, stage, 0, static_cast<uint32_t>(j));
+                    stamp<TRACE>(p, it, 20 + t * 6 + 2);
+                    if (!ptx::mbar_wait_warp(b_of(bar.p_hi[t]), it & 1u)) {
                         ok = false;
                         break;
                     }
-                    if (more && !ptx::mbar_wait(&bar.k_full[sn], ((it + 1) / KV_STAGES) & 1u)) {
-                        flag(p, ERR_MMA);
-                        ok = false;
-                        break;
+                    stamp<TRACE>(p, it, 20 + t * 6 + 3);
+                    ptx::tc_fence_after();
+                    issue_pv(t, stage, 1, 1u);
+                    if (!more) {
+                        ptx::mma_commit_if<1>(b_of(bar.o_final[t]), leader);
                     }
-                    for (int t = 0; t < QT; ++t) {
-                        stamp<TRACE>(p, it, 20 + t * 6 + 0);
-                        if (!ptx::mbar_wait(&bar.p_lo[t], pcount[t] & 1u)) {
-                            flag(p, ERR_MMA);
-                            ok = false;
-                            break;
-                        }
-                        stamp<TRACE>(p, it, 20 + t * 6 + 1);
-                        if (j == 0 && !ptx::mbar_wait(&bar.o_free[t], (wc & 1u) ^ 1u)) {
-                            flag(p, ERR_MMA);
-                            ok = false;
-                            break;
-                        }
-                        ptx::tc_fence_after();
-                        issue_pv(t, s, 0, j != 0);
-                        stamp<TRACE>(p, it, 20 + t * 6 + 2);
-                        if (!ptx::mbar_wait(&bar.p_hi[t], pcount[t] & 1u)) {
-                            flag(p, ERR_MMA);
-                            ok = false;
-                            break;
-                        }
-                        stamp<TRACE>(p, it, 20 + t * 6 + 3);
-                        ++pcount[t];
-                        ptx::tc_fence_after();
-                        issue_pv(t, s, 1, true);
-                        if (!more) {
-                            ptx::mma_commit(&bar.o_final[t]);
-                        }
-                        else {
-                            issue_qk(t, sn);  // S_t is free again: PV_t above is ordered before it
-                        }
-                        stamp<TRACE>(p, it, 20 + t * 6 + 4);
+                    else {
+                        issue_qk(t, next);  // S_t is free again: PV_t above is ordered before it
                     }
-                    if (!ok) {
-                        break;
-                    }
-                    ptx::mma_commit(&bar.v_empty[s]);
-                    if (more) {
-                        ptx::mma_commit(&bar.k_empty[sn]);
-                    }
+                    stamp<TRACE>(p, it, 20 + t * 6 + 4);
                 }
-                ptx::mma_commit(&bar.q_empty);
+                if (!ok) {
+                    break;
+                }
+                ptx::mma_commit_if<1>(b_of(bar.v_empty[0]) + stage * 8, leader);
+                if (more) {
+                    ptx::mma_commit_if<1>(b_of(bar.k_empty[0]) + next * 8, leader);
+                }
+                stage = next;
+                phase = next_phase;
             }
+            ptx::mma_commit_if<1>(b_of(bar.q_empty), leader);
+        }
+        if (!ok) {
+            flag(p, ERR_MMA);
         }
         __syncwarp();
     }
