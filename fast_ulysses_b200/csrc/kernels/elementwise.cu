@@ -18,6 +18,8 @@
 
 #include <cuda_bf16.h>
 
+#include <algorithm>
+
 namespace {
 
 struct NormRopeBwd {
@@ -33,61 +35,151 @@ struct NormRopeBwd {
     float                eps;
 };
 
+// Both kernels below give a row of 128 values (one head of one token) to eight lanes, 16 values each:
+// four rows per warp and instruction, three shuffles per reduction.
+struct RowPart {
+    uint2 w[4];  // 16 bf16 values
+};
+__device__ __forceinline__ RowPart load_part(const void* p)
+{
+    RowPart r;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        asm volatile("ld.global.v2.u32 {%0, %1}, [%2];"
+                     : "=r"(r.w[k].x), "=r"(r.w[k].y)
+                     : "l"(static_cast<const uint8_t*>(p) + k * 64));
+    }
+    return r;
+}
+__device__ __forceinline__ void store_part(void* p, const RowPart& r)
+{
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        *reinterpret_cast<uint2*>(static_cast<uint8_t*>(p) + k * 64) = r.w[k];
+    }
+}
+// Value k of lane `part` is element (k / 4) * 32 + part * 4 + k % 4 of its row (eight lanes move 64
+// contiguous bytes per instruction and an 8-byte alignment is enough).
+constexpr int kPartStride = 32;
+
+__device__ __forceinline__ float sum_of_row(float v)
+{
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) {
+        v += __shfl_xor_sync(0xffffffffu, v, off);
+    }
+    return v;
+}
+
+// d(projection) of one row from the gradient behind RMSNorm -> RoPE; accumulates d(gamma) into dg.
+__device__ __forceinline__ RowPart norm_rope_bwd(const RowPart& g, const RowPart& y, const float* rope, const float* gamma, float eps,
+                                                 int part, float (&dg)[16])
+{
+    float yy[16], dx[16], ss = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 cs = *reinterpret_cast<const float4*>(rope + k * kPartStride + part * 4);  // (c0, s0, c1, s1)
+        const float2 g0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g.w[k].x));
+        const float2 g1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&g.w[k].y));
+        const float2 y0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&y.w[k].x));
+        const float2 y1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&y.w[k].y));
+        // undo the rotation: the transpose of a rotation is the opposite rotation
+        dx[4 * k]     = g0.x * cs.x + g0.y * cs.y;
+        dx[4 * k + 1] = -g0.x * cs.y + g0.y * cs.x;
+        dx[4 * k + 2] = g1.x * cs.z + g1.y * cs.w;
+        dx[4 * k + 3] = -g1.x * cs.w + g1.y * cs.z;
+        yy[4 * k] = y0.x, yy[4 * k + 1] = y0.y, yy[4 * k + 2] = y1.x, yy[4 * k + 3] = y1.y;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            ss += yy[4 * k + i] * yy[4 * k + i];
+        }
+    }
+    const float rstd = rsqrtf(sum_of_row(ss) * (1.0f / 128.0f) + eps);
+    float       dot  = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float4 gm     = *reinterpret_cast<const float4*>(gamma + k * kPartStride + part * 4);
+        const float  gmv[4] = {gm.x, gm.y, gm.z, gm.w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const int   e = 4 * k + i;
+            const float n = yy[e] * rstd;
+            dg[e] += dx[e] * n;
+            dx[e] *= gmv[i];
+            dot += dx[e] * n;
+            yy[e] = n;
+        }
+    }
+    dot = sum_of_row(dot) * (1.0f / 128.0f);
+    RowPart out;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        float o[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            o[i] = rstd * (dx[4 * k + i] - yy[4 * k + i] * dot);
+        }
+        out.w[k].x = fu::ptx::pack_bf16x2(o[0], o[1]);
+        out.w[k].y = fu::ptx::pack_bf16x2(o[2], o[3]);
+    }
+    return out;
+}
+
+// Adds a CTA's d(gamma) to the result: the lanes that hold the same elements by shuffle, the warps through
+// shared memory, one atomic per element and CTA. (All threads of the CTA.)
+__device__ __forceinline__ void add_dgamma(float (&dg)[16], float* dgamma, float (*red)[128])
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int e = 0; e < 16; ++e) {
+        dg[e] += __shfl_xor_sync(0xffffffffu, dg[e], 8);
+        dg[e] += __shfl_xor_sync(0xffffffffu, dg[e], 16);
+    }
+    __syncthreads();
+    if (lane < 8) {
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+            red[warp][(e >> 2) * kPartStride + lane * 4 + (e & 3)] = dg[e];
+        }
+    }
+    __syncthreads();
+    if (dgamma && threadIdx.x < 128) {
+        float s = 0.0f;
+        for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
+            s += red[w][threadIdx.x];
+        }
+        atomicAdd(dgamma + threadIdx.x, s);
+    }
+}
+
 __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(const NormRopeBwd p)
 {
-    const int     lane   = threadIdx.x & 31;
-    const int64_t warp0  = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    const int64_t items  = p.m * p.heads;  // per projection
+    __shared__ float red[8][128];
+    const int        sub    = (threadIdx.x >> 3) & 3, part = threadIdx.x & 7;
+    const int64_t    warp0  = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
+    const int64_t    nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
+    const int64_t    items  = p.m * p.heads;  // per projection
     for (int t = 0; t < 2; ++t) {
-        const float4 gm = *reinterpret_cast<const float4*>(p.gamma[t] + lane * 4);
-        float        dg[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int64_t it = warp0; it < items; it += nwarps) {
+        float dg[16] = {};
+        for (int64_t it0 = warp0 * 4; it0 < items; it0 += nwarps * 4) {
+            const bool    here = it0 + sub < items;  // the warp stays together for the reductions
+            const int64_t it   = here ? it0 + sub : items - 1;
             const int64_t row  = it / p.heads;
-            const int     head = static_cast<int>(it - row * p.heads);
-            const int64_t s    = row % p.s_local;
-            const uint2   gv   = *reinterpret_cast<const uint2*>(p.g[t] + (row * p.heads + head) * 128 + lane * 4);
-            const uint2   yv   = *reinterpret_cast<const uint2*>(p.y + row * p.ld_y + (t * p.heads + head) * 128 + lane * 4);
-            const float2  g01  = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gv.x));
-            const float2  g23  = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gv.y));
-            const float2  y01  = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&yv.x));
-            const float2  y23  = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&yv.y));
-            const float4  cs   = *reinterpret_cast<const float4*>(p.rope + s * 64 + lane * 2);  // (c0, s0, c1, s1)
-            // undo the rotation: the transpose of a rotation is the opposite rotation
-            const float dx[4] = {g01.x * cs.x + g01.y * cs.y, -g01.x * cs.y + g01.y * cs.x,
-                                 g23.x * cs.z + g23.y * cs.w, -g23.x * cs.w + g23.y * cs.z};
-            const float yy[4] = {y01.x, y01.y, y23.x, y23.y};
-            float       ss    = yy[0] * yy[0] + yy[1] * yy[1] + yy[2] * yy[2] + yy[3] * yy[3];
+            const int64_t head = it - row * p.heads;
+            const RowPart g    = load_part(p.g[t] + it * 128 + part * 4);
+            const RowPart y    = load_part(p.y + row * p.ld_y + (t * p.heads + head) * 128 + part * 4);
+            float         own[16] = {};
+            const RowPart out  = norm_rope_bwd(g, y, reinterpret_cast<const float*>(p.rope + (row % p.s_local) * 64), p.gamma[t],
+                                               p.eps, part, own);
+            if (here) {
 #pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                ss += __shfl_xor_sync(0xffffffffu, ss, off);
-            }
-            const float rstd  = rsqrtf(ss * (1.0f / 128.0f) + p.eps);
-            const float gmv[4] = {gm.x, gm.y, gm.z, gm.w};
-            float       n[4], dn[4], dot = 0.0f;
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                n[k]  = yy[k] * rstd;
-                dn[k] = dx[k] * gmv[k];
-                dg[k] += dx[k] * n[k];
-                dot += dn[k] * n[k];
-            }
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                dot += __shfl_xor_sync(0xffffffffu, dot, off);
-            }
-            dot *= (1.0f / 128.0f);
-            uint2 out;
-            out.x = fu::ptx::pack_bf16x2(rstd * (dn[0] - n[0] * dot), rstd * (dn[1] - n[1] * dot));
-            out.y = fu::ptx::pack_bf16x2(rstd * (dn[2] - n[2] * dot), rstd * (dn[3] - n[3] * dot));
-            *reinterpret_cast<uint2*>(p.dy + row * p.ld_dy + (t * p.heads + head) * 128 + lane * 4) = out;
-        }
-        if (p.dgamma[t]) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                atomicAdd(p.dgamma[t] + lane * 4 + k, dg[k]);
+                for (int e = 0; e < 16; ++e) {
+                    dg[e] += own[e];
+                }
+                store_part(p.dy + row * p.ld_dy + (t * p.heads + head) * 128 + part * 4, out);
             }
         }
+        add_dgamma(dg, p.dgamma[t], red);
     }
 }
 
@@ -297,9 +389,16 @@ struct PullGrads {
     uint8_t              owner[MAX_HEADS], local[MAX_HEADS], heads_of[FU_MAX_WORLD];
 };
 
-__global__ void __launch_bounds__(256) pull_qkv_grads_kernel(const __grid_constant__ PullGrads p)
+// Bound by HBM (or the link). 75600 tokens x 40 heads on one GPU, 6.2 GB: @PULL@ ms; 5.0 with a warp per row,
+// whose 64-bit index arithmetic filled the issue slots. 256 tokens x 2 heads: @PULLT@ us; 153 when every warp
+// of a full grid added its d(gamma) with atomics of its own.
+__global__ void __launch_bounds__(256, 2) pull_qkv_grads_kernel(const __grid_constant__ PullGrads p)
 {
-    __shared__ uint32_t ticket;
+    __shared__ uint32_t       ticket;
+    __shared__ const uint8_t* from[3][MAX_HEADS];
+    __shared__ uint32_t       pitch[MAX_HEADS];
+    __shared__ float          red[8][128];
+    constexpr int             kInFlight = 2;
     const int      lane = threadIdx.x & 31;
     const int      warp = threadIdx.x >> 5;
     const uint64_t base = *reinterpret_cast<volatile uint64_t*>(&p.peers.own->epoch);
@@ -313,98 +412,72 @@ __global__ void __launch_bounds__(256) pull_qkv_grads_kernel(const __grid_consta
     }
     __syncthreads();
 
-    const int64_t warp0  = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-    const int64_t items  = p.m * p.heads;  // per projection
+    // A warp takes four neighbouring heads of a token at a time, kInFlight such groups together: a load
+    // from a peer takes microseconds, and with one group the kernel would wait on latency instead of
+    // on the link. Where a head lives is looked up in shared memory (the lanes of a group may differ).
+    for (int i = threadIdx.x; i < p.heads; i += blockDim.x) {
+        const int peer = p.owner[i];
+        pitch[i]       = static_cast<uint32_t>(p.heads_of[peer]) * 256u;
+        for (int t = 0; t < 3; ++t) {
+            from[t][i] = p.src[t][peer] + p.local[i] * 256;
+        }
+    }
+    __syncthreads();
+    const int      sub    = lane >> 3, part = lane & 7;
+    const uint32_t warp0  = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
+    const uint32_t groups = (static_cast<uint32_t>(p.heads) + 3) / 4;
+    const uint32_t s_loc  = static_cast<uint32_t>(p.s_local);
+    const uint32_t items  = static_cast<uint32_t>(p.m) * groups;  // per projection
     for (int t = 0; t < 3; ++t) {
-        float4 gm    = make_float4(0.f, 0.f, 0.f, 0.f);
-        float  dg[4] = {0.f, 0.f, 0.f, 0.f};
-        if (t < 2) {
-            gm = *reinterpret_cast<const float4*>(p.gamma[t] + lane * 4);
-        }
-        // Four rows per warp in flight: a load from a peer takes microseconds, and with one per
-        // warp the kernel would wait on latency instead of on the link.
-        constexpr int kInFlight = 4;
-        for (int64_t it0 = warp0; it0 < items; it0 += nwarps * kInFlight) {
-            uint2   gvs[kInFlight], yvs[kInFlight];
-            int64_t rows[kInFlight];
-            int     hds[kInFlight];
+        float dg[16] = {};
+        for (uint32_t it0 = warp0; it0 < items; it0 += nwarps * kInFlight) {
+            RowPart  g[kInFlight], y[kInFlight];
+            uint32_t rows[kInFlight], ss[kInFlight];
+            int      hds[kInFlight];  // -1: nothing here for this lane
 #pragma unroll
             for (int u = 0; u < kInFlight; ++u) {
-                const int64_t it = it0 + u * nwarps;
-                rows[u]          = -1;
+                const uint32_t it = it0 + u * nwarps;
+                hds[u]            = -1;
                 if (it < items) {
-                    const int64_t  row   = it / p.heads;
-                    const int      head  = static_cast<int>(it - row * p.heads);
-                    const int64_t  batch = row / p.s_local;
-                    const int64_t  s     = row - batch * p.s_local;
-                    const int      peer  = p.owner[head];
-                    const int64_t  hp    = p.heads_of[peer];
-                    const uint8_t* from  = p.src[t][peer]
-                                          + (((batch * p.s_total + p.seq_off + s) * hp + p.local[head]) * 128 + lane * 4) * 2;
-                    asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(gvs[u].x), "=r"(gvs[u].y) : "l"(from));
-                    if (t < 2) {
-                        yvs[u] = *reinterpret_cast<const uint2*>(p.y + row * p.ld_y + (t * p.heads + head) * 128 + lane * 4);
+                    const uint32_t row   = it / groups;
+                    const int      head  = static_cast<int>(it - row * groups) * 4 + sub;
+                    const uint32_t batch = row / s_loc;
+                    rows[u]              = row;
+                    ss[u]                = row - batch * s_loc;
+                    if (head < p.heads) {
+                        hds[u] = head;
+                        g[u]   = load_part(from[t][head] + (batch * p.s_total + p.seq_off + ss[u]) * pitch[head] + part * 8);
+                        if (t < 2) {
+                            y[u] = load_part(p.y + row * p.ld_y + (t * p.heads + head) * 128 + part * 4);
+                        }
                     }
-                    rows[u] = row;
-                    hds[u]  = head;
                 }
             }
 #pragma unroll
             for (int u = 0; u < kInFlight; ++u) {
-                if (rows[u] < 0) {
-                    continue;
+                if (it0 + u * nwarps >= items) {
+                    break;  // warp-uniform
                 }
-                const int64_t row  = rows[u];
-                const int     head = hds[u];
-                const int64_t s    = row % p.s_local;
-                const uint2   gv   = gvs[u];
-                __nv_bfloat16* to = p.dy + row * p.ld_dy + (static_cast<int64_t>(t) * p.heads + head) * 128 + lane * 4;
-                if (t == 2) {
-                    *reinterpret_cast<uint2*>(to) = gv;  // dv needs no transformation
-                    continue;
-                }
-                const uint2  yv  = yvs[u];
-                const float2 g01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gv.x));
-                const float2 g23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&gv.y));
-                const float2 y01 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&yv.x));
-                const float2 y23 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&yv.y));
-                const float4 cs  = *reinterpret_cast<const float4*>(p.rope + s * 64 + lane * 2);  // (c0, s0, c1, s1)
-                // undo the rotation: the transpose of a rotation is the opposite rotation
-                const float dx[4] = {g01.x * cs.x + g01.y * cs.y, -g01.x * cs.y + g01.y * cs.x,
-                                     g23.x * cs.z + g23.y * cs.w, -g23.x * cs.w + g23.y * cs.z};
-                const float yy[4] = {y01.x, y01.y, y23.x, y23.y};
-                float       ss    = yy[0] * yy[0] + yy[1] * yy[1] + yy[2] * yy[2] + yy[3] * yy[3];
+                RowPart out = g[u];  // dv needs no transformation
+                if (t < 2) {
+                    float own[16] = {};
+                    out = norm_rope_bwd(g[u], y[u], reinterpret_cast<const float*>(p.rope + static_cast<int64_t>(ss[u]) * 64),
+                                        p.gamma[t], p.eps, part, own);
+                    if (hds[u] >= 0) {
 #pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    ss += __shfl_xor_sync(0xffffffffu, ss, off);
+                        for (int e = 0; e < 16; ++e) {
+                            dg[e] += own[e];
+                        }
+                    }
                 }
-                const float rstd   = rsqrtf(ss * (1.0f / 128.0f) + p.eps);
-                const float gmv[4] = {gm.x, gm.y, gm.z, gm.w};
-                float       n[4], dn[4], dot = 0.0f;
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    n[k]  = yy[k] * rstd;
-                    dn[k] = dx[k] * gmv[k];
-                    dg[k] += dx[k] * n[k];
-                    dot += dn[k] * n[k];
+                if (hds[u] >= 0) {
+                    store_part(p.dy + rows[u] * p.ld_dy + (static_cast<int64_t>(t) * p.heads + hds[u]) * 128 + part * 4, out);
                 }
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    dot += __shfl_xor_sync(0xffffffffu, dot, off);
-                }
-                dot *= (1.0f / 128.0f);
-                uint2 out;
-                out.x = fu::ptx::pack_bf16x2(rstd * (dn[0] - n[0] * dot), rstd * (dn[1] - n[1] * dot));
-                out.y = fu::ptx::pack_bf16x2(rstd * (dn[2] - n[2] * dot), rstd * (dn[3] - n[3] * dot));
-                *reinterpret_cast<uint2*>(to) = out;
             }
         }
-        if (t < 2 && p.dgamma[t]) {
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                atomicAdd(p.dgamma[t] + lane * 4 + k, dg[k]);
-            }
+        if (t < 2) {
+            add_dgamma(dg, p.dgamma[t], red);
         }
     }
     // Closing: "I have finished reading everybody's gradients", so that their owners may overwrite
@@ -457,7 +530,7 @@ extern "C" int fu_qk_norm_rope_bwd(const FuNormRopeBwdArgs* a, void* stream)
     int dev = 0, sms = 0;
     FU_CUDA_OK(cudaGetDevice(&dev));
     FU_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    qk_norm_rope_bwd_kernel<<<sms * 8, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
+    qk_norm_rope_bwd_kernel<<<static_cast<int>(std::min<int64_t>(sms * 8, (a->m * a->heads + 31) / 32)), 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
     FU_CUDA_OK(cudaGetLastError());
     return FU_OK;
 }
@@ -547,7 +620,11 @@ extern "C" int fu_pull_qkv_grads(const FuPullGradsArgs* a, void* stream)
     // must not be what a peer is waiting for. Every CTA of the first wave gets to run whatever
     // else is on the device, and a resident grid keeps the closing handshake prompt.
     FU_CUDA_OK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, pull_qkv_grads_kernel, 256, 0));
-    const int grid = sms * (per_sm > 0 ? per_sm : 1);
+    const int64_t warps = a->m * ((a->heads + 3) / 4);  // no more CTAs than there are groups of rows
+    if (warps * 2 > 0xffffffffll - (1ll << 22)) {  // index arithmetic is 32 bits wide, one grid of items beyond the last included
+        return fu::fail(FU_E_ARG, "fu_pull_qkv_grads: %lld tokens x %d heads", (long long)a->m, a->heads);
+    }
+    const int grid = static_cast<int>(std::min<int64_t>(sms * (per_sm > 0 ? per_sm : 1), (warps + 7) / 8));
     pull_qkv_grads_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
     FU_CUDA_OK(cudaGetLastError());
     return FU_OK;

@@ -27,49 +27,55 @@ constexpr int D   = 128;
 constexpr int BLK = 128;
 
 // delta[b,h,s] = sum_x O[b,s,h,x] * dO[b,s,h,x]; lse2 = lse * log2(e); padding rows get lse2 = +inf
-// (so that their probabilities vanish) and delta = 0. One warp per (b, h, s).
+// (so that their probabilities vanish) and delta = 0. A CTA takes 32 tokens of one head, eight lanes
+// per row; heads are the fastest CTA index, so the CTAs in flight read whole tokens and each
+// writes 128 contiguous bytes of both statistics. Bound by HBM: 75600 tokens x 40 heads (1.55 GB)
+// @PRE@ ms, 0.91 with a warp per row and the tokens as the fastest index.
 struct PreParams {
     const __nv_bfloat16 *o, *d_o;
     const float*         lse;
     float *              lse2, *delta;
-    int64_t              o_row, o_head, o_batch, do_row, do_head, do_batch;
+    int64_t              o_row, o_head, o_batch;
     int                  B, H, Sq, Sq_pad;
 };
+constexpr int kPreRows = 32;
 
-__global__ void fmha_bwd_pre_kernel(const PreParams p)
+__global__ void __launch_bounds__(8 * kPreRows) fmha_bwd_pre_kernel(const PreParams p)
 {
-    const int64_t gw    = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    const int     lane  = threadIdx.x & 31;
-    const int64_t total = static_cast<int64_t>(p.B) * p.H * p.Sq_pad;
-    if (gw >= total) {
-        return;
-    }
-    const int s = static_cast<int>(gw % p.Sq_pad);
-    const int h = static_cast<int>((gw / p.Sq_pad) % p.H);
-    const int b = static_cast<int>(gw / (static_cast<int64_t>(p.Sq_pad) * p.H));
-    if (s >= p.Sq) {
-        if (lane == 0) {
-            p.lse2[gw]  = INFINITY;
-            p.delta[gw] = 0.0f;
-        }
-        return;
-    }
-    const uint2 ov = *reinterpret_cast<const uint2*>(p.o + b * p.o_batch + static_cast<int64_t>(s) * p.o_row
-                                                     + h * p.o_head + lane * 4);
-    const uint2 dv = *reinterpret_cast<const uint2*>(p.d_o + b * p.do_batch + static_cast<int64_t>(s) * p.do_row
-                                                     + h * p.do_head + lane * 4);
-    const float2 o0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ov.x));
-    const float2 o1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&ov.y));
-    const float2 d0 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&dv.x));
-    const float2 d1 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&dv.y));
-    float        acc = o0.x * d0.x + o0.y * d0.y + o1.x * d1.x + o1.y * d1.y;
+    const uint32_t blks = static_cast<uint32_t>(p.Sq_pad) / kPreRows;
+    const int      h    = static_cast<int>(blockIdx.x % p.H);
+    const uint32_t hb   = blockIdx.x / p.H;
+    const int      b    = static_cast<int>(hb / blks);
+    const int      s    = static_cast<int>(hb - b * blks) * kPreRows + (threadIdx.x >> 3);
+    const int      part = threadIdx.x & 7;
+    const int64_t  at   = (static_cast<int64_t>(b) * p.H + h) * p.Sq_pad + s;
+    float          acc  = 0.0f;
+    if (s < p.Sq) {
+        const int64_t row = b * p.o_batch + static_cast<int64_t>(s) * p.o_row + h * p.o_head + part * 4;
+        uint2         ov[4], dv[4];
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
+        for (int k = 0; k < 4; ++k) {
+            ov[k] = *reinterpret_cast<const uint2*>(p.o + row + k * 32);
+            dv[k] = *reinterpret_cast<const uint2*>(p.d_o + row + k * 32);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            const __nv_bfloat162* oh = reinterpret_cast<const __nv_bfloat162*>(&ov[k]);
+            const __nv_bfloat162* dh = reinterpret_cast<const __nv_bfloat162*>(&dv[k]);
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const float2 of = __bfloat1622float2(oh[j]), df = __bfloat1622float2(dh[j]);
+                acc += of.x * df.x + of.y * df.y;
+            }
+        }
+    }
+#pragma unroll
+    for (int off = 4; off > 0; off >>= 1) {
         acc += __shfl_xor_sync(0xffffffffu, acc, off);
     }
-    if (lane == 0) {
-        p.delta[gw] = acc;
-        p.lse2[gw]  = p.lse[(static_cast<int64_t>(b) * p.H + h) * p.Sq + s] * 1.4426950408889634f;
+    if (part == 0) {
+        p.delta[at] = acc;
+        p.lse2[at]  = s < p.Sq ? p.lse[(static_cast<int64_t>(b) * p.H + h) * p.Sq + s] * 1.4426950408889634f : INFINITY;
     }
 }
 
@@ -127,16 +133,15 @@ extern "C" int fu_fmha_bwd(const FuFmhaArgs* a, void* stream_v)
     pre.lse = a->lse;
     pre.lse2 = a->delta;
     pre.delta = a->delta + stats;
-    pre.o_row = pre.do_row = a->o_row;
-    pre.o_head = pre.do_head = a->o_head;
-    pre.o_batch = pre.do_batch = a->o_batch;
+    pre.o_row = a->o_row;
+    pre.o_head = a->o_head;
+    pre.o_batch = a->o_batch;
     pre.B = a->batch;
     pre.H = a->heads;
     pre.Sq = a->seq_q;
     pre.Sq_pad = sq_pad;
     {
-        const int64_t threads = stats * 32;
-        fmha_bwd_pre_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(pre);
+        fmha_bwd_pre_kernel<<<static_cast<unsigned>(stats / kPreRows), 8 * kPreRows, 0, stream>>>(pre);
         FU_CUDA_OK(cudaGetLastError());
     }
     if (deterministic) {

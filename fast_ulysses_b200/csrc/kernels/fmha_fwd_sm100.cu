@@ -8,12 +8,23 @@
 //   warps 2, 3   idle (they fill warpgroup 0 so that register counts can be set per warpgroup:
 //                warpgroup 0 gives registers away, the softmax warpgroups take them)
 //   warps 4..7   softmax for query tile 0, warps 8..11 for query tile 1: one thread per row;
-//                exp2 with a lazily updated reference maximum, P written back over S in tensor
-//                memory as packed bf16, O rescaled in tensor memory only when the maximum grew by
-//                more than 2^8; final normalisation, bf16 store and log-sum-exp
+//                exponentials against a loose reference, P written back over S in tensor memory as
+//                packed bf16, O rescaled in tensor memory only when a row leaves the reference's range;
+//                final normalisation, bf16 store and log-sum-exp
 // Tensor memory (512 columns): S0 | S1 | O0 | O1, 128 fp32 columns each; P_t aliases S_t.
 // The two query tiles are staggered (QK of tile 0 for step j+1 is issued between the two PV of
 // step j), so each softmax has two MMA slots of cover.
+//
+// What bounds it: a tile's scores, softmax, P V and next scores form one chain through the columns S_t and
+// P_t share, and two tiles are all that fit. The chain is about 2850 clocks per 128 kv rows (SM clock,
+// zeros, no power limit): 100 to load the first scores, 96 exponentials per thread, their hand-over, the
+// last 32 under most of P V, then 2 + 8 MMAs (640) and two barrier wake-ups (300). The exponentials take
+// 9 - 12 clocks each on the special-function unit, whose floor for both tiles is 2050 per step; an
+// eighth of them on the FMA pipe is the best split with random operands at the power limit (16384 tokens
+// x 10 heads: 1.229 ms, 1.244 with none, 1.242 with a quarter, which is the fastest with zeros: 0.965
+// against 0.979 and 1.005). No maximum is taken in an ordinary step (1.253 and 1.010 before). Tried and slower: half steps of 64 kv rows with two score
+// buffers per tile (1.17 ms), two threads per row (1.03), an issuing warp per tile (1.40: the tiles then
+// run in step and contend).
 //
 // q, k, v, o use the (batch, seq, heads, 128) layout of the all-to-all windows, so attention reads
 // what the fused QKV kernel scattered and writes what the output projection pulls, with no copy.
@@ -26,6 +37,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 namespace {
 
@@ -42,8 +54,8 @@ constexpr int SMEM_BYTES = (QT + 2 * KV_STAGES) * TILE_BYTES + 1024;
 constexpr int THREADS    = 32 * 12;            // three warpgroups: {producer, MMA, 2 idle}, softmax 0, softmax 1
 constexpr int REGS_SMALL = 104;                 // warpgroup 0 after it has given registers away
 constexpr int REGS_SOFTMAX = 200;              // per scheduler: 32 x (104 + 2 x 200) = 16128 of 16384 registers
-constexpr float RESCALE_THRESHOLD = 8.0f;     // in log2 units
-constexpr int   kPolyPairs = 0;               // of every 16 exponential pairs, on the FMA pipe by default
+constexpr float RANGE = 32.0f;                // in log2 units
+constexpr int   kPolyPairs = 2;               // of every 16 exponential pairs, on the FMA pipe by default
 
 enum : uint32_t { ERR_LOAD = 11, ERR_MMA = 12, ERR_SOFTMAX = 13 };
 
@@ -73,37 +85,47 @@ struct Barriers {
 };
 
 // exp2 of a pair on the FMA pipe instead of the special-function unit: floor by a round-down add of
-// 1.5 * 2^23 (the integer part lands in the low mantissa bits), a cubic for 2^fraction (relative
-// error 7.5e-5, far below the bf16 rounding of P that follows), and the integer part added to the
-// exponent field. Arguments below -126 are clamped: their exponent field would wrap.
+// 1.5 * 2^23 (the integer part lands in the low mantissa bits), the minimax quintic for 2^fraction on
+// [0, 1) (Remez exchange; relative error 1.5e-7 evaluated in fp32, as good as the special-function
+// unit's), and the integer part added to the exponent field. Arguments below -126 are clamped: their
+// exponent field would wrap.
 __device__ __forceinline__ void ex2_poly2(float& e0, float& e1, float x0, float x1)
 {
     constexpr float MAGIC = 12582912.0f;
-    constexpr float C0 = 0.9999251961708069f, C1 = 0.695833683013916f, C2 = 0.22606723010540009f,
-                    C3 = 0.07802422344684601f;
+    constexpr float C0 = 0.9999999403953552f, C1 = 0.6931530833244324f, C2 = 0.24015361070632935f, C3 = 0.05582631751894951f,
+                    C4 = 0.00898933969438076f, C5 = 0.0018775766948238015f;
     x0 = fmaxf(x0, -126.0f);
     x1 = fmaxf(x1, -126.0f);
     float t0, t1, i0, i1, f0, f1, p0, p1;
     ptx::add2_rm(t0, t1, x0, x1, MAGIC, MAGIC);
     ptx::add2(i0, i1, t0, t1, -MAGIC, -MAGIC);
     ptx::fma2(f0, f1, i0, i1, -1.0f, -1.0f, x0, x1);
-    ptx::fma2(p0, p1, f0, f1, C3, C3, C2, C2);
+    ptx::fma2(p0, p1, f0, f1, C5, C5, C4, C4);
+    ptx::fma2(p0, p1, p0, p1, f0, f1, C3, C3);
+    ptx::fma2(p0, p1, p0, p1, f0, f1, C2, C2);
     ptx::fma2(p0, p1, p0, p1, f0, f1, C1, C1);
     ptx::fma2(p0, p1, p0, p1, f0, f1, C0, C0);
     e0 = __uint_as_float(__float_as_uint(p0) + (__float_as_uint(t0) << 23));
     e1 = __uint_as_float(__float_as_uint(p1) + (__float_as_uint(t1) << 23));
 }
 
-// 32 columns of one row: P = exp2(S * c - m * c) as packed bf16, row sum into l4. NP of every 16
-// pairs take the FMA-pipe path (spread evenly so both pipes stay fed), the rest the special-function unit.
+// Whether pair `i` of 16 takes the FMA-pipe path: NP of them, spread evenly so both pipes stay fed.
 template <int NP>
-__device__ __forceinline__ void exp_chunk(const uint32_t* r, float c, float nmc, float (&l4)[4], uint32_t (&pk)[16])
+__device__ constexpr bool on_fma_pipe(int i)
+{
+    return NP > 0 && (i * NP) % 16 < NP;
+}
+
+// 32 columns of one row: P = exp2(S * c - m * c) as packed bf16, row sum into l4. NP of every 16
+// pairs take the FMA-pipe path, the rest the special-function unit.
+template <int NP>
+__device__ __forceinline__ void exp_chunk(const uint32_t* r, float c, float nmc, float (&l4)[4], uint32_t* pk)
 {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
         float x0, x1, e0, e1;
         ptx::fma2(x0, x1, __uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]), c, c, nmc, nmc);
-        if (NP > 0 && (i * NP) % 16 < NP) {
+        if (on_fma_pipe<NP>(i)) {
             ex2_poly2(e0, e1, x0, x1);
         }
         else {
@@ -248,15 +270,14 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             }
             ptx::mma_commit_if<1>(b_of(bar.s_full[0]) + t * 8, leader);
         };
-        // One half (64 kv rows) of P_t V: the softmax hands P over in two halves so that the
-        // first half's products run under the second half's exponentials.
-        auto issue_pv = [&](int t, uint32_t st, int half, uint32_t accumulate) {
+        // The softmax hands P over in two parts, 96 kv rows and 32, so that most of P_t V runs under the
+        // last exponentials: what is left behind them is on the way to the next step's scores.
+        auto issue_pv = [&](int t, uint32_t st, auto part, uint32_t accumulate) {
             // 16 kv rows = 2048 bytes further down; the two 64-wide halves of d are HALF_BYTES
             // apart (leading byte offset), 8-row groups 1024 bytes apart
             const ptx::Desc va = desc_v.at(st * TILE_BYTES);
 #pragma unroll
-            for (int k4 = 0; k4 < BN / 32; ++k4) {
-                const int kk = half * (BN / 32) + k4;
+            for (int kk = decltype(part)::value ? 6 : 0; kk < (decltype(part)::value ? 8 : 6); ++kk) {
                 ptx::mma_f16_ts_if(tmem + 256 + t * 128, tmem + t * 128 + kk * 8, va.at(kk * 2048), idesc_pv,
                                    accumulate | static_cast<uint32_t>(kk), leader);
             }
@@ -291,7 +312,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                     }
                     stamp<TRACE>(p, it, 20 + t * 6 + 1);
                     ptx::tc_fence_after();
-                    issue_pv(t, stage, 0, static_cast<uint32_t>(j));
+                    issue_pv(t, stage, std::integral_constant<int, 0>{}, static_cast<uint32_t>(j));
                     stamp<TRACE>(p, it, 20 + t * 6 + 2);
                     if (!ptx::mbar_wait_warp(b_of(bar.p_hi[t]), it & 1u)) {
                         ok = false;
@@ -299,7 +320,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                     }
                     stamp<TRACE>(p, it, 20 + t * 6 + 3);
                     ptx::tc_fence_after();
-                    issue_pv(t, stage, 1, 1u);
+                    issue_pv(t, stage, std::integral_constant<int, 1>{}, 1u);
                     if (!more) {
                         ptx::mma_commit_if<1>(b_of(bar.o_final[t]), leader);
                     }
@@ -344,7 +365,15 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             const int h   = (w / p.q_blocks) % p.H;
             const int b   = w / (p.q_blocks * p.H);
             const int row = qb * (QT * BM) + t * BM + row_in;
-            float     m_ref = -INFINITY, l = 0.0f;
+            // Exponentials are taken against a reference that is only roughly the row's maximum: P, O and
+            // the row sum are floating point, so any reference within 2^RANGE of it gives the same relative
+            // precision. It starts at 0 and is moved to a step's maximum when the step's exponentials
+            // leave that range. Whether they do is read off their own sum, so an ordinary step takes no
+            // maximum of the row; only the last quarter, which is handed over later, and the columns on the
+            // FMA pipe, whose exponent field wraps where the special-function unit returns infinity, are
+            // judged by their scores.
+            float m_ref = 0.0f;
+            float l4[4] = {0.f, 0.f, 0.f, 0.f};
 
             for (int j = 0; j < n_kv; ++j, ++scount) {
                 if (!ptx::mbar_wait(&bar.s_full[t], scount & 1u)) {
@@ -355,92 +384,131 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 ptx::tc_fence_after();
                 stamp<TRACE>(p, scount, t * 10 + 0);
                 const int valid = min(BN, p.Skv - j * BN);  // columns of this step that exist
-                // The whole row of S in registers with a single wait: the softmax sits on the
-                // critical path between two MMAs, so its latency matters more than its register use.
+                // The whole row of S in registers; the first quarter is waited for by itself.
                 uint32_t r[BN];
+                ptx::tmem_ld_32x32(ts, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+                ptx::tmem_ld_wait();
 #pragma unroll
-                for (int ch = 0; ch < 4; ++ch) {
+                for (int ch = 1; ch < 4; ++ch) {
                     ptx::tmem_ld_32x32(ts + ch * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[ch * 32]));
                 }
-                ptx::tmem_ld_wait();
                 stamp<TRACE>(p, scount, t * 10 + 1);
-                if (valid < BN) {
+                // The last block of a ragged sequence holds columns that do not exist: they become -inf
+                // (exp2 gives exactly 0) and take the special-function unit only (the FMA-pipe form
+                // clamps instead of returning 0).
+                auto mask = [&](int from) {
 #pragma unroll
-                    for (int i = 0; i < BN; ++i) {
-                        if (i >= valid) {
-                            r[i] = 0xff800000u;  // -inf: exp2 gives exactly 0
+                    for (int i = 0; i < 32; ++i) {
+                        if (from + i >= valid) {
+                            r[from + i] = 0xff800000u;
                         }
                     }
-                }
-                // row maximum with three-input max: 64 instructions in four independent chains
-                float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-#pragma unroll
-                for (int i = 0; i < BN; i += 8) {
-#pragma unroll
-                    for (int u = 0; u < 4; ++u) {
-                        mx4[u] = ptx::max3(mx4[u], __uint_as_float(r[i + 2 * u]), __uint_as_float(r[i + 2 * u + 1]));
-                    }
-                }
-                const float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3]));
-                // lazy reference maximum: rescale only when it grew by more than the threshold
-                const bool grow = (j == 0) || ((mx - m_ref) * c > RESCALE_THRESHOLD);
-                if (__any_sync(0xffffffffu, grow && j != 0)) {
-                    const float alpha = (grow && j != 0) ? ptx::ex2((m_ref - mx) * c) : 1.0f;
-                    l *= alpha;
-#pragma unroll 1
-                    for (int ch = 0; ch < 4; ++ch) {
-                        uint32_t ro[32];
-                        ptx::tmem_ld_32x32(to + ch * 32, ro);
-                        ptx::tmem_ld_wait();
-#pragma unroll
-                        for (int i = 0; i < 32; ++i) {
-                            ro[i] = __float_as_uint(__uint_as_float(ro[i]) * alpha);
-                        }
-                        ptx::tmem_st_32x32(to + ch * 32, ro);
-                    }
-                    ptx::tmem_st_wait();
-                }
-                if (grow) {
-                    m_ref = mx;
-                }
-                stamp<TRACE>(p, scount, t * 10 + 2);
-                const float mc = m_ref * c;
-                // P = exp2(S * c - m_ref * c), written over S as packed bf16
-                const float nmc = -mc;
-                float       l4[4] = {0.f, 0.f, 0.f, 0.f};
-                // The last block of a ragged sequence holds -inf columns: those take the
-                // special-function unit only (the FMA-pipe form clamps instead of returning 0).
-                uint32_t pk[16];
+                };
+                uint32_t pk[48];
+                float    s4[4] = {0.f, 0.f, 0.f, 0.f};
+                float    nmc = -m_ref * c;
+                // P = exp2(S * c - m_ref * c) as packed bf16, three quarters of the row
                 if (valid == BN) {
-                    exp_chunk<NP>(&r[0], c, nmc, l4, pk);
-                    ptx::tmem_st_32x16(ts, pk);
-                    exp_chunk<NP>(&r[32], c, nmc, l4, pk);
-                    ptx::tmem_st_32x16(ts + 16, pk);
-                    // third quarter's exponentials are issued before waiting for the first half's
-                    // stores, so the store latency hides under them
-                    exp_chunk<NP>(&r[64], c, nmc, l4, pk);
+                    exp_chunk<NP>(&r[0], c, nmc, s4, &pk[0]);
+                    ptx::tmem_ld_wait();
+                    exp_chunk<NP>(&r[32], c, nmc, s4, &pk[16]);
+                    exp_chunk<NP>(&r[64], c, nmc, s4, &pk[32]);
                 }
                 else {
-                    exp_chunk<0>(&r[0], c, nmc, l4, pk);
-                    ptx::tmem_st_32x16(ts, pk);
-                    exp_chunk<0>(&r[32], c, nmc, l4, pk);
-                    ptx::tmem_st_32x16(ts + 16, pk);
-                    exp_chunk<0>(&r[64], c, nmc, l4, pk);
+                    mask(0);
+                    exp_chunk<0>(&r[0], c, nmc, s4, &pk[0]);
+                    ptx::tmem_ld_wait();
+                    mask(32);
+                    mask(64);
+                    mask(96);
+                    exp_chunk<0>(&r[32], c, nmc, s4, &pk[16]);
+                    exp_chunk<0>(&r[64], c, nmc, s4, &pk[32]);
+                }
+                float mx2[2] = {-INFINITY, -INFINITY};
+#pragma unroll
+                for (int i = 96; i < BN; i += 4) {
+                    mx2[0] = ptx::max3(mx2[0], __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+                    mx2[1] = ptx::max3(mx2[1], __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+                }
+#pragma unroll
+                for (int i = 0; i < 48; ++i) {
+                    if (on_fma_pipe<NP>(i % 16)) {
+                        mx2[i & 1] = ptx::max3(mx2[i & 1], __uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                    }
+                }
+                const float tail = fmaxf(mx2[0], mx2[1]);
+                const float part = (s4[0] + s4[1]) + (s4[2] + s4[3]);
+                const float last = fmaf(tail, c, nmc);
+                // (written so that a NaN among the scores takes the slow path too and stays one)
+                const bool fine = part < 0x1p32f && last < RANGE && (j != 0 || part > 0x1p-32f);
+                if (__any_sync(0xffffffffu, !fine)) {
+                    // The maximum of the whole row; the first three quarters are still in tensor memory.
+                    float mx = tail;
+#pragma unroll 1
+                    for (int ch = 0; ch < 6; ++ch) {
+                        uint32_t rs[16];
+                        ptx::tmem_ld_32x16(ts + ch * 16, rs);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) {
+                            mx = ch * 16 + i < valid ? fmaxf(mx, __uint_as_float(rs[i])) : mx;
+                        }
+                    }
+                    const float m_new = fine ? m_ref : mx;
+                    if (j != 0) {  // the commit behind S_t also covers the product before it: O is complete
+                        const float alpha = ptx::ex2((m_ref - m_new) * c);
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            l4[u] *= alpha;
+                        }
+#pragma unroll 1
+                        for (int ch = 0; ch < 8; ++ch) {
+                            uint32_t ro[16];
+                            ptx::tmem_ld_32x16(to + ch * 16, ro);
+                            ptx::tmem_ld_wait();
+#pragma unroll
+                            for (int i = 0; i < 16; ++i) {
+                                ro[i] = __float_as_uint(__uint_as_float(ro[i]) * alpha);
+                            }
+                            ptx::tmem_st_32x16(to + ch * 16, ro);
+                        }
+                        ptx::tmem_st_wait();
+                    }
+                    m_ref = m_new;
+                    nmc   = -m_ref * c;
+                    s4[0] = s4[1] = s4[2] = s4[3] = 0.f;
+#pragma unroll
+                    for (int ch = 0; ch < 3; ++ch) {
+                        ptx::tmem_ld_32x32(ts + ch * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[ch * 32]));
+                        ptx::tmem_ld_wait();
+                        if (valid < BN) {
+                            mask(ch * 32);
+                        }
+                        exp_chunk<0>(&r[ch * 32], c, nmc, s4, &pk[ch * 16]);
+                    }
+                }
+                stamp<TRACE>(p, scount, t * 10 + 2);
+                // written over S, of which only the last quarter is still needed and in registers
+#pragma unroll
+                for (int ch = 0; ch < 3; ++ch) {
+                    ptx::tmem_st_32x16(ts + ch * 16, *reinterpret_cast<uint32_t(*)[16]>(&pk[ch * 16]));
+                }
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    l4[u] += s4[u];
                 }
                 stamp<TRACE>(p, scount, t * 10 + 3);
                 ptx::tmem_st_wait();
                 ptx::tc_fence_before();
                 ptx::mbar_arrive_warp(&bar.p_lo[t]);
                 stamp<TRACE>(p, scount, t * 10 + 4);
-                ptx::tmem_st_32x16(ts + 32, pk);
                 if (valid == BN) {
                     exp_chunk<NP>(&r[96], c, nmc, l4, pk);
                 }
                 else {
                     exp_chunk<0>(&r[96], c, nmc, l4, pk);
                 }
-                ptx::tmem_st_32x16(ts + 48, pk);
-                l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
+                ptx::tmem_st_32x16(ts + 48, *reinterpret_cast<uint32_t(*)[16]>(&pk[0]));
                 stamp<TRACE>(p, scount, t * 10 + 5);
                 ptx::tmem_st_wait();
                 ptx::tc_fence_before();
@@ -456,6 +524,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 break;
             }
             ptx::tc_fence_after();
+            const float    l      = (l4[0] + l4[1]) + (l4[2] + l4[3]);
             const float    inv    = 1.0f / l;
             const bool     row_ok = row < p.Sq;
             __nv_bfloat16* dst    = p.o + b * p.o_batch + static_cast<int64_t>(row) * p.o_row + h * p.o_head;

@@ -1,0 +1,61 @@
+"""The forward's exponentials are taken against a loose reference that moves only when a row's scores leave
+its range: scores that leave it in any quarter of a kv step, in the first step or later, upwards or (in
+the first step) downwards, by a little or by hundreds of powers of two, for some rows of a warp or all."""
+
+import pytest
+import torch
+
+from fast_ulysses_b200.ops import attention, gemm
+
+pytestmark = pytest.mark.gpu
+
+
+def run(q, k, v):
+    o, lse = attention.fmha_fwd(q, k, v)
+    gemm.check_errors()
+    o_ref, lse_ref = attention.attention_reference(q, k, v)
+    # P and o are rounded to bf16: 2^-9 each
+    assert ((o.float() - o_ref).norm() / o_ref.norm()).item() < 1e-2
+    # the dominant scores are sums of 128 products in fp32, in another order (|q| |k| bounds the terms)
+    terms = q.float().norm(dim=-1).max() * k.float().norm(dim=-1).max() / 128 ** 0.5
+    bound = 1e-3 + 2.0 ** -20 * lse_ref.abs() + 128 * 2.0 ** -24 * terms
+    assert torch.all((lse - lse_ref).abs() <= bound), (lse - lse_ref).abs().max().item()
+
+
+@pytest.fixture(autouse=True)
+def fp32_oracle():
+    before = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
+    yield
+    torch.backends.cuda.matmul.allow_tf32 = before
+
+
+@pytest.mark.parametrize("where", [0, 40, 70, 100, 127, 128 + 5, 128 + 120, 300])
+@pytest.mark.parametrize("size", [3.0, 12.0, 60.0])
+@pytest.mark.parametrize("rows", ["all", "some"])
+def test_reference_moves_up(where, size, rows):
+    torch.manual_seed(where)
+    q = torch.randn(1, 256, 2, 128, device="cuda").bfloat16()
+    k = torch.randn(1, 333, 2, 128, device="cuda").bfloat16()
+    v = torch.randn(1, 333, 2, 128, device="cuda").bfloat16()
+    hot = q[:, 5] if rows == "some" else q.float().mean(1).bfloat16() * 16
+    k[:, where] = hot * size  # one key that some, or about half, of the queries match very well
+    run(q, k, v)
+
+
+@pytest.mark.parametrize("level", [-40.0, -4.0, 4.0, 40.0])
+def test_reference_of_the_first_step(level):
+    torch.manual_seed(3)
+    q = torch.randn(1, 128, 1, 128, device="cuda").abs().bfloat16()
+    k = (torch.randn(1, 200, 1, 128, device="cuda") * 0.1 + level).bfloat16()  # every score far from zero, all alike
+    v = torch.randn(1, 200, 1, 128, device="cuda").bfloat16()
+    run(q, k, v)
+
+
+def test_first_step_far_below_a_later_one():
+    torch.manual_seed(4)
+    q = torch.randn(1, 128, 1, 128, device="cuda").abs().bfloat16()
+    k = torch.full((1, 512, 1, 128), -30.0, device="cuda").bfloat16()
+    k[:, 384:] = (torch.randn(1, 128, 1, 128, device="cuda") + 30.0).bfloat16()
+    v = torch.randn(1, 512, 1, 128, device="cuda").bfloat16()
+    run(q, k, v)
