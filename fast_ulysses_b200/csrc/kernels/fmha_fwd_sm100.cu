@@ -19,10 +19,10 @@
 // P_t share, and two tiles are all that fit. The chain is about 2850 clocks per 128 kv rows (SM clock,
 // zeros, no power limit): 100 to load the first scores, 96 exponentials per thread, their hand-over, the
 // last 32 under most of P V, then 2 + 8 MMAs (640) and two barrier wake-ups (300). The exponentials take
-// 9 - 12 clocks each on the special-function unit, whose floor for both tiles is 2050 per step; an
-// eighth of them on the FMA pipe is the best split with random operands at the power limit (16384 tokens
-// x 10 heads: 1.229 ms, 1.244 with none, 1.242 with a quarter, which is the fastest with zeros: 0.965
-// against 0.979 and 1.005). No maximum is taken in an ordinary step (1.253 and 1.010 before). Tried and slower: half steps of 64 kv rows with two score
+// 9 - 12 clocks each on the special-function unit, whose floor for both tiles is 2050 per step; a quarter
+// of them on the FMA pipe is the best split (16384 tokens x 10 heads: 1.187 ms with random operands at the
+// power limit and 0.948 with zeros, 1.201 and 0.992 with none, 1.277 and 1.056 with three eighths). No
+// maximum is taken in an ordinary step (1.253 and 1.010 with one, and with O written row by row). Tried and slower: half steps of 64 kv rows with two score
 // buffers per tile (1.17 ms), two threads per row (1.03), an issuing warp per tile (1.40: the tiles then
 // run in step and contend).
 //
@@ -50,12 +50,13 @@ constexpr int BN        = 128;  // kv rows per step
 constexpr int KV_STAGES = 2;
 constexpr int TILE_BYTES = 128 * D * 2;       // 32 KiB: a 128 x 128 bf16 tile as two 64-column halves
 constexpr int HALF_BYTES = TILE_BYTES / 2;
-constexpr int SMEM_BYTES = (QT + 2 * KV_STAGES) * TILE_BYTES + 1024;
+constexpr int OUT_BYTES  = 32 * 128;          // per softmax warp: 32 rows x 64 columns of the result
+constexpr int SMEM_BYTES = (QT + 2 * KV_STAGES) * TILE_BYTES + 8 * OUT_BYTES + 1024;
 constexpr int THREADS    = 32 * 12;            // three warpgroups: {producer, MMA, 2 idle}, softmax 0, softmax 1
 constexpr int REGS_SMALL = 104;                 // warpgroup 0 after it has given registers away
 constexpr int REGS_SOFTMAX = 200;              // per scheduler: 32 x (104 + 2 x 200) = 16128 of 16384 registers
 constexpr float RANGE = 32.0f;                // in log2 units
-constexpr int   kPolyPairs = 2;               // of every 16 exponential pairs, on the FMA pipe by default
+constexpr int   kPolyPairs = 4;               // of every 16 exponential pairs, on the FMA pipe by default
 
 enum : uint32_t { ERR_LOAD = 11, ERR_MMA = 12, ERR_SOFTMAX = 13 };
 
@@ -527,30 +528,51 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             const float    l      = (l4[0] + l4[1]) + (l4[2] + l4[3]);
             const float    inv    = 1.0f / l;
             const bool     row_ok = row < p.Sq;
-            __nv_bfloat16* dst    = p.o + b * p.o_batch + static_cast<int64_t>(row) * p.o_row + h * p.o_head;
+            // A thread has a row; written straight out, every store instruction would touch 32 lines (3700
+            // clocks for the CTA's tile). Through shared memory eight lanes write 128 bytes of one row.
+            const uint32_t stage = sv_addr + KV_STAGES * TILE_BYTES + (warp - 4) * OUT_BYTES;
+            const int      row_w = row - lane;  // first row of this warp
+            __nv_bfloat16* dst   = p.o + b * p.o_batch + static_cast<int64_t>(row_w + (lane >> 3)) * p.o_row + h * p.o_head
+                                 + (lane & 7) * 8;
 #pragma unroll 1
-            for (int ch = 0; ch < 4; ++ch) {
-                uint32_t r[32];
-                ptx::tmem_ld_32x32(to + ch * 32, r);
-                ptx::tmem_ld_wait();
-                if (row_ok) {
-                    uint32_t pk[16];
+            for (int half = 0; half < 2; ++half) {
 #pragma unroll
-                    for (int i = 0; i < 16; ++i) {
-                        pk[i] = ptx::pack_bf16x2(__uint_as_float(r[2 * i]) * inv, __uint_as_float(r[2 * i + 1]) * inv);
+                for (int ch = 0; ch < 2; ++ch) {
+                    uint32_t r[32];
+                    ptx::tmem_ld_32x32(to + half * 64 + ch * 32, r);
+                    ptx::tmem_ld_wait();
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        uint32_t pk[4];
+#pragma unroll
+                        for (int i = 0; i < 4; ++i) {
+                            pk[i] = ptx::pack_bf16x2(__uint_as_float(r[8 * g + 2 * i]) * inv, __uint_as_float(r[8 * g + 2 * i + 1]) * inv);
+                        }
+                        ptx::st_shared_v4(stage + lane * 128 + (((ch * 4 + g) ^ (lane & 7)) << 4), make_uint4(pk[0], pk[1], pk[2], pk[3]));
                     }
-                    uint4* out = reinterpret_cast<uint4*>(dst + ch * 32);
+                }
+                if (half == 1) {  // O is in registers or on its way out: the next item's first product may overwrite it
+                    ptx::tc_fence_before();
+                    ptx::mbar_arrive_warp(&bar.o_free[t]);
+                }
+                __syncwarp();
+                uint4 v[8];
 #pragma unroll
-                    for (int q4 = 0; q4 < 4; ++q4) {
-                        out[q4] = make_uint4(pk[4 * q4], pk[4 * q4 + 1], pk[4 * q4 + 2], pk[4 * q4 + 3]);
+                for (int i = 0; i < 8; ++i) {
+                    const int r = i * 4 + (lane >> 3);
+                    v[i]        = ptx::ld_shared_v4(stage + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+                }
+                __syncwarp();
+#pragma unroll
+                for (int i = 0; i < 8; ++i) {
+                    if (row_w + i * 4 + (lane >> 3) < p.Sq) {
+                        ptx::st_v4(dst + half * 64 + i * 4 * p.o_row, v[i]);
                     }
                 }
             }
             if (row_ok && p.lse) {
                 p.lse[(static_cast<int64_t>(b) * p.H + h) * p.Sq + row] = (m_ref * c + ptx::lg2(l)) * 0.6931471805599453f;
             }
-            ptx::tc_fence_before();
-            ptx::mbar_arrive_warp(&bar.o_free[t]);
         }
     }
 

@@ -61,17 +61,17 @@ struct PlainEpi {
     __device__ void open(int) {}
     __device__ void close(int) {}
 
-    __device__ __forceinline__ static void pack_row(const float (&v)[64], uint8_t* stage, int lane)
+    __device__ __forceinline__ static void pack_row(const float (&v)[64], uint32_t stage, int lane)
     {
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
-            *stage_unit(stage, lane, g) = make_uint4(pack_bf16(v[8 * g], v[8 * g + 1]), pack_bf16(v[8 * g + 2], v[8 * g + 3]),
-                                                     pack_bf16(v[8 * g + 4], v[8 * g + 5]), pack_bf16(v[8 * g + 6], v[8 * g + 7]));
+            ptx::st_shared_v4(stage_unit(stage, lane, g), make_uint4(pack_bf16(v[8 * g], v[8 * g + 1]), pack_bf16(v[8 * g + 2], v[8 * g + 3]),
+                                                                     pack_bf16(v[8 * g + 4], v[8 * g + 5]), pack_bf16(v[8 * g + 6], v[8 * g + 7])));
         }
     }
 
     template <int H>
-    __device__ __forceinline__ void half(const uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage) const
+    __device__ __forceinline__ void half(const uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage) const
     {
         float v[64];
 #pragma unroll
@@ -79,7 +79,8 @@ struct PlainEpi {
             v[j] = __uint_as_float(r[H * 64 + j]);
         }
         if (bias) {
-            if (col0 + 64 <= N && !bias_bf16) {
+            const bool whole = col0 + 64 <= N && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;  // uniform
+            if (whole && !bias_bf16) {
                 const float4* b = reinterpret_cast<const float4*>(static_cast<const float*>(bias) + col0);
 #pragma unroll
                 for (int j = 0; j < 16; ++j) {
@@ -87,7 +88,7 @@ struct PlainEpi {
                     v[4 * j] += f.x, v[4 * j + 1] += f.y, v[4 * j + 2] += f.z, v[4 * j + 3] += f.w;
                 }
             }
-            else if (col0 + 64 <= N) {
+            else if (whole) {
                 const uint4* b = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(bias) + col0);
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
@@ -124,7 +125,7 @@ struct PlainEpi {
             stage_in(stage, aux, ldc, row0, col0, M, N, lane);
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
-                const uint4           q = *stage_unit(stage, lane, g);
+                const uint4           q = ptx::ld_shared_v4(stage_unit(stage, lane, g));
                 const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -138,7 +139,7 @@ struct PlainEpi {
             stage_in(stage, residual, ldc, row0, col0, M, N, lane);
 #pragma unroll
             for (int g = 0; g < 8; ++g) {
-                const uint4           q = *stage_unit(stage, lane, g);
+                const uint4           q = ptx::ld_shared_v4(stage_unit(stage, lane, g));
                 const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -152,7 +153,7 @@ struct PlainEpi {
         stage_out(stage, c, ldc, row0, col0, M, N, lane);
     }
 
-    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage) const
+    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage) const
     {
         if (row0 >= M || col0 >= N) {
             return;  // warp-uniform
@@ -202,6 +203,7 @@ struct QkvParams {
     uint8_t       heads_of[FU_MAX_WORLD];
     int           handshake;
     int           n_types, n_normed;
+    int           tables_aligned;  // rope and both gammas to 16 bytes
     __nv_bfloat16* y_save;
     int64_t       ld_y;
 };
@@ -256,23 +258,32 @@ struct QkvEpi {
         }
     }
 
+    // Four neighbours of a table that the caller need not have aligned to more than its elements.
+    __device__ __forceinline__ float4 load4(const float* p) const
+    {
+        if (this->p.tables_aligned) {
+            return __ldg(reinterpret_cast<const float4*>(p));
+        }
+        return make_float4(p[0], p[1], p[2], p[3]);
+    }
+
     // 64 columns of a head: rotate (NORMED), round, and store each row's 128 bytes to its owner. The
     // staging buffer makes every store instruction write whole 128-byte lines: written straight from
     // the accumulator layout (a lane is a row) each would scatter 32 separate 16-byte pieces, which
     // NVLink carries at a fraction of its rate.
     template <int H, bool NORMED>
     __device__ __forceinline__ void half(const uint32_t (&r)[128], float scale, const float* gamma, const float2* cs,
-                                         unsigned long long my_dst, int lane, uint8_t* stage) const
+                                         unsigned long long my_dst, int lane, uint32_t stage) const
     {
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
             uint32_t o[4];
             if (NORMED) {
-                const float4 g0 = __ldg(reinterpret_cast<const float4*>(gamma + H * 64 + g * 8));
-                const float4 g1 = __ldg(reinterpret_cast<const float4*>(gamma + H * 64 + g * 8 + 4));
+                const float4 g0 = load4(gamma + H * 64 + g * 8);
+                const float4 g1 = load4(gamma + H * 64 + g * 8 + 4);
                 const float  gm[8] = {g0.x, g0.y, g0.z, g0.w, g1.x, g1.y, g1.z, g1.w};
-                const float4 t0 = __ldg(reinterpret_cast<const float4*>(cs + H * 32 + g * 4));
-                const float4 t1 = __ldg(reinterpret_cast<const float4*>(cs + H * 32 + g * 4 + 2));
+                const float4 t0 = load4(&cs[H * 32 + g * 4].x);
+                const float4 t1 = load4(&cs[H * 32 + g * 4 + 2].x);
                 const float  cc[4] = {t0.x, t0.z, t1.x, t1.z}, sn[4] = {t0.y, t0.w, t1.y, t1.w};
 #pragma unroll
                 for (int k = 0; k < 4; ++k) {
@@ -287,23 +298,28 @@ struct QkvEpi {
                     o[k] = pack_bf16(__uint_as_float(r[H * 64 + g * 8 + 2 * k]), __uint_as_float(r[H * 64 + g * 8 + 2 * k + 1]));
                 }
             }
-            *stage_unit(stage, lane, g) = make_uint4(o[0], o[1], o[2], o[3]);
+            ptx::st_shared_v4(stage_unit(stage, lane, g), make_uint4(o[0], o[1], o[2], o[3]));
         }
         __syncwarp();
+        uint4              v[8];
+        unsigned long long to[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-            const int                from = i * 4 + (lane >> 3);
-            const unsigned long long to   = __shfl_sync(0xffffffffu, my_dst, from);
-            const uint4              v    = *stage_unit(stage, from, lane & 7);
-            if (to) {
-                ptx::st_v4(reinterpret_cast<uint4*>(to) + H * 8 + (lane & 7), v);
+            const int from = i * 4 + (lane >> 3);
+            v[i]           = ptx::ld_shared_v4(stage_unit(stage, from, lane & 7));
+            to[i]          = __shfl_sync(0xffffffffu, my_dst, from);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (to[i]) {
+                ptx::st_v4(reinterpret_cast<uint4*>(to[i]) + H * 8 + (lane & 7), v[i]);
             }
         }
         __syncwarp();  // the buffer may be refilled
     }
 
     template <int H>
-    __device__ __forceinline__ void save(const uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage) const
+    __device__ __forceinline__ void save(const uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage) const
     {
 #pragma unroll
         for (int g = 0; g < 8; ++g) {
@@ -312,12 +328,12 @@ struct QkvEpi {
             for (int k = 0; k < 4; ++k) {
                 o[k] = pack_bf16(__uint_as_float(r[H * 64 + g * 8 + 2 * k]), __uint_as_float(r[H * 64 + g * 8 + 2 * k + 1]));
             }
-            *stage_unit(stage, lane, g) = make_uint4(o[0], o[1], o[2], o[3]);
+            ptx::st_shared_v4(stage_unit(stage, lane, g), make_uint4(o[0], o[1], o[2], o[3]));
         }
         stage_out(stage, p.y_save, p.ld_y, row0, col0 + H * 64, p.M, 0x7fffffff, lane);
     }
 
-    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage) const
+    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage) const
     {
         const int head_global = col0 / HEAD_DIM;
         const int type        = head_global / p.heads;  // 0 q, 1 k, 2 v
@@ -679,8 +695,8 @@ int pair_capacity()
 // Which core and tile a problem gets, from its size alone: the one whose estimated time is lowest. The
 // estimate is a start-and-end time plus, per wave of CTAs, a time per 64-wide K-block, both measured
 // (us, SM clock 1.9 GHz, problems of 64 - 2048 rows and 256 - 5120 columns and K):
-//   128 x 128 tiles on single CTAs   5 + 0.225 per K-block and wave of 148
-//   256 x 256 blocks on pairs        8 + 0.305 per K-block and block of each wave of 74 (a whole tile is two
+//   128 x 128 tiles on single CTAs   3.2 + 0.225 per K-block and wave of 148
+//   256 x 256 blocks on pairs        6 + 0.305 per K-block and block of each wave of 74 (a whole tile is two
 //                                    blocks; a block by itself takes 1.05)
 // Of the two wide orientations, which move the same bytes, the one with the fuller last wave wins; when at
 // most half as many tiles as pairs are left over, those are split into blocks.
@@ -718,7 +734,7 @@ Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int fla
         return wide;
     }
     const double kb = static_cast<double>((k + BK - 1) / BK);
-    return 5.0 + 0.225 * kb * ((t128 + sms - 1) / sms) < 8.0 + 0.305 * kb * wide_cost(wide, pairs) ? small : wide;
+    return 3.2 + 0.225 * kb * ((t128 + sms - 1) / sms) < 6.0 + 0.305 * kb * wide_cost(wide, pairs) ? small : wide;
 }
 
 int fill_core(Core& core, const void* a, const void* b, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb, uint32_t* err)
@@ -995,6 +1011,8 @@ extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream_v)
     e.rope             = reinterpret_cast<const float2*>(q->rope);
     e.gamma_q          = q->gamma_q;
     e.gamma_k          = q->gamma_k;
+    e.tables_aligned   = ((reinterpret_cast<uintptr_t>(q->rope) | reinterpret_cast<uintptr_t>(q->gamma_q)
+                         | reinterpret_cast<uintptr_t>(q->gamma_k)) & 15u) == 0;
     e.eps              = q->eps;
     e.M                = a.core.M;
     e.heads            = q->heads;

@@ -221,8 +221,8 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src, Aux aux
 // soon as the registers are loaded, before any arithmetic or store. Epi requirements:
 //   static constexpr bool kPeers          whether open() / close() run (kernels that touch peers)
 //   void open(int epi_tid), close(int epi_tid)          all epilogue threads, once before / after the tiles
-//   void unit(uint32_t (&r)[128], int row0, int col0, int lane, uint8_t* stage)
-// `stage` is 4 KiB of shared memory of this warp's own (32 rows x 128 bytes).
+//   void unit(uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage)
+// `stage` is the address of 4 KiB of shared memory of this warp's own (32 rows x 128 bytes).
 constexpr int UNIT_STAGE_BYTES = 32 * 128;
 
 __device__ __forceinline__ void load_unit(uint32_t taddr, uint32_t (&r)[128])
@@ -522,7 +522,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
         const int epi_warp = warp - WIDE_FIRST_EPI;
         const int quarter  = warp & 3;        // the TMEM lane quarter this warp may access
         const int cg       = epi_warp >> 2;   // which 128 of a block's 256 columns
-        uint8_t*  stage    = ring + WIDE_STAGES * WIDE_STAGE_BYTES + epi_warp * UNIT_STAGE_BYTES;
+        const uint32_t stage = base + WIDE_STAGES * WIDE_STAGE_BYTES + epi_warp * UNIT_STAGE_BYTES;
         if (Epi::kPeers) {
             epi.open(threadIdx.x - 32 * WIDE_FIRST_EPI);
         }
@@ -694,7 +694,7 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
     else {
         const int epi_warp = warp - 2;
         const int quarter  = warp & 3;
-        uint8_t*  stage    = ring + SMALL_STAGES * SMALL_STAGE_BYTES + epi_warp * UNIT_STAGE_BYTES;
+        const uint32_t stage = base + SMALL_STAGES * SMALL_STAGE_BYTES + epi_warp * UNIT_STAGE_BYTES;
         if (Epi::kPeers) {
             epi.open(threadIdx.x - 64);
         }
@@ -732,69 +732,94 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
 // ---- a unit's 64-column halves through the staging buffer ----------------------------------------------------
 // A thread holds a row, so its global accesses would be 32 scattered pieces per instruction. They go
 // through the warp's staging buffer instead: eight lanes move the 128 bytes of one row, four rows per
-// instruction. 16-byte units are XOR-swizzled by the row: neither side has bank conflicts.
-__device__ __forceinline__ uint4* stage_unit(uint8_t* stage, int row, int unit)
+// instruction. 16-byte units are XOR-swizzled by the row: neither side has bank conflicts. All eight
+// accesses of a lane are in flight together: with each store waiting for its load, writing a unit out took
+// 3700 clocks, most of a small GEMM's time.
+__device__ __forceinline__ uint32_t stage_unit(uint32_t stage, int row, int unit)
 {
-    return reinterpret_cast<uint4*>(stage + row * 128 + ((unit ^ (row & 7)) << 4));
+    return stage + row * 128 + ((unit ^ (row & 7)) << 4);
 }
 
 // 32 rows x 64 columns of a bf16 matrix into the staging buffer; what lies outside reads as zero.
-__device__ __forceinline__ void stage_in(uint8_t* stage, const __nv_bfloat16* src, int64_t ld, int row0, int col0, int M, int N,
+__device__ __forceinline__ void stage_in(uint32_t stage, const __nv_bfloat16* src, int64_t ld, int row0, int col0, int M, int N,
                                          int lane)
 {
     const int unit = lane & 7, col = col0 + unit * 8;
     uint4     v[8];
+    if (row0 + 32 <= M && col0 + 64 <= N) {  // warp-uniform
+        const __nv_bfloat16* p = src + static_cast<int64_t>(row0 + (lane >> 3)) * ld + col;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int row = row0 + i * 4 + (lane >> 3);
-        v[i]          = make_uint4(0u, 0u, 0u, 0u);
-        if (row < M) {
-            const __nv_bfloat16* p = src + static_cast<int64_t>(row) * ld + col;
-            if (col + 8 <= N) {
-                v[i] = *reinterpret_cast<const uint4*>(p);
-            }
-            else if (col < N) {
-                __nv_bfloat16 e[8] = {};
-                for (int j = 0; j < N - col; ++j) {
-                    e[j] = p[j];
+        for (int i = 0; i < 8; ++i) {
+            v[i] = *reinterpret_cast<const uint4*>(p + i * 4 * ld);
+        }
+    }
+    else {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int row = row0 + i * 4 + (lane >> 3);
+            v[i]          = make_uint4(0u, 0u, 0u, 0u);
+            if (row < M) {
+                const __nv_bfloat16* p = src + static_cast<int64_t>(row) * ld + col;
+                if (col + 8 <= N) {
+                    v[i] = *reinterpret_cast<const uint4*>(p);
                 }
-                v[i] = *reinterpret_cast<const uint4*>(e);
+                else if (col < N) {
+                    __nv_bfloat16 e[8] = {};
+                    for (int j = 0; j < N - col; ++j) {
+                        e[j] = p[j];
+                    }
+                    v[i] = *reinterpret_cast<const uint4*>(e);
+                }
             }
         }
     }
     __syncwarp();  // the buffer's previous contents have been read
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        *stage_unit(stage, i * 4 + (lane >> 3), unit) = v[i];
+        ptx::st_shared_v4(stage_unit(stage, i * 4 + (lane >> 3), unit), v[i]);
     }
     __syncwarp();
 }
 
 // The rows of the staging buffer to a bf16 matrix. The caller's threads have each written their row.
-__device__ __forceinline__ void stage_out(uint8_t* stage, __nv_bfloat16* dst, int64_t ld, int row0, int col0, int M, int N,
+__device__ __forceinline__ void stage_out(uint32_t stage, __nv_bfloat16* dst, int64_t ld, int row0, int col0, int M, int N,
                                           int lane)
 {
     const int unit = lane & 7, col = col0 + unit * 8;
+    uint4     v[8];
     __syncwarp();
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-        const int   r   = i * 4 + (lane >> 3);
-        const int   row = row0 + r;
-        const uint4 v   = *stage_unit(stage, r, unit);
+        v[i] = ptx::ld_shared_v4(stage_unit(stage, i * 4 + (lane >> 3), unit));
+    }
+    __syncwarp();  // the buffer may be refilled
+    if (row0 + 32 <= M && col0 + 64 <= N) {  // warp-uniform
+        __nv_bfloat16* p = dst + static_cast<int64_t>(row0 + (lane >> 3)) * ld + col;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            ptx::st_v4(p + i * 4 * ld, v[i]);
+        }
+        return;
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const int row = row0 + i * 4 + (lane >> 3);
         if (row < M) {
             __nv_bfloat16* p = dst + static_cast<int64_t>(row) * ld + col;
             if (col + 8 <= N) {
-                *reinterpret_cast<uint4*>(p) = v;
+                ptx::st_v4(p, v[i]);
             }
             else if (col < N) {
-                const __nv_bfloat16* e = reinterpret_cast<const __nv_bfloat16*>(&v);
-                for (int j = 0; j < N - col; ++j) {
-                    p[j] = e[j];
+                const uint32_t w[4] = {v[i].x, v[i].y, v[i].z, v[i].w};
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                    if (j < N - col) {
+                        p[j] = __ushort_as_bfloat16(static_cast<unsigned short>(w[j >> 1] >> (16 * (j & 1))));
+                    }
                 }
             }
         }
     }
-    __syncwarp();  // the buffer may be refilled
 }
 
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi)
