@@ -37,6 +37,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <mutex>
 #include <type_traits>
 
 namespace {
@@ -67,6 +68,7 @@ struct Params {
     int64_t        o_row, o_head, o_batch;  // element strides of o
     int            B, H, Sq, Skv;
     int            q_blocks, total_work, n_kv;
+    int            first;       // split kernel: the item of cluster 0
     float          scale, scale_log2;
     uint32_t*      err;
     uint64_t*      trace;
@@ -149,7 +151,128 @@ __device__ __forceinline__ void stamp(const Params& p, uint32_t step, int ev)
     }
 }
 
-template <int NP, bool TRACE>
+// The end of an item whose kv tiles were shared by the CTAs of a cluster: every CTA holds an unnormalised
+// O (256 x 128 in tensor memory), and for each row its reference and sum. The result is cut into eight
+// units of one query tile x 32 columns, dealt to the CTAs in order; each sends the others' units of its O
+// through distributed shared memory, so all of them send, receive and write at once, and the sum over
+// the shares runs in their order. The operand tiles are done with by then: units received lie at
+// their place, 16 KiB each, the (reference, sum) pairs behind them. Executed by the softmax warps; the
+// other warps take part in the two cluster barriers.
+constexpr int UNITS       = 8;
+constexpr int UNIT_BYTES  = BM * 128;         // 128 rows x 32 fp32
+constexpr int PAIRS_OFF   = 160 * 1024;       // (cluster size - 1) x units of a CTA <= 10 for 2..6 and 8 CTAs
+static_assert(PAIRS_OFF + 8 * QT * BM * 8 <= (QT + 2 * KV_STAGES) * TILE_BYTES, "exchange area");
+
+__device__ __forceinline__ void join_shares(const Params& p, int b, int h, int row, int t, int quarter, int lane, uint32_t to,
+                                            float m_log2, float l, int crank, int csize, uint32_t base, uint32_t stage)
+{
+    ptx::tc_fence_after();
+    const int row_in = quarter * 32 + lane;
+    auto first_unit = [&](int r) { return (r * UNITS + csize - 1) / csize; };  // units [first_unit(r), first_unit(r + 1)) are CTA r's
+    ptx::cluster_sync();  // every CTA's products are complete: its operand tiles may be overwritten
+    for (int r = 0; r < csize; ++r) {
+        ptx::st_cluster_v2f(ptx::cluster_addr(base + PAIRS_OFF + ((crank * QT + t) * BM + row_in) * 8, r), m_log2, l);
+    }
+#pragma unroll 1
+    for (int ch = 0; ch < 4; ++ch) {
+        const int u     = t * 4 + ch;
+        const int owner = u * csize / UNITS;
+        if (owner == crank) {
+            continue;
+        }
+        const int      slot = (crank - (crank > owner ? 1 : 0)) * (first_unit(owner + 1) - first_unit(owner)) + u - first_unit(owner);
+        // through the warp's staging buffer, so that a store instruction writes 512 contiguous bytes of the
+        // other CTA's memory (a row per lane, 32 separate pieces, took three times as long)
+        const uint32_t dst = ptx::cluster_addr(base + slot * UNIT_BYTES + quarter * OUT_BYTES + lane * 16, owner);
+        uint32_t       r[32];
+        ptx::tmem_ld_32x32(to + ch * 32, r);
+        ptx::tmem_ld_wait();
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            ptx::st_shared_v4(stage + lane * 128 + ((g ^ (lane & 7)) << 4), make_uint4(r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]));
+        }
+        __syncwarp();
+        uint4 v[8];
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            v[g] = ptx::ld_shared_v4(stage + g * 512 + lane * 16);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+            ptx::st_cluster_v4(dst + g * 512, v[g].x, v[g].y, v[g].z, v[g].w);
+        }
+    }
+    ptx::cluster_sync();
+    const int first = first_unit(crank), mine = first_unit(crank + 1) - first;
+    if (first + mine <= t * 4 || first >= t * 4 + 4) {
+        return;  // none of this query tile
+    }
+    const uint32_t pairs = base + PAIRS_OFF + (t * BM + row_in) * 8;
+    float          top = -INFINITY, sum = 0.0f;
+    for (int r = 0; r < csize; ++r) {
+        top = fmaxf(top, ptx::ld_shared_v2f(pairs + r * QT * BM * 8).x);
+    }
+    for (int r = 0; r < csize; ++r) {
+        const float2 ml = ptx::ld_shared_v2f(pairs + r * QT * BM * 8);
+        sum += ptx::ex2(ml.x - top) * ml.y;
+    }
+    const float inv   = 1.0f / sum;
+    const int   row_w = row - lane;
+#pragma unroll 1
+    for (int ch = max(0, first - t * 4); ch < min(4, first + mine - t * 4); ++ch) {
+        float acc[32];
+#pragma unroll
+        for (int i = 0; i < 32; ++i) {
+            acc[i] = 0.0f;
+        }
+#pragma unroll 1
+        for (int r = 0; r < csize; ++r) {
+            const float w = ptx::ex2(ptx::ld_shared_v2f(pairs + r * QT * BM * 8).x - top) * inv;
+            if (r == crank) {
+                uint32_t o[32];
+                ptx::tmem_ld_32x32(to + ch * 32, o);
+                ptx::tmem_ld_wait();
+#pragma unroll
+                for (int i = 0; i < 32; ++i) {
+                    acc[i] += __uint_as_float(o[i]) * w;
+                }
+            }
+            else {
+                const uint32_t src = base + ((r - (r > crank ? 1 : 0)) * mine + t * 4 + ch - first) * UNIT_BYTES + row_in * 128;
+#pragma unroll
+                for (int g = 0; g < 8; ++g) {
+                    const uint4 v = ptx::ld_shared_v4(src + ((g ^ (lane & 7)) << 4));
+                    acc[4 * g] += __uint_as_float(v.x) * w;
+                    acc[4 * g + 1] += __uint_as_float(v.y) * w;
+                    acc[4 * g + 2] += __uint_as_float(v.z) * w;
+                    acc[4 * g + 3] += __uint_as_float(v.w) * w;
+                }
+            }
+        }
+        __syncwarp();
+#pragma unroll
+        for (int g = 0; g < 4; ++g) {
+            ptx::st_shared_v4(stage + lane * 128 + ((g ^ (lane & 7)) << 4),
+                              make_uint4(ptx::pack_bf16x2(acc[8 * g], acc[8 * g + 1]), ptx::pack_bf16x2(acc[8 * g + 2], acc[8 * g + 3]),
+                                         ptx::pack_bf16x2(acc[8 * g + 4], acc[8 * g + 5]), ptx::pack_bf16x2(acc[8 * g + 6], acc[8 * g + 7])));
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {  // four lanes per row
+            const int   r = i * 8 + (lane >> 2);
+            const uint4 v = ptx::ld_shared_v4(stage + r * 128 + (((lane & 3) ^ (r & 7)) << 4));
+            if (row_w + r < p.Sq) {
+                ptx::st_v4(p.o + b * p.o_batch + static_cast<int64_t>(row_w + r) * p.o_row + h * p.o_head + ch * 32 + (lane & 3) * 8, v);
+            }
+        }
+        if (ch == 0 && row < p.Sq && p.lse) {
+            p.lse[(static_cast<int64_t>(b) * p.H + h) * p.Sq + row] = (top + ptx::lg2(sum)) * 0.6931471805599453f;
+        }
+    }
+}
+
+template <int NP, bool TRACE, bool SPLIT>
 __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_constant__ Params p)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -194,7 +317,16 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
     __syncthreads();
     ptx::tc_fence_after();
     const uint32_t tmem = ptx::uniform(tmem_holder);
-    const int      n_kv = p.n_kv;
+    // The items of this CTA and the kv tiles of each: every gridDim.x-th item and all of its tiles; or
+    // (SPLIT) one item per cluster, each CTA its share of the tiles.
+    const int crank = SPLIT ? static_cast<int>(ptx::uniform(ptx::cluster_ctarank())) : 0;
+    const int csize = SPLIT ? static_cast<int>(ptx::uniform(ptx::cluster_nctarank())) : 1;
+    const int w_0   = SPLIT ? p.first + static_cast<int>(blockIdx.x) / csize : static_cast<int>(blockIdx.x);
+    const int w_end = SPLIT ? w_0 + 1 : p.total_work;
+    const int w_inc = SPLIT ? 1 : static_cast<int>(gridDim.x);
+    const int share = SPLIT ? (p.n_kv + csize - 1) / csize : p.n_kv;
+    const int j_0   = crank * share;
+    const int n_kv  = SPLIT ? min(share, p.n_kv - j_0) : p.n_kv;
 
     if (warp < 4) {
     ptx::setmaxnreg_dec<REGS_SMALL>();
@@ -205,7 +337,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
         // ---------------------------------------------------------------- producer
         uint32_t stage = 0, phase = 1, wc = 0;
         bool     ok = true;
-        for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
+        for (int w = w_0; w < w_end && ok; w += w_inc, ++wc) {
             const int qb = w % p.q_blocks;
             const int h  = (w / p.q_blocks) % p.H;
             const int b  = w / (p.q_blocks * p.H);
@@ -228,7 +360,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 }
                 ptx::mbar_expect_tx_if(kf, TILE_BYTES, leader);
                 for (int half = 0; half < 2; ++half) {
-                    ptx::tma_load_4d_if(sk_addr + stage * TILE_BYTES + half * HALF_BYTES, &p.map_k, half * 64, j * BN, h, b, kf,
+                    ptx::tma_load_4d_if(sk_addr + stage * TILE_BYTES + half * HALF_BYTES, &p.map_k, half * 64, (j_0 + j) * BN, h, b, kf,
                                         leader);
                 }
                 if (!ptx::mbar_wait_warp(b_of(bar.v_empty[0]) + stage * 8, phase)) {
@@ -237,7 +369,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 }
                 ptx::mbar_expect_tx_if(vf, TILE_BYTES, leader);
                 for (int half = 0; half < 2; ++half) {
-                    ptx::tma_load_4d_if(sv_addr + stage * TILE_BYTES + half * HALF_BYTES, &p.map_v, half * 64, j * BN, h, b, vf,
+                    ptx::tma_load_4d_if(sv_addr + stage * TILE_BYTES + half * HALF_BYTES, &p.map_v, half * 64, (j_0 + j) * BN, h, b, vf,
                                         leader);
                 }
                 if (++stage == KV_STAGES) {
@@ -284,7 +416,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             }
         };
 
-        for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
+        for (int w = w_0; w < w_end && ok; w += w_inc, ++wc) {
             // prologue: S for both query tiles of kv step 0
             if (!ptx::mbar_wait_warp(b_of(bar.q_full), wc & 1u)
                 || !ptx::mbar_wait_warp(b_of(bar.k_full[0]) + stage * 8, phase)) {
@@ -347,6 +479,10 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
         }
         __syncwarp();
     }
+    if (SPLIT) {  // the softmax warps' exchange
+        ptx::cluster_sync();
+        ptx::cluster_sync();
+    }
     }
     else {
         ptx::setmaxnreg_inc<REGS_SOFTMAX>();
@@ -361,7 +497,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
         uint32_t       scount = 0, wc = 0;
         bool           ok = true;
 
-        for (int w = blockIdx.x; w < p.total_work && ok; w += gridDim.x, ++wc) {
+        for (int w = w_0; w < w_end && ok; w += w_inc, ++wc) {
             const int qb  = w % p.q_blocks;
             const int h   = (w / p.q_blocks) % p.H;
             const int b   = w / (p.q_blocks * p.H);
@@ -384,7 +520,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 }
                 ptx::tc_fence_after();
                 stamp<TRACE>(p, scount, t * 10 + 0);
-                const int valid = min(BN, p.Skv - j * BN);  // columns of this step that exist
+                const int valid = min(BN, p.Skv - (j_0 + j) * BN);  // columns of this step that exist
                 // The whole row of S in registers; the first quarter is waited for by itself.
                 uint32_t r[BN];
                 ptx::tmem_ld_32x32(ts, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
@@ -516,6 +652,15 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 ptx::mbar_arrive_warp(&bar.p_hi[t]);
                 stamp<TRACE>(p, scount, t * 10 + 6);
             }
+            if (SPLIT) {
+                ok = ok && ptx::mbar_wait(&bar.o_final[t], wc & 1u);
+                if (!ok) {
+                    flag(p, ERR_SOFTMAX);
+                }
+                join_shares(p, b, h, row, t, quarter, lane, to, m_ref * c, (l4[0] + l4[1]) + (l4[2] + l4[3]), crank, csize, base,
+                            sv_addr + KV_STAGES * TILE_BYTES + (warp - 4) * OUT_BYTES);
+                break;
+            }
             if (!ok) {
                 break;
             }
@@ -583,6 +728,80 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
     }
 }
 
+cudaLaunchAttribute cluster_attr(int csize)
+{
+    cudaLaunchAttribute attr = {};
+    attr.id                  = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x    = static_cast<unsigned>(csize);
+    attr.val.clusterDim.y    = 1;
+    attr.val.clusterDim.z    = 1;
+    return attr;
+}
+
+// How many clusters of `csize` CTAs of the split kernel the device holds at once (a cluster stays inside
+// a GPC); 0 when it cannot be asked. Asked once per device and size.
+int split_capacity(int csize, int dev)
+{
+    static std::mutex lock;
+    static int        cached[64][9] = {};
+    if (dev < 0 || dev >= 64) {
+        return 0;
+    }
+    const std::lock_guard<std::mutex> guard(lock);
+    if (cached[dev][csize] == 0) {
+        auto                kernel = fmha_fwd_kernel<kPolyPairs, false, true>;
+        cudaLaunchConfig_t  cfg    = {};
+        cudaLaunchAttribute attr   = cluster_attr(csize);
+        cfg.gridDim                = dim3(static_cast<unsigned>(csize), 1, 1);
+        cfg.blockDim               = dim3(THREADS, 1, 1);
+        cfg.dynamicSmemBytes       = SMEM_BYTES;
+        cfg.attrs                  = &attr;
+        cfg.numAttrs               = 1;
+        int n                      = 0;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess
+            || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+            (void)cudaGetLastError();
+            n = -1;
+        }
+        cached[dev][csize] = n;
+    }
+    return std::max(0, cached[dev][csize]);
+}
+
+// Items beyond whole waves of one per SM are shared out: each to a cluster whose CTAs take a part of the
+// kv tiles. Times in kv tiles (1.45 us), measured: an item costs 3 beyond its own (launch, first loads,
+// write-out), the exchange of a cluster 4.5 more, a second launch 2. 8191 tokens x 10 heads (320 items on
+// 148 SMs): 304 -> 249 us; 1000 x 10 (40 items): 17.4 -> 15.9.
+struct SplitPlan {
+    int whole, csize;  // items of the plain kernel; cluster size of the rest (1: no split)
+};
+SplitPlan plan_split(int items, int n_kv, int sms, int dev)
+{
+    const int    whole = items / sms * sms, rest = items - whole;
+    SplitPlan    best{items, 1};
+    double       best_cost = static_cast<double>((items + sms - 1) / sms) * (n_kv + 3);
+    if (rest == 0) {
+        return best;
+    }
+    for (const int csize : {2, 3, 4, 5, 6, 8}) {
+        const int share = (n_kv + csize - 1) / csize;
+        if (csize > n_kv || (n_kv + share - 1) / share != csize) {
+            continue;  // a CTA would have nothing to do
+        }
+        const int cap = split_capacity(csize, dev);
+        if (cap < 1) {
+            continue;
+        }
+        const double cost = static_cast<double>(whole / sms) * (n_kv + 3) + static_cast<double>((rest + cap - 1) / cap) * (share + 7.5)
+                            + (whole > 0 ? 2 : 0);
+        if (cost < best_cost) {
+            best      = {whole, csize};
+            best_cost = cost;
+        }
+    }
+    return best;
+}
+
 }  // namespace
 
 extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
@@ -629,8 +848,6 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
     int dev = 0, sms = 0;
     FU_CUDA_OK(cudaGetDevice(&dev));
     FU_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    int grid = a->ctas > 0 ? std::min(a->ctas, sms) : sms;
-    grid     = std::max(1, std::min(grid, p.total_work));
     // how many of every 16 exponential pairs go to the FMA pipe: FU_FMHA_POLY(n) in flags, default kPolyPairs
     const int np = (a->flags & FU_FMHA_POLY_SET) ? ((a->flags >> 8) & 15) : kPolyPairs;
     if (np < 0 || np > 6 || (np & 1)) {
@@ -644,22 +861,48 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
                 configured[dev][np] = true;
             }
         }
+        int grid = a->ctas > 0 ? std::min(a->ctas, sms) : sms;
+        grid     = std::max(1, std::min(grid, p.total_work));
         kernel<<<grid, THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(p);
         FU_CUDA_OK(cudaGetLastError());
         return FU_OK;
     };
     p.trace = a->trace;
     if (a->trace) {
-        if (np != 0) {
+        if (np != kPolyPairs) {
             return fu::fail(FU_E_ARG, "fu_fmha_fwd: the timeline build exists for the default exponential split only");
         }
-        return launch(fmha_fwd_kernel<0, true>);
+        return launch(fmha_fwd_kernel<kPolyPairs, true, false>);
+    }
+    if (np == kPolyPairs && a->ctas <= 0) {
+        const SplitPlan plan = plan_split(p.total_work, p.n_kv, sms, dev);
+        if (plan.csize > 1) {
+            const int items = p.total_work;
+            p.total_work    = plan.whole;
+            if (plan.whole > 0) {
+                rc = launch(fmha_fwd_kernel<kPolyPairs, false, false>);
+                if (rc != FU_OK) {
+                    return rc;
+                }
+            }
+            p.first                   = plan.whole;
+            cudaLaunchConfig_t  cfg   = {};
+            cudaLaunchAttribute attr  = cluster_attr(plan.csize);
+            cfg.gridDim               = dim3(static_cast<unsigned>((items - plan.whole) * plan.csize), 1, 1);
+            cfg.blockDim              = dim3(THREADS, 1, 1);
+            cfg.dynamicSmemBytes      = SMEM_BYTES;
+            cfg.stream                = static_cast<cudaStream_t>(stream);
+            cfg.attrs                 = &attr;
+            cfg.numAttrs              = 1;
+            FU_CUDA_OK(cudaLaunchKernelEx(&cfg, fmha_fwd_kernel<kPolyPairs, false, true>, p));
+            return FU_OK;
+        }
     }
     switch (np) {
-    case 0: return launch(fmha_fwd_kernel<0, false>);
-    case 2: return launch(fmha_fwd_kernel<2, false>);
-    case 4: return launch(fmha_fwd_kernel<4, false>);
-    case 6: return launch(fmha_fwd_kernel<6, false>);
+    case 0: return launch(fmha_fwd_kernel<0, false, false>);
+    case 2: return launch(fmha_fwd_kernel<2, false, false>);
+    case 4: return launch(fmha_fwd_kernel<4, false, false>);
+    case 6: return launch(fmha_fwd_kernel<6, false, false>);
     default: return fu::fail(FU_E_ARG, "fu_fmha_fwd: %d of 16 exponential pairs on the FMA pipe is not built (0, 2, 4, 6)", np);
     }
 }

@@ -59,3 +59,21 @@ def test_first_step_far_below_a_later_one():
     k[:, 384:] = (torch.randn(1, 128, 1, 128, device="cuda") + 30.0).bfloat16()
     v = torch.randn(1, 512, 1, 128, device="cuda").bfloat16()
     run(q, k, v)
+
+
+# 256 query rows are an item; items beyond whole waves of one per SM are shared out to clusters of up to
+# eight CTAs, each with a part of the 128-row kv tiles
+@pytest.mark.parametrize("b,h,sq,skv", [(1, 1, 1, 129), (1, 1, 256, 256), (1, 2, 300, 384), (1, 1, 257, 500), (2, 1, 130, 640),
+                                        (1, 1, 64, 1025), (1, 3, 700, 1111), (1, 1, 256, 8 * 128 + 1), (1, 1, 100, 6000),
+                                        (1, 8, 1000, 1000), (1, 20, 1024, 400), (1, 37, 1000, 300), (2, 19, 1030, 1500)])
+def test_kv_tiles_shared_by_a_cluster(b, h, sq, skv):
+    torch.manual_seed(sq + skv)
+    q = torch.randn(b, sq, h, 128, device="cuda").bfloat16()
+    k = torch.randn(b, skv, h, 128, device="cuda").bfloat16()
+    v = torch.randn(b, skv, h, 128, device="cuda").bfloat16()
+    k[:, skv // 2:] *= 1.5  # the shares see different ranges of scores
+    run(q, k, v)
+    k[:, skv - 1] = q[:, sq // 2] * 20.0  # the last share moves its reference for some rows
+    run(q, k, v)
+    first = attention.fmha_fwd(q, k, v)
+    assert all(torch.equal(x, y) for x, y in zip(first, attention.fmha_fwd(q, k, v)))
