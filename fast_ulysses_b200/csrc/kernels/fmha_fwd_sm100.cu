@@ -29,6 +29,7 @@
 // q, k, v, o use the (batch, seq, heads, 128) layout of the all-to-all windows, so attention reads
 // what the fused QKV kernel scattered and writes what the output projection pulls, with no copy.
 // The reference has no attention kernel (examples/dit_attention.py:57 calls torch SDPA).
+#include "cluster_plan.h"
 #include "fu_kernels.h"
 #include "host_util.h"
 #include "ptx.cuh"
@@ -37,7 +38,6 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
-#include <mutex>
 #include <type_traits>
 
 namespace {
@@ -728,78 +728,14 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
     }
 }
 
-cudaLaunchAttribute cluster_attr(int csize)
+// Items beyond whole waves of one per SM are shared out, see cluster_plan.h. Times in kv tiles (1.45 us).
+// 8191 tokens x 10 heads (320 items on 148 SMs): 304 -> 249 us; 1000 x 10 (40 items): 17.4 -> 15.9.
+fu::ClusterPlan plan_split(int items, int n_kv, int sms, int dev)
 {
-    cudaLaunchAttribute attr = {};
-    attr.id                  = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x    = static_cast<unsigned>(csize);
-    attr.val.clusterDim.y    = 1;
-    attr.val.clusterDim.z    = 1;
-    return attr;
-}
-
-// How many clusters of `csize` CTAs of the split kernel the device holds at once (a cluster stays inside
-// a GPC); 0 when it cannot be asked. Asked once per device and size.
-int split_capacity(int csize, int dev)
-{
-    static std::mutex lock;
-    static int        cached[64][9] = {};
-    if (dev < 0 || dev >= 64) {
-        return 0;
-    }
-    const std::lock_guard<std::mutex> guard(lock);
-    if (cached[dev][csize] == 0) {
-        auto                kernel = fmha_fwd_kernel<kPolyPairs, false, true>;
-        cudaLaunchConfig_t  cfg    = {};
-        cudaLaunchAttribute attr   = cluster_attr(csize);
-        cfg.gridDim                = dim3(static_cast<unsigned>(csize), 1, 1);
-        cfg.blockDim               = dim3(THREADS, 1, 1);
-        cfg.dynamicSmemBytes       = SMEM_BYTES;
-        cfg.attrs                  = &attr;
-        cfg.numAttrs               = 1;
-        int n                      = 0;
-        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) != cudaSuccess
-            || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
-            (void)cudaGetLastError();
-            n = -1;
-        }
-        cached[dev][csize] = n;
-    }
-    return std::max(0, cached[dev][csize]);
-}
-
-// Items beyond whole waves of one per SM are shared out: each to a cluster whose CTAs take a part of the
-// kv tiles. Times in kv tiles (1.45 us), measured: an item costs 3 beyond its own (launch, first loads,
-// write-out), the exchange of a cluster 4.5 more, a second launch 2. 8191 tokens x 10 heads (320 items on
-// 148 SMs): 304 -> 249 us; 1000 x 10 (40 items): 17.4 -> 15.9.
-struct SplitPlan {
-    int whole, csize;  // items of the plain kernel; cluster size of the rest (1: no split)
-};
-SplitPlan plan_split(int items, int n_kv, int sms, int dev)
-{
-    const int    whole = items / sms * sms, rest = items - whole;
-    SplitPlan    best{items, 1};
-    double       best_cost = static_cast<double>((items + sms - 1) / sms) * (n_kv + 3);
-    if (rest == 0) {
-        return best;
-    }
-    for (const int csize : {2, 3, 4, 5, 6, 8}) {
-        const int share = (n_kv + csize - 1) / csize;
-        if (csize > n_kv || (n_kv + share - 1) / share != csize) {
-            continue;  // a CTA would have nothing to do
-        }
-        const int cap = split_capacity(csize, dev);
-        if (cap < 1) {
-            continue;
-        }
-        const double cost = static_cast<double>(whole / sms) * (n_kv + 3) + static_cast<double>((rest + cap - 1) / cap) * (share + 7.5)
-                            + (whole > 0 ? 2 : 0);
-        if (cost < best_cost) {
-            best      = {whole, csize};
-            best_cost = cost;
-        }
-    }
-    return best;
+    static fu::ClusterCapacity capacity;
+    return fu::plan_clusters(items, n_kv, sms, {3.0, 4.5, 2.0}, [&](int csize) {
+        return capacity.of(fmha_fwd_kernel<kPolyPairs, false, true>, csize, dev, THREADS, SMEM_BYTES);
+    });
 }
 
 }  // namespace
@@ -875,7 +811,7 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
         return launch(fmha_fwd_kernel<kPolyPairs, true, false>);
     }
     if (np == kPolyPairs && a->ctas <= 0) {
-        const SplitPlan plan = plan_split(p.total_work, p.n_kv, sms, dev);
+        const fu::ClusterPlan plan = plan_split(p.total_work, p.n_kv, sms, dev);
         if (plan.csize > 1) {
             const int items = p.total_work;
             p.total_work    = plan.whole;
@@ -887,7 +823,7 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
             }
             p.first                   = plan.whole;
             cudaLaunchConfig_t  cfg   = {};
-            cudaLaunchAttribute attr  = cluster_attr(plan.csize);
+            cudaLaunchAttribute attr  = fu::cluster_attr(plan.csize);
             cfg.gridDim               = dim3(static_cast<unsigned>((items - plan.whole) * plan.csize), 1, 1);
             cfg.blockDim              = dim3(THREADS, 1, 1);
             cfg.dynamicSmemBytes      = SMEM_BYTES;

@@ -77,3 +77,29 @@ def test_kv_tiles_shared_by_a_cluster(b, h, sq, skv):
     run(q, k, v)
     first = attention.fmha_fwd(q, k, v)
     assert all(torch.equal(x, y) for x, y in zip(first, attention.fmha_fwd(q, k, v)))
+
+
+# backward: 128 kv rows are an item, and the 128-row query blocks are what a cluster shares
+@pytest.mark.parametrize("b,h,sq,skv", [(1, 1, 256, 40), (1, 1, 1025, 64), (1, 1, 640, 129), (1, 2, 2000, 300), (2, 3, 1111, 700),
+                                        (1, 1, 8 * 128 + 1, 128), (1, 8, 1500, 1000), (1, 20, 1024, 1024), (1, 37, 1500, 600)])
+def test_query_blocks_shared_by_a_cluster(b, h, sq, skv):
+    torch.manual_seed(sq + skv)
+    q = torch.randn(b, sq, h, 128, device="cuda").bfloat16()
+    k = torch.randn(b, skv, h, 128, device="cuda").bfloat16()
+    v = torch.randn(b, skv, h, 128, device="cuda").bfloat16()
+    o, lse = attention.fmha_fwd(q, k, v)
+    d_o = torch.randn_like(o)
+    grads = attention.fmha_bwd(q, k, v, o, lse, d_o)
+    again = attention.fmha_bwd(q, k, v, o, lse, d_o)
+    whole = attention.fmha_bwd(q, k, v, o, lse, d_o, ctas=148)  # an explicit grid shares nothing
+    gemm.check_errors()
+    assert torch.equal(grads[1], again[1]) and torch.equal(grads[2], again[2])
+    qr, kr, vr = (t.float().requires_grad_() for t in (q, k, v))
+    o_ref, _ = attention.attention_reference(qr, kr, vr)
+    o_ref.backward(d_o.float())
+    for name, got, want, plain in zip("qkv", grads, (qr.grad, kr.grad, vr.grad), whole):
+        # P, dS and the gradient are rounded to bf16: 2^-9 each
+        assert ((got.float() - want).norm() / want.norm().clamp_min(1e-6)).item() < 1e-2, name
+        # the same terms, summed in fp32 in another order and rounded once: one step of bf16 apart at most
+        # where the sum is not cancelled, so 2^-9 in the norm with room to spare
+        assert ((got.float() - plain.float()).norm() / plain.float().norm().clamp_min(1e-6)).item() < 2.0 ** -9, name
