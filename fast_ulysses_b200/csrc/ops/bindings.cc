@@ -325,8 +325,9 @@ at::Tensor run_async(Group& g, const at::Tensor& input, int64_t mode, const Spli
         const c10::cuda::CUDAStreamGuard on_caller(caller);
         p = prepare(g, input, mode, seq, heads, out, Role::kAsync, lend);
     }
-    if (p.output.defined() && !out.has_value() && !p.out_is_window) {
-        // Allocated while the caller's stream was current; the comm stream writes it.
+    if (p.output.defined() && !out.has_value() && !p.out_is_window && !hold_caller) {
+        // Allocated while the caller's stream was current; the comm stream writes it. (Held, the
+        // caller's stream waits for that write before anything that could reuse the block.)
         c10::cuda::CUDACachingAllocator::recordStream(p.output.storage().data_ptr(), comm);
     }
     g.order_streams(caller.stream(), comm.stream());
@@ -529,8 +530,13 @@ std::pair<at::Tensor, bool> direct_async(const GroupRef& ref, const at::Tensor& 
         y = run_async(*ref.group, input, mode, seq, heads, out, caller.id(), caller.device_index(), lend, hold_caller);
     }
     const bool registered = register_stream_completion(y, reinterpret_cast<int64_t>(comm.stream()));
-    c10::cuda::CUDACachingAllocator::recordStream(y.storage().data_ptr(), comm);
-    c10::cuda::CUDACachingAllocator::recordStream(y.storage().data_ptr(), caller);
+    // A fresh result of a held call belongs to the caller's stream in every respect. Recording streams on
+    // it would put off its reuse until both have passed: a loop that drops each result ran ahead of
+    // the device and into cudaMalloc.
+    if (!hold_caller || out.has_value()) {
+        c10::cuda::CUDACachingAllocator::recordStream(y.storage().data_ptr(), comm);
+        c10::cuda::CUDACachingAllocator::recordStream(y.storage().data_ptr(), caller);
+    }
     return {y, registered};
 }
 
