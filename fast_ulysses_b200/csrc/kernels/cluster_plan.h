@@ -55,7 +55,8 @@ private:
 };
 
 struct ClusterPlan {
-    int whole, csize;  // items of the plain kernel; cluster size of the rest (1: no split)
+    int    whole, csize;  // items of the plain kernel; cluster size of the rest (1: no split)
+    double cost;          // in steps
 };
 // Measured, in steps: what an item costs beyond its own steps (launch, first loads, write-out), what the
 // exchange of a cluster adds, and what a second launch does.
@@ -67,8 +68,7 @@ template <typename Capacity>
 ClusterPlan plan_clusters(int items, int steps, int sms, const ClusterCosts& cost, Capacity capacity)
 {
     const int   whole = items / sms * sms, rest = items - whole;
-    ClusterPlan best{items, 1};
-    double      best_cost = static_cast<double>((items + sms - 1) / sms) * (steps + cost.item);
+    ClusterPlan best{items, 1, static_cast<double>((items + sms - 1) / sms) * (steps + cost.item)};
     if (rest == 0) {
         return best;
     }
@@ -83,9 +83,8 @@ ClusterPlan plan_clusters(int items, int steps, int sms, const ClusterCosts& cos
         }
         const double c = static_cast<double>(whole / sms) * (steps + cost.item)
                          + static_cast<double>((rest + cap - 1) / cap) * (share + cost.item + cost.exchange) + (whole > 0 ? cost.launch : 0.0);
-        if (c < best_cost) {
-            best      = {whole, csize};
-            best_cost = c;
+        if (c < best.cost) {
+            best = {whole, csize, c};
         }
     }
     return best;

@@ -693,7 +693,7 @@ int fu_fmha_bwd_fused_launch(const FuFmhaArgs* a, const float* lse2, const float
         }
     }
     const int             items = p.total_work;
-    const fu::ClusterPlan plan  = a->ctas > 0 || a->trace ? fu::ClusterPlan{items, 1} : plan_split(items, p.n_q, sms, dev);
+    const fu::ClusterPlan plan  = a->ctas > 0 || a->trace ? fu::ClusterPlan{items, 1, 0.0} : plan_split(items, p.n_q, sms, dev);
     p.total_work                = plan.whole;
     p.first                     = plan.whole;
     if (plan.whole > 0) {

@@ -84,7 +84,7 @@ __device__ __forceinline__ void flag(const Params& p, uint32_t code)
 struct Barriers {
     uint64_t q_full, q_empty;
     uint64_t k_full[KV_STAGES], k_empty[KV_STAGES], v_full[KV_STAGES], v_empty[KV_STAGES];
-    uint64_t s_full[QT], p_lo[QT], p_hi[QT], o_final[QT], o_free[QT];
+    uint64_t s_full[QT], p_lo[QT], p_hi[QT], o_final[QT], o_free[QT], merge;
 };
 
 // exp2 of a pair on the FMA pipe instead of the special-function unit: floor by a round-down add of
@@ -272,9 +272,20 @@ __device__ __forceinline__ void join_shares(const Params& p, int b, int h, int r
     }
 }
 
-template <int NP, bool TRACE, bool SPLIT>
+// What a CTA takes for an item. kTwoTiles: two query tiles, all kv tiles. kShared: the same two query tiles,
+// but the CTAs of a cluster take a part of the kv tiles each. kOneTile: one query tile, whose even kv
+// tiles go through the first half of the kernel (scores, P, O) and the odd ones through the second; the two
+// results meet in the epilogue, which reads both from tensor memory. Half as many steps per
+// item and twice as many items, for problems that leave SMs idle; every K and V tile then serves 128
+// rows instead of 256, so it reads them twice as often.
+enum class Form { kTwoTiles, kShared, kOneTile };
+
+template <int NP, bool TRACE, Form FORM>
 __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_constant__ Params p)
 {
+    constexpr bool SPLIT    = FORM == Form::kShared;
+    constexpr bool ONE      = FORM == Form::kOneTile;
+    constexpr int  ROWS     = ONE ? BM : QT * BM;  // query rows of an item
     extern __shared__ uint8_t smem_raw[];
     __shared__ Barriers       bar;
     __shared__ uint32_t       tmem_holder;
@@ -302,8 +313,9 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             ptx::mbar_init(&bar.p_lo[t], 4);  // one arrival per warp
             ptx::mbar_init(&bar.p_hi[t], 4);
             ptx::mbar_init(&bar.o_final[t], 1);
-            ptx::mbar_init(&bar.o_free[t], 4);
+            ptx::mbar_init(&bar.o_free[t], ONE ? 8 : 4);  // every warp that reads it
         }
+        ptx::mbar_init(&bar.merge, 8);
         ptx::mbar_fence_init();
         ptx::tma_prefetch_desc(&p.map_q);
         ptx::tma_prefetch_desc(&p.map_k);
@@ -345,11 +357,11 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 ok = false;
                 break;
             }
-            ptx::mbar_expect_tx_if(b_of(bar.q_full), QT * TILE_BYTES, leader);
-            for (int t = 0; t < QT; ++t) {
+            ptx::mbar_expect_tx_if(b_of(bar.q_full), ROWS / BM * TILE_BYTES, leader);
+            for (int t = 0; t < ROWS / BM; ++t) {
                 for (int half = 0; half < 2; ++half) {
                     ptx::tma_load_4d_if(sq_addr + t * TILE_BYTES + half * HALF_BYTES, &p.map_q, half * 64,
-                                        qb * (QT * BM) + t * BM, h, b, b_of(bar.q_full), leader);
+                                        qb * ROWS + t * BM, h, b, b_of(bar.q_full), leader);
                 }
             }
             for (int j = 0; j < n_kv; ++j) {
@@ -395,7 +407,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
         bool            ok = true;
 
         auto issue_qk = [&](int t, uint32_t st) {
-            const ptx::Desc qa = desc_q.at(t * TILE_BYTES), ka = desc_k.at(st * TILE_BYTES);
+            const ptx::Desc qa = desc_q.at(ONE ? 0 : t * TILE_BYTES), ka = desc_k.at(st * TILE_BYTES);
 #pragma unroll
             for (int kk = 0; kk < D / 16; ++kk) {
                 const uint32_t off = (kk >> 2) * HALF_BYTES + (kk & 3) * 32;
@@ -416,6 +428,57 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             }
         };
 
+        if constexpr (ONE) {
+            // kv tile n of the CTA's sequence of tiles is in stage n % 2 and that stage's n / 2-th fill
+            static_assert(KV_STAGES == 2, "stages by parity");
+            uint32_t steps[QT] = {0, 0}, n_0 = 0;
+            auto     qk = [&](int t, uint32_t n) {
+                if (!ptx::mbar_wait_warp(b_of(bar.k_full[0]) + (n & 1u) * 8, (n >> 1) & 1u)) {
+                    return false;
+                }
+                ptx::tc_fence_after();
+                issue_qk(t, n & 1u);
+                ptx::mma_commit_if<1>(b_of(bar.k_empty[0]) + (n & 1u) * 8, leader);
+                return true;
+            };
+            for (int w = w_0; w < w_end && ok; w += w_inc, ++wc, n_0 += n_kv) {
+                ok = ptx::mbar_wait_warp(b_of(bar.q_full), wc & 1u) && qk(0, n_0) && (n_kv < 2 || qk(1, n_0 + 1));
+                for (int j = 0; j < n_kv && ok; j += 2) {
+#pragma unroll
+                    for (int t = 0; t < QT; ++t) {
+                        if (j + t >= n_kv) {
+                            break;
+                        }
+                        const uint32_t n = n_0 + j + t;
+                        ok = ptx::mbar_wait_warp(b_of(bar.v_full[0]) + (n & 1u) * 8, (n >> 1) & 1u)
+                             && ptx::mbar_wait_warp(b_of(bar.p_lo[t]), steps[t] & 1u)
+                             && (j != 0 || ptx::mbar_wait_warp(b_of(bar.o_free[t]), (wc & 1u) ^ 1u));
+                        if (!ok) {
+                            break;
+                        }
+                        ptx::tc_fence_after();
+                        issue_pv(t, n & 1u, std::integral_constant<int, 0>{}, static_cast<uint32_t>(j));
+                        ok = ptx::mbar_wait_warp(b_of(bar.p_hi[t]), steps[t] & 1u);
+                        if (!ok) {
+                            break;
+                        }
+                        ptx::tc_fence_after();
+                        issue_pv(t, n & 1u, std::integral_constant<int, 1>{}, 1u);
+                        ptx::mma_commit_if<1>(b_of(bar.v_empty[0]) + (n & 1u) * 8, leader);
+                        if (j + t + 2 >= n_kv) {
+                            ptx::mma_commit_if<1>(b_of(bar.o_final[t]), leader);
+                        }
+                        else if (!qk(t, n + 2)) {
+                            ok = false;
+                            break;
+                        }
+                        ++steps[t];
+                    }
+                }
+                ptx::mma_commit_if<1>(b_of(bar.q_empty), leader);
+            }
+        }
+        else {
         for (int w = w_0; w < w_end && ok; w += w_inc, ++wc) {
             // prologue: S for both query tiles of kv step 0
             if (!ptx::mbar_wait_warp(b_of(bar.q_full), wc & 1u)
@@ -474,6 +537,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             }
             ptx::mma_commit_if<1>(b_of(bar.q_empty), leader);
         }
+        }
         if (!ok) {
             flag(p, ERR_MMA);
         }
@@ -501,7 +565,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             const int qb  = w % p.q_blocks;
             const int h   = (w / p.q_blocks) % p.H;
             const int b   = w / (p.q_blocks * p.H);
-            const int row = qb * (QT * BM) + t * BM + row_in;
+            const int row = qb * ROWS + (ONE ? 0 : t * BM) + row_in;
             // Exponentials are taken against a reference that is only roughly the row's maximum: P, O and
             // the row sum are floating point, so any reference within 2^RANGE of it gives the same relative
             // precision. It starts at 0 and is moved to a step's maximum when the step's exponentials
@@ -512,7 +576,8 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             float m_ref = 0.0f;
             float l4[4] = {0.f, 0.f, 0.f, 0.f};
 
-            for (int j = 0; j < n_kv; ++j, ++scount) {
+            const int j_first = ONE ? t : 0;
+            for (int j = j_first; j < n_kv; j += ONE ? 2 : 1, ++scount) {
                 if (!ptx::mbar_wait(&bar.s_full[t], scount & 1u)) {
                     flag(p, ERR_SOFTMAX);
                     ok = false;
@@ -577,7 +642,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 const float part = (s4[0] + s4[1]) + (s4[2] + s4[3]);
                 const float last = fmaf(tail, c, nmc);
                 // (written so that a NaN among the scores takes the slow path too and stays one)
-                const bool fine = part < 0x1p32f && last < RANGE && (j != 0 || part > 0x1p-32f);
+                const bool fine = part < 0x1p32f && last < RANGE && (j != j_first || part > 0x1p-32f);
                 if (__any_sync(0xffffffffu, !fine)) {
                     // The maximum of the whole row; the first three quarters are still in tensor memory.
                     float mx = tail;
@@ -592,7 +657,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                         }
                     }
                     const float m_new = fine ? m_ref : mx;
-                    if (j != 0) {  // the commit behind S_t also covers the product before it: O is complete
+                    if (j != j_first) {  // the commit behind S_t also covers the product before it: O is complete
                         const float alpha = ptx::ex2((m_ref - m_new) * c);
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
@@ -669,8 +734,23 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 flag(p, ERR_SOFTMAX);
                 break;
             }
+            float l = (l4[0] + l4[1]) + (l4[2] + l4[3]), m_log2 = m_ref * c;
+            float weight[QT] = {1.0f, 1.0f};  // of the two O of a row (kOneTile)
+            if (ONE) {
+                const uint32_t pair = sq_addr + TILE_BYTES + row_in * 8;  // where the second query tile would be
+                ptx::st_shared_v2f(pair + t * BM * 8, m_log2, l);
+                ptx::mbar_arrive_warp(&bar.merge);
+                if (!ptx::mbar_wait(&bar.merge, wc & 1u) || !ptx::mbar_wait(&bar.o_final[t ^ 1], wc & 1u)) {
+                    flag(p, ERR_SOFTMAX);
+                    break;
+                }
+                const float2 a = ptx::ld_shared_v2f(pair), d = ptx::ld_shared_v2f(pair + BM * 8);
+                m_log2    = fmaxf(a.x, d.x);
+                weight[0] = ptx::ex2(a.x - m_log2);
+                weight[1] = ptx::ex2(d.x - m_log2);
+                l         = weight[0] * a.y + weight[1] * d.y;
+            }
             ptx::tc_fence_after();
-            const float    l      = (l4[0] + l4[1]) + (l4[2] + l4[3]);
             const float    inv    = 1.0f / l;
             const bool     row_ok = row < p.Sq;
             // A thread has a row; written straight out, every store instruction would touch 32 lines (3700
@@ -680,12 +760,24 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             __nv_bfloat16* dst   = p.o + b * p.o_batch + static_cast<int64_t>(row_w + (lane >> 3)) * p.o_row + h * p.o_head
                                  + (lane & 7) * 8;
 #pragma unroll 1
-            for (int half = 0; half < 2; ++half) {
+            for (int half = ONE ? t : 0; half < (ONE ? t + 1 : 2); ++half) {  // kOneTile: 64 columns for each half of the warps
 #pragma unroll
                 for (int ch = 0; ch < 2; ++ch) {
                     uint32_t r[32];
-                    ptx::tmem_ld_32x32(to + half * 64 + ch * 32, r);
-                    ptx::tmem_ld_wait();
+                    if (ONE) {
+                        uint32_t r1[32];
+                        ptx::tmem_ld_32x32(tmem + 256 + lane_off + half * 64 + ch * 32, r);
+                        ptx::tmem_ld_32x32(tmem + 384 + lane_off + half * 64 + ch * 32, r1);
+                        ptx::tmem_ld_wait();
+#pragma unroll
+                        for (int i = 0; i < 32; ++i) {
+                            r[i] = __float_as_uint(__uint_as_float(r[i]) * weight[0] + __uint_as_float(r1[i]) * weight[1]);
+                        }
+                    }
+                    else {
+                        ptx::tmem_ld_32x32(to + half * 64 + ch * 32, r);
+                        ptx::tmem_ld_wait();
+                    }
 #pragma unroll
                     for (int g = 0; g < 4; ++g) {
                         uint32_t pk[4];
@@ -696,7 +788,12 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                         ptx::st_shared_v4(stage + lane * 128 + (((ch * 4 + g) ^ (lane & 7)) << 4), make_uint4(pk[0], pk[1], pk[2], pk[3]));
                     }
                 }
-                if (half == 1) {  // O is in registers or on its way out: the next item's first product may overwrite it
+                if (ONE) {
+                    ptx::tc_fence_before();
+                    ptx::mbar_arrive_warp(&bar.o_free[0]);
+                    ptx::mbar_arrive_warp(&bar.o_free[1]);
+                }
+                else if (half == 1) {  // O is in registers or on its way out: the next item's first product may overwrite it
                     ptx::tc_fence_before();
                     ptx::mbar_arrive_warp(&bar.o_free[t]);
                 }
@@ -715,8 +812,8 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                     }
                 }
             }
-            if (row_ok && p.lse) {
-                p.lse[(static_cast<int64_t>(b) * p.H + h) * p.Sq + row] = (m_ref * c + ptx::lg2(l)) * 0.6931471805599453f;
+            if (row_ok && p.lse && (!ONE || t == 0)) {
+                p.lse[(static_cast<int64_t>(b) * p.H + h) * p.Sq + row] = (m_log2 + ptx::lg2(l)) * 0.6931471805599453f;
             }
         }
     }
@@ -734,7 +831,7 @@ fu::ClusterPlan plan_split(int items, int n_kv, int sms, int dev)
 {
     static fu::ClusterCapacity capacity;
     return fu::plan_clusters(items, n_kv, sms, {3.0, 4.5, 2.0}, [&](int csize) {
-        return capacity.of(fmha_fwd_kernel<kPolyPairs, false, true>, csize, dev, THREADS, SMEM_BYTES);
+        return capacity.of(fmha_fwd_kernel<kPolyPairs, false, Form::kShared>, csize, dev, THREADS, SMEM_BYTES);
     });
 }
 
@@ -790,11 +887,11 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
         return fu::fail(FU_E_ARG, "fu_fmha_fwd: %d of 16 exponential pairs on the FMA pipe is not built (0, 2, 4, 6)", np);
     }
     static bool configured[64][8] = {};
-    auto launch = [&](auto kernel) -> int {
-        if (dev >= 64 || a->trace || !configured[dev][np]) {
+    auto launch = [&](auto kernel, int slot) -> int {
+        if (dev >= 64 || a->trace || !configured[dev][slot]) {
             FU_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
             if (dev < 64) {
-                configured[dev][np] = true;
+                configured[dev][slot] = true;
             }
         }
         int grid = a->ctas > 0 ? std::min(a->ctas, sms) : sms;
@@ -808,15 +905,24 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
         if (np != kPolyPairs) {
             return fu::fail(FU_E_ARG, "fu_fmha_fwd: the timeline build exists for the default exponential split only");
         }
-        return launch(fmha_fwd_kernel<kPolyPairs, true, false>);
+        return launch(fmha_fwd_kernel<kPolyPairs, true, Form::kTwoTiles>, np);
     }
     if (np == kPolyPairs && a->ctas <= 0) {
         const fu::ClusterPlan plan = plan_split(p.total_work, p.n_kv, sms, dev);
+        // One query tile per item where that takes fewer steps of the busiest SM; its steps are a tenth longer
+        // (K and V are read twice as often). 2 x 1000 tokens x 5 heads (80 items instead of 40 in clusters of
+        // three): 16.0 -> 11.8 us; 4000 x 4: 35.2 -> 30.7; 1000 x 20 would take two waves, 20.8 for 18.0.
+        const int one_blocks = (a->seq_q + BM - 1) / BM, one_items = one_blocks * p.H * p.B;
+        if (p.n_kv > 1 && ((one_items + sms - 1) / sms) * 1.1 * ((p.n_kv + 1) / 2 + 3.0) < plan.cost) {
+            p.q_blocks   = one_blocks;
+            p.total_work = one_items;
+            return launch(fmha_fwd_kernel<kPolyPairs, false, Form::kOneTile>, 7);
+        }
         if (plan.csize > 1) {
             const int items = p.total_work;
             p.total_work    = plan.whole;
             if (plan.whole > 0) {
-                rc = launch(fmha_fwd_kernel<kPolyPairs, false, false>);
+                rc = launch(fmha_fwd_kernel<kPolyPairs, false, Form::kTwoTiles>, np);
                 if (rc != FU_OK) {
                     return rc;
                 }
@@ -830,15 +936,15 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
             cfg.stream                = static_cast<cudaStream_t>(stream);
             cfg.attrs                 = &attr;
             cfg.numAttrs              = 1;
-            FU_CUDA_OK(cudaLaunchKernelEx(&cfg, fmha_fwd_kernel<kPolyPairs, false, true>, p));
+            FU_CUDA_OK(cudaLaunchKernelEx(&cfg, fmha_fwd_kernel<kPolyPairs, false, Form::kShared>, p));
             return FU_OK;
         }
     }
     switch (np) {
-    case 0: return launch(fmha_fwd_kernel<0, false, false>);
-    case 2: return launch(fmha_fwd_kernel<2, false, false>);
-    case 4: return launch(fmha_fwd_kernel<4, false, false>);
-    case 6: return launch(fmha_fwd_kernel<6, false, false>);
+    case 0: return launch(fmha_fwd_kernel<0, false, Form::kTwoTiles>, np);
+    case 2: return launch(fmha_fwd_kernel<2, false, Form::kTwoTiles>, np);
+    case 4: return launch(fmha_fwd_kernel<4, false, Form::kTwoTiles>, np);
+    case 6: return launch(fmha_fwd_kernel<6, false, Form::kTwoTiles>, np);
     default: return fu::fail(FU_E_ARG, "fu_fmha_fwd: %d of 16 exponential pairs on the FMA pipe is not built (0, 2, 4, 6)", np);
     }
 }

@@ -65,7 +65,8 @@ def test_first_step_far_below_a_later_one():
 # eight CTAs, each with a part of the 128-row kv tiles
 @pytest.mark.parametrize("b,h,sq,skv", [(1, 1, 1, 129), (1, 1, 256, 256), (1, 2, 300, 384), (1, 1, 257, 500), (2, 1, 130, 640),
                                         (1, 1, 64, 1025), (1, 3, 700, 1111), (1, 1, 256, 8 * 128 + 1), (1, 1, 100, 6000),
-                                        (1, 8, 1000, 1000), (1, 20, 1024, 400), (1, 37, 1000, 300), (2, 19, 1030, 1500)])
+                                        (1, 8, 1000, 1000), (1, 20, 1024, 400), (1, 37, 1000, 300), (2, 19, 1030, 1500),
+                                        (1, 1, 257, 3000), (1, 3, 700, 4111), (1, 10, 1000, 3333), (1, 9, 2000, 2600), (1, 40, 1024, 2000)])
 def test_kv_tiles_shared_by_a_cluster(b, h, sq, skv):
     torch.manual_seed(sq + skv)
     q = torch.randn(b, sq, h, 128, device="cuda").bfloat16()
@@ -77,6 +78,22 @@ def test_kv_tiles_shared_by_a_cluster(b, h, sq, skv):
     run(q, k, v)
     first = attention.fmha_fwd(q, k, v)
     assert all(torch.equal(x, y) for x, y in zip(first, attention.fmha_fwd(q, k, v)))
+
+
+# one query tile per item, its even and odd kv tiles through either half of the kernel
+@pytest.mark.parametrize("b,h,sq,skv", [(1, 1, 1, 129), (1, 2, 128, 256), (1, 3, 257, 300), (2, 1, 130, 384), (1, 5, 1000, 640),
+                                        (2, 5, 1000, 1000), (1, 20, 1000, 1025), (1, 148, 128, 200), (1, 149, 128, 500)])
+def test_kv_tiles_by_parity(b, h, sq, skv):
+    torch.manual_seed(sq * 5 + skv)
+    q = torch.randn(b, sq, h, 128, device="cuda").bfloat16()
+    k = torch.randn(b, skv, h, 128, device="cuda").bfloat16()
+    v = torch.randn(b, skv, h, 128, device="cuda").bfloat16()
+    run(q, k, v)
+    first = attention.fmha_fwd(q, k, v)
+    assert all(torch.equal(x, y) for x, y in zip(first, attention.fmha_fwd(q, k, v)))
+    for at, size in ((0, 20.0), (min(130, skv - 1), 40.0), (skv - 1, 90.0)):  # either half moves its reference, and far
+        k[:, at] = q[:, sq // 2] * size
+        run(q, k, v)
 
 
 # backward: 128 kv rows are an item, and the 128-row query blocks are what a cluster shares
