@@ -280,6 +280,7 @@ struct Linear : public torch::autograd::Function<Linear> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w, const MaybeTensor& bias,
                           const MaybeTensor& residual)
     {
+        const at::AutoDispatchBelowAutograd below;
         const Tensor x2 = rows_of(x, x.size(-1));
         ctx->save_for_backward({x2, w});
         ctx->saved_data["x_shape"]  = x.sizes().vec();
@@ -290,6 +291,7 @@ struct Linear : public torch::autograd::Function<Linear> {
 
     static variable_list backward(AutogradContext* ctx, variable_list grads)
     {
+        const at::AutoDispatchBelowADInplaceOrView below;
         const variable_list        saved = ctx->get_saved_variables();
         const Tensor               x2 = saved[0], w = saved[1], gy = grads[0];
         const c10::cuda::CUDAGuard on(gy.device());
@@ -340,6 +342,7 @@ struct FeedForward : public torch::autograd::Function<FeedForward> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& w1, const MaybeTensor& b1, const Tensor& w2,
                           const MaybeTensor& b2, const MaybeTensor& residual)
     {
+        const at::AutoDispatchBelowAutograd below;
         const Tensor x2 = rows_of(x, x.size(-1));
         GemmExtra    e;
         e.bias         = bias_ready(or_none(b1));
@@ -356,6 +359,7 @@ struct FeedForward : public torch::autograd::Function<FeedForward> {
 
     static variable_list backward(AutogradContext* ctx, variable_list grads)
     {
+        const at::AutoDispatchBelowADInplaceOrView below;
         const variable_list        saved = ctx->get_saved_variables();
         const Tensor               x2 = saved[0], w1 = saved[1], w2 = saved[2], pre = saved[3], h = saved[4], gy = grads[0];
         const c10::cuda::CUDAGuard on(gy.device());
@@ -451,6 +455,7 @@ Tensor layer_norm_backward(const Tensor& gy, const Tensor& x2, const Tensor& sta
 struct LayerNorm : public torch::autograd::Function<LayerNorm> {
     static Tensor forward(AutogradContext* ctx, const Tensor& x, double eps)
     {
+        const at::AutoDispatchBelowAutograd below;
         const Tensor x2        = layer_norm_rows(x);
         const auto [y, stats] = layer_norm_forward(x2, eps);
         ctx->save_for_backward({x2, stats});
@@ -459,6 +464,7 @@ struct LayerNorm : public torch::autograd::Function<LayerNorm> {
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads)
     {
+        const at::AutoDispatchBelowADInplaceOrView below;
         const variable_list        saved = ctx->get_saved_variables();
         const c10::cuda::CUDAGuard on(saved[0].device());
         return {layer_norm_backward(grads[0], saved[0], saved[1], Tensor(), ctx->saved_data["shape"].toIntVector()), Tensor()};
@@ -470,6 +476,7 @@ struct LayerNorm : public torch::autograd::Function<LayerNorm> {
 struct LayerNormFork : public torch::autograd::Function<LayerNormFork> {
     static variable_list forward(AutogradContext* ctx, const Tensor& x, double eps)
     {
+        const at::AutoDispatchBelowAutograd below;
         const Tensor x2        = layer_norm_rows(x);
         const auto [y, stats] = layer_norm_forward(x2, eps);
         ctx->save_for_backward({x2, stats});
@@ -479,6 +486,7 @@ struct LayerNormFork : public torch::autograd::Function<LayerNormFork> {
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads)
     {
+        const at::AutoDispatchBelowADInplaceOrView below;
         const variable_list saved = ctx->get_saved_variables();
         if (!grads[0].defined()) {
             return {grads[1], Tensor()};
@@ -620,6 +628,7 @@ std::tuple<Tensor, Tensor, Tensor> fmha_bwd(const Tensor& q, const Tensor& k, co
 struct Attention : public torch::autograd::Function<Attention> {
     static Tensor forward(AutogradContext* ctx, const Tensor& q, const Tensor& k, const Tensor& v, std::optional<double> scale)
     {
+        const at::AutoDispatchBelowAutograd below;
         const auto [o, lse] = fmha_fwd(q, k, v, scale, std::nullopt, 0, 0, std::nullopt);
         ctx->save_for_backward({q, k, v, o, lse});
         if (scale.has_value()) {
@@ -629,6 +638,7 @@ struct Attention : public torch::autograd::Function<Attention> {
     }
     static variable_list backward(AutogradContext* ctx, variable_list grads)
     {
+        const at::AutoDispatchBelowADInplaceOrView below;
         const variable_list   s = ctx->get_saved_variables();
         std::optional<double> scale;
         if (ctx->saved_data.count("scale")) {
@@ -849,6 +859,7 @@ struct SpAttentionFn : public torch::autograd::Function<SpAttentionFn> {
                           const Tensor& gamma_k, const Tensor& w_o, const MaybeTensor& b_o, const MaybeTensor& residual,
                           const Tensor& rope, const SpPtr& mod)
     {
+        const at::AutoDispatchBelowAutograd below;
         const auto f = mod->forward(x, w_qkv, gamma_q, gamma_k, w_o, or_none(b_o), or_none(residual), rope, true);
         ctx->saved_data["b_o"]      = b_o.has_value();
         ctx->saved_data["residual"] = residual.has_value();
@@ -861,6 +872,7 @@ struct SpAttentionFn : public torch::autograd::Function<SpAttentionFn> {
 
     static variable_list backward(AutogradContext* ctx, variable_list grads)
     {
+        const at::AutoDispatchBelowADInplaceOrView below;
         const variable_list s = ctx->get_saved_variables();
         const Tensor        x2 = s[0], w_qkv = s[1], gamma_q = s[2], gamma_k = s[3], w_o = s[4], y_save = s[5], gather = s[6],
                      lse = s[7], rope = s[8], dy = grads[0];
@@ -903,7 +915,8 @@ struct SpAttentionFn : public torch::autograd::Function<SpAttentionFn> {
         }
         // dq, dk, dv come home inside the kernel that undoes RoPE and RMSNorm (mode-1 direction)
         const Tensor dyqkv = empty_bf16({m, 3 * heads * kHeadDim}, dy);
-        const Tensor dg    = at::zeros({2, kHeadDim}, at::TensorOptions().dtype(at::kFloat).device(dy.device()));
+        const Tensor dg    = empty_f32({2, kHeadDim}, dy);
+        C10_CUDA_CHECK(cudaMemsetAsync(dg.data_ptr(), 0, dg.nbytes(), stream_of(dy)));
         {
             const NvtxRange r("fast_ulysses_b200::pull_qkv_grads");
             const Tensor    gq = SpAttention::f32(gamma_q, mod->gq_cache), gk = SpAttention::f32(gamma_k, mod->gk_cache);
