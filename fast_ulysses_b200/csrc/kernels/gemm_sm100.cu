@@ -9,6 +9,7 @@
 //
 // The reference has no GEMM: its example wraps nn.Linear + separate norm/RoPE around two
 // all_to_all_4d calls (examples/dit_attention.py:45-63). These kernels replace that composition.
+#include "cluster_plan.h"
 #include "fu_kernels.h"
 #include "gemm_sm100.cuh"
 #include "host_util.h"
@@ -61,29 +62,29 @@ struct PlainEpi {
     __device__ void open(int) {}
     __device__ void close(int) {}
 
-    __device__ __forceinline__ static void pack_row(const float (&v)[64], uint32_t stage, int lane)
+    template <int W>
+    __device__ __forceinline__ static void pack_row(const float (&v)[W], uint32_t stage, int lane)
     {
 #pragma unroll
-        for (int g = 0; g < 8; ++g) {
+        for (int g = 0; g < W / 8; ++g) {
             ptx::st_shared_v4(stage_unit(stage, lane, g), make_uint4(pack_bf16(v[8 * g], v[8 * g + 1]), pack_bf16(v[8 * g + 2], v[8 * g + 3]),
                                                                      pack_bf16(v[8 * g + 4], v[8 * g + 5]), pack_bf16(v[8 * g + 6], v[8 * g + 7])));
         }
     }
 
-    template <int H>
-    __device__ __forceinline__ void half(const uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage) const
+    // W columns of 32 rows, a row per thread
+    template <int W>
+    __device__ __forceinline__ void piece(float (&v)[W], int row0, int col0, int lane, uint32_t stage) const
     {
-        float v[64];
-#pragma unroll
-        for (int j = 0; j < 64; ++j) {
-            v[j] = __uint_as_float(r[H * 64 + j]);
+        if (row0 >= M || col0 >= N) {
+            return;  // warp-uniform
         }
         if (bias) {
-            const bool whole = col0 + 64 <= N && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;  // uniform
+            const bool whole = col0 + W <= N && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;  // uniform
             if (whole && !bias_bf16) {
                 const float4* b = reinterpret_cast<const float4*>(static_cast<const float*>(bias) + col0);
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
+                for (int j = 0; j < W / 4; ++j) {
                     const float4 f = __ldg(b + j);
                     v[4 * j] += f.x, v[4 * j + 1] += f.y, v[4 * j + 2] += f.z, v[4 * j + 3] += f.w;
                 }
@@ -91,7 +92,7 @@ struct PlainEpi {
             else if (whole) {
                 const uint4* b = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(bias) + col0);
 #pragma unroll
-                for (int j = 0; j < 8; ++j) {
+                for (int j = 0; j < W / 8; ++j) {
                     const uint4           q = __ldg(b + j);
                     const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
@@ -103,7 +104,7 @@ struct PlainEpi {
             }
             else {
 #pragma unroll
-                for (int j = 0; j < 64; ++j) {
+                for (int j = 0; j < W; ++j) {
                     if (col0 + j < N) {
                         v[j] += bias_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[col0 + j])
                                           : static_cast<const float*>(bias)[col0 + j];
@@ -113,18 +114,18 @@ struct PlainEpi {
         }
         if (c_pre) {
             pack_row(v, stage, lane);
-            stage_out(stage, c_pre, ldc, row0, col0, M, N, lane);
+            stage_out<W>(stage, c_pre, ldc, row0, col0, M, N, lane);
         }
         if (ACT == 1 || ACT == 2) {
 #pragma unroll
-            for (int j = 0; j < 64; ++j) {
+            for (int j = 0; j < W; ++j) {
                 v[j] = ACT == 1 ? gelu_tanh(v[j]) : gelu_erf(v[j]);
             }
         }
         if (ACT == 3) {
-            stage_in(stage, aux, ldc, row0, col0, M, N, lane);
+            stage_in<W>(stage, aux, ldc, row0, col0, M, N, lane);
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
+            for (int g = 0; g < W / 8; ++g) {
                 const uint4           q = ptx::ld_shared_v4(stage_unit(stage, lane, g));
                 const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
@@ -136,9 +137,9 @@ struct PlainEpi {
             }
         }
         if (residual) {
-            stage_in(stage, residual, ldc, row0, col0, M, N, lane);
+            stage_in<W>(stage, residual, ldc, row0, col0, M, N, lane);
 #pragma unroll
-            for (int g = 0; g < 8; ++g) {
+            for (int g = 0; g < W / 8; ++g) {
                 const uint4           q = ptx::ld_shared_v4(stage_unit(stage, lane, g));
                 const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
 #pragma unroll
@@ -150,18 +151,22 @@ struct PlainEpi {
             }
         }
         pack_row(v, stage, lane);
-        stage_out(stage, c, ldc, row0, col0, M, N, lane);
+        stage_out<W>(stage, c, ldc, row0, col0, M, N, lane);
     }
 
     __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage) const
     {
-        if (row0 >= M || col0 >= N) {
-            return;  // warp-uniform
+        float v[64];
+#pragma unroll
+        for (int j = 0; j < 64; ++j) {
+            v[j] = __uint_as_float(r[j]);
         }
-        half<0>(r, row0, col0, lane, stage);
-        if (col0 + 64 < N) {
-            half<1>(r, row0, col0 + 64, lane, stage);
+        piece<64>(v, row0, col0, lane, stage);
+#pragma unroll
+        for (int j = 0; j < 64; ++j) {
+            v[j] = __uint_as_float(r[64 + j]);
         }
+        piece<64>(v, row0, col0 + 64, lane, stage);
     }
 };
 
@@ -182,7 +187,14 @@ template <int ACT>
 __global__ void __launch_bounds__(SMALL_THREADS, 1) gemm_small_kernel(const __grid_constant__ PlainArgs<ACT> a)
 {
     PlainEpi<ACT> epi = a.epi;
-    run_small(a.core, epi);
+    run_small<false>(a.core, epi);
+}
+
+template <int ACT>
+__global__ void __launch_bounds__(SMALL_THREADS, 1) gemm_split_kernel(const __grid_constant__ PlainArgs<ACT> a)
+{
+    PlainEpi<ACT> epi = a.epi;
+    run_small<true>(a.core, epi);
 }
 
 // ---- fused QKV epilogue: RMSNorm + 3D RoPE + scatter ---------------------------------------------------
@@ -330,7 +342,7 @@ struct QkvEpi {
             }
             ptx::st_shared_v4(stage_unit(stage, lane, g), make_uint4(o[0], o[1], o[2], o[3]));
         }
-        stage_out(stage, p.y_save, p.ld_y, row0, col0 + H * 64, p.M, 0x7fffffff, lane);
+        stage_out<64>(stage, p.y_save, p.ld_y, row0, col0 + H * 64, p.M, 0x7fffffff, lane);
     }
 
     __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage) const
@@ -388,7 +400,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WIDE_THREADS, 1) qkv
 __global__ void __launch_bounds__(SMALL_THREADS, 1) qkv_small_kernel(const __grid_constant__ QkvArgs a)
 {
     QkvEpi<32 * SMALL_EPI_WARPS> epi(a.epi);
-    run_small(a.core, epi);
+    run_small<false>(a.core, epi);
 }
 
 // ---- fused mode-1 path: pull attention output from peers, feed the output projection -----------------
@@ -702,39 +714,69 @@ int pair_capacity()
 // most half as many tiles as pairs are left over, those are split into blocks.
 enum class Shape { kSmall, kTall, kBroad };  // 128 x 128; 512 x 256; 256 x 512
 struct Choice {
-    Shape shape;
-    int   tiles_m, tiles_n, full, items;
+    Shape  shape;
+    int    tiles_m, tiles_n, full, items;
+    double cost;
 };
 
-Choice wide_choice(int64_t m, int64_t n, Shape shape, int pairs)
+Choice wide_choice(int64_t m, int64_t n, double kb, Shape shape, int pairs)
 {
     const int64_t tm    = shape == Shape::kTall ? (m + 511) / 512 : (m + 255) / 256;
     const int64_t tn    = shape == Shape::kTall ? (n + 255) / 256 : (n + 511) / 512;
     const int64_t tiles = tm * tn, left = tiles % pairs;
     const int64_t full = 2 * left <= pairs ? tiles - left : tiles;
-    return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(full), static_cast<int>(full + 2 * (tiles - full))};
-}
-
-double wide_cost(const Choice& c, int pairs)
-{
-    return 2.0 * ((c.full + pairs - 1) / pairs) + 1.05 * ((c.items - c.full + pairs - 1) / pairs);
+    const int64_t items = full + 2 * (tiles - full);
+    return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(full), static_cast<int>(items),
+            6.0 + 0.305 * kb * (2.0 * ((full + pairs - 1) / pairs) + 1.05 * ((items - full + pairs - 1) / pairs))};
 }
 
 Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int flags)
 {
     const int64_t t128 = ((m + 127) / 128) * ((n + 127) / 128);
+    const double  kb   = static_cast<double>((k + BK - 1) / BK);
     const Choice  small{Shape::kSmall, static_cast<int>((m + 127) / 128), static_cast<int>((n + 127) / 128), 0,
-                       static_cast<int>(t128)};
+                       static_cast<int>(t128), 3.2 + 0.225 * kb * ((t128 + sms - 1) / sms)};
     if (flags & FU_GEMM_SINGLE) {
         return small;
     }
-    const Choice tall = wide_choice(m, n, Shape::kTall, pairs), broad = wide_choice(m, n, Shape::kBroad, pairs);
-    const Choice wide = wide_cost(tall, pairs) < wide_cost(broad, pairs) ? tall : broad;
+    const Choice tall = wide_choice(m, n, kb, Shape::kTall, pairs), broad = wide_choice(m, n, kb, Shape::kBroad, pairs);
+    const Choice wide = tall.cost < broad.cost ? tall : broad;
     if (flags & FU_GEMM_PAIR) {
         return wide;
     }
-    const double kb = static_cast<double>((k + BK - 1) / BK);
-    return 3.2 + 0.225 * kb * ((t128 + sms - 1) / sms) < 6.0 + 0.305 * kb * wide_cost(wide, pairs) ? small : wide;
+    return small.cost < wide.cost ? small : wide;
+}
+
+// How many CTAs share the K-blocks of a 128 x 128 tile (1: none do), see run_small, when that is estimated
+// to be faster than `best`. The exchange takes 1.8, 2.4 and 2.8 us beyond the tile's own time (measured, for
+// two, four and eight CTAs). 64 x 2000 x 8000: 30.6 -> 13.3 us with four, 64 x 512 x 2048: 10.6 -> 7.0 with eight,
+// 512 x 1536 x 4096: 18.0 -> 13.2 with two; the 160 tiles of 512 x 5120 x 5120 stay as they are.
+int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k)
+{
+    static fu::ClusterCapacity capacity;
+    const int64_t              t128 = ((m + 127) / 128) * ((n + 127) / 128), kb = (k + BK - 1) / BK;
+    int                        dev = 0, chosen = 1;
+    double                     cost = best.cost;
+    if (cudaGetDevice(&dev) != cudaSuccess) {
+        return 1;
+    }
+    for (const int csize : {2, 4, 8}) {
+        const int64_t share = (kb + csize - 1) / csize;
+        const double  once  = 3.2 + (csize == 2 ? 1.8 : csize == 4 ? 2.4 : 2.8) + 0.225 * share;
+        if ((kb + share - 1) / share != csize || once >= cost) {
+            continue;  // a CTA would have nothing to do, or no gain even in one wave
+        }
+        const int cap = capacity.of(gemm_split_kernel<0>, csize, dev, SMALL_THREADS, SMALL_SMEM_BYTES);
+        if (cap < 1) {
+            continue;
+        }
+        const double c = static_cast<double>((t128 + cap - 1) / cap) * once;
+        if (c < cost) {
+            cost   = c;
+            chosen = csize;
+        }
+    }
+    return chosen;
 }
 
 int fill_core(Core& core, const void* a, const void* b, int64_t m, int64_t n, int64_t k, int64_t lda, int64_t ldb, uint32_t* err)
@@ -831,9 +873,32 @@ int launch_small(Kernel kernel, const Args& a, int ctas, cudaStream_t stream)
 }
 
 template <int ACT>
-int launch_plain(const FuGemmArgs* g, const Choice& c, int pairs, int flags, cudaStream_t stream)
+int launch_split(const PlainArgs<ACT>& a, int csize, cudaStream_t stream)
+{
+    const int rc = set_smem(gemm_split_kernel<ACT>, SMALL_SMEM_BYTES);
+    if (rc != FU_OK) {
+        return rc;
+    }
+    cudaLaunchConfig_t  cfg  = {};
+    cudaLaunchAttribute attr = fu::cluster_attr(csize);
+    cfg.gridDim              = dim3(static_cast<unsigned>(a.core.items * csize), 1, 1);
+    cfg.blockDim             = dim3(SMALL_THREADS, 1, 1);
+    cfg.dynamicSmemBytes     = SMALL_SMEM_BYTES;
+    cfg.stream               = stream;
+    cfg.attrs                = &attr;
+    cfg.numAttrs             = 1;
+    FU_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_split_kernel<ACT>, a));
+    return FU_OK;
+}
+
+template <int ACT>
+int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream_t stream)
 {
     PlainArgs<ACT> a{};
+    const int      csize = g->ctas > 0 || (flags & (FU_GEMM_SINGLE | FU_GEMM_PAIR)) ? 1 : choose_split(c, g->m, g->n, g->k);
+    if (csize > 1) {
+        c = choose_shape(g->m, g->n, g->k, pairs, 1, FU_GEMM_SINGLE);
+    }
     const int      rc = fill_wide(a.core, c, g->a, g->b, g->m, g->n, g->k, g->lda, g->ldb, g->err, flags);
     if (rc != FU_OK) {
         return rc;
@@ -847,6 +912,9 @@ int launch_plain(const FuGemmArgs* g, const Choice& c, int pairs, int flags, cud
     a.epi.N         = a.core.N;
     a.epi.aux       = static_cast<const __nv_bfloat16*>(g->aux);
     a.epi.c_pre     = static_cast<__nv_bfloat16*>(g->c_pre);
+    if (csize > 1) {
+        return launch_split<ACT>(a, csize, stream);
+    }
     switch (c.shape) {
     case Shape::kTall: return launch_pairs(gemm_wide_kernel<2, 1, ACT>, a, pairs, stream);
     case Shape::kBroad: return launch_pairs(gemm_wide_kernel<1, 2, ACT>, a, pairs, stream);

@@ -20,6 +20,8 @@
 #include "handshake.cuh"
 #include "ptx.cuh"
 
+#include <type_traits>
+
 namespace fu {
 namespace gemm {
 
@@ -567,13 +569,17 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
 // epilogue, and nothing shared between SMs. Bound by shared memory (its MMAs read 128 B/clk by
 // themselves) at about half the tensor pipe's rate, which a problem of this size does not reach anyway.
 // The two halves of the tensor memory in use alternate between tiles.
+//
+// SPLIT: the CTAs of a cluster (2, 4 or 8) take a part of the K-blocks of one tile each, for problems whose
+// tiles leave SMs idle. They add up their fp32 sums through distributed shared memory, every CTA 128 / size
+// columns of the tile in the order of the CTAs, and each finishes and writes its columns.
 constexpr int SMALL_STAGES      = 6;
 constexpr int SMALL_STAGE_BYTES = 2 * WIDE_BLOCK_BYTES;
 constexpr int SMALL_EPI_WARPS   = 4;
 constexpr int SMALL_THREADS     = 32 * (2 + SMALL_EPI_WARPS);
 constexpr int SMALL_SMEM_BYTES  = SMALL_STAGES * SMALL_STAGE_BYTES + SMALL_EPI_WARPS * UNIT_STAGE_BYTES + 1024;
 
-template <class Epi>
+template <bool SPLIT, class Epi>
 __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
 {
     extern __shared__ uint8_t smem_raw[];
@@ -586,6 +592,11 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
     const int      lane = threadIdx.x & 31;
     const int      tiles   = core.tiles_m * core.tiles_n;  // of 128 x 128 here
     const int      kblocks = (core.K + BK - 1) / BK;
+    const int      csize   = SPLIT ? static_cast<int>(ptx::uniform(ptx::cluster_nctarank())) : 1;
+    const int      crank   = SPLIT ? static_cast<int>(ptx::uniform(ptx::cluster_ctarank())) : 0;
+    const int      share   = SPLIT ? (kblocks + csize - 1) / csize : kblocks;
+    const int      kb_0 = crank * share, kb_n = SPLIT ? min(kblocks, kb_0 + share) : kblocks;  // this CTA's K-blocks
+    const int      t_0 = SPLIT ? blockIdx.x / csize : blockIdx.x, t_inc = SPLIT ? gridDim.x / csize : gridDim.x;
 
     if (warp == 0 && lane == 0) {
         ptx::tma_prefetch_desc(&core.map_a);
@@ -614,10 +625,10 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
     if (warp == 0) {
         uint32_t stage = 0, phase = 1;
         bool     ok    = true;
-        for (int t = blockIdx.x; t < tiles && ok; t += gridDim.x) {
+        for (int t = t_0; t < tiles && ok; t += t_inc) {
             int mt, nt;
             pair_tile_coords(core.tiles_m, core.tiles_n, 16, t, mt, nt);
-            for (int kb = 0; kb < kblocks; ++kb) {
+            for (int kb = kb_0; kb < kb_n; ++kb) {
                 if (!ptx::mbar_wait_warp(empty_b + stage * 8, phase)) {
                     ok = false;
                     break;
@@ -657,14 +668,14 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
         const uint32_t  tfull_b = ptx::smem_addr(tmem_full), tempty_b = ptx::smem_addr(tmem_empty);
         uint32_t        stage = 0, phase = 0, tcount = 0;
         uint32_t        gave_up = ERR_NONE;
-        for (int t = blockIdx.x; t < tiles && !gave_up; t += gridDim.x, ++tcount) {
+        for (int t = t_0; t < tiles && !gave_up; t += t_inc, ++tcount) {
             const uint32_t acc = tcount & 1u;
             if (!ptx::mbar_wait_warp(tempty_b + acc * 8, ((tcount >> 1) & 1u) ^ 1u)) {
                 gave_up = ERR_MMA_WAIT_TMEM;
                 break;
             }
             ptx::tc_fence_after();
-            for (int kb = 0; kb < kblocks; ++kb) {
+            for (int kb = kb_0; kb < kb_n; ++kb) {
                 if (!ptx::mbar_wait_warp(full_b + stage * 8, phase)) {
                     gave_up = ERR_MMA_WAIT_FULL;
                     break;
@@ -674,7 +685,7 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; ++k) {
                     ptx::mma_f16_ss_if<1>(tmem_base + acc * 128, a.at(a_step * k), b.at(b_step * k), idesc,
-                                          static_cast<uint32_t>(kb | k), leader);
+                                          static_cast<uint32_t>((kb - kb_0) | k), leader);
                 }
                 ptx::mma_commit_if<1>(empty_b + stage * 8, leader);
                 if (++stage == SMALL_STAGES) {
@@ -699,15 +710,70 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
             epi.open(threadIdx.x - 64);
         }
         uint32_t tcount = 0;
-        for (int t = blockIdx.x; t < tiles; t += gridDim.x, ++tcount) {
+        for (int t = t_0; t < tiles; t += t_inc, ++tcount) {
             const uint32_t acc = tcount & 1u;
-            if (!ptx::mbar_wait(&tmem_full[acc], (tcount >> 1) & 1u)) {
+            const bool     ok  = ptx::mbar_wait(&tmem_full[acc], (tcount >> 1) & 1u);
+            if (!ok) {
                 flag_error(core.err, ERR_EPI_WAIT);
+            }
+            int mt, nt;
+            pair_tile_coords(core.tiles_m, core.tiles_n, 16, t, mt, nt);
+            if constexpr (SPLIT) {  // one tile per cluster; also after a timeout: the other CTAs wait in its barriers
+                ptx::tc_fence_after();
+                const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+                const int      row0 = mt * 128 + quarter * 32, width = 128 / csize;
+                const uint32_t slot = base + quarter * 16384 + lane * 16;  // this warp's rows: [columns / 4][lane] of 16 bytes per CTA
+                ptx::cluster_sync();  // every CTA's products are complete: its stages may be overwritten
+#pragma unroll 1
+                for (int ch = 0; ch < 8; ++ch) {  // the next CTA's columns first, so that not all write to one
+                    const int      col = (ch * 16 + (crank + 1) * width) & 127, owner = col / width;
+                    const uint32_t dst = ptx::cluster_addr(slot + (crank * width + col - owner * width) * 128, owner);
+                    uint32_t       r[16];
+                    ptx::tmem_ld_32x16(taddr + col, r);
+                    ptx::tmem_ld_wait();
+#pragma unroll
+                    for (int g = 0; g < 4; ++g) {
+                        ptx::st_cluster_v4(dst + g * 512, r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+                    }
+                }
+                ptx::cluster_sync();
+                auto finish = [&](auto w) {
+                    constexpr int W = decltype(w)::value;
+                    float         v[W];
+#pragma unroll
+                    for (int k = 0; k < W; ++k) {
+                        v[k] = 0.0f;
+                    }
+#pragma unroll 1
+                    for (int from = 0; from < csize; ++from) {
+#pragma unroll
+                        for (int g = 0; g < W / 4; ++g) {
+                            const uint4 q = ptx::ld_shared_v4(slot + (from * W + g * 4) * 128);
+                            v[4 * g] += __uint_as_float(q.x);
+                            v[4 * g + 1] += __uint_as_float(q.y);
+                            v[4 * g + 2] += __uint_as_float(q.z);
+                            v[4 * g + 3] += __uint_as_float(q.w);
+                        }
+                    }
+                    epi.template piece<W>(v, row0, nt * 128 + crank * W, lane, stage);
+                };
+                if (ok) {
+                    if (csize == 2) {
+                        finish(std::integral_constant<int, 64>{});
+                    }
+                    else if (csize == 4) {
+                        finish(std::integral_constant<int, 32>{});
+                    }
+                    else {
+                        finish(std::integral_constant<int, 16>{});
+                    }
+                }
+                break;
+            }
+            if (!ok) {
                 break;
             }
             ptx::tc_fence_after();
-            int mt, nt;
-            pair_tile_coords(core.tiles_m, core.tiles_n, 16, t, mt, nt);
             uint32_t r[128];
             load_unit(tmem_base + acc * 128 + (static_cast<uint32_t>(quarter * 32) << 16), r);
             ptx::tc_fence_before();
@@ -722,6 +788,10 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
         }
     }
 
+    if (SPLIT && warp < 2) {  // the epilogue warps' exchange
+        ptx::cluster_sync();
+        ptx::cluster_sync();
+    }
     ptx::tc_fence_before();
     __syncthreads();
     if (warp == 1) {
@@ -729,10 +799,10 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
     }
 }
 
-// ---- a unit's 64-column halves through the staging buffer ----------------------------------------------------
+// ---- W columns of a unit through the staging buffer -----------------------------------------------------------
 // A thread holds a row, so its global accesses would be 32 scattered pieces per instruction. They go
-// through the warp's staging buffer instead: eight lanes move the 128 bytes of one row, four rows per
-// instruction. 16-byte units are XOR-swizzled by the row: neither side has bank conflicts. All eight
+// through the warp's staging buffer instead: W / 8 lanes move the W columns of one row (eight lanes and 128
+// bytes for half a unit). 16-byte units are XOR-swizzled by the row: neither side has bank conflicts. All
 // accesses of a lane are in flight together: with each store waiting for its load, writing a unit out took
 // 3700 clocks, most of a small GEMM's time.
 __device__ __forceinline__ uint32_t stage_unit(uint32_t stage, int row, int unit)
@@ -740,23 +810,25 @@ __device__ __forceinline__ uint32_t stage_unit(uint32_t stage, int row, int unit
     return stage + row * 128 + ((unit ^ (row & 7)) << 4);
 }
 
-// 32 rows x 64 columns of a bf16 matrix into the staging buffer; what lies outside reads as zero.
+// 32 rows x W columns of a bf16 matrix into the staging buffer; what lies outside reads as zero.
+template <int W>
 __device__ __forceinline__ void stage_in(uint32_t stage, const __nv_bfloat16* src, int64_t ld, int row0, int col0, int M, int N,
                                          int lane)
 {
-    const int unit = lane & 7, col = col0 + unit * 8;
-    uint4     v[8];
-    if (row0 + 32 <= M && col0 + 64 <= N) {  // warp-uniform
-        const __nv_bfloat16* p = src + static_cast<int64_t>(row0 + (lane >> 3)) * ld + col;
+    constexpr int U = W / 8, ROWS = 32 / U;  // lanes a row, rows an access
+    const int     unit = lane % U, col = col0 + unit * 8, first = lane / U;
+    uint4         v[U];
+    if (row0 + 32 <= M && col0 + W <= N) {  // warp-uniform
+        const __nv_bfloat16* p = src + static_cast<int64_t>(row0 + first) * ld + col;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            v[i] = *reinterpret_cast<const uint4*>(p + i * 4 * ld);
+        for (int i = 0; i < U; ++i) {
+            v[i] = *reinterpret_cast<const uint4*>(p + i * ROWS * ld);
         }
     }
     else {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            const int row = row0 + i * 4 + (lane >> 3);
+        for (int i = 0; i < U; ++i) {
+            const int row = row0 + i * ROWS + first;
             v[i]          = make_uint4(0u, 0u, 0u, 0u);
             if (row < M) {
                 const __nv_bfloat16* p = src + static_cast<int64_t>(row) * ld + col;
@@ -775,35 +847,37 @@ __device__ __forceinline__ void stage_in(uint32_t stage, const __nv_bfloat16* sr
     }
     __syncwarp();  // the buffer's previous contents have been read
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        ptx::st_shared_v4(stage_unit(stage, i * 4 + (lane >> 3), unit), v[i]);
+    for (int i = 0; i < U; ++i) {
+        ptx::st_shared_v4(stage_unit(stage, i * ROWS + first, unit), v[i]);
     }
     __syncwarp();
 }
 
 // The rows of the staging buffer to a bf16 matrix. The caller's threads have each written their row.
+template <int W>
 __device__ __forceinline__ void stage_out(uint32_t stage, __nv_bfloat16* dst, int64_t ld, int row0, int col0, int M, int N,
                                           int lane)
 {
-    const int unit = lane & 7, col = col0 + unit * 8;
-    uint4     v[8];
+    constexpr int U = W / 8, ROWS = 32 / U;
+    const int     unit = lane % U, col = col0 + unit * 8, first = lane / U;
+    uint4         v[U];
     __syncwarp();
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        v[i] = ptx::ld_shared_v4(stage_unit(stage, i * 4 + (lane >> 3), unit));
+    for (int i = 0; i < U; ++i) {
+        v[i] = ptx::ld_shared_v4(stage_unit(stage, i * ROWS + first, unit));
     }
     __syncwarp();  // the buffer may be refilled
-    if (row0 + 32 <= M && col0 + 64 <= N) {  // warp-uniform
-        __nv_bfloat16* p = dst + static_cast<int64_t>(row0 + (lane >> 3)) * ld + col;
+    if (row0 + 32 <= M && col0 + W <= N) {  // warp-uniform
+        __nv_bfloat16* p = dst + static_cast<int64_t>(row0 + first) * ld + col;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            ptx::st_v4(p + i * 4 * ld, v[i]);
+        for (int i = 0; i < U; ++i) {
+            ptx::st_v4(p + i * ROWS * ld, v[i]);
         }
         return;
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const int row = row0 + i * 4 + (lane >> 3);
+    for (int i = 0; i < U; ++i) {
+        const int row = row0 + i * ROWS + first;
         if (row < M) {
             __nv_bfloat16* p = dst + static_cast<int64_t>(row) * ld + col;
             if (col + 8 <= N) {

@@ -57,3 +57,34 @@ def test_epilogues_on_ragged_tiles(pair, act, m, n, k):
         torch.nn.functional.gelu(x, approximate="tanh").sum().backward()
         y = y * x.grad
     assert rel_err(got, (y + res.double()).float()) < 4e-3
+
+
+# few tiles and a long K: two, four or eight CTAs share the K-blocks of a tile, the last with fewer
+@pytest.mark.parametrize("act", [0, 1, 3])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 8192), (128, 128, 4104), (129, 264, 3000), (64, 1000, 8000), (300, 520, 5000),
+                                   (500, 1600, 4096), (700, 1416, 4160), (1000, 1024, 6000)])
+def test_k_shared_by_a_cluster(act, m, n, k):
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda").bfloat16()
+    b = (torch.randn(n, k, device="cuda") * 0.02).bfloat16()
+    bias, res, aux = torch.randn(n, device="cuda"), torch.randn(m, n, device="cuda").bfloat16(), torch.randn(m, n, device="cuda").bfloat16()
+    pre = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
+    kw = dict(bias=bias, residual=res, act=act, aux=aux if act == 3 else None)
+    got = gemm.gemm_bf16(a, b, store_pre=pre, **kw)
+    again = gemm.gemm_bf16(a, b, **kw)
+    whole = gemm.gemm_bf16(a, b, pair=False, **kw)
+    turned = gemm.gemm_bf16(a.t().contiguous(), b.t().contiguous(), a_km=True, b_kn=True, **kw) if m % 8 == 0 else got
+    gemm.check_errors()
+    assert torch.equal(got, again) and torch.equal(got, turned)
+    y = a.double() @ b.double().t() + bias.double()
+    assert rel_err(pre, y.float()) < 4e-3
+    # the same products summed in fp32 in another order, then rounded to bf16 once: equal but for a few
+    # results that lie at the edge between two bf16 numbers
+    assert rel_err(got, whole.float()) < 1e-3
+    if act == 1:
+        y = torch.nn.functional.gelu(y, approximate="tanh")
+    elif act == 3:
+        x = aux.double().requires_grad_()
+        torch.nn.functional.gelu(x, approximate="tanh").sum().backward()
+        y = y * x.grad
+    assert rel_err(got, (y + res.double()).float()) < 4e-3
