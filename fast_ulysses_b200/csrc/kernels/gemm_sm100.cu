@@ -180,7 +180,14 @@ template <int MB, int NB, int ACT>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WIDE_THREADS, 1) gemm_wide_kernel(const __grid_constant__ PlainArgs<ACT> a)
 {
     PlainEpi<ACT> epi = a.epi;
-    run_wide<MB, NB>(a.core, epi);
+    run_wide<MB, NB, false>(a.core, epi);
+}
+
+template <int ACT>
+__global__ void __launch_bounds__(WIDE_THREADS, 1) gemm_wide_split_kernel(const __grid_constant__ PlainArgs<ACT> a)
+{
+    PlainEpi<ACT> epi = a.epi;
+    run_wide<1, 2, true>(a.core, epi);
 }
 
 template <int ACT>
@@ -394,7 +401,7 @@ template <int MB, int NB>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WIDE_THREADS, 1) qkv_wide_kernel(const __grid_constant__ QkvArgs a)
 {
     QkvEpi<32 * WIDE_EPI_WARPS> epi(a.epi);
-    run_wide<MB, NB>(a.core, epi);
+    run_wide<MB, NB, false>(a.core, epi);
 }
 
 __global__ void __launch_bounds__(SMALL_THREADS, 1) qkv_small_kernel(const __grid_constant__ QkvArgs a)
@@ -717,6 +724,7 @@ struct Choice {
     Shape  shape;
     int    tiles_m, tiles_n, full, items;
     double cost;
+    int    rest = 0, csize = 1;  // kBroad: blocks beyond `items`, shared by clusters of `csize` CTAs
 };
 
 Choice wide_choice(int64_t m, int64_t n, double kb, Shape shape, int pairs)
@@ -745,6 +753,47 @@ Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int fla
         return wide;
     }
     return small.cost < wide.cost ? small : wide;
+}
+
+// The broad tiles with what whole waves leave over shared by clusters (gemm_wide_split_kernel), when that is
+// estimated to be faster than `best`. Measured (us): a wave of clusters takes 8.1 (two pairs) or 9.4 (four) and
+// 0.29 per K-block of a pair's share; behind another launch 1.5 of that are hidden. 2000 x 5120 x 5120 (80 tiles
+// on 74 pairs): 83.5 -> 79.5, 1000 x 5120 x 13824 (40 tiles: a wave of blocks and six more): 130 -> 115.
+Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, int pairs)
+{
+    static fu::ClusterCapacity capacity;
+    const int64_t              kb = (k + BK - 1) / BK;
+    Choice                     chosen = best;
+    const Choice               broad  = wide_choice(m, n, static_cast<double>(kb), Shape::kBroad, pairs);
+    const int64_t              tiles = static_cast<int64_t>(broad.tiles_m) * broad.tiles_n, full = tiles / pairs * pairs;
+    const int64_t              blocks = 2 * (tiles - full), single = blocks / pairs * pairs, rest = blocks - single;
+    int                        dev = 0;
+    if (rest == 0 || cudaGetDevice(&dev) != cudaSuccess) {
+        return best;
+    }
+    const double before =
+        full + single > 0 ? 6.0 - 1.5 + 0.305 * kb * (2.0 * (full / pairs) + 1.05 * (single / pairs)) : 0.0;
+    for (const int csize : {4, 8}) {
+        const int64_t parts = csize / 2, share = (kb + parts - 1) / parts;
+        const double  wave  = (csize == 4 ? 8.1 : 9.4) + 0.29 * share;
+        if ((kb + share - 1) / share != parts || before + wave >= chosen.cost) {
+            continue;  // a pair would have nothing to do, or no gain even in one wave
+        }
+        const int cap = capacity.of(gemm_wide_split_kernel<0>, csize, dev, WIDE_THREADS, WIDE_SMEM_BYTES);
+        if (cap < 1) {
+            continue;
+        }
+        const double cost = before + static_cast<double>((rest + cap - 1) / cap) * wave;
+        if (cost < chosen.cost) {
+            chosen       = broad;
+            chosen.full  = static_cast<int>(full);
+            chosen.items = static_cast<int>(full + single);
+            chosen.cost  = cost;
+            chosen.rest  = static_cast<int>(rest);
+            chosen.csize = csize;
+        }
+    }
+    return chosen;
 }
 
 // How many CTAs share the K-blocks of a 128 x 128 tile (1: none do), see run_small, when that is estimated
@@ -873,21 +922,22 @@ int launch_small(Kernel kernel, const Args& a, int ctas, cudaStream_t stream)
 }
 
 template <int ACT>
-int launch_split(const PlainArgs<ACT>& a, int csize, cudaStream_t stream)
+int launch_clusters(void (*kernel)(PlainArgs<ACT>), const PlainArgs<ACT>& a, int clusters, int csize, int threads, int smem,
+                    cudaStream_t stream)
 {
-    const int rc = set_smem(gemm_split_kernel<ACT>, SMALL_SMEM_BYTES);
+    const int rc = set_smem(kernel, smem);
     if (rc != FU_OK) {
         return rc;
     }
     cudaLaunchConfig_t  cfg  = {};
     cudaLaunchAttribute attr = fu::cluster_attr(csize);
-    cfg.gridDim              = dim3(static_cast<unsigned>(a.core.items * csize), 1, 1);
-    cfg.blockDim             = dim3(SMALL_THREADS, 1, 1);
-    cfg.dynamicSmemBytes     = SMALL_SMEM_BYTES;
+    cfg.gridDim              = dim3(static_cast<unsigned>(clusters * csize), 1, 1);
+    cfg.blockDim             = dim3(static_cast<unsigned>(threads), 1, 1);
+    cfg.dynamicSmemBytes     = static_cast<size_t>(smem);
     cfg.stream               = stream;
     cfg.attrs                = &attr;
     cfg.numAttrs             = 1;
-    FU_CUDA_OK(cudaLaunchKernelEx(&cfg, gemm_split_kernel<ACT>, a));
+    FU_CUDA_OK(cudaLaunchKernelEx(&cfg, kernel, a));
     return FU_OK;
 }
 
@@ -895,7 +945,11 @@ template <int ACT>
 int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream_t stream)
 {
     PlainArgs<ACT> a{};
-    const int      csize = g->ctas > 0 || (flags & (FU_GEMM_SINGLE | FU_GEMM_PAIR)) ? 1 : choose_split(c, g->m, g->n, g->k);
+    int            csize = 1;
+    if (g->ctas <= 0 && !(flags & (FU_GEMM_SINGLE | FU_GEMM_PAIR))) {
+        c     = choose_wide_split(c, g->m, g->n, g->k, pairs);
+        csize = choose_split(c, g->m, g->n, g->k);
+    }
     if (csize > 1) {
         c = choose_shape(g->m, g->n, g->k, pairs, 1, FU_GEMM_SINGLE);
     }
@@ -913,7 +967,13 @@ int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream
     a.epi.aux       = static_cast<const __nv_bfloat16*>(g->aux);
     a.epi.c_pre     = static_cast<__nv_bfloat16*>(g->c_pre);
     if (csize > 1) {
-        return launch_split<ACT>(a, csize, stream);
+        return launch_clusters<ACT>(gemm_split_kernel<ACT>, a, a.core.items, csize, SMALL_THREADS, SMALL_SMEM_BYTES, stream);
+    }
+    if (c.rest > 0) {
+        a.core.first = c.items;
+        const int rc = c.items > 0 ? launch_pairs(gemm_wide_kernel<1, 2, ACT>, a, pairs, stream) : FU_OK;
+        return rc != FU_OK ? rc
+                           : launch_clusters<ACT>(gemm_wide_split_kernel<ACT>, a, c.rest, c.csize, WIDE_THREADS, WIDE_SMEM_BYTES, stream);
     }
     switch (c.shape) {
     case Shape::kTall: return launch_pairs(gemm_wide_kernel<2, 1, ACT>, a, pairs, stream);

@@ -280,6 +280,9 @@ __device__ __forceinline__ void pair_tile_coords(int tiles_m, int tiles_n, int b
     mt                   = band * band_rows + (r - nt * rows);
 }
 
+// SPLIT: what whole waves leave over. A cluster of two or four pairs takes one block, each pair a part of its
+// K-blocks; the CTAs with the same rows add up their sums as run_small's do, 256 / pairs columns each.
+//
 // The schedule: `full` whole tiles, then the remaining tiles block by block (two items each), which the
 // host asks for when half as many items as pairs are left, so that the last wave is half as long.
 struct WideCore {
@@ -287,6 +290,7 @@ struct WideCore {
     int         M, N, K;
     int         tiles_m, tiles_n;  // of MB * 256 x NB * 256
     int         full, items;
+    int         first;             // split kernel: the item of cluster 0
     int         a_mn, b_mn;
     uint32_t*   err;
 };
@@ -323,7 +327,7 @@ struct WideItem {
     __device__ __forceinline__ int col(int u) const { return n0 + (NB == 2 ? u * 256 : 0); }
 };
 
-template <int MB, int NB, class Epi>
+template <int MB, int NB, bool SPLIT, class Epi>
 __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
 {
     static_assert(MB * NB == 2, "two blocks of 256 x 256");
@@ -335,9 +339,15 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
     uint8_t*       ring = smem_raw + (base - ptx::smem_addr(smem_raw));
     const int      warp = static_cast<int>(ptx::uniform(threadIdx.x >> 5));
     const int      lane = threadIdx.x & 31;
-    const int      half = static_cast<int>(ptx::uniform(ptx::cluster_ctarank()));  // 0: issues the MMAs; 1: the other rows
-    const int      pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
-    const int      kblocks = (core.K + BK - 1) / BK;
+    const int      crank = static_cast<int>(ptx::uniform(ptx::cluster_ctarank()));
+    const int      csize = SPLIT ? static_cast<int>(ptx::uniform(ptx::cluster_nctarank())) : 2;
+    const int      half  = crank & 1;  // 0: issues the MMAs; 1: the other rows
+    const int      part = crank >> 1, parts = csize >> 1;
+    const uint32_t even = static_cast<uint32_t>(crank & ~1);  // the pair's issuing CTA
+    const int      all_kb = (core.K + BK - 1) / BK, share = SPLIT ? (all_kb + parts - 1) / parts : all_kb;
+    const int      kb_0 = part * share, kblocks = SPLIT ? min(share, all_kb - kb_0) : all_kb;  // this pair's K-blocks
+    const int      w_0 = SPLIT ? core.first + static_cast<int>(blockIdx.x) / csize : static_cast<int>(blockIdx.x >> 1);
+    const int      w_end = SPLIT ? w_0 + 1 : core.items, w_inc = SPLIT ? 1 : static_cast<int>(gridDim.x >> 1);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < WIDE_STAGES; ++s) {
@@ -369,7 +379,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
     if (warp == 0) {
         uint32_t stage = 0, phase = 1;
         bool     ok    = true;
-        for (int w = pair; w < core.items && ok; w += npairs) {
+        for (int w = w_0; w < w_end && ok; w += w_inc) {
             const WideItem<MB, NB> item(core, w);
             if (item.u0 == item.u1) {
                 continue;
@@ -392,11 +402,11 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                     const int      m  = item.m0 + u * 256 + half * 128;
                     const uint32_t to = sa + u * WIDE_BLOCK_BYTES;
                     if (!core.a_mn) {
-                        ptx::tma_load_2d_pair_if(to, &core.map_a, kb * BK, m, bar, leader);
+                        ptx::tma_load_2d_pair_if(to, &core.map_a, (kb_0 + kb) * BK, m, bar, leader);
                     }
                     else {  // 64 (k) x 64 (m) blocks of 8 KiB
-                        ptx::tma_load_2d_pair_if(to, &core.map_a, m, kb * BK, bar, leader);
-                        ptx::tma_load_2d_pair_if(to + 8192, &core.map_a, m + 64, kb * BK, bar, leader);
+                        ptx::tma_load_2d_pair_if(to, &core.map_a, m, (kb_0 + kb) * BK, bar, leader);
+                        ptx::tma_load_2d_pair_if(to + 8192, &core.map_a, m + 64, (kb_0 + kb) * BK, bar, leader);
                     }
                 }
 #pragma unroll
@@ -407,11 +417,11 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                     const int      n  = item.n0 + u * 256 + half * 128;
                     const uint32_t to = sb + u * WIDE_BLOCK_BYTES;
                     if (!core.b_mn) {
-                        ptx::tma_load_2d_pair_if(to, &core.map_b, kb * BK, n, bar, leader);
+                        ptx::tma_load_2d_pair_if(to, &core.map_b, (kb_0 + kb) * BK, n, bar, leader);
                     }
                     else {
-                        ptx::tma_load_2d_pair_if(to, &core.map_b, n, kb * BK, bar, leader);
-                        ptx::tma_load_2d_pair_if(to + 8192, &core.map_b, n + 64, kb * BK, bar, leader);
+                        ptx::tma_load_2d_pair_if(to, &core.map_b, n, (kb_0 + kb) * BK, bar, leader);
+                        ptx::tma_load_2d_pair_if(to + 8192, &core.map_b, n + 64, (kb_0 + kb) * BK, bar, leader);
                     }
                 }
                 if (++stage == WIDE_STAGES) {
@@ -436,6 +446,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
             const uint32_t  tfull_b = ptx::smem_addr(tmem_full), tempty_b = ptx::smem_addr(tmem_empty);
             uint32_t        stage = 0, phase = 0, uses0 = 0, uses1 = 0;
             uint32_t        gave_up = ERR_NONE;
+            const uint32_t  both = 3u << even;
             auto issue = [&](int u, uint32_t s, uint32_t accumulate) {  // one K-block into block u
                 const ptx::Desc a = a_desc.at(s * WIDE_STAGE_BYTES + (MB == 2 ? u * WIDE_BLOCK_BYTES : 0));
                 const ptx::Desc b = b_desc.at(s * WIDE_STAGE_BYTES + (NB == 2 ? u * WIDE_BLOCK_BYTES : 0));
@@ -450,7 +461,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                     ph ^= 1u;
                 }
             };
-            for (int w = pair; w < core.items && !gave_up; w += npairs) {
+            for (int w = w_0; w < w_end && !gave_up; w += w_inc) {
                 const WideItem<MB, NB> item(core, w);
                 if (item.u0 == item.u1) {
                     continue;
@@ -468,7 +479,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                             ptx::tc_fence_after();
                             issue(0, stage, 1u);
                             issue(1, stage, 1u);
-                            ptx::mma_commit_if<2>(empty_b + stage * 8, leader);
+                            ptx::mma_commit_if<2>(empty_b + stage * 8, leader, both);
                             advance(stage, phase);
                         }
                         kb += n;
@@ -499,12 +510,12 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                             }
                             issue(u, s, static_cast<uint32_t>(kb | i));
                             if (u + 1 == item.u1) {
-                                ptx::mma_commit_if<2>(empty_b + s * 8, leader);
+                                ptx::mma_commit_if<2>(empty_b + s * 8, leader, both);
                             }
                             advance(s, ph);
                         }
                         if (!gave_up && run == left) {
-                            ptx::mma_commit_if<2>(tfull_b + u * 8, leader);
+                            ptx::mma_commit_if<2>(tfull_b + u * 8, leader, both);
                         }
                     }
                     stage = s;
@@ -518,6 +529,10 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
         }
         __syncwarp();
     }
+    if (SPLIT) {  // the epilogue warps' exchange
+        ptx::cluster_sync();
+        ptx::cluster_sync();
+    }
     }
     else {
         ptx::setmaxnreg_inc<WIDE_REGS_EPI>();
@@ -528,9 +543,64 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
         if (Epi::kPeers) {
             epi.open(threadIdx.x - 32 * WIDE_FIRST_EPI);
         }
+        if constexpr (SPLIT) {
+            const WideItem<MB, NB> item(core, w_0);
+            bool                   ok = item.u0 != item.u1;  // an empty item only takes part in the barriers
+            if (ok && !ptx::mbar_wait(&tmem_full[item.u0], 0u)) {
+                flag_error(core.err, ERR_EPI_WAIT);
+                ok = false;
+            }
+            ptx::tc_fence_after();
+            const uint32_t taddr = tmem_base + item.u0 * 256 + (static_cast<uint32_t>(quarter * 32) << 16);
+            const int      width = 256 / parts;
+            const uint32_t slot  = base + quarter * 32768 + lane * 16;  // this warp's rows: [columns / 4][lane] of 16 bytes per pair
+            ptx::cluster_sync();  // every pair's products are complete: its stages may be overwritten
+#pragma unroll 1
+            for (int ch = 0; ok && ch < 8; ++ch) {
+                const int      col = cg * 128 + ((ch + 2 * part) & 7) * 16, owner = col / width;
+                const uint32_t dst = ptx::cluster_addr(slot + (part * width + col - owner * width) * 128, owner * 2 + half);
+                uint32_t       r[16];
+                ptx::tmem_ld_32x16(taddr + col, r);
+                ptx::tmem_ld_wait();
+#pragma unroll
+                for (int g = 0; g < 4; ++g) {
+                    ptx::st_cluster_v4(dst + g * 512, r[4 * g], r[4 * g + 1], r[4 * g + 2], r[4 * g + 3]);
+                }
+            }
+            ptx::cluster_sync();
+            auto finish = [&](auto w) {
+                constexpr int W = decltype(w)::value;
+                float         v[W];
+#pragma unroll
+                for (int k = 0; k < W; ++k) {
+                    v[k] = 0.0f;
+                }
+#pragma unroll 1
+                for (int from = 0; from < parts; ++from) {
+#pragma unroll
+                    for (int g = 0; g < W / 4; ++g) {
+                        const uint4 q = ptx::ld_shared_v4(slot + (from * 2 * W + cg * W + g * 4) * 128);
+                        v[4 * g] += __uint_as_float(q.x);
+                        v[4 * g + 1] += __uint_as_float(q.y);
+                        v[4 * g + 2] += __uint_as_float(q.z);
+                        v[4 * g + 3] += __uint_as_float(q.w);
+                    }
+                }
+                epi.template piece<W>(v, item.row(item.u0) + half * 128 + quarter * 32, item.col(item.u0) + (2 * part + cg) * W, lane, stage);
+            };
+            if (ok) {
+                if (parts == 2) {
+                    finish(std::integral_constant<int, 64>{});
+                }
+                else {
+                    finish(std::integral_constant<int, 32>{});
+                }
+            }
+        }
+        else {
         uint32_t uses[2] = {0, 0};
         bool     ok      = true;
-        for (int w = pair; w < core.items && ok; w += npairs) {
+        for (int w = w_0; w < w_end && ok; w += w_inc) {
             const WideItem<MB, NB> item(core, w);
             for (int u = item.u0; u < item.u1; ++u) {
                 if (!ptx::mbar_wait(&tmem_full[u], uses[u] & 1u)) {
@@ -545,10 +615,11 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                 ptx::tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
-                    ptx::mbar_arrive_cluster(ptx::cluster_addr(&tmem_empty[u], 0));
+                    ptx::mbar_arrive_cluster(ptx::cluster_addr(&tmem_empty[u], even));
                 }
                 epi.unit(r, item.row(u) + half * 128 + quarter * 32, item.col(u) + cg * 128, lane, stage);
             }
+        }
         }
         if (Epi::kPeers) {
             epi.close(threadIdx.x - 32 * WIDE_FIRST_EPI);

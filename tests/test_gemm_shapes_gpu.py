@@ -88,3 +88,26 @@ def test_k_shared_by_a_cluster(act, m, n, k):
         torch.nn.functional.gelu(x, approximate="tanh").sum().backward()
         y = y * x.grad
     assert rel_err(got, (y + res.double()).float()) < 4e-3
+
+
+# more 256 x 256 blocks than whole waves of pairs: the rest, some of it outside the result, is shared by
+# clusters of two or four pairs along K; with and without a launch before it, ragged in every direction
+@pytest.mark.parametrize("act", [0, 1, 3])
+@pytest.mark.parametrize("m,n,k", [(1000, 5120, 5120), (512, 5120, 6016), (2000, 5128, 2568), (1800, 5000, 4104), (257, 10000, 4096),
+                                   (4100, 4096, 1544), (2048, 5120, 5120)])
+def test_rest_shared_by_clusters_of_pairs(act, m, n, k):
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda").bfloat16()
+    b = (torch.randn(n, k, device="cuda") * 0.02).bfloat16()
+    bias, res, aux = torch.randn(n, device="cuda"), torch.randn(m, n, device="cuda").bfloat16(), torch.randn(m, n, device="cuda").bfloat16()
+    pre = torch.empty(m, n, device="cuda", dtype=torch.bfloat16)
+    kw = dict(bias=bias, residual=res, act=act, aux=aux if act == 3 else None)
+    got = gemm.gemm_bf16(a, b, store_pre=pre, **kw)
+    again = gemm.gemm_bf16(a, b, **kw)
+    whole = gemm.gemm_bf16(a, b, pair=True, **kw)
+    turned = gemm.gemm_bf16(a.t().contiguous(), b.t().contiguous(), a_km=True, b_kn=True, **kw) if m % 8 == 0 else got
+    gemm.check_errors()
+    assert torch.equal(got, again) and torch.equal(got, turned)
+    # the same products summed in fp32 in another order, then rounded to bf16 once
+    assert rel_err(got, whole.float()) < 1e-3
+    assert rel_err(pre, a.float() @ b.float().t() + bias) < 4e-3
