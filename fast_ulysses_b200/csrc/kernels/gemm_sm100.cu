@@ -72,9 +72,9 @@ struct PlainEpi {
         }
     }
 
-    // W columns of 32 rows, a row per thread
+    // W columns of 32 rows, a row per thread; none from column N on
     template <int W>
-    __device__ __forceinline__ void piece(float (&v)[W], int row0, int col0, int lane, uint32_t stage) const
+    __device__ __forceinline__ void piece(float (&v)[W], int row0, int col0, int N, int lane, uint32_t stage) const
     {
         if (row0 >= M || col0 >= N) {
             return;  // warp-uniform
@@ -154,19 +154,20 @@ struct PlainEpi {
         stage_out<W>(stage, c, ldc, row0, col0, M, N, lane);
     }
 
-    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage) const
+    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int col_end, int lane, uint32_t stage) const
     {
-        float v[64];
+        const int end = min(N, col_end);
+        float     v[64];
 #pragma unroll
         for (int j = 0; j < 64; ++j) {
             v[j] = __uint_as_float(r[j]);
         }
-        piece<64>(v, row0, col0, lane, stage);
+        piece<64>(v, row0, col0, end, lane, stage);
 #pragma unroll
         for (int j = 0; j < 64; ++j) {
             v[j] = __uint_as_float(r[64 + j]);
         }
-        piece<64>(v, row0, col0 + 64, lane, stage);
+        piece<64>(v, row0, col0 + 64, end, lane, stage);
     }
 };
 
@@ -352,7 +353,7 @@ struct QkvEpi {
         stage_out<64>(stage, p.y_save, p.ld_y, row0, col0 + H * 64, p.M, 0x7fffffff, lane);
     }
 
-    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage) const
+    __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int, int lane, uint32_t stage) const
     {
         const int head_global = col0 / HEAD_DIM;
         const int type        = head_global / p.heads;  // 0 q, 1 k, 2 v
@@ -713,44 +714,89 @@ int pair_capacity()
 
 // Which core and tile a problem gets, from its size alone: the one whose estimated time is lowest. The
 // estimate is a start-and-end time plus, per wave of CTAs, a time per 64-wide K-block, both measured
-// (us, SM clock 1.9 GHz, problems of 64 - 2048 rows and 256 - 5120 columns and K):
+// (us, SM clock 1.9 GHz, problems of 64 - 4100 rows and 256 - 13824 columns and K):
 //   128 x 128 tiles on single CTAs   3.2 + 0.225 per K-block and wave of 148
-//   256 x 256 blocks on pairs        6 + 0.305 per K-block and block of each wave of 74 (a whole tile is two
-//                                    blocks; a block by itself takes 1.05)
-// Of the two wide orientations, which move the same bytes, the one with the fuller last wave wins; when at
-// most half as many tiles as pairs are left over, those are split into blocks.
-enum class Shape { kSmall, kTall, kBroad };  // 128 x 128; 512 x 256; 256 x 512
+//   two 256 x 256 blocks on pairs    6 + 0.61 per K-block and wave of 74, 0.32 for a wave of single blocks
+//   one 256 x 256 block on pairs     6 + 0.30
+// Rows of an operand that do not all start on a 32-byte sector (a pitch that is an odd multiple of 16 bytes)
+// reach shared memory more slowly: the K-blocks of a 128 x 128 tile take 0.265 us with one such operand and 0.385
+// with two, those of a single block on a pair 0.34 and 0.37, of two blocks 0.65 and 0.69 (256 x 3328 x 4096 with
+// small tiles: 18.1, 21.3 and 28.6 us). The pair kernels' time per K-block shrinks with the width of the block, see block_clocks(). At most half as
+// many tiles of two blocks as pairs left over are split into blocks.
+// What the widths and the single block gave, against two blocks of 256 columns or the small tiles: 1000 x 5120 x
+// 5120 53.0 -> 41.8 us (two of 160), 512 x 5120 x 13824 81.6 -> 61.6 and 512 x 5120 x 5120 30.4 -> 25.8 (one of
+// 160), 4100 x 1536 x 4096 58.9 -> 47.2 (two of 192).
+enum class Shape { kSmall, kTall, kBroad, kOne };  // 128 x 128; 512 x width; 256 x 2 width; 256 x width
 struct Choice {
     Shape  shape;
     int    tiles_m, tiles_n, full, items;
     double cost;
+    int    width = 256;
     int    rest = 0, csize = 1;  // kBroad: blocks beyond `items`, shared by clusters of `csize` CTAs
 };
 
-Choice wide_choice(int64_t m, int64_t n, double kb, Shape shape, int pairs)
+// What bounds a K-block of a pair's tile of mb x nb blocks: the tensor pipe takes width / 2 clocks per MMA; shared
+// memory moves 128 bytes a clock, 4 KiB of A and 16 * width bytes of B for each MMA and the operands' own
+// 16 KiB per block row and 64 * width bytes per block column once.
+double block_clocks(int mb, int nb, int width)
 {
-    const int64_t tm    = shape == Shape::kTall ? (m + 511) / 512 : (m + 255) / 256;
-    const int64_t tn    = shape == Shape::kTall ? (n + 255) / 256 : (n + 511) / 512;
-    const int64_t tiles = tm * tn, left = tiles % pairs;
-    const int64_t full = 2 * left <= pairs ? tiles - left : tiles;
-    const int64_t items = full + 2 * (tiles - full);
-    return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(full), static_cast<int>(items),
-            6.0 + 0.305 * kb * (2.0 * ((full + pairs - 1) / pairs) + 1.05 * ((items - full + pairs - 1) / pairs))};
+    const double tensor = 4.0 * mb * nb * width / 2;
+    const double shared = (4.0 * mb * nb * (4096 + 16 * width) + 16384.0 * mb + 64.0 * width * nb) / 128;
+    return std::max(tensor, shared);
 }
 
-Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int flags)
+// us per K-block, by how many of the two operands lie off the 32-byte sectors
+constexpr double kSmallBlock[3] = {0.225, 0.265, 0.385}, kOneBlock[3] = {0.30, 0.34, 0.37}, kTwoBlocks[3] = {0.61, 0.65, 0.69};
+
+int off_sectors(const void* a, int64_t lda, const void* b, int64_t ldb)
+{
+    auto off = [](const void* p, int64_t ld) { return ld % 16 != 0 || (reinterpret_cast<uintptr_t>(p) & 31u) != 0; };
+    return (off(a, lda) ? 1 : 0) + (off(b, ldb) ? 1 : 0);
+}
+
+Choice wide_choice(int64_t m, int64_t n, double kb, Shape shape, int width, int pairs, int off)
+{
+    const int     mb = shape == Shape::kTall ? 2 : 1, nb = shape == Shape::kBroad ? 2 : 1;
+    const int64_t tm = (m + 256 * mb - 1) / (256 * mb), tn = (n + width * nb - 1) / (width * nb), tiles = tm * tn;
+    if (shape == Shape::kOne) {
+        return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(tiles), static_cast<int>(tiles),
+                6.0 + kb * kOneBlock[off] / 512 * block_clocks(1, 1, width) * ((tiles + pairs - 1) / pairs), width};
+    }
+    const int64_t left = tiles % pairs, full = 2 * left <= pairs ? tiles - left : tiles, items = full + 2 * (tiles - full);
+    return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(full), static_cast<int>(items),
+            6.0 + kb * (kTwoBlocks[off] / 1024 * block_clocks(mb, nb, width) * ((full + pairs - 1) / pairs)
+                        + 1.05 * kOneBlock[off] / 512 * block_clocks(1, 1, width) * ((items - full + pairs - 1) / pairs)), width};
+}
+
+// `narrow`: the epilogue takes blocks of any width (the heads of the QKV projection need 128 columns at once).
+Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int flags, bool narrow, int off)
 {
     const int64_t t128 = ((m + 127) / 128) * ((n + 127) / 128);
     const double  kb   = static_cast<double>((k + BK - 1) / BK);
     const Choice  small{Shape::kSmall, static_cast<int>((m + 127) / 128), static_cast<int>((n + 127) / 128), 0,
-                       static_cast<int>(t128), 3.2 + 0.225 * kb * ((t128 + sms - 1) / sms)};
+                       static_cast<int>(t128), 3.2 + kSmallBlock[off] * kb * ((t128 + sms - 1) / sms)};
     if (flags & FU_GEMM_SINGLE) {
         return small;
     }
-    const Choice tall = wide_choice(m, n, kb, Shape::kTall, pairs), broad = wide_choice(m, n, kb, Shape::kBroad, pairs);
-    const Choice wide = tall.cost < broad.cost ? tall : broad;
+    const Choice tall = wide_choice(m, n, kb, Shape::kTall, 256, pairs, off), broad = wide_choice(m, n, kb, Shape::kBroad, 256, pairs, off);
+    Choice       wide = tall.cost < broad.cost ? tall : broad;
     if (flags & FU_GEMM_PAIR) {
         return wide;
+    }
+    if (narrow) {
+        Choice best = wide;
+        for (int width = 256; width >= 96; width -= 32) {
+            if ((flags & FU_GEMM_B_KN) && width % 128 != 0) {
+                continue;  // such a B comes in blocks of 64 columns, half of them for each CTA
+            }
+            for (const Shape shape : {Shape::kTall, Shape::kBroad, Shape::kOne}) {
+                const Choice c = wide_choice(m, n, kb, shape, width, pairs, off);
+                best           = c.cost < best.cost ? c : best;
+            }
+        }
+        if (best.cost < 0.96 * wide.cost) {  // whole blocks where it makes little difference: they take less power
+            wide = best;
+        }
     }
     return small.cost < wide.cost ? small : wide;
 }
@@ -759,12 +805,12 @@ Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int fla
 // estimated to be faster than `best`. Measured (us): a wave of clusters takes 8.1 (two pairs) or 9.4 (four) and
 // 0.29 per K-block of a pair's share; behind another launch 1.5 of that are hidden. 2000 x 5120 x 5120 (80 tiles
 // on 74 pairs): 83.5 -> 79.5, 1000 x 5120 x 13824 (40 tiles: a wave of blocks and six more): 130 -> 115.
-Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, int pairs)
+Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, int pairs, int off)
 {
     static fu::ClusterCapacity capacity;
     const int64_t              kb = (k + BK - 1) / BK;
     Choice                     chosen = best;
-    const Choice               broad  = wide_choice(m, n, static_cast<double>(kb), Shape::kBroad, pairs);
+    const Choice               broad  = wide_choice(m, n, static_cast<double>(kb), Shape::kBroad, 256, pairs, off);
     const int64_t              tiles = static_cast<int64_t>(broad.tiles_m) * broad.tiles_n, full = tiles / pairs * pairs;
     const int64_t              blocks = 2 * (tiles - full), single = blocks / pairs * pairs, rest = blocks - single;
     int                        dev = 0;
@@ -772,12 +818,12 @@ Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, in
         return best;
     }
     const double before =
-        full + single > 0 ? 6.0 - 1.5 + 0.305 * kb * (2.0 * (full / pairs) + 1.05 * (single / pairs)) : 0.0;
+        full + single > 0 ? 6.0 - 1.5 + kb * (kTwoBlocks[off] * (full / pairs) + 1.05 * kOneBlock[off] * (single / pairs)) : 0.0;
     for (const int csize : {4, 8}) {
         const int64_t parts = csize / 2, share = (kb + parts - 1) / parts;
-        const double  wave  = (csize == 4 ? 8.1 : 9.4) + 0.29 * share;
-        if ((kb + share - 1) / share != parts || before + wave >= chosen.cost) {
-            continue;  // a pair would have nothing to do, or no gain even in one wave
+        const double  wave  = (csize == 4 ? 8.1 : 9.4) + 0.97 * kOneBlock[off] * share;
+        if ((kb + share - 1) / share != parts || before + wave >= 0.96 * best.cost) {
+            continue;  // a pair would have nothing to do, or no gain beyond the estimate's error even in one wave
         }
         const int cap = capacity.of(gemm_wide_split_kernel<0>, csize, dev, WIDE_THREADS, WIDE_SMEM_BYTES);
         if (cap < 1) {
@@ -800,7 +846,7 @@ Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, in
 // to be faster than `best`. The exchange takes 1.8, 2.4 and 2.8 us beyond the tile's own time (measured, for
 // two, four and eight CTAs). 64 x 2000 x 8000: 30.6 -> 13.3 us with four, 64 x 512 x 2048: 10.6 -> 7.0 with eight,
 // 512 x 1536 x 4096: 18.0 -> 13.2 with two; the 160 tiles of 512 x 5120 x 5120 stay as they are.
-int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k)
+int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k, int off)
 {
     static fu::ClusterCapacity capacity;
     const int64_t              t128 = ((m + 127) / 128) * ((n + 127) / 128), kb = (k + BK - 1) / BK;
@@ -811,7 +857,7 @@ int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k)
     }
     for (const int csize : {2, 4, 8}) {
         const int64_t share = (kb + csize - 1) / csize;
-        const double  once  = 3.2 + (csize == 2 ? 1.8 : csize == 4 ? 2.4 : 2.8) + 0.225 * share;
+        const double  once  = 3.2 + (csize == 2 ? 1.8 : csize == 4 ? 2.4 : 2.8) + kSmallBlock[off] * share;
         if ((kb + share - 1) / share != csize || once >= cost) {
             continue;  // a CTA would have nothing to do, or no gain even in one wave
         }
@@ -862,7 +908,7 @@ int fill_wide(WideCore& core, const Choice& c, const void* a, const void* b, int
     if (rc != FU_OK) {
         return rc;
     }
-    rc = core.b_mn ? make_map_2d(&core.map_b, b, 2, k, n, ldb, 64, 64) : make_map_2d(&core.map_b, b, 2, n, k, ldb, 128, BK);
+    rc = core.b_mn ? make_map_2d(&core.map_b, b, 2, k, n, ldb, 64, 64) : make_map_2d(&core.map_b, b, 2, n, k, ldb, c.shape == Shape::kSmall ? 128 : c.width / 2, BK);
     if (rc != FU_OK) {
         return rc;
     }
@@ -873,6 +919,7 @@ int fill_wide(WideCore& core, const Choice& c, const void* a, const void* b, int
     core.tiles_n = c.tiles_n;
     core.full    = c.full;
     core.items   = c.items;
+    core.width   = c.width;
     core.err     = err;
     return FU_OK;
 }
@@ -945,13 +992,14 @@ template <int ACT>
 int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream_t stream)
 {
     PlainArgs<ACT> a{};
+    const int      off = off_sectors(g->a, g->lda, g->b, g->ldb);
     int            csize = 1;
     if (g->ctas <= 0 && !(flags & (FU_GEMM_SINGLE | FU_GEMM_PAIR))) {
-        c     = choose_wide_split(c, g->m, g->n, g->k, pairs);
-        csize = choose_split(c, g->m, g->n, g->k);
+        c     = choose_wide_split(c, g->m, g->n, g->k, pairs, off);
+        csize = choose_split(c, g->m, g->n, g->k, off);
     }
     if (csize > 1) {
-        c = choose_shape(g->m, g->n, g->k, pairs, 1, FU_GEMM_SINGLE);
+        c = choose_shape(g->m, g->n, g->k, pairs, 1, FU_GEMM_SINGLE, false, off);
     }
     const int      rc = fill_wide(a.core, c, g->a, g->b, g->m, g->n, g->k, g->lda, g->ldb, g->err, flags);
     if (rc != FU_OK) {
@@ -978,6 +1026,7 @@ int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream
     switch (c.shape) {
     case Shape::kTall: return launch_pairs(gemm_wide_kernel<2, 1, ACT>, a, pairs, stream);
     case Shape::kBroad: return launch_pairs(gemm_wide_kernel<1, 2, ACT>, a, pairs, stream);
+    case Shape::kOne: return launch_pairs(gemm_wide_kernel<1, 1, ACT>, a, pairs, stream);
     default: return launch_small(gemm_small_kernel<ACT>, a, g->ctas, stream);
     }
 }
@@ -1017,7 +1066,7 @@ extern "C" int fu_gemm_bf16(const FuGemmArgs* g, void* stream_v)
     const bool   forced = pair_default && !(g->flags & FU_GEMM_SINGLE);
     const int    flags  = forced ? (g->flags | FU_GEMM_PAIR) : g->flags;
     const int    sms    = g->ctas > 0 ? std::min(g->ctas, device_sms()) : device_sms();
-    const Choice c      = choose_shape(g->m, g->n, g->k, pairs, sms, flags);
+    const Choice c      = choose_shape(g->m, g->n, g->k, pairs, sms, flags, true, off_sectors(g->a, g->lda, g->b, g->ldb));
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     switch (g->act) {
     case 0: return launch_plain<0>(g, c, pairs, flags, stream);
@@ -1100,7 +1149,7 @@ extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream_v)
     }
     const int    sms   = q->ctas > 0 ? std::min(q->ctas, device_sms()) : device_sms();
     const int    flags = (q->flags & FU_QKV_W_KN) ? FU_GEMM_B_KN : 0;
-    const Choice c     = choose_shape(q->m, n, q->k, pairs, sms, flags);
+    const Choice c     = choose_shape(q->m, n, q->k, pairs, sms, flags, false, off_sectors(q->x, q->ldx, q->w, q->ldw));
     rc = fill_wide(a.core, c, q->x, q->w, q->m, n, q->k, q->ldx, q->ldw, q->err, flags);
     if (rc != FU_OK) {
         return rc;

@@ -223,8 +223,8 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src, Aux aux
 // soon as the registers are loaded, before any arithmetic or store. Epi requirements:
 //   static constexpr bool kPeers          whether open() / close() run (kernels that touch peers)
 //   void open(int epi_tid), close(int epi_tid)          all epilogue threads, once before / after the tiles
-//   void unit(uint32_t (&r)[128], int row0, int col0, int lane, uint32_t stage)
-// `stage` is the address of 4 KiB of shared memory of this warp's own (32 rows x 128 bytes).
+//   void unit(uint32_t (&r)[128], int row0, int col0, int col_end, int lane, uint32_t stage)
+// Columns from `col_end` on are not the unit's. `stage` is the address of 4 KiB of shared memory of this warp's own (32 rows x 128 bytes).
 constexpr int UNIT_STAGE_BYTES = 32 * 128;
 
 __device__ __forceinline__ void load_unit(uint32_t taddr, uint32_t (&r)[128])
@@ -254,11 +254,16 @@ __device__ __forceinline__ void load_unit(uint32_t taddr, uint32_t (&r)[128])
 // 1390 TFLOP/s on the feed-forward shapes, 9450 x 13824 x 5120 and its relatives (cuBLAS 1320 - 1430; the
 // 128 x 256 single-CTA tiles before this kernel 1120 - 1200).
 //
-// There is no second accumulator buffer, so the blocks' order hides the epilogue instead: the first
+// A block may be narrower, `width` = 32 .. 256 columns in steps of 32, and a pair may own a single block (MB =
+// NB = 1, whose accumulators alternate between the halves of tensor memory): both so that a problem of a few
+// waves fills the last one. A narrow or single block makes less of each byte in shared memory, see
+// block_clocks().
+//
+// With two blocks there is no second accumulator buffer, so the blocks' order hides the epilogue instead: the first
 // kStages K-blocks of a tile are multiplied into block 0 and then into block 1, and so are the last
 // ones. Block 0 is finished (and read out) four stages before block 1, and the next tile can start in
 // block 0 while block 1 is still being read out.
-constexpr int WIDE_STAGES      = 4;
+constexpr int WIDE_STAGES      = 4;  // of 48 KiB; six of 32 KiB with one block per pair
 constexpr int WIDE_BLOCK_BYTES = 128 * BK * 2;  // 128 rows of one operand, one K-block
 constexpr int WIDE_STAGE_BYTES = 3 * WIDE_BLOCK_BYTES;
 constexpr int WIDE_EPI_WARPS   = 8;
@@ -288,7 +293,8 @@ __device__ __forceinline__ void pair_tile_coords(int tiles_m, int tiles_n, int b
 struct WideCore {
     CUtensorMap map_a, map_b;
     int         M, N, K;
-    int         tiles_m, tiles_n;  // of MB * 256 x NB * 256
+    int         tiles_m, tiles_n;  // of MB * 256 x NB * width
+    int         width;             // columns of a block
     int         full, items;
     int         first;             // split kernel: the item of cluster 0
     int         a_mn, b_mn;
@@ -302,37 +308,45 @@ __device__ __forceinline__ void flag_error(uint32_t* err, uint32_t code)
     }
 }
 
+// `n`: how many items this pair has had before.
 template <int MB, int NB>
 struct WideItem {
-    int m0, n0, u0, u1;
-    __device__ __forceinline__ WideItem(const WideCore& c, int item)
+    int m0, n0, u0, u1, width;
+    __device__ __forceinline__ WideItem(const WideCore& c, int item, uint32_t n) : width(c.width)
     {
-        const bool whole = item < c.full;
+        const bool whole = MB * NB == 1 || item < c.full;
         const int  rest  = item - c.full;
         int        mt, nt;
         pair_tile_coords(c.tiles_m, c.tiles_n, WIDE_BAND_ROWS / (MB * 256), whole ? item : c.full + (rest >> 1), mt, nt);
         m0 = mt * MB * 256;
-        n0 = nt * NB * 256;
+        n0 = nt * NB * width;
+        if (MB * NB == 1) {
+            u0 = n & 1u;
+            u1 = u0 + 1;
+            return;
+        }
         u0 = whole ? 0 : (rest & 1);
         u1 = whole ? 2 : u0 + 1;
         // a block that lies outside the result altogether is not computed
-        if (u1 == 2 && (MB == 2 ? m0 + 256 >= c.M : n0 + 256 >= c.N)) {
+        if (u1 == 2 && (MB == 2 ? m0 + 256 >= c.M : n0 + width >= c.N)) {
             u1 = 1;
         }
-        if (u0 == 1 && (MB == 2 ? m0 + 256 >= c.M : n0 + 256 >= c.N)) {
+        if (u0 == 1 && (MB == 2 ? m0 + 256 >= c.M : n0 + width >= c.N)) {
             u1 = u0;  // empty
         }
     }
     __device__ __forceinline__ int row(int u) const { return m0 + (MB == 2 ? u * 256 : 0); }
-    __device__ __forceinline__ int col(int u) const { return n0 + (NB == 2 ? u * 256 : 0); }
+    __device__ __forceinline__ int col(int u) const { return n0 + (NB == 2 ? u * width : 0); }
 };
 
 template <int MB, int NB, bool SPLIT, class Epi>
 __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
 {
-    static_assert(MB * NB == 2, "two blocks of 256 x 256");
+    static_assert(MB * NB <= 2, "tensor memory holds two blocks of 256 x 256");
+    constexpr int STAGES      = MB * NB == 2 ? WIDE_STAGES : WIDE_STAGES * 3 / 2;
+    constexpr int STAGE_BYTES = (MB + NB) * WIDE_BLOCK_BYTES;
     extern __shared__ uint8_t smem_raw[];
-    __shared__ uint64_t       full[WIDE_STAGES], empty[WIDE_STAGES], tmem_full[2], tmem_empty[2];
+    __shared__ uint64_t       full[STAGES], empty[STAGES], tmem_full[2], tmem_empty[2];
     __shared__ uint32_t       tmem_holder;
 
     const uint32_t base = (ptx::smem_addr(smem_raw) + 1023u) & ~1023u;
@@ -350,7 +364,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
     const int      w_end = SPLIT ? w_0 + 1 : core.items, w_inc = SPLIT ? 1 : static_cast<int>(gridDim.x >> 1);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < WIDE_STAGES; ++s) {
+        for (int s = 0; s < STAGES; ++s) {
             ptx::mbar_init(&full[s], 1);
             ptx::mbar_init(&empty[s], 1);
         }
@@ -379,20 +393,23 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
     if (warp == 0) {
         uint32_t stage = 0, phase = 1;
         bool     ok    = true;
+        // of an operand's 128 rows (or, stored the other way, two 64 x 64 blocks) B may need only a part
+        const int      b_rows  = core.width / 2;
+        const uint32_t b_bytes = core.b_mn ? (b_rows + 63) / 64 * 8192u : b_rows * 128u;
         for (int w = w_0; w < w_end && ok; w += w_inc) {
-            const WideItem<MB, NB> item(core, w);
+            const WideItem<MB, NB> item(core, w, 0);
             if (item.u0 == item.u1) {
                 continue;
             }
-            const uint32_t blocks = (MB == 2 ? item.u1 - item.u0 : 1) + (NB == 2 ? item.u1 - item.u0 : 1);
+            const uint32_t bytes = (MB == 2 ? item.u1 - item.u0 : 1) * WIDE_BLOCK_BYTES + (NB == 2 ? item.u1 - item.u0 : 1) * b_bytes;
             for (int kb = 0; kb < kblocks; ++kb) {
                 if (!ptx::mbar_wait_warp(empty_b + stage * 8, phase)) {
                     ok = false;
                     break;
                 }
-                const uint32_t sa = base + stage * WIDE_STAGE_BYTES, sb = sa + MB * WIDE_BLOCK_BYTES, bar = full_b + stage * 8;
+                const uint32_t sa = base + stage * STAGE_BYTES, sb = sa + MB * WIDE_BLOCK_BYTES, bar = full_b + stage * 8;
                 if (half == 0) {
-                    ptx::mbar_expect_tx_if(bar, 2 * blocks * WIDE_BLOCK_BYTES, leader);  // both CTAs' bytes
+                    ptx::mbar_expect_tx_if(bar, 2 * bytes, leader);  // both CTAs' bytes
                 }
 #pragma unroll
                 for (int u = 0; u < MB; ++u) {
@@ -414,17 +431,19 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                     if (NB == 2 && (u < item.u0 || u >= item.u1)) {
                         continue;
                     }
-                    const int      n  = item.n0 + u * 256 + half * 128;
+                    const int      n  = item.col(u) + half * b_rows;
                     const uint32_t to = sb + u * WIDE_BLOCK_BYTES;
                     if (!core.b_mn) {
                         ptx::tma_load_2d_pair_if(to, &core.map_b, (kb_0 + kb) * BK, n, bar, leader);
                     }
                     else {
                         ptx::tma_load_2d_pair_if(to, &core.map_b, n, (kb_0 + kb) * BK, bar, leader);
-                        ptx::tma_load_2d_pair_if(to + 8192, &core.map_b, n + 64, (kb_0 + kb) * BK, bar, leader);
+                        if (b_rows > 64) {
+                            ptx::tma_load_2d_pair_if(to + 8192, &core.map_b, n + 64, (kb_0 + kb) * BK, bar, leader);
+                        }
                     }
                 }
-                if (++stage == WIDE_STAGES) {
+                if (++stage == STAGES) {
                     stage = 0;
                     phase ^= 1u;
                 }
@@ -437,7 +456,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
     }
     else if (warp == 1) {
         if (half == 0) {
-            const uint32_t  idesc = ptx::make_idesc(1, 1, 256, 256, core.a_mn ? 1 : 0, core.b_mn ? 1 : 0);
+            const uint32_t  idesc = ptx::make_idesc(1, 1, 256, core.width, core.a_mn ? 1 : 0, core.b_mn ? 1 : 0);
             // K-major: 16 bf16 along K are 32 bytes inside the swizzle atom. MN-major: 16 rows of K are
             // 2048 bytes, 64-column blocks 8 KiB apart.
             const uint32_t  a_step = core.a_mn ? 2048u : 32u, b_step = core.b_mn ? 2048u : 32u;
@@ -448,29 +467,29 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
             uint32_t        gave_up = ERR_NONE;
             const uint32_t  both = 3u << even;
             auto issue = [&](int u, uint32_t s, uint32_t accumulate) {  // one K-block into block u
-                const ptx::Desc a = a_desc.at(s * WIDE_STAGE_BYTES + (MB == 2 ? u * WIDE_BLOCK_BYTES : 0));
-                const ptx::Desc b = b_desc.at(s * WIDE_STAGE_BYTES + (NB == 2 ? u * WIDE_BLOCK_BYTES : 0));
+                const ptx::Desc a = a_desc.at(s * STAGE_BYTES + (MB == 2 ? u * WIDE_BLOCK_BYTES : 0));
+                const ptx::Desc b = b_desc.at(s * STAGE_BYTES + (NB == 2 ? u * WIDE_BLOCK_BYTES : 0));
 #pragma unroll
                 for (int k = 0; k < BK / UMMA_K; ++k) {
                     ptx::mma_f16_ss_if<2>(tmem_base + u * 256, a.at(a_step * k), b.at(b_step * k), idesc, accumulate | k, leader);
                 }
             };
             auto advance = [](uint32_t& s, uint32_t& ph) {
-                if (++s == WIDE_STAGES) {
+                if (++s == STAGES) {
                     s = 0;
                     ph ^= 1u;
                 }
             };
             for (int w = w_0; w < w_end && !gave_up; w += w_inc) {
-                const WideItem<MB, NB> item(core, w);
+                const WideItem<MB, NB> item(core, w, uses0 + uses1);
                 if (item.u0 == item.u1) {
                     continue;
                 }
                 for (int kb = 0; kb < kblocks && !gave_up;) {
                     const int left = kblocks - kb;
-                    if (kb > 0 && left > WIDE_STAGES && item.u1 - item.u0 == 2) {
+                    if (kb > 0 && left > STAGES && item.u1 - item.u0 == 2) {
                         // the middle of a whole tile: both blocks, one K-block after another
-                        const int n = left - WIDE_STAGES;
+                        const int n = left - STAGES;
                         for (int i = 0; i < n; ++i) {
                             if (!ptx::mbar_wait_warp(full_b + stage * 8, phase)) {
                                 gave_up = ERR_MMA_WAIT_FULL;
@@ -486,7 +505,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                         continue;
                     }
                     // the first K-blocks of a tile, its last ones, or any of a single block
-                    const int run = min(left, WIDE_STAGES);
+                    const int run = min(left, STAGES);
                     uint32_t  s = stage, ph = phase;
                     for (int u = item.u0; u < item.u1 && !gave_up; ++u) {
                         if (kb == 0) {
@@ -539,12 +558,12 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
         const int epi_warp = warp - WIDE_FIRST_EPI;
         const int quarter  = warp & 3;        // the TMEM lane quarter this warp may access
         const int cg       = epi_warp >> 2;   // which 128 of a block's 256 columns
-        const uint32_t stage = base + WIDE_STAGES * WIDE_STAGE_BYTES + epi_warp * UNIT_STAGE_BYTES;
+        const uint32_t stage = base + STAGES * STAGE_BYTES + epi_warp * UNIT_STAGE_BYTES;
         if (Epi::kPeers) {
             epi.open(threadIdx.x - 32 * WIDE_FIRST_EPI);
         }
         if constexpr (SPLIT) {
-            const WideItem<MB, NB> item(core, w_0);
+            const WideItem<MB, NB> item(core, w_0, 0);
             bool                   ok = item.u0 != item.u1;  // an empty item only takes part in the barriers
             if (ok && !ptx::mbar_wait(&tmem_full[item.u0], 0u)) {
                 flag_error(core.err, ERR_EPI_WAIT);
@@ -586,7 +605,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                         v[4 * g + 3] += __uint_as_float(q.w);
                     }
                 }
-                epi.template piece<W>(v, item.row(item.u0) + half * 128 + quarter * 32, item.col(item.u0) + (2 * part + cg) * W, lane, stage);
+                epi.template piece<W>(v, item.row(item.u0) + half * 128 + quarter * 32, item.col(item.u0) + (2 * part + cg) * W, core.N, lane, stage);
             };
             if (ok) {
                 if (parts == 2) {
@@ -601,7 +620,8 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
         uint32_t uses[2] = {0, 0};
         bool     ok      = true;
         for (int w = w_0; w < w_end && ok; w += w_inc) {
-            const WideItem<MB, NB> item(core, w);
+            const WideItem<MB, NB> item(core, w, uses[0] + uses[1]);
+            const int              cols = core.width / 2, col0 = cg * cols;  // a warp's share of a block
             for (int u = item.u0; u < item.u1; ++u) {
                 if (!ptx::mbar_wait(&tmem_full[u], uses[u] & 1u)) {
                     flag_error(core.err, ERR_EPI_WAIT);
@@ -611,13 +631,13 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
                 ++uses[u];
                 ptx::tc_fence_after();
                 uint32_t r[128];
-                load_unit(tmem_base + u * 256 + cg * 128 + (static_cast<uint32_t>(quarter * 32) << 16), r);
+                load_unit(tmem_base + u * 256 + col0 + (static_cast<uint32_t>(quarter * 32) << 16), r);
                 ptx::tc_fence_before();
                 __syncwarp();
                 if (lane == 0) {
                     ptx::mbar_arrive_cluster(ptx::cluster_addr(&tmem_empty[u], even));
                 }
-                epi.unit(r, item.row(u) + half * 128 + quarter * 32, item.col(u) + cg * 128, lane, stage);
+                epi.unit(r, item.row(u) + half * 128 + quarter * 32, item.col(u) + col0, item.col(u) + col0 + cols, lane, stage);
             }
         }
         }
@@ -826,7 +846,7 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
                             v[4 * g + 3] += __uint_as_float(q.w);
                         }
                     }
-                    epi.template piece<W>(v, row0, nt * 128 + crank * W, lane, stage);
+                    epi.template piece<W>(v, row0, nt * 128 + crank * W, core.N, lane, stage);
                 };
                 if (ok) {
                     if (csize == 2) {
@@ -852,7 +872,7 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
             if (lane == 0) {
                 ptx::mbar_arrive(&tmem_empty[acc]);
             }
-            epi.unit(r, mt * 128 + quarter * 32, nt * 128, lane, stage);
+            epi.unit(r, mt * 128 + quarter * 32, nt * 128, nt * 128 + 128, lane, stage);
         }
         if (Epi::kPeers) {
             epi.close(threadIdx.x - 64);
