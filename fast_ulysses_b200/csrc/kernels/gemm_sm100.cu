@@ -817,12 +817,13 @@ Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, in
     if (rest == 0 || cudaGetDevice(&dev) != cudaSuccess) {
         return best;
     }
+    double       limit = 0.96 * best.cost;
     const double before =
         full + single > 0 ? 6.0 - 1.5 + kb * (kTwoBlocks[off] * (full / pairs) + 1.05 * kOneBlock[off] * (single / pairs)) : 0.0;
     for (const int csize : {4, 8}) {
         const int64_t parts = csize / 2, share = (kb + parts - 1) / parts;
         const double  wave  = (csize == 4 ? 8.1 : 9.4) + 0.97 * kOneBlock[off] * share;
-        if ((kb + share - 1) / share != parts || before + wave >= 0.96 * best.cost) {
+        if ((kb + share - 1) / share != parts || before + wave >= limit) {
             continue;  // a pair would have nothing to do, or no gain beyond the estimate's error even in one wave
         }
         const int cap = capacity.of(gemm_wide_split_kernel<0>, csize, dev, WIDE_THREADS, WIDE_SMEM_BYTES);
@@ -830,7 +831,8 @@ Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, in
             continue;
         }
         const double cost = before + static_cast<double>((rest + cap - 1) / cap) * wave;
-        if (cost < chosen.cost) {
+        if (cost < limit) {
+            limit        = cost;
             chosen       = broad;
             chosen.full  = static_cast<int>(full);
             chosen.items = static_cast<int>(full + single);
