@@ -46,6 +46,32 @@ void expect(bool good, const Args&... what)
     }
 }
 
+// Operands of one launch lie on one GPU: an address of another device, or of the host, would reach the
+// kernels as if it were this one's.
+void expect_on_device_of(const Tensor& x, std::initializer_list<const Tensor*> operands, const char* what)
+{
+    expect(x.is_cuda(), what, ": expected CUDA tensors, got one on ", x.device());
+    for (const Tensor* t : operands) {
+        if (t->defined()) {
+            expect(t->device() == x.device(), what, ": expected every operand on ", x.device(), ", got one on ", t->device());
+        }
+    }
+}
+
+// What an epilogue reads beside a product of `rows` x w.size(0): one bias value per column, and a residual with
+// the product's values, which it reads as bf16.
+void expect_epilogue(const Tensor& w, const Tensor& bias, const Tensor& residual, int64_t rows, const char* what)
+{
+    const int64_t n = w.size(0);
+    if (bias.defined()) {
+        expect(bias.numel() == n, what, ": expected a bias of ", n, " values, got ", bias.sizes());
+    }
+    if (residual.defined()) {
+        expect(residual.scalar_type() == at::kBFloat16 && residual.numel() == rows * n, what, ": expected a bf16 residual of ", rows,
+               " rows of ", n, " values, got ", residual.scalar_type(), " ", residual.sizes());
+    }
+}
+
 cudaStream_t stream_of(const Tensor& t)
 {
     return at::cuda::getCurrentCUDAStream(t.device().index());
@@ -331,8 +357,10 @@ Tensor linear_entry(const Tensor& x, const Tensor& w, const MaybeTensor& bias, c
     expect(x.is_cuda() && w.is_cuda() && x.scalar_type() == at::kBFloat16 && w.scalar_type() == at::kBFloat16,
            "linear: x and weight must be bf16 CUDA tensors");
     expect(w.dim() == 2 && x.dim() >= 1 && x.size(-1) == w.size(1), "linear: ", x.sizes(), " x ", w.sizes());
+    const Tensor b = or_none(bias), r = or_none(residual);
+    expect_on_device_of(x, {&w, &b, &r}, "linear");
+    expect_epilogue(w, b, r, c10::multiply_integers(x.sizes().slice(0, x.dim() - 1)), "linear");
     const c10::cuda::CUDAGuard on(x.device());
-    const Tensor               b = or_none(bias), r = or_none(residual);
     if (wants_grad({&x, &w, &b, &r})) {
         return Linear::apply(x, w, maybe(b), maybe(r));
     }
@@ -416,8 +444,12 @@ Tensor feed_forward_entry(const Tensor& x, const Tensor& w1, const MaybeTensor& 
            "feed_forward: x and both weights must be bf16 CUDA tensors");
     expect(w1.dim() == 2 && w2.dim() == 2 && x.dim() >= 1 && x.size(-1) == w1.size(1) && w2.size(1) == w1.size(0),
            "feed_forward: ", x.sizes(), " x ", w1.sizes(), " x ", w2.sizes());
+    const Tensor  c1 = or_none(b1), c2 = or_none(b2), r = or_none(residual);
+    const int64_t rows = c10::multiply_integers(x.sizes().slice(0, x.dim() - 1));
+    expect_on_device_of(x, {&w1, &c1, &w2, &c2, &r}, "feed_forward");
+    expect_epilogue(w1, c1, Tensor(), rows, "feed_forward");
+    expect_epilogue(w2, c2, r, rows, "feed_forward");
     const c10::cuda::CUDAGuard on(x.device());
-    const Tensor               c1 = or_none(b1), c2 = or_none(b2), r = or_none(residual);
     if (wants_grad({&x, &w1, &c1, &w2, &c2, &r})) {
         return FeedForward::apply(x, w1, maybe(c1), w2, maybe(c2), maybe(r));
     }
@@ -986,6 +1018,13 @@ Tensor sp_attention_entry(const SpPtr& mod, const Tensor& x, const Tensor& w_qkv
     const Tensor r = or_none(residual), b = or_none(b_o);
     expect(!r.defined() || (r.sizes() == x.sizes() && r.scalar_type() == at::kBFloat16),
            "UlyssesSelfAttention: the residual must be bf16 and shaped like the input");
+    expect_on_device_of(x, {&w_qkv, &gamma_q, &gamma_k, &w_o, &b, &r, &rope}, "UlyssesSelfAttention");
+    expect(gamma_q.numel() == kHeadDim && gamma_k.numel() == kHeadDim && rope.is_contiguous() && rope.scalar_type() == at::kFloat
+               && rope.numel() == mod->s_local * kHeadDim,
+           "UlyssesSelfAttention: norm weights of ", kHeadDim, " values and a dense fp32 table of ", mod->s_local, " positions, got ",
+           gamma_q.sizes(), ", ", gamma_k.sizes(), " and ", rope.sizes());
+    expect(w_o.dim() == 2, "UlyssesSelfAttention: output weight ", w_o.sizes());
+    expect_epilogue(w_o, b, r, mod->batch * mod->s_local, "UlyssesSelfAttention");
     const c10::cuda::CUDAGuard on(x.device());
     if (wants_grad({&x, &w_qkv, &gamma_q, &gamma_k, &w_o, &b, &r})) {
         return SpAttentionFn::apply(x, w_qkv, gamma_q, gamma_k, w_o, maybe(b), maybe(r), rope, mod);

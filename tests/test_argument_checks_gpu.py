@@ -1,0 +1,81 @@
+"""What the differentiable entry points refuse. Each refusal is made on the host, before a kernel starts: an
+operand on another device, or one that is shorter than what an epilogue reads, would otherwise be an address
+that the kernel may not touch."""
+
+import pytest
+import torch
+
+import fast_ulysses_b200 as fu
+from fast_ulysses_b200.models.attention import UlyssesSelfAttention
+from fast_ulysses_b200.ops import gemm
+
+pytestmark = pytest.mark.gpu
+
+M, K, N = 24, 64, 40
+
+
+def bf16(*shape):
+    return torch.randn(*shape, device="cuda").bfloat16()
+
+
+def short_epilogues(rows, n):
+    """Name, bias and residual of a product of ``rows`` x ``n`` that an epilogue must not be given."""
+    return [("a bias that is too short", bf16(n - 8), None), ("a bias on the host", bf16(n).cpu(), None),
+            ("a residual that would broadcast", None, bf16(1, n)), ("a residual of too few rows", None, bf16(rows - 1, n)),
+            ("an fp32 residual", None, torch.randn(rows, n, device="cuda")), ("a residual on the host", None, bf16(rows, n).cpu())]
+
+
+@pytest.mark.parametrize("train", [False, True])
+def test_linear_refuses(train):
+    x, w = bf16(2, M // 2, K).requires_grad_(train), bf16(N, K)
+    for what, bias, residual in short_epilogues(M, N):
+        with pytest.raises(AssertionError):
+            gemm.linear(x, w, bias, residual)
+            pytest.fail(what)
+    with pytest.raises(AssertionError):
+        gemm.linear(x, w.cpu())
+    # and takes what it always took: a bias of another type or with a leading axis, a flat residual
+    for bias in (torch.randn(N, device="cuda"), torch.randn(N, device="cuda").half(), bf16(1, N)):
+        assert gemm.linear(x, w, bias, bf16(M, N)).shape == (2, M // 2, N)
+
+
+@pytest.mark.parametrize("train", [False, True])
+def test_feed_forward_refuses(train):
+    x, w1, w2 = bf16(2, M // 2, K).requires_grad_(train), bf16(N, K), bf16(K, N)
+    good = [x, w1, bf16(N), w2, bf16(K)]
+    gemm.feed_forward(*good, residual=bf16(2, M // 2, K))
+    for at in (1, 2, 3, 4):  # every weight and bias, left on the host
+        args = list(good)
+        args[at] = args[at].cpu()
+        with pytest.raises(AssertionError):
+            gemm.feed_forward(*args)
+    with pytest.raises(AssertionError):
+        gemm.feed_forward(x, w1, bf16(N - 8), w2, None)
+    for what, bias, residual in short_epilogues(M, K):
+        with pytest.raises(AssertionError):
+            gemm.feed_forward(x, w1, None, w2, bias, residual)
+            pytest.fail(what)
+
+
+@pytest.mark.parametrize("name,value", [("w_qkv", lambda p: p.cpu()), ("w_o", lambda p: p.cpu()), ("b_o", lambda p: p.cpu()),
+                                        ("b_o", lambda p: p[:-8]), ("gamma_q", lambda p: p[:64]), ("gamma_k", lambda p: p.cpu())])
+def test_attention_block_refuses_a_parameter_it_cannot_read(name, value):
+    g = fu.UlyssesGroup(device="cuda")
+    attn = UlyssesSelfAttention(g, 256, 2, grid=(1, 4, 8))
+    x = bf16(1, 32, 256)
+    assert attn(x, residual=x).shape == x.shape
+    setattr(attn, name, torch.nn.Parameter(value(getattr(attn, name).detach())))
+    with pytest.raises(AssertionError):
+        attn(x, residual=x)
+    gemm.check_errors()
+    g.check()
+    g.destroy()
+
+
+def test_attention_block_refuses_a_residual_on_the_host():
+    g = fu.UlyssesGroup(device="cuda")
+    attn = UlyssesSelfAttention(g, 256, 2, grid=(1, 4, 8))
+    x = bf16(1, 32, 256)
+    with pytest.raises(AssertionError):
+        attn(x, residual=x.cpu())
+    g.destroy()
