@@ -629,21 +629,24 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 float mx2[2] = {-INFINITY, -INFINITY};
 #pragma unroll
                 for (int i = 96; i < BN; i += 4) {
-                    mx2[0] = ptx::max3(mx2[0], __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
-                    mx2[1] = ptx::max3(mx2[1], __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
+                    mx2[0] = ptx::max3_nan(mx2[0], __uint_as_float(r[i]), __uint_as_float(r[i + 1]));
+                    mx2[1] = ptx::max3_nan(mx2[1], __uint_as_float(r[i + 2]), __uint_as_float(r[i + 3]));
                 }
 #pragma unroll
                 for (int i = 0; i < 48; ++i) {
                     if (on_fma_pipe<NP>(i % 16)) {
-                        mx2[i & 1] = ptx::max3(mx2[i & 1], __uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+                        mx2[i & 1] = ptx::max3_nan(mx2[i & 1], __uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
                     }
                 }
-                const float tail = fmaxf(mx2[0], mx2[1]);
+                const float tail = ptx::max3_nan(mx2[0], mx2[1], mx2[1]);
                 const float part = (s4[0] + s4[1]) + (s4[2] + s4[3]);
                 const float last = fmaf(tail, c, nmc);
-                // (written so that a NaN among the scores takes the slow path too and stays one)
+                // A NaN among the scores reaches `part` or `last` and fails their test: the slow path and the last
+                // quarter behind it then run on the special-function unit, which keeps it (the FMA-pipe form's clamp
+                // would turn it into a number).
                 const bool fine = part < 0x1p32f && last < RANGE && (j != j_first || part > 0x1p-32f);
-                if (__any_sync(0xffffffffu, !fine)) {
+                const bool slow = __any_sync(0xffffffffu, !fine);
+                if (slow) {
                     // The maximum of the whole row; the first three quarters are still in tensor memory.
                     float mx = tail;
 #pragma unroll 1
@@ -704,7 +707,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 ptx::tc_fence_before();
                 ptx::mbar_arrive_warp(&bar.p_lo[t]);
                 stamp<TRACE>(p, scount, t * 10 + 4);
-                if (valid == BN) {
+                if (valid == BN && !slow) {
                     exp_chunk<NP>(&r[96], c, nmc, l4, pk);
                 }
                 else {

@@ -120,3 +120,32 @@ def test_query_blocks_shared_by_a_cluster(b, h, sq, skv):
         # the same terms, summed in fp32 in another order and rounded once: one step of bf16 apart at most
         # where the sum is not cancelled, so 2^-9 in the norm with room to spare
         assert ((got.float() - plain.float()).norm() / plain.float().norm().clamp_min(1e-6)).item() < 2.0 ** -9, name
+
+
+# two query tiles per item, clusters that share the kv tiles, and one query tile with its kv tiles by parity
+FORMS = [(1, 1, 256, 700, 148), (1, 10, 4000, 1500, 0), (1, 2, 300, 700, 0)]
+
+
+@pytest.mark.parametrize("b,h,sq,skv,ctas", FORMS)
+@pytest.mark.parametrize("where", [0, 1, 2, 5, 96, 97, 127, 128, 136, 300, -60, -59, -2, -1])  # from -60 on: the ragged last tile
+def test_nan_in_a_key_reaches_every_row(b, h, sq, skv, ctas, where):
+    torch.manual_seed(where + 60)
+    q, k, v = (torch.randn(b, s, h, 128, device="cuda").bfloat16() for s in (sq, skv, skv))
+    k[:, where, 0, 7] = float("nan")
+    o, lse = attention.fmha_fwd(q, k, v, ctas=ctas)
+    gemm.check_errors()
+    assert o[:, :, 0].isnan().all() and lse[:, 0].isnan().all()
+    assert not o[:, :, 1:].isnan().any() and not lse[:, 1:].isnan().any()  # the other heads
+
+
+@pytest.mark.parametrize("b,h,sq,skv,ctas", FORMS)
+def test_nan_in_a_query_stays_in_its_row(b, h, sq, skv, ctas):
+    torch.manual_seed(5)
+    q, k, v = (torch.randn(b, s, h, 128, device="cuda").bfloat16() for s in (sq, skv, skv))
+    q[:, 77, 0, 3] = float("nan")
+    o, lse = attention.fmha_fwd(q, k, v, ctas=ctas)
+    gemm.check_errors()
+    bad = torch.zeros(b, sq, h, dtype=torch.bool, device="cuda")
+    bad[:, 77, 0] = True
+    assert torch.equal(o.isnan().any(-1), bad) and torch.equal(o.isnan().all(-1), bad)
+    assert torch.equal(lse.isnan(), bad.transpose(1, 2))
