@@ -90,15 +90,16 @@ struct Barriers {
 // exp2 of a pair on the FMA pipe instead of the special-function unit: floor by a round-down add of
 // 1.5 * 2^23 (the integer part lands in the low mantissa bits), the minimax quintic for 2^fraction on
 // [0, 1) (Remez exchange; relative error 1.5e-7 evaluated in fp32, as good as the special-function
-// unit's), and the integer part added to the exponent field. Arguments below -126 are clamped: their
-// exponent field would wrap.
+// unit's), and the integer part added to the exponent field. That field would wrap below -127: such arguments
+// become the next number above it, whose result is 2^-143 and thus a bf16 zero, as the special-function
+// unit's is (a weight of 2^-126 is not nothing beside a value of 2^127).
 __device__ __forceinline__ void ex2_poly2(float& e0, float& e1, float x0, float x1)
 {
     constexpr float MAGIC = 12582912.0f;
     constexpr float C0 = 0.9999999403953552f, C1 = 0.6931530833244324f, C2 = 0.24015361070632935f, C3 = 0.05582631751894951f,
                     C4 = 0.00898933969438076f, C5 = 0.0018775766948238015f;
-    x0 = fmaxf(x0, -126.0f);
-    x1 = fmaxf(x1, -126.0f);
+    x0 = fmaxf(x0, -0x1.fbfffep6f);
+    x1 = fmaxf(x1, -0x1.fbfffep6f);
     float t0, t1, i0, i1, f0, f1, p0, p1;
     ptx::add2_rm(t0, t1, x0, x1, MAGIC, MAGIC);
     ptx::add2(i0, i1, t0, t1, -MAGIC, -MAGIC);

@@ -149,3 +149,20 @@ def test_nan_in_a_query_stays_in_its_row(b, h, sq, skv, ctas):
     bad[:, 77, 0] = True
     assert torch.equal(o.isnan().any(-1), bad) and torch.equal(o.isnan().all(-1), bad)
     assert torch.equal(lse.isnan(), bad.transpose(1, 2))
+
+
+@pytest.mark.parametrize("b,h,sq,skv,ctas", FORMS)
+def test_a_weight_that_underflows_is_zero(b, h, sq, skv, ctas):
+    """Half the keys of every tile score hundreds of powers of two below the rest, and their values are the
+    largest there are (2^127): a weight of exactly zero keeps them out."""
+    torch.manual_seed(6)
+    q = torch.randn(b, sq, h, 128, device="cuda").abs().bfloat16()
+    k, v = (torch.randn(b, skv, h, 128, device="cuda").bfloat16() for _ in range(2))
+    hidden = torch.arange(skv, device="cuda") % 16 < 8
+    k[:, hidden] = -50.0
+    v[:, hidden] = 2.0 ** 127
+    o, lse = attention.fmha_fwd(q, k, v, ctas=ctas)
+    gemm.check_errors()
+    o_ref, lse_ref = attention.attention_reference(q, k[:, ~hidden], v[:, ~hidden])
+    assert ((o.float() - o_ref).norm() / o_ref.norm()).item() < 1e-2  # P and o are rounded to bf16: 2^-9 each
+    assert ((lse - lse_ref).abs().max()).item() < 1e-3
