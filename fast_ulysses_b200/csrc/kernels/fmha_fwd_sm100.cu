@@ -573,8 +573,10 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             // leave that range. Whether they do is read off their own sum, so an ordinary step takes no
             // maximum of the row; only the last quarter, which is handed over later, and the columns on the
             // FMA pipe, whose exponent field wraps where the special-function unit returns infinity, are
-            // judged by their scores.
+            // judged by their scores. A row whose scores have all been -inf so far has no reference yet and takes
+            // the one of the first step that has others.
             float m_ref = 0.0f;
+            bool  begun = false;
             float l4[4] = {0.f, 0.f, 0.f, 0.f};
 
             const int j_first = ONE ? t : 0;
@@ -645,7 +647,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 // A NaN among the scores reaches `part` or `last` and fails their test: the slow path and the last
                 // quarter behind it then run on the special-function unit, which keeps it (the FMA-pipe form's clamp
                 // would turn it into a number).
-                const bool fine = part < 0x1p32f && last < RANGE && (j != j_first || part > 0x1p-32f);
+                const bool fine = part < 0x1p32f && last < RANGE && (begun || part > 0x1p-32f);
                 const bool slow = __any_sync(0xffffffffu, !fine);
                 if (slow) {
                     // The maximum of the whole row; the first three quarters are still in tensor memory.
@@ -660,9 +662,9 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                             mx = ch * 16 + i < valid ? fmaxf(mx, __uint_as_float(rs[i])) : mx;
                         }
                     }
-                    const float m_new = fine ? m_ref : mx;
+                    const float m_new = fine || mx == -INFINITY ? m_ref : mx;
                     if (j != j_first) {  // the commit behind S_t also covers the product before it: O is complete
-                        const float alpha = ptx::ex2((m_ref - m_new) * c);
+                        const float alpha = begun ? ptx::ex2((m_ref - m_new) * c) : 1.0f;
 #pragma unroll
                         for (int u = 0; u < 4; ++u) {
                             l4[u] *= alpha;
@@ -681,6 +683,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                         ptx::tmem_st_wait();
                     }
                     m_ref = m_new;
+                    begun = begun || mx != -INFINITY;
                     nmc   = -m_ref * c;
                     s4[0] = s4[1] = s4[2] = s4[3] = 0.f;
 #pragma unroll
@@ -692,6 +695,9 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                         }
                         exp_chunk<0>(&r[ch * 32], c, nmc, s4, &pk[ch * 16]);
                     }
+                }
+                else {
+                    begun = true;
                 }
                 stamp<TRACE>(p, scount, t * 10 + 2);
                 // written over S, of which only the last quarter is still needed and in registers
@@ -726,7 +732,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 if (!ok) {
                     flag(p, ERR_SOFTMAX);
                 }
-                join_shares(p, b, h, row, t, quarter, lane, to, m_ref * c, (l4[0] + l4[1]) + (l4[2] + l4[3]), crank, csize, base,
+                join_shares(p, b, h, row, t, quarter, lane, to, begun ? m_ref * c : -INFINITY, (l4[0] + l4[1]) + (l4[2] + l4[3]), crank, csize, base,
                             sv_addr + KV_STAGES * TILE_BYTES + (warp - 4) * OUT_BYTES);
                 break;
             }
@@ -738,7 +744,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 flag(p, ERR_SOFTMAX);
                 break;
             }
-            float l = (l4[0] + l4[1]) + (l4[2] + l4[3]), m_log2 = m_ref * c;
+            float l = (l4[0] + l4[1]) + (l4[2] + l4[3]), m_log2 = begun ? m_ref * c : -INFINITY;
             float weight[QT] = {1.0f, 1.0f};  // of the two O of a row (kOneTile)
             if (ONE) {
                 const uint32_t pair = sq_addr + TILE_BYTES + row_in * 8;  // where the second query tile would be

@@ -166,3 +166,23 @@ def test_a_weight_that_underflows_is_zero(b, h, sq, skv, ctas):
     o_ref, lse_ref = attention.attention_reference(q, k[:, ~hidden], v[:, ~hidden])
     assert ((o.float() - o_ref).norm() / o_ref.norm()).item() < 1e-2  # P and o are rounded to bf16: 2^-9 each
     assert ((lse - lse_ref).abs().max()).item() < 1e-3
+
+
+@pytest.mark.parametrize("b,h,sq,skv,ctas", FORMS)
+@pytest.mark.parametrize("first,last", [(0, 1), (0, 128), (128, 256), (0, 256), (256, 512), (100, 400), (0, 690), (512, 700)])
+def test_steps_whose_scores_are_all_minus_infinity(b, h, sq, skv, ctas, first, last):
+    """Keys ruled out by a score of -inf, a whole kv step or several of them, wherever a form begins: its first
+    step, the first of the odd steps, the first of a share. Only every other query rules them out."""
+    torch.manual_seed(first + last)
+    q, k, v = (torch.randn(b, s, h, 128, device="cuda").bfloat16() for s in (sq, skv, skv))
+    q[..., 0] = 1.0
+    q[:, 1::2, :, 0] = 0.0
+    keep = torch.ones(skv, dtype=torch.bool, device="cuda")
+    keep[first:last] = False
+    k[:, ~keep, :, 0] = -torch.inf
+    o, lse = attention.fmha_fwd(q, k, v, ctas=ctas)
+    gemm.check_errors()
+    o_ref, lse_ref = attention.attention_reference(q[:, ::2], k[:, keep], v[:, keep])
+    assert ((o[:, ::2].float() - o_ref).norm() / o_ref.norm()).item() < 1e-2  # P and o are rounded to bf16: 2^-9 each
+    assert ((lse[..., ::2] - lse_ref).abs().max()).item() < 1e-3
+    assert o[:, 1::2].isnan().all()  # 0 x -inf
