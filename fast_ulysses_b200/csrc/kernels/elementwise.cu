@@ -19,6 +19,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <initializer_list>
 
 namespace {
 
@@ -501,6 +502,12 @@ __global__ void __launch_bounds__(256, 2) pull_qkv_grads_kernel(const __grid_con
     }
 }
 
+// The tables are read four floats, the rows four bf16 values at a time.
+bool misaligned(uintptr_t bytes, std::initializer_list<const void*> operands)
+{
+    return std::any_of(operands.begin(), operands.end(), [&](const void* p) { return reinterpret_cast<uintptr_t>(p) % bytes != 0; });
+}
+
 }  // namespace
 
 extern "C" int fu_qk_norm_rope_bwd(const FuNormRopeBwdArgs* a, void* stream)
@@ -510,6 +517,9 @@ extern "C" int fu_qk_norm_rope_bwd(const FuNormRopeBwdArgs* a, void* stream)
     }
     if (a->m <= 0 || a->heads <= 0 || a->s_local <= 0 || (a->ld_y % 4) || (a->ld_dy % 4)) {
         return fu::fail(FU_E_ARG, "fu_qk_norm_rope_bwd: bad shape");
+    }
+    if (misaligned(16, {a->rope, a->gamma_q, a->gamma_k}) || misaligned(8, {a->dq, a->dk, a->y, a->dy})) {
+        return fu::fail(FU_E_ARG, "fu_qk_norm_rope_bwd: rope and norm weights need 16-byte alignment, rows 8-byte");
     }
     NormRopeBwd p{};
     p.g[0]      = static_cast<const __nv_bfloat16*>(a->dq);
@@ -552,12 +562,18 @@ extern "C" int fu_pull_qkv_grads_check(const FuPullGradsArgs* a)
         return fu::fail(FU_E_ARG, "fu_pull_qkv_grads: rows %lld..%lld do not lie inside a sequence of %lld",
                         (long long)a->seq_off, (long long)(a->seq_off + a->s_local), (long long)a->s_total);
     }
+    if (misaligned(16, {a->rope, a->gamma_q, a->gamma_k}) || misaligned(8, {a->y, a->dy})) {
+        return fu::fail(FU_E_ARG, "fu_pull_qkv_grads: rope and norm weights need 16-byte alignment, y and dy 8-byte");
+    }
     int heads_seen = 0;
     const int64_t batches = a->m / a->s_local;
     for (int p = 0; p < a->world; ++p) {
         if (a->head_splits[p] < 0 || a->head_splits[p] > 255 || !a->peer_dq[p] || !a->peer_dk[p] || !a->peer_dv[p]
             || !a->peer_ctrl[p]) {
             return fu::fail(FU_E_ARG, "fu_pull_qkv_grads: bad shard or missing buffer for rank %d", p);
+        }
+        if (misaligned(8, {a->peer_dq[p], a->peer_dk[p], a->peer_dv[p]})) {
+            return fu::fail(FU_E_ARG, "fu_pull_qkv_grads: the buffers of rank %d need 8-byte alignment", p);
         }
         heads_seen += a->head_splits[p];
         // row (batch, seq_off + s) of rank p's buffers starts at ((batch * s_total + seq_off + s) * head_splits[p]) * 256

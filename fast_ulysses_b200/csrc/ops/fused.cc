@@ -724,7 +724,8 @@ struct SpAttention : public torch::CustomClassHolder {
     {
         const Tensor p = param.detach();
         if (p.scalar_type() == at::kFloat && p.is_contiguous()) {
-            return p;
+            // a slice of a flat parameter buffer may start anywhere; the gradient kernel reads four values at a time
+            return reinterpret_cast<uintptr_t>(p.data_ptr()) % 16 == 0 ? p : p.clone();
         }
         const uint32_t version = param._version();
         if (!c.f32.defined() || c.version != version || c.ptr != p.data_ptr()) {

@@ -171,6 +171,31 @@ def test_pull_of_the_gradients_past_a_peer_buffer_is_refused():
     assert ck.lib().fu_pull_qkv_grads_check(C.byref(a)) != 0 and "do not lie inside a sequence of 30" in last_error()
 
 
+def grads_args():
+    a = ck.FuPullGradsArgs()
+    a.y, a.dy, a.rope, a.gamma_q, a.gamma_k = (BASE + i * (1 << 30) for i in range(5))
+    a.m = a.s_local = a.s_total = 10
+    a.heads, a.world, a.ld_y, a.ld_dy = 2, 1, 512, 768
+    a.head_splits[0] = 2
+    a.peer_dq[0], a.peer_dk[0], a.peer_dv[0], a.peer_ctrl[0] = (BASE + i * (1 << 30) for i in range(6, 10))
+    a.src_bytes = 10 * 2 * 256
+    return a
+
+
+@pytest.mark.parametrize("field,step", [("rope", 8), ("gamma_q", 4), ("gamma_k", 8), ("y", 2), ("dy", 4), ("peer_dq", 2),
+                                        ("peer_dk", 4), ("peer_dv", 6)])
+def test_pull_of_the_gradients_refuses_an_operand_its_loads_are_too_wide_for(field, step):
+    """Tables are read 16 bytes at a time, rows 8."""
+    a = grads_args()
+    assert ck.lib().fu_pull_qkv_grads_check(C.byref(a)) == 0, last_error()
+    if field.startswith("peer"):
+        getattr(a, field)[0] += step
+    else:
+        setattr(a, field, getattr(a, field) + step)
+    assert ck.lib().fu_pull_qkv_grads_check(C.byref(a)) != 0
+    assert "alignment" in last_error()
+
+
 def test_fp8_exchange_route_past_the_packed_window_is_refused():
     a = ck.FuA2AFp8Args()
     a.src, a.out = BASE, BASE + (1 << 40)

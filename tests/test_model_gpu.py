@@ -83,3 +83,28 @@ def test_backward_after_a_later_forward_is_refused():
     assert torch.allclose(attn.w_o.grad.float(), 2 * first.float(), rtol=2e-2, atol=1e-3)
     gemm.check_errors()
     g.destroy()
+
+
+def test_norm_weights_may_be_slices_of_a_flat_buffer():
+    """Parameters kept in one flat buffer start on any element, not on the 16 bytes a vector load needs."""
+    torch.manual_seed(3)
+    g = fu.UlyssesGroup(device="cuda")
+    attn = UlyssesSelfAttention(g, 256, 2, grid=(2, 4, 8))
+    x = torch.randn(1, 64, 256, device="cuda").bfloat16()
+    dy = torch.randn_like(x)
+    flat = torch.rand(3 + 2 * 129, device="cuda") + 0.5
+    grads = []
+    for at in (3, 4):  # 4: 16-byte aligned slices of the same values
+        flat[at:at + 128] = torch.linspace(0.5, 1.5, 128, device="cuda")
+        flat[at + 128:at + 256] = torch.linspace(1.5, 0.5, 128, device="cuda")
+        attn.gamma_q = torch.nn.Parameter(flat[at:at + 128])
+        attn.gamma_k = torch.nn.Parameter(flat[at + 128:at + 256])
+        attn.w_qkv.grad = None
+        y = attn(x)
+        y.backward(dy)
+        grads.append((y.detach(), attn.w_qkv.grad, attn.gamma_q.grad, attn.gamma_k.grad))
+    gemm.check_errors()
+    for name, a, b in zip(("y", "w_qkv", "gamma_q", "gamma_k"), *grads):
+        # dq and d(gamma) are summed in fp32 in another order from call to call
+        assert rel_err(a, b) < 2e-3, name
+    g.destroy()
