@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <initializer_list>
 
 namespace {
 
@@ -130,6 +131,20 @@ extern "C" int fu_fmha_bwd(const FuFmhaArgs* a, void* stream_v)
     }
     if (a->batch < 1 || a->heads < 1 || a->seq_q < 1 || a->seq_kv < 1) {
         return fu::fail(FU_E_ARG, "fu_fmha_bwd: empty problem");
+    }
+    // Every kernel below reads or writes rows in pieces of 8 or 16 bytes; the tensor maps check only what TMA loads,
+    // and only after the pre-pass has been launched.
+    const std::initializer_list<const void*> operands = {a->q, a->k, a->v, a->o, a->d_o, a->dq, a->dk, a->dv, a->delta, a->dq_acc};
+    for (const void* p : operands) {
+        if (reinterpret_cast<uintptr_t>(p) & 15u) {
+            return fu::fail(FU_E_ARG, "fu_fmha_bwd: every operand needs 16-byte alignment, got %p", p);
+        }
+    }
+    for (const int64_t stride : {a->q_row, a->q_head, a->q_batch, a->k_row, a->k_head, a->k_batch, a->v_row, a->v_head, a->v_batch,
+                                 a->o_row, a->o_head, a->o_batch}) {
+        if (stride % 8) {
+            return fu::fail(FU_E_ARG, "fu_fmha_bwd: strides need to be multiples of 8 elements");
+        }
     }
     cudaStream_t  stream = static_cast<cudaStream_t>(stream_v);
     const int     sq_pad = (a->seq_q + BLK - 1) / BLK * BLK;

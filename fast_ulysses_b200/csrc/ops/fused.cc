@@ -109,6 +109,12 @@ uint32_t* error_ptr(const Tensor& t)
     return cached[d];
 }
 
+// A tensor that starts on 16 bytes, as vector loads need, with its strides: a gradient can be a view of any offset.
+Tensor aligned(const Tensor& t)
+{
+    return reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0 ? t : t.clone();
+}
+
 Tensor empty_bf16(at::IntArrayRef shape, const Tensor& like)
 {
     return at::detail::empty_cuda(shape, at::kBFloat16, like.device(), std::nullopt);
@@ -626,7 +632,7 @@ std::tuple<Tensor, Tensor, Tensor> fmha_bwd(const Tensor& q, const Tensor& k, co
 {
     const c10::cuda::CUDAGuard on(q.device());
     const int64_t              b = q.size(0), sq = q.size(1), h = q.size(2);
-    Tensor                     o = o_in, d_o = do_in;
+    Tensor                     o = o_in, d_o = aligned(do_in);
     if (d_o.strides() != o.strides()) {
         d_o = d_o.contiguous();
         o   = o.contiguous();

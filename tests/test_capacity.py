@@ -196,6 +196,19 @@ def test_pull_of_the_gradients_refuses_an_operand_its_loads_are_too_wide_for(fie
     assert "alignment" in last_error()
 
 
+@pytest.mark.parametrize("field,step", [("o", 4), ("d_o", 2), ("d_o", 8), ("dq", 8), ("dk", 8), ("dv", 2), ("delta", 4), ("dq_acc", 8)])
+def test_attention_backward_refuses_a_misaligned_operand_before_its_first_launch(field, step):
+    a = ck.FuFmhaArgs()
+    for i, name in enumerate(("q", "k", "v", "o", "lse", "d_o", "dq", "dk", "dv", "delta", "dq_acc")):
+        setattr(a, name, BASE + i * (1 << 30))
+    a.batch, a.heads, a.seq_q, a.seq_kv, a.head_dim = 1, 2, 64, 64, 128
+    for name in "qkvo":
+        setattr(a, f"{name}_row", 256), setattr(a, f"{name}_head", 128), setattr(a, f"{name}_batch", 64 * 256)
+    setattr(a, field, getattr(a, field) + step)
+    assert ck.lib().fu_fmha_bwd(C.byref(a), None) != 0
+    assert "alignment" in last_error()
+
+
 def test_fp8_exchange_route_past_the_packed_window_is_refused():
     a = ck.FuA2AFp8Args()
     a.src, a.out = BASE, BASE + (1 << 40)
