@@ -1225,8 +1225,8 @@ extern "C" int fu_pull_outproj_check(const FuPullArgs* q)
         return fu::fail(FU_E_ARG, "fu_pull_outproj: m=%lld is not a multiple of s_local=%lld", (long long)q->m,
                         (long long)q->s_local);
     }
-    if ((q->ldc % 8) || (reinterpret_cast<uintptr_t>(q->c) & 15u)) {
-        return fu::fail(FU_E_ARG, "fu_pull_outproj: C needs 16-byte aligned rows");
+    if ((q->ldc % 8) || (reinterpret_cast<uintptr_t>(q->c) & 15u) || (reinterpret_cast<uintptr_t>(q->residual) & 15u)) {
+        return fu::fail(FU_E_ARG, "fu_pull_outproj: C and the residual need 16-byte aligned rows");
     }
     int heads_seen = 0;
     for (int p = 0; p < q->world; ++p) {

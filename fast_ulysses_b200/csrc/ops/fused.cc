@@ -493,7 +493,7 @@ Tensor layer_norm_backward(const Tensor& gy, const Tensor& x2, const Tensor& sta
 {
     const int64_t rows = x2.size(0), cols = x2.size(1);
     const Tensor  g2 = gy.reshape({rows, cols}).contiguous(), xc = x2.contiguous();
-    Tensor        a2 = add.defined() ? add.reshape({rows, cols}).contiguous() : add;
+    Tensor        a2 = add.defined() ? aligned(add.reshape({rows, cols}).contiguous()) : add;
     Tensor        dx = empty_bf16({rows, cols}, gy);
     ok(fu_layernorm_bwd_add(g2.data_ptr(), xc.data_ptr(), static_cast<const float*>(stats.data_ptr()),
                             a2.defined() ? a2.data_ptr() : nullptr, dx.data_ptr(), rows, cols, cols, stream_of(gy)));
@@ -895,7 +895,7 @@ struct SpAttention : public torch::CustomClassHolder {
         }
         const NvtxRange r("fast_ulysses_b200::pull_outproj");
         std::tie(f.out, f.gather) =
-            pull_outproj(w_o, b_o, residual.defined() ? residual.reshape({m, hidden}).contiguous() : residual);
+            pull_outproj(w_o, b_o, residual.defined() ? aligned(residual.reshape({m, hidden}).contiguous()) : residual);
         f.out = f.out.view(x.sizes());
         return f;
     }

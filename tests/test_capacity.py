@@ -153,6 +153,15 @@ def test_pull_with_a_buffer_that_is_too_small_is_refused(field, text):
     assert text in last_error()
 
 
+def test_pull_refuses_a_residual_off_16_bytes():
+    q = pull_args()
+    q.residual = BASE + (8 << 30)
+    assert ck.lib().fu_pull_outproj_check(C.byref(q)) == 0, last_error()
+    q.residual += 8
+    assert ck.lib().fu_pull_outproj_check(C.byref(q)) != 0
+    assert "16-byte aligned" in last_error()
+
+
 def test_pull_of_the_gradients_past_a_peer_buffer_is_refused():
     a = ck.FuPullGradsArgs()
     head_splits, s_local, s_total = (2, 3), 10, 30

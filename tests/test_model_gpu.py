@@ -6,7 +6,7 @@ import torch
 
 import fast_ulysses_b200 as fu
 from fast_ulysses_b200.models.attention import UlyssesSelfAttention, reference_attention
-from fast_ulysses_b200.models.dit import DiTStack, reference_forward
+from fast_ulysses_b200.models.dit import DiTBlock, DiTStack, reference_forward
 from fast_ulysses_b200.ops import gemm
 
 pytestmark = pytest.mark.gpu
@@ -107,4 +107,24 @@ def test_norm_weights_may_be_slices_of_a_flat_buffer():
     for name, a, b in zip(("y", "w_qkv", "gamma_q", "gamma_k"), *grads):
         # dq and d(gamma) are summed in fp32 in another order from call to call
         assert rel_err(a, b) < 2e-3, name
+    g.destroy()
+
+
+def test_block_takes_a_gradient_that_starts_anywhere():
+    """The gradient of the result is also that of the second half's residual: a dense tensor at an odd offset of a
+    larger buffer is no different from its copy. Nor is such a residual of the attention block."""
+    torch.manual_seed(4)
+    g = fu.UlyssesGroup(device="cuda")
+    block = DiTBlock(g, 256, 2, 512, grid=(2, 4, 8))
+    x = torch.randn(1, 64, 256, device="cuda").bfloat16().requires_grad_()
+    odd = torch.randn(64 * 256 + 3, device="cuda").bfloat16()[3:].view(1, 64, 256)
+    grads = []
+    for dy in (odd, odd.clone()):
+        x.grad = None
+        block(x).backward(dy)
+        grads.append(x.grad)
+    assert rel_err(*grads) < 2e-3  # dq is summed in fp32 in another order from call to call
+    with torch.no_grad():
+        assert torch.equal(block.attn(x, residual=odd), block.attn(x, residual=odd.clone()))
+    gemm.check_errors()
     g.destroy()
