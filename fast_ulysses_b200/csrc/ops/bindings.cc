@@ -62,12 +62,12 @@ void require_backend(const Group& g, const at::Tensor& t, const char* name)
 
 // What a call has decided before anything collective happens.
 struct Prepared {
-    const Plan* plan = nullptr;
-    at::Tensor  x;              // the tensor the kernel reads (the input, or a densified copy)
-    at::Tensor  output;
-    Window*     window        = nullptr;
-    bool        out_is_window = false;
-    int         pool_slot     = 0;  // > 0: `output` is that buffer of the output pool
+    std::shared_ptr<const Plan> plan;
+    at::Tensor                  x;  // the tensor the kernel reads (the input, or a densified copy)
+    at::Tensor                  output;
+    Window*                     window        = nullptr;
+    bool                        out_is_window = false;
+    int                         pool_slot     = 0;  // > 0: `output` is that buffer of the output pool
     // Every rank evaluates the same condition (role, no out=, pool switched on, no capture): when it
     // holds, any rank may ask for this call's payload in one of its pool buffers; when it does not,
     // no rank can, and the kernel is told that there is no pool at all.
@@ -109,7 +109,7 @@ Prepared prepare(Group& g, const at::Tensor& input, int64_t mode, const Splits& 
             p.x = p.x.clone();
         }
     }
-    p.plan = &g.plan(p.x.sizes(), strides, p.x.scalar_type(), mode, seq, heads);
+    p.plan = g.plan(p.x.sizes(), strides, p.x.scalar_type(), mode, seq, heads);
     const auto    dtype        = p.x.scalar_type();
     const int64_t elem         = static_cast<int64_t>(c10::elementSize(dtype));
     const int64_t window_bytes = p.plan->window_numel * elem;
@@ -230,7 +230,7 @@ std::vector<int64_t> output_shape_for(const Group& g, const at::Tensor& input, i
 {
     // Shape rule only; shares the validation with the real kernel through a throw-away plan.
     Group& mut = const_cast<Group&>(g);
-    return mut.plan(input.sizes(), {}, input.scalar_type(), mode, seq, heads).out_shape;
+    return mut.plan(input.sizes(), {}, input.scalar_type(), mode, seq, heads)->out_shape;
 }
 
 }  // namespace
@@ -375,9 +375,9 @@ at::Tensor empty_output(const GroupPtr& group, const at::Tensor& input, int64_t 
 {
     group->check_alive();
     require_backend(*group, input, "input");
-    const Plan&   plan = group->plan(input.sizes(), {}, input.scalar_type(), mode, seq, heads);
+    const auto    plan = group->plan(input.sizes(), {}, input.scalar_type(), mode, seq, heads);
     const int64_t elem = static_cast<int64_t>(input.element_size());
-    return group->make_output(plan.out_shape, input.scalar_type(), plan.window_numel * elem);
+    return group->make_output(plan->out_shape, input.scalar_type(), plan->window_numel * elem);
 }
 
 at::Tensor empty_output_meta(const GroupPtr&, const at::Tensor&, int64_t, const Splits&, const Splits&)

@@ -1050,7 +1050,8 @@ Tensor fp8_exchange(const GroupRef& ref, const Tensor& x_in, int64_t mode, const
     const c10::cuda::CUDAGuard                 on(x_in.device());
     const at::AutoDispatchBelowADInplaceOrView below;
     Tensor                                     x    = x_in.contiguous();
-    const Plan&                                plan = g.plan(x.sizes(), {}, x.scalar_type(), mode, seq, heads);
+    const std::shared_ptr<const Plan>          kept = g.plan(x.sizes(), {}, x.scalar_type(), mode, seq, heads);
+    const Plan&                                plan = *kept;
     Tensor                                     out  = empty_bf16(plan.out_shape, x);
     const int                                  world = g.world(), rank = g.rank();
     if (world == 1) {

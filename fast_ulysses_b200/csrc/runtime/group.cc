@@ -130,24 +130,24 @@ void Group::check_alive() const
     TORCH_CHECK(alive_, "this UlyssesGroup has been destroyed; build a new one");
 }
 
-const Plan& Group::plan(at::IntArrayRef sizes, at::IntArrayRef strides, at::ScalarType dtype, int64_t mode,
-                        const Splits& seq, const Splits& heads)
+std::shared_ptr<const Plan> Group::plan(at::IntArrayRef sizes, at::IntArrayRef strides, at::ScalarType dtype, int64_t mode,
+                                        const Splits& seq, const Splits& heads)
 {
     const std::lock_guard<std::mutex> lock(plan_mutex_);
     const bool plain = !seq.has_value() && !heads.has_value() && sizes.size() == 4 && (strides.empty() || strides.size() == 4);
     if (plain && last_plan_.plan && last_plan_.mode == mode && last_plan_.dtype == dtype
         && std::equal(sizes.begin(), sizes.end(), last_plan_.sizes) && last_plan_.strided == !strides.empty()
         && (strides.empty() || std::equal(strides.begin(), strides.end(), last_plan_.strides))) {
-        return *last_plan_.plan;
+        return last_plan_.plan;
     }
-    auto remember = [&](const Plan& found) -> const Plan& {
+    auto remember = [&](const std::shared_ptr<const Plan>& found) {
         if (plain) {
             last_plan_.mode    = mode;
             last_plan_.dtype   = dtype;
             last_plan_.strided = !strides.empty();
             std::copy(sizes.begin(), sizes.end(), last_plan_.sizes);
             std::copy(strides.begin(), strides.end(), last_plan_.strides);
-            last_plan_.plan = &found;  // map nodes do not move; clear() below forgets it
+            last_plan_.plan = found;
         }
         return found;
     };
@@ -189,10 +189,9 @@ const Plan& Group::plan(at::IntArrayRef sizes, at::IntArrayRef strides, at::Scal
                 "this call moves no data: every rank's shard is empty. Check the shape and the splits -- a "
                 "sequence or head axis of 0 on ALL ranks has nothing to exchange");
     if (plans_.size() >= kPlanCacheCap) {
-        last_plan_.plan = nullptr;
         plans_.clear();
     }
-    return remember(plans_.emplace(std::move(key), std::move(p)).first->second);
+    return remember(plans_.emplace(std::move(key), std::make_shared<const Plan>(std::move(p))).first->second);
 }
 
 Window Group::allocate(int64_t bytes)
@@ -660,8 +659,11 @@ void Group::destroy()
         const c10::cuda::CUDAGuard guard(static_cast<c10::DeviceIndex>(device_index_));
         cudaDeviceSynchronize();
     }
-    last_plan_.plan = nullptr;
-    plans_.clear();
+    {
+        const std::lock_guard<std::mutex> lock(plan_mutex_);
+        last_plan_.plan = nullptr;
+        plans_.clear();
+    }
     windows_.clear();
     pool_.clear();
     pool_capacity_ = 0;

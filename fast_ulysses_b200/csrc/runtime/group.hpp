@@ -73,8 +73,9 @@ public:
 
     // Validation on rank-uniform quantities only, then the cached plan. Throws before anything
     // collective has happened, so a rejected argument is rejected on every rank together.
-    const Plan& plan(at::IntArrayRef sizes, at::IntArrayRef strides, at::ScalarType dtype, int64_t mode,
-                     const Splits& seq, const Splits& heads);
+    // The caller shares the plan: another thread may empty the cache while this call still uses it.
+    std::shared_ptr<const Plan> plan(at::IntArrayRef sizes, at::IntArrayRef strides, at::ScalarType dtype, int64_t mode,
+                                     const Splits& seq, const Splits& heads);
 
     Window&       window(Role role, int64_t bytes);
     Window&       lend_window(int64_t bytes);
@@ -151,14 +152,14 @@ private:
     cudaEvent_t order_event_ = nullptr;
 
     std::mutex                           plan_mutex_;  // autograd's thread and the caller's may both ask
-    std::map<std::vector<int64_t>, Plan> plans_;
+    std::map<std::vector<int64_t>, std::shared_ptr<const Plan>> plans_;
     // The call before this one: a loop over layers asks for the same plan again and again.
     struct LastPlan {
-        int64_t        mode = -1;
-        at::ScalarType dtype = at::kByte;
-        bool           strided = false;
-        int64_t        sizes[4] = {}, strides[4] = {};
-        const Plan*    plan = nullptr;
+        int64_t                     mode = -1;
+        at::ScalarType              dtype = at::kByte;
+        bool                        strided = false;
+        int64_t                     sizes[4] = {}, strides[4] = {};
+        std::shared_ptr<const Plan> plan;
     } last_plan_;
     std::map<int64_t, Window>            windows_;  // by role
     std::array<Window, kLentSlots>       lent_;

@@ -250,3 +250,32 @@ def test_mode_1_undoes_mode_0_for_any_layout(lay):
     back, _ = replay(b, seq, heads, d, 1, [np.ascontiguousarray(m) for m in mid])
     for r in range(len(seq)):
         assert np.array_equal(back[r], inputs[r])
+
+
+def test_a_plan_in_use_outlives_the_cache_that_held_it():
+    """Calls run without the GIL: while one is moving its rows, other threads may ask for so many other shapes
+    that the cache of 512 plans is emptied, and its memory taken for theirs."""
+    import threading
+
+    group = fast_ulysses_b200.UlyssesGroup(device="cpu")
+    x = torch.arange(400_000 * 3 * 4, dtype=torch.int32).view(1, 400_000, 3, 4).view(torch.float32)
+    done = threading.Event()
+
+    def ask_for_other_shapes():
+        s = 0
+        while not done.is_set():
+            s = s % 5000 + 1
+            group.all_to_all_4d(torch.empty(1, s, 1, 16, dtype=torch.int8))
+
+    others = [threading.Thread(target=ask_for_other_shapes) for _ in range(3)]
+    for t in others:
+        t.start()
+    try:
+        for _ in range(20):
+            y = group.all_to_all_4d(x, mode=1)
+            assert torch.equal(y.view(torch.int32), x.view(torch.int32))
+    finally:
+        done.set()
+        for t in others:
+            t.join()
+    group.destroy()
