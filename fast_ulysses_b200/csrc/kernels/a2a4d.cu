@@ -1063,12 +1063,10 @@ extern "C" int fu_a2a4d(const FuA2AArgs* args, void* stream_v)
         a2a4d_kernel<false><<<ctas, kLdstThreads, 0, stream>>>(k);
     }
     else {
-        static bool configured[64] = {};
-        const int   smem_bytes     = kStages * kStageBytes;
-        if (dev < 64 && !configured[dev]) {
-            FU_CUDA_OK(cudaFuncSetAttribute(a2a4d_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                            smem_bytes));
-            configured[dev] = true;
+        const int smem_bytes = kStages * kStageBytes;
+        const int limit      = fu::raise_smem_limit(a2a4d_kernel<true>, smem_bytes);
+        if (limit != FU_OK) {
+            return limit;
         }
         a2a4d_kernel<true><<<ctas, 32, smem_bytes, stream>>>(k);
     }

@@ -2,6 +2,8 @@
 // CTAs take a part of the item's steps (kv tiles forward, query blocks backward) and join their results.
 #pragma once
 
+#include "host_util.h"
+
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -20,7 +22,7 @@ inline cudaLaunchAttribute cluster_attr(int csize)
 }
 
 // How many clusters of `csize` CTAs of a kernel the device holds at once (a cluster stays inside a GPC);
-// 0 when it cannot be asked. Asked once per device and size; also sets the kernel's shared-memory limit.
+// 0 when it cannot be asked. Asked once per device and size; also raises the kernel's shared-memory limit.
 class ClusterCapacity {
 public:
     template <typename Kernel>
@@ -39,8 +41,7 @@ public:
             cfg.attrs                = &attr;
             cfg.numAttrs             = 1;
             int n                    = 0;
-            if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_bytes) != cudaSuccess
-                || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+            if (raise_smem_limit(kernel, smem_bytes) != FU_OK || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
                 (void)cudaGetLastError();
                 n = -1;
             }

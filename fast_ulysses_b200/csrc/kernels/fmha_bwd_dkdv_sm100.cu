@@ -379,10 +379,9 @@ int fu_fmha_bwd_dkdv_launch(const FuFmhaArgs* a, const float* lse2, const float*
     int dev = 0, sms = 0;
     FU_CUDA_OK(cudaGetDevice(&dev));
     FU_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    static bool configured[64] = {};
-    if (dev < 64 && !configured[dev]) {
-        FU_CUDA_OK(cudaFuncSetAttribute(fmha_bwd_dkdv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        configured[dev] = true;
+    rc = fu::raise_smem_limit(fmha_bwd_dkdv_kernel, SMEM_BYTES);
+    if (rc != FU_OK) {
+        return rc;
     }
     int grid = a->ctas > 0 ? std::min(a->ctas, sms) : sms;
     grid     = std::max(1, std::min(grid, p.total_work));

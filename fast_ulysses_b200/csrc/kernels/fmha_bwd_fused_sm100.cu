@@ -685,12 +685,9 @@ int fu_fmha_bwd_fused_launch(const FuFmhaArgs* a, const float* lse2, const float
     int dev = 0, sms = 0;
     FU_CUDA_OK(cudaGetDevice(&dev));
     FU_CUDA_OK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-    static bool configured[64] = {};
-    if (dev >= 64 || !configured[dev]) {
-        FU_CUDA_OK(cudaFuncSetAttribute(fmha_bwd_fused_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-        if (dev < 64) {
-            configured[dev] = true;
-        }
+    rc = fu::raise_smem_limit(fmha_bwd_fused_kernel<false>, SMEM_BYTES);
+    if (rc != FU_OK) {
+        return rc;
     }
     const int             items = p.total_work;
     const fu::ClusterPlan plan  = a->ctas > 0 || a->trace ? fu::ClusterPlan{items, 1, 0.0} : plan_split(items, p.n_q, sms, dev);

@@ -18,6 +18,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <atomic>
 #include <initializer_list>
 
 namespace {
@@ -231,8 +232,8 @@ extern "C" int fu_fmha_bwd_noalloc(const FuFmhaArgs* a, void* stream)
     // per device, with that device current. This happens on the first call on each device. The
     // address is remembered for the life of the process: after cudaDeviceReset() it is stale, and
     // this entry point must not be used again in that process.
-    static void* base[64] = {};
-    int          dev      = 0;
+    static std::atomic<void*> base[64] = {};
+    int                       dev      = 0;
     FU_CUDA_OK(cudaGetDevice(&dev));
     if (dev < 0 || dev >= 64) {
         return fu::fail(FU_E_UNSUPPORTED, "fu_fmha_bwd_noalloc: device index %d", dev);
@@ -243,8 +244,8 @@ extern "C" int fu_fmha_bwd_noalloc(const FuFmhaArgs* a, void* stream)
         base[dev] = ptr;
     }
     FuFmhaArgs local = *a;
-    local.delta      = reinterpret_cast<float*>(base[dev]);
-    local.dq_acc     = reinterpret_cast<float*>(static_cast<unsigned char*>(base[dev]) + kNoAllocStatsBytes);
+    local.delta      = static_cast<float*>(base[dev].load());
+    local.dq_acc     = reinterpret_cast<float*>(static_cast<unsigned char*>(base[dev].load()) + kNoAllocStatsBytes);
     // fu_fmha_bwd zeroes the accumulator and rewrites every statistic it reads, so nothing of an
     // earlier call survives into this one.
     return fu_fmha_bwd(&local, stream);

@@ -896,13 +896,10 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
     if (np < 0 || np > 6 || (np & 1)) {
         return fu::fail(FU_E_ARG, "fu_fmha_fwd: %d of 16 exponential pairs on the FMA pipe is not built (0, 2, 4, 6)", np);
     }
-    static bool configured[64][8] = {};
-    auto launch = [&](auto kernel, int slot) -> int {
-        if (dev >= 64 || a->trace || !configured[dev][slot]) {
-            FU_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES));
-            if (dev < 64) {
-                configured[dev][slot] = true;
-            }
+    auto launch = [&](auto kernel) -> int {
+        const int limit = fu::raise_smem_limit(kernel, SMEM_BYTES);
+        if (limit != FU_OK) {
+            return limit;
         }
         int grid = a->ctas > 0 ? std::min(a->ctas, sms) : sms;
         grid     = std::max(1, std::min(grid, p.total_work));
@@ -915,7 +912,7 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
         if (np != kPolyPairs) {
             return fu::fail(FU_E_ARG, "fu_fmha_fwd: the timeline build exists for the default exponential split only");
         }
-        return launch(fmha_fwd_kernel<kPolyPairs, true, Form::kTwoTiles>, np);
+        return launch(fmha_fwd_kernel<kPolyPairs, true, Form::kTwoTiles>);
     }
     if (np == kPolyPairs && a->ctas <= 0) {
         const fu::ClusterPlan plan = plan_split(p.total_work, p.n_kv, sms, dev);
@@ -926,13 +923,13 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
         if (p.n_kv > 1 && ((one_items + sms - 1) / sms) * 1.1 * ((p.n_kv + 1) / 2 + 3.0) < plan.cost) {
             p.q_blocks   = one_blocks;
             p.total_work = one_items;
-            return launch(fmha_fwd_kernel<kPolyPairs, false, Form::kOneTile>, 7);
+            return launch(fmha_fwd_kernel<kPolyPairs, false, Form::kOneTile>);
         }
         if (plan.csize > 1) {
             const int items = p.total_work;
             p.total_work    = plan.whole;
             if (plan.whole > 0) {
-                rc = launch(fmha_fwd_kernel<kPolyPairs, false, Form::kTwoTiles>, np);
+                rc = launch(fmha_fwd_kernel<kPolyPairs, false, Form::kTwoTiles>);
                 if (rc != FU_OK) {
                     return rc;
                 }
@@ -951,10 +948,10 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
         }
     }
     switch (np) {
-    case 0: return launch(fmha_fwd_kernel<0, false, Form::kTwoTiles>, np);
-    case 2: return launch(fmha_fwd_kernel<2, false, Form::kTwoTiles>, np);
-    case 4: return launch(fmha_fwd_kernel<4, false, Form::kTwoTiles>, np);
-    case 6: return launch(fmha_fwd_kernel<6, false, Form::kTwoTiles>, np);
+    case 0: return launch(fmha_fwd_kernel<0, false, Form::kTwoTiles>);
+    case 2: return launch(fmha_fwd_kernel<2, false, Form::kTwoTiles>);
+    case 4: return launch(fmha_fwd_kernel<4, false, Form::kTwoTiles>);
+    case 6: return launch(fmha_fwd_kernel<6, false, Form::kTwoTiles>);
     default: return fu::fail(FU_E_ARG, "fu_fmha_fwd: %d of 16 exponential pairs on the FMA pipe is not built (0, 2, 4, 6)", np);
     }
 }

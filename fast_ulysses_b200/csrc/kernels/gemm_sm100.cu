@@ -16,8 +16,8 @@
 #include "tma_host.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
-#include <mutex>
 
 namespace {
 
@@ -622,8 +622,8 @@ __global__ void __launch_bounds__(THREADS + 128, 1) pull_outproj_kernel(const __
 
 int device_sms()
 {
-    static int cached[64] = {};
-    int        dev        = 0;
+    static std::atomic<int> cached[64] = {};
+    int                     dev        = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
         return 148;
     }
@@ -642,40 +642,12 @@ int launch_grid(int ctas, int tiles)
     return std::max(1, std::min(g, tiles));
 }
 
-// Raises a kernel's dynamic shared-memory limit once per (device, kernel). Keyed by the kernel's
-// address: two kernels with the same signature share one instantiation of this template.
-template <class K>
-int set_smem(K kernel, int bytes = SMEM_BYTES)
-{
-    struct Done {
-        int         dev;
-        const void* fn;
-    };
-    static std::mutex lock;
-    static Done       done[256];
-    static int        n_done = 0;
-    int               dev    = 0;
-    FU_CUDA_OK(cudaGetDevice(&dev));
-    const void*                       fn = reinterpret_cast<const void*>(kernel);
-    const std::lock_guard<std::mutex> guard(lock);
-    for (int i = 0; i < n_done; ++i) {
-        if (done[i].dev == dev && done[i].fn == fn) {
-            return FU_OK;
-        }
-    }
-    FU_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
-    if (n_done < 256) {
-        done[n_done++] = Done{dev, fn};
-    }
-    return FU_OK;
-}
-
 // How many CTA pairs of the wide kernels the device holds at once (GPCs with an odd number of SMs
 // leave one SM without a partner). Asked once per device; all of them have the same shape.
 int pair_capacity()
 {
-    static int cached[64] = {};
-    int        dev        = 0;
+    static std::atomic<int> cached[64] = {};
+    int                     dev        = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev >= 64) {
         return 0;
     }
@@ -693,7 +665,7 @@ int pair_capacity()
         cfg.attrs             = &attr;
         cfg.numAttrs          = 1;
         int n                 = 0;
-        if (set_smem(kernel, WIDE_SMEM_BYTES) != FU_OK || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess
+        if (raise_smem_limit(kernel, WIDE_SMEM_BYTES) != FU_OK || cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess
             || n < 1) {
             (void)cudaGetLastError();
             // the kernel carries its cluster shape itself; ask again without naming it
@@ -709,7 +681,7 @@ int pair_capacity()
         }
         cached[dev] = n > 0 ? n : -1;
     }
-    return cached[dev] > 0 ? cached[dev] : 0;
+    return std::max(0, cached[dev].load());
 }
 
 // Which core and tile a problem gets, from its size alone: the one whose estimated time is lowest. The
@@ -949,7 +921,7 @@ int pairs_for(int ctas)
 template <class Kernel, class Args>
 int launch_pairs(Kernel kernel, const Args& a, int pairs, cudaStream_t stream)
 {
-    const int rc = set_smem(kernel, WIDE_SMEM_BYTES);
+    const int rc = raise_smem_limit(kernel, WIDE_SMEM_BYTES);
     if (rc != FU_OK) {
         return rc;
     }
@@ -961,7 +933,7 @@ int launch_pairs(Kernel kernel, const Args& a, int pairs, cudaStream_t stream)
 template <class Kernel, class Args>
 int launch_small(Kernel kernel, const Args& a, int ctas, cudaStream_t stream)
 {
-    const int rc = set_smem(kernel, SMALL_SMEM_BYTES);
+    const int rc = raise_smem_limit(kernel, SMALL_SMEM_BYTES);
     if (rc != FU_OK) {
         return rc;
     }
@@ -974,7 +946,7 @@ template <int ACT>
 int launch_clusters(void (*kernel)(PlainArgs<ACT>), const PlainArgs<ACT>& a, int clusters, int csize, int threads, int smem,
                     cudaStream_t stream)
 {
-    const int rc = set_smem(kernel, smem);
+    const int rc = raise_smem_limit(kernel, smem);
     if (rc != FU_OK) {
         return rc;
     }
@@ -1314,7 +1286,7 @@ extern "C" int fu_pull_outproj(const FuPullArgs* q, void* stream_v)
     a.epi.ldc          = q->ldc;
     a.epi.M            = a.core.M;
     a.epi.N            = a.core.N;
-    rc                 = set_smem(pull_outproj_kernel);
+    rc                 = raise_smem_limit(pull_outproj_kernel, SMEM_BYTES);
     if (rc != FU_OK) {
         return rc;
     }

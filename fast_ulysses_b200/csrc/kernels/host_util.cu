@@ -1,11 +1,29 @@
 #include "fu_kernels.h"
 #include "host_util.h"
 
+#include <mutex>
+#include <set>
+#include <utility>
+
 namespace fu {
 char* error_buffer()
 {
     static thread_local char buf[512] = {0};
     return buf;
+}
+
+int raise_smem_limit(const void* kernel, int bytes)
+{
+    static std::mutex                            lock;
+    static std::set<std::pair<int, const void*>> raised;
+    int                                          dev = 0;
+    FU_CUDA_OK(cudaGetDevice(&dev));
+    const std::lock_guard<std::mutex> guard(lock);
+    if (raised.count({dev, kernel}) == 0) {
+        FU_CUDA_OK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+        raised.insert({dev, kernel});
+    }
+    return FU_OK;
 }
 }  // namespace fu
 

@@ -1,6 +1,8 @@
 #pragma once
 // Host-side helpers shared by the launchers: a thread-local error string and CUDA call checking
 // that reports instead of aborting, because these launchers are called from inside a framework.
+#include "fu_kernels.h"
+
 #include <cuda_runtime.h>
 #include <cstdarg>
 #include <cstdio>
@@ -16,6 +18,16 @@ inline int fail(int code, const char* fmt, ...)
     vsnprintf(error_buffer(), 512, fmt, ap);
     va_end(ap);
     return code;
+}
+
+// Raises a kernel's dynamic shared-memory limit on the current device, once per device and kernel. Launches come
+// from several threads (autograd's beside the caller's): the record of what has been raised is locked.
+int raise_smem_limit(const void* kernel, int bytes);
+
+template <class Kernel>
+int raise_smem_limit(Kernel kernel, int bytes)
+{
+    return raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes);
 }
 
 }  // namespace fu

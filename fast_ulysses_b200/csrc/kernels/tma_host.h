@@ -3,6 +3,7 @@
 // the library needs no link-time dependency on libcuda and loads on a machine without a GPU.
 #include <cuda.h>
 #include <cuda_runtime.h>
+#include <atomic>
 #include <cstdint>
 
 #include "fu_kernels.h"
@@ -24,8 +25,8 @@ inline EncodeTiledFn encode_tiled_fn()
         cudaFree(nullptr);
         bound = true;
     }
-    static EncodeTiledFn fn = nullptr;
-    if (!fn) {
+    static std::atomic<EncodeTiledFn> fn = nullptr;
+    if (!fn.load()) {
         void*                           p = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess

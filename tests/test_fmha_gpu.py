@@ -144,3 +144,21 @@ def test_gradient_that_starts_off_16_bytes(offset):
     assert torch.equal(grads[0][1], grads[1][1]) and torch.equal(grads[0][2], grads[1][2])
     # dq is summed in fp32 in another order from call to call, then rounded to bf16
     assert ((grads[0][0].float() - grads[1][0].float()).norm() / grads[1][0].float().norm()).item() < 2e-3
+
+
+def test_a_plain_launch_behind_the_instrumented_one():
+    """Each build of the kernel has its shared-memory limit raised for itself, whichever runs first in a process."""
+    import pathlib
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from fast_ulysses_b200.ops import attention, gemm
+q, k, v = (torch.randn(1, 256, 148, 128, device="cuda").bfloat16() for _ in range(3))
+traced, _ = attention.fmha_fwd(q, k, v, trace=torch.zeros(256, dtype=torch.int64, device="cuda"))
+plain, _ = attention.fmha_fwd(q, k, v, ctas=148)
+gemm.check_errors()
+assert torch.equal(traced, plain)
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=pathlib.Path(__file__).parents[1])
