@@ -1086,7 +1086,8 @@ Tensor fp8_exchange(const GroupRef& ref, const Tensor& x_in, int64_t mode, const
             }
         }
     }
-    a.timeout_ms = 10000;
+    a.flags      = g.test_flags();
+    a.timeout_ms = g.timeout_ms();
     ok(fu_a2a4d_fp8(&a, stream_of(x)));
     return out;
 }

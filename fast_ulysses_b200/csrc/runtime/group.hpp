@@ -125,8 +125,10 @@ public:
     int64_t epoch(int64_t role_or_ptr, const at::Tensor& probe);
     std::vector<int64_t> stamps(int64_t role);
 
-    void set_timeout_ms(int64_t ms) { timeout_ms_ = static_cast<uint32_t>(ms); }
+    void     set_timeout_ms(int64_t ms) { timeout_ms_ = static_cast<uint32_t>(ms); }
+    uint32_t timeout_ms() const { return timeout_ms_; }
     void set_test_flags(int64_t flags) { test_flags_ = static_cast<int>(flags); }
+    int  test_flags() const { return test_flags_; }
     void set_ctas(int64_t ctas) { ctas_ = static_cast<int>(ctas); }
     int64_t windows_allocated() const { return allocations_; }
 

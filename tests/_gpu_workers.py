@@ -2,6 +2,8 @@
 the library is bounded, so a protocol error ends as a status (checked with group.check()) or a
 mismatch, never as a hang. No test here faults, traps or hangs a GPU on purpose."""
 
+import time
+
 import torch
 import torch.distributed as dist
 
@@ -644,6 +646,28 @@ def peer_timeout_is_reported(rank, world):
         raised = "timed out" in str(e) and f"waiting on rank {world - 1}" in str(e)
     # the silent rank itself may or may not have run out of time waiting for the others
     assert raised or rank == world - 1, "the missing announcement was not reported"
+
+    # the fp8 exchange waits no longer than its group does either
+    from fast_ulysses_b200.ops import fp8
+
+    x = torch.randn(1, 64, 2 * world, 128, device=dev, dtype=torch.bfloat16)
+    fp8.all_to_all_4d_fp8(g, x)
+    g.check()
+    dist.barrier()
+    if rank == world - 1:
+        g._handle.set_test_flags(16)  # FU_A2A_MUTE
+    t0 = time.monotonic()
+    fp8.all_to_all_4d_fp8(g, x)
+    torch.cuda.synchronize()
+    took = time.monotonic() - t0
+    g._handle.set_test_flags(0)
+    raised = False
+    try:
+        g.check()
+    except RuntimeError as e:
+        raised = "timed out" in str(e) and "fp8 window" in str(e)
+    assert raised or rank == world - 1, "the missing announcement was not reported"
+    assert took < 5.0, f"waited {took:.1f} s in a group with a limit of 0.3 s"
     assert torch.ones(8, device=dev).sum().item() == 8  # context alive
     dist.barrier()
     g.destroy()
