@@ -386,6 +386,9 @@ FU_API int fu_fp8_round_trip(const void* src, void* dst, int64_t rows, void* str
 FU_API int fu_a2a4d_fp8(const FuA2AFp8Args* args, void* stream);
 FU_API int fu_a2a4d_fp8_check(const FuA2AFp8Args* args);  // the argument checks alone; no CUDA call
 
+// The address, on the current device, of a word that kernels given it as `err` set when one of their bounded waits
+// runs out. One per device, zero at first.
+FU_API int fu_error_word(void** word);
 FU_API const char* fu_last_error(void);
 FU_API const char* fu_build_info(void);  // "sm_100a;<nvcc version>;<library version>"
 

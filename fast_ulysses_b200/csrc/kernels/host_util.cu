@@ -27,6 +27,19 @@ int raise_smem_limit(const void* kernel, int bytes)
 }
 }  // namespace fu
 
+// The word lies in the library's image, zero from the moment it is loaded: nothing is allocated, filled or waited
+// for when it is first asked for, which may be inside a stream capture.
+static __device__ uint32_t g_error_word;
+
+extern "C" int fu_error_word(void** word)
+{
+    if (!word) {
+        return fu::fail(FU_E_ARG, "fu_error_word: null argument");
+    }
+    FU_CUDA_OK(cudaGetSymbolAddress(word, g_error_word));
+    return FU_OK;
+}
+
 #define FU_STR2(x) #x
 #define FU_STR(x) FU_STR2(x)
 

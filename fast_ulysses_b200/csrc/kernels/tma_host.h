@@ -19,11 +19,12 @@ inline EncodeTiledFn encode_tiled_fn()
 {
     // The encoder is a driver call and wants a current context on the calling thread. A thread that
     // has made no runtime call yet (an autograd worker whose first CUDA work is one of these
-    // launches) has none: a no-op runtime call binds the device's primary context to it.
+    // launches) has none: choosing the current device again binds its primary context to it, also while a
+    // stream is being captured.
     static thread_local bool bound = false;
     if (!bound) {
-        cudaFree(nullptr);
-        bound = true;
+        int dev = 0;
+        bound   = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
     }
     static std::atomic<EncodeTiledFn> fn = nullptr;
     if (!fn.load()) {

@@ -8,7 +8,6 @@
 #include <torch/csrc/utils/pybind.h>
 
 #include <cmath>
-#include <mutex>
 
 namespace py = pybind11;
 
@@ -80,24 +79,16 @@ cudaStream_t stream_of(const Tensor& t)
 // One device word per GPU that kernels set when one of their bounded waits ran out.
 Tensor error_word(int64_t device)
 {
-    static std::mutex                lock;
-    static std::map<int64_t, Tensor> words;
-    const std::lock_guard<std::mutex> guard(lock);
-    auto                              it = words.find(device);
-    if (it == words.end()) {
-        const c10::Device dev(c10::DeviceType::CUDA, static_cast<c10::DeviceIndex>(device));
-        // zeroed before any stream can use it: the word is shared by all of them
-        Tensor w = at::zeros({1}, at::TensorOptions().dtype(at::kInt).device(dev));
-        const c10::cuda::CUDAGuard on(dev);
-        cudaStreamSynchronize(at::cuda::getCurrentCUDAStream(dev.index()));
-        it = words.emplace(device, w).first;
-    }
-    return it->second;
+    const c10::Device          dev(c10::DeviceType::CUDA, static_cast<c10::DeviceIndex>(device));
+    const c10::cuda::CUDAGuard on(dev);
+    void*                      word = nullptr;
+    ok(fu_error_word(&word));
+    return at::from_blob(word, {1}, at::TensorOptions().dtype(at::kInt).device(dev));
 }
 
 uint32_t* error_ptr(const Tensor& t)
 {
-    // the map is looked up once per device and thread
+    // asked for once per device and thread
     static thread_local uint32_t* cached[16] = {};
     const int64_t                 d = t.device().index();
     if (d < 0 || d >= 16) {

@@ -99,3 +99,31 @@ def test_layer_norm_fork_joins_both_gradients(rows, cols):
     x.grad = None
     norm.layer_norm_fork(x)[1].backward(gr)  # only the residual is used
     assert torch.equal(x.grad, gr)
+
+
+def test_first_call_of_a_process_inside_a_graph_capture():
+    """Nothing an operator sets up on its first call is refused, or recorded, by a capture."""
+    import pathlib
+    import subprocess
+    import sys
+
+    code = """
+import torch
+from fast_ulysses_b200.ops import attention, gemm, norm
+x = torch.randn(1, 256, 512, device="cuda").bfloat16()
+w = torch.randn(512, 512, device="cuda").bfloat16()
+
+def step():
+    h = norm.layer_norm(x)
+    q = gemm.linear(h, w).view(1, 256, 4, 128)
+    return attention.attention(q, q, q)
+
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    y = step()
+gemm.check_errors()
+graph.replay()
+gemm.check_errors()
+assert torch.equal(y, step())
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=300, cwd=pathlib.Path(__file__).parents[1])
