@@ -110,6 +110,18 @@ Tensor empty_bf16(at::IntArrayRef shape, const Tensor& like)
 {
     return at::detail::empty_cuda(shape, at::kBFloat16, like.device(), std::nullopt);
 }
+// `t` with the strides of `out`, which an epilogue reads it by: a tensor saved for backward comes back dense where
+// hooks have packed it (moved to the host, say), whatever its pitch was.
+Tensor laid_out_like(const Tensor& out, const Tensor& t)
+{
+    if (t.strides() == out.strides() && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0) {
+        return t;
+    }
+    Tensor copy = at::empty_strided(out.sizes(), out.strides(), out.options());
+    copy.copy_(t);
+    return copy;
+}
+
 // A matrix of this library's own, read by later GEMMs: rows on 32-byte sectors, which TMA moves up to 1.7 times
 // as fast as rows that are not.
 Tensor empty_operand(int64_t rows, int64_t cols, const Tensor& like)
@@ -409,10 +421,10 @@ struct FeedForward : public torch::autograd::Function<FeedForward> {
         }
         if (wanted[0] || wanted[1] || wanted[2]) {
             GemmExtra e;  // d(pre-activation) = (gy W2) * gelu'(pre)
-            e.b_kn            = true;
-            e.act             = 3;
-            e.aux             = pre;
-            e.out             = empty_operand(gy2.size(0), w2.size(1), gy2);
+            e.b_kn = true;
+            e.act  = 3;
+            e.out  = empty_operand(gy2.size(0), w2.size(1), gy2);
+            e.aux  = laid_out_like(e.out, pre);
             const Tensor gpre = gemm(gy2, w2, e);
             if (wanted[1]) {
                 out[1] = gemm(gpre, x2, wgrad);

@@ -168,3 +168,18 @@ def test_linear_with_residual_in_the_epilogue():
     want = x.detach().float() @ w.detach().float().t() + r.detach().float()
     assert rel_err(y, want) < 1e-2
     assert torch.equal(r.grad, torch.ones_like(r))
+
+
+@pytest.mark.parametrize("ffn", [256, 264])  # 264: the hidden layer is kept with a wider pitch
+def test_feed_forward_under_hooks_that_move_what_it_saves(ffn):
+    torch.manual_seed(ffn)
+    args = [torch.randn(*s, device="cuda").mul_(0.3).bfloat16().requires_grad_()
+            for s in ((40, 64), (ffn, 64), (ffn,), (64, ffn), (64,), (40, 64))]
+    gy = torch.randn(40, 64, device="cuda").bfloat16()
+    want = torch.autograd.grad(gemm.feed_forward(*args), args, gy)
+    with torch.autograd.graph.save_on_cpu():
+        y = gemm.feed_forward(*args)
+    got = torch.autograd.grad(y, args, gy)
+    gemm.check_errors()
+    for a, b in zip(got, want):
+        assert torch.equal(a, b)
