@@ -133,13 +133,13 @@ Tensor empty_f32(at::IntArrayRef shape, const Tensor& like)
     return at::detail::empty_cuda(shape, at::kFloat, like.device(), std::nullopt);
 }
 
+// Whether a call goes through its autograd node. A forward-mode tangent does too, whatever the grad mode: the node
+// has no rule for one and says so, instead of a result without it.
 bool wants_grad(std::initializer_list<const Tensor*> ts)
 {
-    if (!at::GradMode::is_enabled()) {
-        return false;
-    }
+    const bool reverse = at::GradMode::is_enabled();
     for (const Tensor* t : ts) {
-        if (t->defined() && t->requires_grad()) {
+        if (t->defined() && ((reverse && t->requires_grad()) || t->_fw_grad(/*level=*/0).defined())) {
             return true;
         }
     }

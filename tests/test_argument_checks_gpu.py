@@ -7,7 +7,7 @@ import torch
 
 import fast_ulysses_b200 as fu
 from fast_ulysses_b200.models.attention import UlyssesSelfAttention
-from fast_ulysses_b200.ops import gemm
+from fast_ulysses_b200.ops import attention, gemm, norm
 
 pytestmark = pytest.mark.gpu
 
@@ -78,4 +78,23 @@ def test_attention_block_refuses_a_residual_on_the_host():
     x = bf16(1, 32, 256)
     with pytest.raises(AssertionError):
         attn(x, residual=x.cpu())
+    g.destroy()
+
+
+@pytest.mark.parametrize("mode", [torch.enable_grad, torch.no_grad])
+def test_forward_mode_tangents_are_refused_and_not_dropped(mode):
+    import torch.autograd.forward_ad as fw
+
+    g = fu.UlyssesGroup(device="cuda")
+    attn = UlyssesSelfAttention(g, 256, 2, grid=(1, 4, 8))
+    q = bf16(1, 32, 2, 128)
+    calls = [(lambda t: gemm.linear(t, bf16(N, K)), bf16(M, K)), (lambda t: gemm.linear(bf16(M, K), t), bf16(N, K)),
+             (lambda t: gemm.feed_forward(t, bf16(N, K), None, bf16(K, N), None), bf16(M, K)),
+             (norm.layer_norm, bf16(M, K)), (norm.layer_norm_fork, bf16(M, K)), (lambda t: attention.attention(q, t, q), bf16(1, 32, 2, 128)),
+             (attn, bf16(1, 32, 256))]
+    with fw.dual_level(), mode():
+        for call, x in calls:
+            call(x)
+            with pytest.raises(RuntimeError, match="jvp|forward AD"):
+                call(fw.make_dual(x, torch.randn_like(x)))
     g.destroy()
