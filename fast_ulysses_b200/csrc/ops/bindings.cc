@@ -515,10 +515,12 @@ void direct_all_to_all_4d_out(const GroupRef& ref, const at::Tensor& input, int6
 // The whole asynchronous call: the exchange on the comm stream, its completion event bound to the
 // result in torch's work registry, and the allocator told about both streams. Returns the result
 // and whether a registry exists.
-std::pair<at::Tensor, bool> direct_async(const GroupRef& ref, const at::Tensor& input, int64_t mode, const Splits& seq,
+std::pair<at::Tensor, bool> direct_async(const GroupRef& ref, const at::Tensor& given, int64_t mode, const Splits& seq,
                                          const Splits& heads, const std::optional<at::Tensor>& out, bool lend,
                                          int64_t comm_stream_id, bool hold_caller)
 {
+    // Holding the caller stands in for a private copy of the input, but not where the result goes over it.
+    const at::Tensor input = hold_caller && out.has_value() && given.is_alias_of(*out) ? given.clone() : given;
     const at::AutoDispatchBelowADInplaceOrView below;
     const c10::Device                 dev = input.device();
     const c10::cuda::CUDAGuard        guard(dev);

@@ -63,6 +63,20 @@ def test_staged_async_call_protects_its_input_and_orders_its_output(group):
     assert torch.equal(plain.wait(), keep)
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+def test_staged_async_call_may_write_over_its_input(group, mode):
+    buf = group.empty_output(torch.empty(2, 3000, 8, 64, device="cuda", dtype=torch.bfloat16), mode=mode)
+    plain = torch.empty_like(buf)
+    want = torch.randn(2, 3000, 8, 64, device="cuda").bfloat16()
+    for out in (buf, plain):  # a symmetric buffer that the call writes directly, and an ordinary tensor
+        out.copy_(want)
+        assert torch.equal(group.all_to_all_4d_async(out, mode=mode, out=out).wait(), want)
+    packed = torch.randn(2, 3000, 3, 8, 64, device="cuda").bfloat16()
+    want = packed[:, :, 1].clone()
+    out = packed.view(-1)[:want.numel()].view_as(want)  # overlaps the view it is filled from, row for other row
+    assert torch.equal(group.all_to_all_4d_async(packed[:, :, 1], mode=mode, out=out).wait(), want)
+
+
 @pytest.mark.parametrize("rows", [1, 31, 64, 65, 1000])
 def test_fp8_exchange_of_a_single_rank_is_quantise_and_dequantise(group, rows):
     gen = torch.Generator(device="cuda").manual_seed(rows)
