@@ -23,12 +23,20 @@ from .. import _C  # noqa: F401  (registers torch.ops.fast_ulysses_b200)
 _OPS = torch.ops.fast_ulysses_b200
 _is_compiling = torch.compiler.is_compiling
 _torch_function_mode = torch._C._is_torch_function_mode_enabled
+_dispatch_modes = torch._C._len_torch_dispatch_stack
+_functorch_level = torch._C._functorch.maybe_current_level
 
 
 def _direct(x) -> bool:
     """Whether a call may skip torch.ops' argument parsing (csrc/ops/bindings.cc: GroupRef). A tensor
     subclass, a TorchFunctionMode or a tracing compiler has to see the torch.ops call itself."""
     return type(x) is torch.Tensor and not _is_compiling() and not _torch_function_mode()
+
+
+def _undispatched(x) -> bool:
+    """Whether a call may skip the dispatcher as well: no TorchDispatchMode and no functorch transform is there to
+    see (or refuse) the operator."""
+    return _direct(x) and _dispatch_modes() == 0 and _functorch_level() is None
 
 
 class CompletedHandle:
@@ -220,7 +228,7 @@ class UlyssesGroup:
         hold_caller = stage and self.world_size == 1
         if stage and not hold_caller:
             x = x.clone()
-        if _direct(x) and (out is None or _direct(out)):
+        if _undispatched(x) and (out is None or _direct(out)):
             y, registered = _C.all_to_all_4d_async(self._ref, x, mode, seq_splits, head_splits, out, lend,
                                                    self._comm_stream.stream_id, hold_caller)
             return AsyncCollectiveTensor(y) if registered else CompletedHandle(y)

@@ -63,6 +63,27 @@ def test_staged_async_call_protects_its_input_and_orders_its_output(group):
     assert torch.equal(plain.wait(), keep)
 
 
+def test_async_call_is_seen_by_dispatch_modes_and_refused_by_vmap(group):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    seen = []
+
+    class Recorder(TorchDispatchMode):
+        def __torch_dispatch__(self, func, types, args=(), kwargs=None):
+            seen.append(str(func))
+            return func(*args, **(kwargs or {}))
+
+    x = torch.randn(2, 16, 4, 64, device="cuda").bfloat16()
+    out = group.empty_output(x)
+    with Recorder():
+        y = group.all_to_all_4d_async(x)
+        z = group.all_to_all_4d_async(x, out=out, stage=False)
+    assert torch.equal(y.wait(), x) and torch.equal(z.wait(), x)
+    assert any("all_to_all_4d_staged.default" in s for s in seen) and any("all_to_all_4d_staged_out.default" in s for s in seen)
+    with pytest.raises(RuntimeError, match="does not support torch.vmap"):
+        torch.vmap(lambda t: group.all_to_all_4d_async(t).wait())(x.unsqueeze(0))
+
+
 @pytest.mark.parametrize("mode", [0, 1])
 def test_staged_async_call_may_write_over_its_input(group, mode):
     buf = group.empty_output(torch.empty(2, 3000, 8, 64, device="cuda", dtype=torch.bfloat16), mode=mode)
