@@ -722,28 +722,9 @@ struct SpAttention : public torch::CustomClassHolder {
     Tensor               ready;  // flags of the pull kernel, grown on demand
     int64_t              comm_stream = 0;  // the group's comm stream (0: none)
     int64_t              forwards    = 0;  // q, k, v and o belong to the latest forward
-    // fp32 copies of norm weights kept in another type, remade when the parameter has changed
-    struct Cached {
-        uint32_t    version = 0;
-        const void* ptr     = nullptr;
-        Tensor      f32;
-    } gq_cache, gk_cache;
-
-    static Tensor f32(const Tensor& param, Cached& c)
-    {
-        const Tensor p = param.detach();
-        if (p.scalar_type() == at::kFloat && p.is_contiguous()) {
-            // a slice of a flat parameter buffer may start anywhere; the gradient kernel reads four values at a time
-            return reinterpret_cast<uintptr_t>(p.data_ptr()) % 16 == 0 ? p : p.clone();
-        }
-        const uint32_t version = param._version();
-        if (!c.f32.defined() || c.version != version || c.ptr != p.data_ptr()) {
-            c.f32     = p.to(at::kFloat).contiguous();
-            c.version = version;
-            c.ptr     = p.data_ptr();
-        }
-        return c.f32;
-    }
+    // A norm weight as the kernels read it: dense fp32 that starts on 16 bytes (a slice of a flat parameter buffer may
+    // start anywhere). Made anew for each call: a write through `.data` leaves no trace that a kept copy could be judged by.
+    static Tensor f32(const Tensor& param) { return aligned(param.detach().to(at::kFloat).contiguous()); }
 
     // How many CTAs a fused GEMM kernel of this block may take right now (0 = the whole device).
     //
@@ -890,7 +871,7 @@ struct SpAttention : public torch::CustomClassHolder {
         }
         {
             const NvtxRange r("fast_ulysses_b200::qkv_norm_rope_scatter");
-            scatter(f.x2, w_qkv, qkv_base, qkv_ctrl, 3, 2, rope, f32(gamma_q, gq_cache), f32(gamma_k, gk_cache), f.y_save, false);
+            scatter(f.x2, w_qkv, qkv_base, qkv_ctrl, 3, 2, rope, f32(gamma_q), f32(gamma_k), f.y_save, false);
         }
         {
             const NvtxRange r("fast_ulysses_b200::fmha_fwd");
@@ -971,7 +952,7 @@ struct SpAttentionFn : public torch::autograd::Function<SpAttentionFn> {
         C10_CUDA_CHECK(cudaMemsetAsync(dg.data_ptr(), 0, dg.nbytes(), stream_of(dy)));
         {
             const NvtxRange r("fast_ulysses_b200::pull_qkv_grads");
-            const Tensor    gq = SpAttention::f32(gamma_q, mod->gq_cache), gk = SpAttention::f32(gamma_k, mod->gk_cache);
+            const Tensor    gq = SpAttention::f32(gamma_q), gk = SpAttention::f32(gamma_k);
             FuPullGradsArgs a{};
             for (int64_t p = 0; p < mod->world; ++p) {
                 a.peer_dq[p]     = reinterpret_cast<const void*>(mod->dqkv_base[p]);
@@ -1136,8 +1117,8 @@ void bind_fused(py::module_& m)
         .def("scatter_qkv",
              [](SpAttention& s, const Tensor& x2, const Tensor& w, const Tensor& rope, const Tensor& gq, const Tensor& gk,
                 const MaybeTensor& y_save) {
-                 s.scatter(x2, w, s.qkv_base, s.qkv_ctrl, 3, 2, rope, SpAttention::f32(gq, s.gq_cache),
-                           SpAttention::f32(gk, s.gk_cache), or_none(y_save), false);
+                 s.scatter(x2, w, s.qkv_base, s.qkv_ctrl, 3, 2, rope, SpAttention::f32(gq),
+                           SpAttention::f32(gk), or_none(y_save), false);
              })
         .def("scatter_dout",
              [](SpAttention& s, const Tensor& dy2, const Tensor& w_o) {

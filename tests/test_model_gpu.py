@@ -128,3 +128,24 @@ def test_block_takes_a_gradient_that_starts_anywhere():
         assert torch.equal(block.attn(x, residual=odd), block.attn(x, residual=odd.clone()))
     gemm.check_errors()
     g.destroy()
+
+
+def test_bf16_norm_weights_written_through_data_are_seen():
+    g = fu.UlyssesGroup(device="cuda")
+    attn = UlyssesSelfAttention(g, 256, 2, grid=(2, 4, 8))
+    attn.gamma_q = torch.nn.Parameter(attn.gamma_q.detach().bfloat16())
+    x = torch.randn(1, 64, 256, device="cuda").bfloat16()
+    dy = torch.randn_like(x)
+    for value in (1.0, 3.0):
+        attn.gamma_q.data.fill_(value)  # as an optimizer that keeps fp32 master weights does
+        attn.zero_grad()
+        y = attn(x)
+        y.backward(dy)
+        got = y.detach(), attn.gamma_k.grad
+        attn.gamma_q = torch.nn.Parameter(torch.full((128,), value, device="cuda", dtype=torch.bfloat16))
+        attn.zero_grad()
+        fresh = attn(x)
+        fresh.backward(dy)
+        assert torch.equal(got[0], fresh)
+        assert rel_err(got[1], attn.gamma_k.grad) < 1e-4  # summed in fp32 in another order from call to call
+    g.destroy()
