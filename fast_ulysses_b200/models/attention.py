@@ -60,7 +60,7 @@ class UlyssesSelfAttention(nn.Module):
                  seq_splits: list[int] | None = None, head_splits: list[int] | None = None, eps: float = 1e-6,
                  out_bias: bool = True, timeout_ms: int = 10000):
         super().__init__()
-        self.group, self.hidden, self.heads, self.grid, self.eps = group, hidden, heads, grid, eps
+        self.group, self.hidden, self.heads, self.grid = group, hidden, heads, grid
         self.rank, self.world = group.rank, group.world_size
         total = grid[0] * grid[1] * grid[2]
         if seq_splits is None:
@@ -74,7 +74,7 @@ class UlyssesSelfAttention(nn.Module):
         self.s_total, self.s_local = total, seq_splits[self.rank]
         self.seq_off = sum(seq_splits[: self.rank])
         self.n_local = head_splits[self.rank]
-        self.batch, self.timeout_ms = batch, timeout_ms
+        self.batch = batch
         dev = group.device
 
         self.w_qkv = nn.Parameter(torch.randn(3 * heads * HEAD_DIM, hidden, device=dev).mul_(0.02).bfloat16())
@@ -113,6 +113,22 @@ class UlyssesSelfAttention(nn.Module):
                       [self.q_view, self.k_view, self.v_view, self.o_view, self.do_view, self.dq_view, self.dk_view,
                        self.dv_view])
         self._native = n
+
+    @property
+    def eps(self) -> float:
+        return self._native.eps
+
+    @eps.setter
+    def eps(self, value: float) -> None:
+        self._native.eps = value
+
+    @property
+    def timeout_ms(self) -> int:
+        return self._native.timeout_ms
+
+    @timeout_ms.setter
+    def timeout_ms(self, value: int) -> None:
+        self._native.timeout_ms = int(value)
 
     def forward(self, x: torch.Tensor, residual: torch.Tensor | None = None) -> torch.Tensor:
         """``residual`` (same shape as the result) is added in the output projection's epilogue."""

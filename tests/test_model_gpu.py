@@ -149,3 +149,18 @@ def test_bf16_norm_weights_written_through_data_are_seen():
         assert torch.equal(got[0], fresh)
         assert rel_err(got[1], attn.gamma_k.grad) < 1e-4  # summed in fp32 in another order from call to call
     g.destroy()
+
+
+def test_eps_and_timeout_set_later_take_effect():
+    torch.manual_seed(6)
+    g = fu.UlyssesGroup(device="cuda")
+    attn = UlyssesSelfAttention(g, 256, 2, grid=(2, 4, 8), eps=1e-6, timeout_ms=700)
+    x = torch.randn(1, 64, 256, device="cuda").bfloat16()
+    with torch.no_grad():
+        before = attn(x)
+        attn.eps, attn.timeout_ms = 0.5, 900
+        after = attn(x)
+        want = reference_attention(x, attn.w_qkv, attn.gamma_q, attn.gamma_k, attn.w_o, attn.b_o, 2, (2, 4, 8), eps=0.5)
+    assert not torch.equal(before, after) and rel_err(after, want) < 2e-2
+    assert (attn.eps, attn.timeout_ms, attn._native.timeout_ms) == (0.5, 900, 900)
+    g.destroy()
