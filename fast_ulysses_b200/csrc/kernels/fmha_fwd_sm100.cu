@@ -56,7 +56,8 @@ constexpr int SMEM_BYTES = (QT + 2 * KV_STAGES) * TILE_BYTES + 8 * OUT_BYTES + 1
 constexpr int THREADS    = 32 * 12;            // three warpgroups: {producer, MMA, 2 idle}, softmax 0, softmax 1
 constexpr int REGS_SMALL = 104;                 // warpgroup 0 after it has given registers away
 constexpr int REGS_SOFTMAX = 200;              // per scheduler: 32 x (104 + 2 x 200) = 16128 of 16384 registers
-constexpr float RANGE = 32.0f;                // in log2 units
+constexpr float RANGE = 8.0f;                 // in log2 units
+constexpr float RANGE_SUM = 256.0f;            // 2^RANGE
 constexpr int   kPolyPairs = 4;               // of every 16 exponential pairs, on the FMA pipe by default
 
 enum : uint32_t { ERR_LOAD = 11, ERR_MMA = 12, ERR_SOFTMAX = 13 };
@@ -567,12 +568,13 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
             const int h   = (w / p.q_blocks) % p.H;
             const int b   = w / (p.q_blocks * p.H);
             const int row = qb * ROWS + (ONE ? 0 : t * BM) + row_in;
-            // Exponentials are taken against a reference that is only roughly the row's maximum: P, O and
-            // the row sum are floating point, so any reference within 2^RANGE of it gives the same relative
-            // precision. It starts at 0 and is moved to a step's maximum when the step's exponentials
-            // leave that range. Whether they do is read off their own sum, so an ordinary step takes no
-            // maximum of the row; only the last quarter, which is handed over later, and the columns on the
-            // FMA pipe, whose exponent field wraps where the special-function unit returns infinity, are
+            // Exponentials are taken against a reference that is only roughly the row's maximum: that of the row's
+            // first step, until a step's exponentials leave a range of 2^RANGE above it; then it moves to that
+            // step's maximum. The weight of the key it was taken from is exactly 1, and weights are rounded to
+            // bf16, so a reference near the largest weight is also the more precise one (one key: the result is its
+            // value). Whether a step stays inside is read off the sum of its exponentials, so an ordinary
+            // step takes no maximum of the row; only the last quarter, which is handed over later, and the columns
+            // on the FMA pipe, whose exponent field wraps where the special-function unit returns infinity, are
             // judged by their scores. A row whose scores have all been -inf so far has no reference yet and takes
             // the one of the first step that has others.
             float m_ref = 0.0f;
@@ -609,6 +611,26 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                         }
                     }
                 };
+                if (j == j_first) {
+                    ptx::tmem_ld_wait();
+                    if (valid < BN) {
+                        mask(0);
+                        mask(32);
+                        mask(64);
+                        mask(96);
+                    }
+                    float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+                    for (int i = 0; i < BN; i += 8) {
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            mx4[u] = ptx::max3_nan(mx4[u], __uint_as_float(r[i + 2 * u]), __uint_as_float(r[i + 2 * u + 1]));
+                        }
+                    }
+                    const float mx = ptx::max3_nan(ptx::max3_nan(mx4[0], mx4[1], mx4[2]), mx4[3], mx4[3]);
+                    begun          = mx != -INFINITY;
+                    m_ref          = begun ? mx : 0.0f;
+                }
                 uint32_t pk[48];
                 float    s4[4] = {0.f, 0.f, 0.f, 0.f};
                 float    nmc = -m_ref * c;
@@ -647,7 +669,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 // A NaN among the scores reaches `part` or `last` and fails their test: the slow path and the last
                 // quarter behind it then run on the special-function unit, which keeps it (the FMA-pipe form's clamp
                 // would turn it into a number).
-                const bool fine = part < 0x1p32f && last < RANGE && (begun || part > 0x1p-32f);
+                const bool fine = part < RANGE_SUM && last < RANGE && begun;
                 const bool slow = __any_sync(0xffffffffu, !fine);
                 if (slow) {
                     // The maximum of the whole row; the first three quarters are still in tensor memory.
@@ -695,9 +717,6 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                         }
                         exp_chunk<0>(&r[ch * 32], c, nmc, s4, &pk[ch * 16]);
                     }
-                }
-                else {
-                    begun = true;
                 }
                 stamp<TRACE>(p, scount, t * 10 + 2);
                 // written over S, of which only the last quarter is still needed and in registers

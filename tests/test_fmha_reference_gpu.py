@@ -1,6 +1,6 @@
-"""The forward's exponentials are taken against a loose reference that moves only when a row's scores leave
-its range: scores that leave it in any quarter of a kv step, in the first step or later, upwards or (in
-the first step) downwards, by a little or by hundreds of powers of two, for some rows of a warp or all."""
+"""The forward's exponentials are taken against a loose reference, the first step's maximum, that moves only when a
+row's scores leave its range: scores that leave it in any quarter of a kv step, in the first step or later,
+by a little or by hundreds of powers of two, for some rows of a warp or all; scores that are NaN or infinite."""
 
 import pytest
 import torch
@@ -186,3 +186,33 @@ def test_steps_whose_scores_are_all_minus_infinity(b, h, sq, skv, ctas, first, l
     assert ((o[:, ::2].float() - o_ref).norm() / o_ref.norm()).item() < 1e-2  # P and o are rounded to bf16: 2^-9 each
     assert ((lse[..., ::2] - lse_ref).abs().max()).item() < 1e-3
     assert o[:, 1::2].isnan().all()  # 0 x -inf
+
+
+@pytest.mark.parametrize("b,h,sq,skv,ctas", FORMS + [(1, 2, 200, 1, 0), (1, 2, 200, 128, 0)])
+@pytest.mark.parametrize("where", [0, 1, 50, 127, 128, 200, -1])
+def test_a_weight_of_one_is_exact(b, h, sq, skv, ctas, where):
+    """One key outweighs all others by 2^28: the result is its value, bit for bit, because a reference taken from it
+    makes its weight 1 in bf16."""
+    torch.manual_seed(where + 1)
+    q, k = torch.zeros(b, sq, h, 128, device="cuda"), torch.zeros(b, skv, h, 128, device="cuda")
+    v = torch.randn(b, skv, h, 128, device="cuda").bfloat16()
+    where = min(where, skv - 1)
+    q[..., 0], k[:, where, :, 0] = 7.0, 31.375  # x log2(e) / sqrt(128): 28.006, whose power of two lies between two bf16 numbers
+    o, lse = attention.fmha_fwd(q.bfloat16(), k.bfloat16(), v, ctas=ctas)
+    gemm.check_errors()
+    assert torch.equal(o, v[:, where].unsqueeze(1).expand_as(o))
+
+
+@pytest.mark.parametrize("b,h,sq,skv,ctas", FORMS)
+@pytest.mark.parametrize("score", [1.0078125, 1.9765625, 3.9375])  # x 8 log2(e) / sqrt(128): their powers of two, too
+def test_equal_scores_average_the_values(b, h, sq, skv, ctas, score):
+    """Every weight is the same and rounds the same way: only a weight that bf16 holds leaves no error behind."""
+    torch.manual_seed(7)
+    q, k = torch.zeros(b, sq, h, 128, device="cuda"), torch.zeros(b, skv, h, 128, device="cuda")
+    v = (torch.randn(b, skv, h, 128, device="cuda") + 2.0).bfloat16()
+    q[..., 0], k[..., 0] = 8.0, score
+    o, _ = attention.fmha_fwd(q.bfloat16(), k.bfloat16(), v, ctas=ctas)
+    gemm.check_errors()
+    mean = v.double().mean(1, keepdim=True).expand_as(o)
+    # one rounding to bf16 (half a unit in the last of 8 bits) and fp32 sums of a thousand terms
+    assert torch.all((o.double() - mean).abs() <= mean.abs() * 2.0 ** -8 * 1.002 + 1e-5)
