@@ -238,6 +238,10 @@ Tensor gemm_entry(const Tensor& a, const Tensor& b, const MaybeTensor& bias, con
     const int64_t m = a.size(a_km ? 1 : 0), n = b.size(b_kn ? 1 : 0);
     expect(a.size(a_km ? 0 : 1) == b.size(b_kn ? 0 : 1), "gemm_bf16: ", a.sizes(), " and ", b.sizes(),
            " do not share a contraction (a_km=", a_km, ", b_kn=", b_kn, ")");
+    for (const MaybeTensor* t : {&bias, &residual, &out, &aux, &store_pre}) {
+        const Tensor given = or_none(*t);
+        expect_on_device_of(a, {&b, &given}, "gemm_bf16");
+    }
     GemmExtra x;
     x.act  = static_cast<int>(act);
     x.a_km = a_km;
@@ -585,9 +589,14 @@ void attention_operand(const Tensor& t)
 
 FuFmhaArgs attention_args(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o, std::optional<double> scale)
 {
+    expect_on_device_of(q, {&k, &v, &o}, "attention");
     for (const Tensor* t : {&q, &k, &v, &o}) {
         attention_operand(*t);
     }
+    expect(k.size(0) == q.size(0) && k.size(2) == q.size(2) && k.sizes() == v.sizes() && o.size(0) >= q.size(0)
+               && o.size(1) >= q.size(1) && o.size(2) >= q.size(2),
+           "attention: q ",
+           q.sizes(), ", k ", k.sizes(), ", v ", v.sizes(), ", result ", o.sizes());
     FuFmhaArgs a{};
     a.q        = q.data_ptr();
     a.k        = k.data_ptr();
@@ -640,11 +649,20 @@ std::tuple<Tensor, Tensor, Tensor> fmha_bwd(const Tensor& q, const Tensor& k, co
         d_o = d_o.contiguous();
         o   = o.contiguous();
     }
+    expect_on_device_of(q, {&d_o, &lse}, "fmha_bwd");
+    expect(d_o.sizes() == o.sizes() && d_o.scalar_type() == at::kBFloat16, "fmha_bwd: the gradient of a result of ", o.sizes(),
+           " is ", d_o.scalar_type(), " ", d_o.sizes());
+    expect(lse.scalar_type() == at::kFloat && lse.is_contiguous() && lse.numel() == b * h * sq, "fmha_bwd: lse is (b, h, sq) dense fp32, got ",
+           lse.scalar_type(), " ", lse.sizes());
     Tensor dq, dk, dv;
     if (out.has_value()) {
         expect(out->size() == 3, "fmha_bwd: out is (dq, dk, dv)");
         dq = (*out)[0], dk = (*out)[1], dv = (*out)[2];
+        expect_on_device_of(q, {&dq, &dk, &dv}, "fmha_bwd");
         expect(dq.is_contiguous() && dk.is_contiguous() && dv.is_contiguous(), "fmha_bwd: out tensors must be dense");
+        expect(dq.sizes() == q.sizes() && dk.sizes() == k.sizes() && dv.sizes() == v.sizes() && dq.scalar_type() == at::kBFloat16
+                   && dk.scalar_type() == at::kBFloat16 && dv.scalar_type() == at::kBFloat16,
+               "fmha_bwd: out is bf16 shaped like q, k, v, got ", dq.sizes(), ", ", dk.sizes(), ", ", dv.sizes());
     }
     else {
         dq = empty_bf16(q.sizes(), q);

@@ -98,3 +98,35 @@ def test_forward_mode_tangents_are_refused_and_not_dropped(mode):
             with pytest.raises(RuntimeError, match="jvp|forward AD"):
                 call(fw.make_dual(x, torch.randn_like(x)))
     g.destroy()
+
+
+def test_attention_refuses_operands_it_cannot_read():
+    q, k, v = bf16(2, 30, 3, 128), bf16(2, 50, 3, 128), bf16(2, 50, 3, 128)
+    o, lse = attention.fmha_fwd(q, k, v)
+    d_o = torch.randn_like(o)
+    attention.fmha_bwd(q, k, v, o, lse, d_o)
+    for args in ((q, k.cpu(), v), (q, k, v.cpu()), (q, k[:, :, :2], v[:, :, :2]), (q, k[:1], v[:1]), (q, k, v[:, :40])):
+        with pytest.raises(AssertionError):
+            attention.attention(*args)
+        with pytest.raises(AssertionError):
+            attention.fmha_bwd(*args, o, lse, d_o)
+    with pytest.raises(AssertionError):
+        attention.fmha_fwd(q, k, v, out=torch.empty(2, 29, 3, 128, device="cuda", dtype=torch.bfloat16))
+    for bad in ((o, lse.cpu(), d_o), (o, lse[:1], d_o), (o, lse.double(), d_o), (o, lse, d_o.cpu()), (o, lse, d_o[:, :20]),
+                (o[:, :20], lse, d_o[:, :20])):
+        with pytest.raises(AssertionError):
+            attention.fmha_bwd(q, k, v, *bad)
+    for bad in ((q, k, v[:, :40].contiguous()), (q, k.cpu(), v), (q.float(), k, v)):
+        with pytest.raises(AssertionError):
+            attention.fmha_bwd(q, k, v, o, lse, d_o, out=tuple(torch.empty_like(t) for t in bad))
+
+
+@pytest.mark.parametrize("name", ["bias", "residual", "out", "aux", "store_pre"])
+def test_gemm_refuses_an_operand_on_the_host(name):
+    a, b = bf16(M, K), bf16(N, K)
+    extra = {name: torch.zeros(N) if name == "bias" else torch.zeros(M, N).bfloat16()}
+    with pytest.raises(AssertionError):
+        gemm.gemm_bf16(a, b, **extra)
+    with pytest.raises(AssertionError):
+        gemm.gemm_bf16(a, b.cpu())
+    assert gemm.gemm_bf16(a, b, **{k: v.cuda() for k, v in extra.items()}).shape == (M, N)
