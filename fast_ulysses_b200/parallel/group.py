@@ -202,7 +202,8 @@ class UlyssesGroup:
 
         ``x`` may be overwritten or freed the moment this returns: by default the call first takes
         a private copy of ``x`` on the caller's stream (``stage=True``, the reference's contract,
-        src/group.cc:320-404 there). ``stage=False`` skips that copy and lets the kernel read ``x``
+        src/group.cc:320-404 there), or on one rank makes the caller's stream wait for the move
+        itself. ``stage=False`` does neither and lets the kernel read ``x``
         in place on the comm stream: freeing ``x`` is still safe (the caching allocator is told
         about the cross-stream use), but writing into ``x`` on the caller's stream before waiting
         on the result is then a race the library cannot see.
