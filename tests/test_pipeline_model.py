@@ -1,6 +1,6 @@
-"""The GEMM core's mbarrier pipeline as a model, checked over every interleaving of its roles.
+"""The GEMM cores' mbarrier pipelines as models, checked over every interleaving of their roles.
 
-`fu::gemm::run` (csrc/kernels/gemm_sm100.cuh) has three roles that never share a program counter:
+`fu::gemm::run` (csrc/kernels/gemm_sm100.cuh; the core of the pulling kernel) has three roles that never share a program counter:
 a TMA producer filling a ring of STAGES operand buffers, one MMA thread consuming them into one of
 two tensor-memory accumulators, and epilogue warps draining a finished accumulator while the next
 tile's main loop already runs. They meet only in mbarriers, and which PHASE PARITY each side waits
@@ -26,9 +26,11 @@ does not divide and an odd number of tiles, and checks in every reachable state 
   * nobody waits for ever.
 
 Negative controls: the same search with the producer's parity un-flipped, and with the accumulator
-barrier counting one warp too few, must each find a violation. The CTA-pair kernel (`run_pair`) has
-the same structure with the `tmem_empty` count doubled (both CTAs' epilogue warps arrive on the even
-CTA's barrier); `warps` below stands for that count.
+barrier counting one warp too few, must each find a violation. `run_small` has the same structure on
+128 x 128 tiles.
+
+`fu::gemm::run_wide` (pairs of CTAs, two accumulator blocks or one) orders its work differently and is searched
+by itself: see `explore_wide`.
 """
 
 import pytest
@@ -148,3 +150,148 @@ def test_a_producer_waiting_for_the_wrong_parity_is_found():
 def test_an_accumulator_barrier_that_counts_one_warp_too_few_is_found():
     found = explore(3, 2, 5, 2, empty_count=1)
     assert found is not None and ("before every epilogue warp" in found or "finds" in found or "deadlock" in found)
+
+
+# ---- pairs of CTAs --------------------------------------------------------------------------------------------
+def mma_program(items, stages, kblocks, release_early=False):
+    """What the issuing warp of `run_wide` does for the blocks (u0, u1) of each item, as in the kernel: the first
+    `stages` K-blocks of a tile go into block 0 and then into block 1, and so do the last ones; those
+    between, into both. `release_early` gives a stage back after the first block that has read it."""
+    ops, stage, phase, uses = [], 0, 0, [0, 0]
+
+    def advance(s, ph):
+        return (0, ph ^ 1) if s + 1 == stages else (s + 1, ph)
+
+    for item, (u0, u1) in enumerate(items):
+        if u0 == u1:
+            continue
+        kb = 0
+        while kb < kblocks:
+            left = kblocks - kb
+            if kb > 0 and left > stages and u1 - u0 == 2:
+                for _ in range(left - stages):
+                    ops += [("wait_full", stage, phase), ("mma", item, 0, kb, stage), ("mma", item, 1, kb, stage), ("empty", stage)]
+                    stage, phase = advance(stage, phase)
+                    kb += 1
+                continue
+            run = min(left, stages)
+            for u in range(u0, u1):
+                if kb == 0:
+                    ops.append(("wait_tempty", u, (uses[u] & 1) ^ 1))
+                    uses[u] += 1
+                s, ph = stage, phase
+                for i in range(run):
+                    if u == u0:
+                        ops.append(("wait_full", s, ph))
+                    ops.append(("mma", item, u, kb + i, s))
+                    if u + 1 == u1 or release_early:
+                        ops.append(("empty", s))
+                    s, ph = advance(s, ph)
+                if run == left:
+                    ops.append(("tfull", u))
+            stage, phase = s, ph
+            kb += run
+    return ops
+
+
+def explore_wide(items, stages=2, kblocks=3, warps=1, flip=1, empty_warps=None, release_early=False):
+    """Every interleaving of the two producers (a stage is full when both CTAs' loads have landed), the issuing warp
+    of the even CTA, whose commits reach both CTAs, and `warps` epilogue warps per CTA, which all arrive on the even
+    CTA's barrier when they have copied a block out. Returns what goes wrong, or None."""
+    loads = [(n, kb) for n, (u0, u1) in enumerate(items) if u0 != u1 for kb in range(kblocks)]
+    blocks = [(n, u) for n, (u0, u1) in enumerate(items) for u in range(u0, u1)]
+    ops = mma_program(items, stages, kblocks, release_early)
+    total = 2 * warps
+    empty_count = total if empty_warps is None else empty_warps
+    reads_of = [items[n][1] - items[n][0] for n in range(len(items))]
+    # producers' positions, MMA program counter, positions of the epilogue warps;
+    # full (one barrier, on the even CTA), empty (one per CTA), tmem_full, tmem_empty; what each CTA's half of a stage
+    # holds and how many blocks have read it; each accumulator's (item, K-blocks added) and who has still to drain it
+    init = ((0, 0), 0, (0,) * total, (Bar.new(2),) * stages, (Bar.new(1),) * stages, (Bar.new(1),) * 2, (Bar.new(empty_count),) * 2,
+            ((None, 0),) * (2 * stages), ((-1, 0),) * 2, (0,) * 2)
+    seen, stack = {init}, [init]
+
+    def put(t, at, value):
+        return t[:at] + (value,) + t[at + 1:]
+
+    while stack:
+        prod, pc, epi, full, empty, tfull, tempty, held, acc, todo = stack.pop()
+        nxt = []
+        for c in range(2):
+            if prod[c] < len(loads):
+                s, ph = prod[c] % stages, ((prod[c] // stages) & 1) ^ flip
+                if Bar.passes(empty[s], ph):  # the commit reaches both CTAs' barriers at once
+                    item, reads = held[2 * s + c]
+                    if item is not None and reads < reads_of[item[0]]:
+                        return f"CTA {c} refills stage {s} ({item}) after {reads} reads"
+                    nxt.append((put(prod, c, prod[c] + 1), pc, epi, put(full, s, Bar.arrive(full[s])), empty, tfull, tempty,
+                                put(held, 2 * s + c, (loads[prod[c]], 0)), acc, todo))
+        if pc < len(ops):
+            op = ops[pc]
+            state = None
+            if op[0] == "wait_full":
+                if Bar.passes(full[op[1]], op[2]):
+                    state = (prod, pc + 1, epi, full, empty, tfull, tempty, held, acc, todo)
+            elif op[0] == "wait_tempty":
+                if Bar.passes(tempty[op[1]], op[2]):
+                    if todo[op[1]]:
+                        return f"the MMA starts block {op[1]} before every epilogue warp has drained it"
+                    state = (prod, pc + 1, epi, full, empty, tfull, tempty, held, acc, todo)
+            elif op[0] == "mma":
+                _, item, u, kb, s = op
+                new = held
+                for c in range(2):
+                    if held[2 * s + c][0] != (item, kb):
+                        return f"the MMA of {(item, u, kb)} finds {held[2 * s + c][0]} in stage {s} of CTA {c}"
+                    new = put(new, 2 * s + c, ((item, kb), held[2 * s + c][1] + 1))
+                if kb != 0 and acc[u] != (item, kb):
+                    return f"the MMA of {(item, u, kb)} adds to {acc[u]}"
+                state = (prod, pc + 1, epi, full, empty, tfull, tempty, new, put(acc, u, (item, kb + 1)), todo)
+            elif op[0] == "empty":
+                state = (prod, pc + 1, epi, full, put(empty, op[1], Bar.arrive(empty[op[1]])), tfull, tempty, held, acc, todo)
+            else:
+                state = (prod, pc + 1, epi, full, empty, put(tfull, op[1], Bar.arrive(tfull[op[1]])), tempty, held, acc,
+                         put(todo, op[1], total))
+            if state is not None:
+                nxt.append(state)
+        for w in range(total):
+            if epi[w] < len(blocks):
+                item, u = blocks[epi[w]]
+                uses = sum(1 for b in blocks[:epi[w]] if b[1] == u)
+                if Bar.passes(tfull[u], uses & 1):
+                    if acc[u] != (item, kblocks):
+                        return f"epilogue warp {w} reads block {u} for item {item} and finds {acc[u]}"
+                    nxt.append((prod, pc, put(epi, w, epi[w] + 1), full, empty, tfull, put(tempty, u, Bar.arrive(tempty[u])), held, acc,
+                                put(todo, u, todo[u] - 1)))
+        if not nxt and (pc < len(ops) or min(prod) < len(loads) or min(epi) < len(blocks)):
+            return f"deadlock: producers at {prod}, MMA at {ops[pc:pc + 1]}, epilogue at {epi}"
+        for n in nxt:
+            if n not in seen:
+                seen.add(n)
+                stack.append(n)
+    return None
+
+
+WHOLE, FIRST, SECOND, OUTSIDE = (0, 2), (0, 1), (1, 2), (1, 1)
+
+
+# K shorter than the ring, as long, one more, twice, and with K-blocks in the middle of a tile; whole tiles, then
+# single blocks of them, some outside the result
+@pytest.mark.parametrize("stages,kblocks", [(2, 1), (2, 2), (2, 3), (2, 4), (2, 6), (3, 2), (3, 5), (3, 7)])
+@pytest.mark.parametrize("items", [(WHOLE, WHOLE, WHOLE), (WHOLE, FIRST, SECOND), (FIRST, WHOLE), (WHOLE, SECOND, OUTSIDE, FIRST),
+                                   (SECOND, FIRST, SECOND)])
+def test_two_blocks_of_a_pair_hold_in_every_interleaving(stages, kblocks, items):
+    assert explore_wide(items, stages, kblocks) is None
+
+
+# one block per pair: its accumulators alternate between the halves of tensor memory
+@pytest.mark.parametrize("stages,kblocks", [(2, 1), (2, 3), (3, 2), (3, 4)])
+def test_alternating_blocks_of_a_pair_hold_in_every_interleaving(stages, kblocks):
+    assert explore_wide((FIRST, SECOND, FIRST, SECOND, FIRST), stages, kblocks) is None
+
+
+@pytest.mark.parametrize("fault,text", [(dict(flip=0), ("deadlock", "refills")), (dict(empty_warps=1), ("before every", "finds", "adds", "deadlock")),
+                                        (dict(release_early=True), ("refills", "finds", "deadlock"))])
+def test_faults_of_the_pair_schedule_are_found(fault, text):
+    found = explore_wide((WHOLE, WHOLE, WHOLE), 2, 3, **fault)
+    assert found is not None and any(t in found for t in text), found
