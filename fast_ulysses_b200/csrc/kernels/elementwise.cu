@@ -666,7 +666,7 @@ extern "C" int fu_layernorm_bwd_add(const void* dy, const void* x, const float* 
     if (!dy || !x || !stats || !dx || rows <= 0 || cols <= 0 || (cols % 8) || (ld % 8)
         || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(dy) | reinterpret_cast<uintptr_t>(dx)
              | reinterpret_cast<uintptr_t>(add)) & 15u)) {
-        return fu::fail(FU_E_ARG, "fu_layernorm_bwd: needs 16-byte aligned rows of a multiple of 8 columns");
+        return fu::fail(FU_E_ARG, "fu_layernorm_bwd_add: needs 16-byte aligned rows of a multiple of 8 columns");
     }
     const unsigned blocks = static_cast<unsigned>((rows + 7) / 8);
     layernorm_bwd_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
@@ -674,12 +674,6 @@ extern "C" int fu_layernorm_bwd_add(const void* dy, const void* x, const float* 
         static_cast<const __nv_bfloat16*>(add), static_cast<__nv_bfloat16*>(dx), rows, cols, ld);
     FU_CUDA_OK(cudaGetLastError());
     return FU_OK;
-}
-
-extern "C" int fu_layernorm_bwd(const void* dy, const void* x, const float* stats, void* dx, int64_t rows, int64_t cols,
-                                int64_t ld, void* stream)
-{
-    return fu_layernorm_bwd_add(dy, x, stats, nullptr, dx, rows, cols, ld, stream);
 }
 
 extern "C" int fu_colsum_bf16(const void* x, void* out, int64_t rows, int64_t cols, int64_t ld, void* stream)

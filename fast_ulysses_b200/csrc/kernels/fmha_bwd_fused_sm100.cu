@@ -630,8 +630,8 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_bwd_fused_kernel(const __grid
 }
 
 // Items beyond whole waves of one per SM are shared out, see cluster_plan.h. Times in query blocks (2.1 us).
-// 8191 tokens x 10 heads (640 items on 148 SMs): 860 -> 777 us, 4000 x 5 (160 items): 163 -> 113, 1000 x 5
-// (40 items): 30.0 -> 22.5.
+// 8191 tokens x 10 heads (640 items on 148 SMs): 844 -> 777 us, 4000 x 5 (160 items): 166 -> 113, 1000 x 5
+// (40 items): 31.7 -> 22.5.
 fu::ClusterPlan plan_split(int items, int n_q, int sms, int dev)
 {
     static fu::ClusterCapacity capacity;

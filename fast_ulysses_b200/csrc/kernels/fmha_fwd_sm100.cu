@@ -855,7 +855,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
 }
 
 // Items beyond whole waves of one per SM are shared out, see cluster_plan.h. Times in kv tiles (1.45 us).
-// 8191 tokens x 10 heads (320 items on 148 SMs): 304 -> 249 us; 1000 x 10 (40 items): 17.4 -> 15.9.
+// 8191 tokens x 10 heads (320 items on 148 SMs): 304 -> 249 us; 4000 x 10 (160 items): 104 -> 75.
 fu::ClusterPlan plan_split(int items, int n_kv, int sms, int dev)
 {
     static fu::ClusterCapacity capacity;

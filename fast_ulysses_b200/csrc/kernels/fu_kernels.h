@@ -140,8 +140,8 @@ FU_API int fu_barrier(FuCtrl* const* peer_ctrl, int rank, int world, uint32_t ti
 enum {
     FU_GEMM_A_KM = 1,
     FU_GEMM_B_KN = 2,
-    FU_GEMM_PAIR = 4,    // run on CTA pairs (256 x 256 tiles, tcgen05 cta_group::2) whatever the default is
-    FU_GEMM_SINGLE = 8,  // run on single CTAs (128 x 256 tiles) whatever the default is
+    FU_GEMM_PAIR = 4,    // run on CTA pairs (two 256 x 256 blocks each, tcgen05 cta_group::2) whatever the size
+    FU_GEMM_SINGLE = 8,  // run on single CTAs (128 x 128 tiles) whatever the size
     FU_GEMM_BIAS_BF16 = 16,  // `bias` points to bf16 values
 };
 typedef struct FuGemmArgs {
@@ -351,8 +351,6 @@ FU_API int fu_layernorm_fwd(const void* x, void* y, float* stats, int64_t rows, 
 // dx = rstd * (dy - mean(dy) - xhat * mean(dy * xhat)), xhat recomputed from x and the saved statistics.
 // `add` (nullable, laid out like dx) is added before the one rounding to bf16: the gradient that reached x
 // past the norm, through a residual connection.
-FU_API int fu_layernorm_bwd(const void* dy, const void* x, const float* stats, void* dx, int64_t rows, int64_t cols,
-                            int64_t ld, void* stream);
 FU_API int fu_layernorm_bwd_add(const void* dy, const void* x, const float* stats, const void* add, void* dx, int64_t rows,
                                 int64_t cols, int64_t ld, void* stream);
 // out[c] = bf16(sum over rows of x[r, c]), x bf16 with leading dimension ld, summed in fp32 in a fixed order.

@@ -65,9 +65,6 @@ def lib() -> C.CDLL:
         _lib.fu_layernorm_fwd.restype = C.c_int
         _lib.fu_layernorm_fwd.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64, C.c_int64,
                                           C.c_float, C.c_void_p]
-        _lib.fu_layernorm_bwd.restype = C.c_int
-        _lib.fu_layernorm_bwd.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int64, C.c_int64, C.c_int64,
-                                          C.c_void_p]
         _lib.fu_pull_qkv_grads.restype = C.c_int
         _lib.fu_pull_qkv_grads.argtypes = [C.c_void_p, C.c_void_p]
         _lib.fu_a2a4d_fp8.restype = C.c_int

@@ -1,5 +1,5 @@
 """LayerNorm without affine parameters as one kernel forward and one backward
-(csrc/kernels/elementwise.cu: fu_layernorm_fwd / fu_layernorm_bwd; autograd in csrc/ops/fused.cc): bf16
+(csrc/kernels/elementwise.cu: fu_layernorm_fwd / fu_layernorm_bwd_add; autograd in csrc/ops/fused.cc): bf16
 in and out, statistics in fp32. The DiT blocks normalise with it so that no eager elementwise kernel
 runs between the GEMMs."""
 
