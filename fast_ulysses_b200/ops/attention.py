@@ -59,7 +59,7 @@ def fmha_bwd(q, k, v, o, lse, d_o, *, scale: float | None = None, ctas: int = 0,
     strides. Returns ``(dq, dk, dv)`` shaped and strided like q, k, v (dense). The default is one
     software-pipelined pass that sums dQ over the K/V blocks with fp32 reductions (dK and dV are
     bit-reproducible, dQ to rounding); ``deterministic=True`` runs two passes without atomics
-    (dK/dV with the K/V block stationary, then dQ with the query rows stationary) at about 1.5x
+    (dK/dV with the K/V block stationary, then dQ with the query rows stationary) at about 2.4x
     the time."""
     return _C.fmha_bwd(q, k, v, o, lse, d_o, scale, ctas, None if out is None else list(out), deterministic, trace)
 
