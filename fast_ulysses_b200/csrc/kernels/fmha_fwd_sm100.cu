@@ -122,9 +122,10 @@ __device__ constexpr bool on_fma_pipe(int i)
 }
 
 // 32 columns of one row: P = exp2(S * c - m * c) as packed bf16, row sum into l4. NP of every 16
-// pairs take the FMA-pipe path, the rest the special-function unit.
-template <int NP>
-__device__ __forceinline__ void exp_chunk(const uint32_t* r, float c, float nmc, float (&l4)[4], uint32_t* pk)
+// pairs take the FMA-pipe path, the rest the special-function unit. RAGGED: columns from `valid` on do not
+// exist and weigh nothing, whatever the scale makes of their -inf.
+template <int NP, bool RAGGED = false>
+__device__ __forceinline__ void exp_chunk(const uint32_t* r, float c, float nmc, float (&l4)[4], uint32_t* pk, int valid = 32)
 {
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
@@ -136,6 +137,10 @@ __device__ __forceinline__ void exp_chunk(const uint32_t* r, float c, float nmc,
         else {
             e0 = ptx::ex2(x0);
             e1 = ptx::ex2(x1);
+        }
+        if (RAGGED) {
+            e0 = 2 * i < valid ? e0 : 0.0f;
+            e1 = 2 * i + 1 < valid ? e1 : 0.0f;
         }
         ptx::add2(l4[(2 * i) & 3], l4[(2 * i + 1) & 3], l4[(2 * i) & 3], l4[(2 * i + 1) & 3], e0, e1);
         pk[i] = ptx::pack_bf16x2(e0, e1);
@@ -600,9 +605,8 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                     ptx::tmem_ld_32x32(ts + ch * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[ch * 32]));
                 }
                 stamp<TRACE>(p, scount, t * 10 + 1);
-                // The last block of a ragged sequence holds columns that do not exist: they become -inf
-                // (exp2 gives exactly 0) and take the special-function unit only (the FMA-pipe form
-                // clamps instead of returning 0).
+                // The last block of a ragged sequence holds columns that do not exist: they become -inf, which
+                // no maximum sees, and exp_chunk gives them no weight.
                 auto mask = [&](int from) {
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
@@ -643,13 +647,13 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                 }
                 else {
                     mask(0);
-                    exp_chunk<0>(&r[0], c, nmc, s4, &pk[0]);
+                    exp_chunk<0, true>(&r[0], c, nmc, s4, &pk[0], valid);
                     ptx::tmem_ld_wait();
                     mask(32);
                     mask(64);
                     mask(96);
-                    exp_chunk<0>(&r[32], c, nmc, s4, &pk[16]);
-                    exp_chunk<0>(&r[64], c, nmc, s4, &pk[32]);
+                    exp_chunk<0, true>(&r[32], c, nmc, s4, &pk[16], valid - 32);
+                    exp_chunk<0, true>(&r[64], c, nmc, s4, &pk[32], valid - 64);
                 }
                 float mx2[2] = {-INFINITY, -INFINITY};
 #pragma unroll
@@ -715,7 +719,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                         if (valid < BN) {
                             mask(ch * 32);
                         }
-                        exp_chunk<0>(&r[ch * 32], c, nmc, s4, &pk[ch * 16]);
+                        exp_chunk<0, true>(&r[ch * 32], c, nmc, s4, &pk[ch * 16], valid - ch * 32);
                     }
                 }
                 stamp<TRACE>(p, scount, t * 10 + 2);
@@ -737,7 +741,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
                     exp_chunk<NP>(&r[96], c, nmc, l4, pk);
                 }
                 else {
-                    exp_chunk<0>(&r[96], c, nmc, l4, pk);
+                    exp_chunk<0, true>(&r[96], c, nmc, l4, pk, valid - 96);
                 }
                 ptx::tmem_st_32x16(ts + 48, *reinterpret_cast<uint32_t(*)[16]>(&pk[0]));
                 stamp<TRACE>(p, scount, t * 10 + 5);

@@ -216,3 +216,32 @@ def test_equal_scores_average_the_values(b, h, sq, skv, ctas, score):
     mean = v.double().mean(1, keepdim=True).expand_as(o)
     # one rounding to bf16 (half a unit in the last of 8 bits) and fp32 sums of a thousand terms
     assert torch.all((o.double() - mean).abs() <= mean.abs() * 2.0 ** -8 * 1.002 + 1e-5)
+
+
+@pytest.mark.parametrize("b,h,sq,skv,ctas", FORMS)
+@pytest.mark.parametrize("scale", [-0.1, 0.0, 0.7])
+def test_any_scale(b, h, sq, skv, ctas, scale):
+    """The reference is a maximum of scores before they are scaled: with a negative scale, the smallest exponent."""
+    torch.manual_seed(8)
+    q, k, v = (torch.randn(b, s, h, 128, device="cuda").bfloat16() for s in (sq, skv, skv))
+    o, lse = attention.fmha_fwd(q, k, v, scale=scale, ctas=ctas)
+    gemm.check_errors()
+    o_ref, lse_ref = attention.attention_reference(q, k, v, scale=scale)
+    assert ((o.float() - o_ref).norm() / o_ref.norm()).item() < 1e-2  # P and o are rounded to bf16: 2^-9 each
+    assert ((lse - lse_ref).abs().max()).item() < 1e-3
+
+
+@pytest.mark.parametrize("deterministic", [False, True])
+@pytest.mark.parametrize("scale", [-0.1, 0.0])
+def test_gradients_at_any_scale(scale, deterministic):
+    torch.manual_seed(9)
+    q, k, v = (torch.randn(1, s, 2, 128, device="cuda").bfloat16() for s in (200, 300, 300))
+    o, lse = attention.fmha_fwd(q, k, v, scale=scale)
+    d_o = torch.randn_like(o)
+    grads = attention.fmha_bwd(q, k, v, o, lse, d_o, scale=scale, deterministic=deterministic)
+    gemm.check_errors()
+    ref = [t.float().requires_grad_() for t in (q, k, v)]
+    attention.attention_reference(*ref, scale=scale)[0].backward(d_o.float())
+    for got, want in zip(grads, ref):
+        # P, dS and the gradient are rounded to bf16: 2^-9 each
+        assert ((got.float() - want.grad).norm() / want.grad.norm().clamp_min(1e-6)).item() < 1e-2
