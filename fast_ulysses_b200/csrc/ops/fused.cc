@@ -742,7 +742,11 @@ struct SpAttention : public torch::CustomClassHolder {
     int64_t              forwards    = 0;  // q, k, v and o belong to the latest forward
     // A norm weight as the kernels read it: dense fp32 that starts on 16 bytes (a slice of a flat parameter buffer may
     // start anywhere). Made anew for each call: a write through `.data` leaves no trace that a kept copy could be judged by.
-    static Tensor f32(const Tensor& param) { return aligned(param.detach().to(at::kFloat).contiguous()); }
+    static Tensor f32(const Tensor& param)
+    {
+        const Tensor p = param.detach();
+        return aligned(p.scalar_type() == at::kFloat && p.is_contiguous() ? p : p.to(at::kFloat).contiguous());
+    }
 
     // How many CTAs a fused GEMM kernel of this block may take right now (0 = the whole device).
     //
