@@ -162,12 +162,14 @@ struct PlainEpi {
         for (int j = 0; j < 64; ++j) {
             v[j] = __uint_as_float(r[j]);
         }
-        piece<64>(v, row0, col0, end, lane, stage);
+#pragma unroll 1
+        for (int h = 0; h < 2; ++h) {
+            piece<64>(v, row0, col0 + h * 64, end, lane, stage);
 #pragma unroll
-        for (int j = 0; j < 64; ++j) {
-            v[j] = __uint_as_float(r[64 + j]);
+            for (int j = 0; j < 64; ++j) {
+                v[j] = __uint_as_float(r[64 + j]);
+            }
         }
-        piece<64>(v, row0, col0 + 64, end, lane, stage);
     }
 };
 
