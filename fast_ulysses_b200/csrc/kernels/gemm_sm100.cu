@@ -690,13 +690,18 @@ int pair_capacity()
 // estimate is a start-and-end time plus, per wave of CTAs, a time per 64-wide K-block, both measured
 // (us, SM clock 1.9 GHz, problems of 64 - 4100 rows and 256 - 13824 columns and K):
 //   128 x 128 tiles on single CTAs   3.2 + 0.225 per K-block and wave of 148
-//   two 256 x 256 blocks on pairs    6 + 0.61 per K-block and wave of 74, 0.32 for a wave of single blocks
-//   one 256 x 256 block on pairs     6 + 0.30
+//   two 256 x 256 blocks on pairs    6 + 0.60 per K-block and wave of 74, 0.33 for a wave of single blocks
+//   one 256 x 256 block on pairs     6 + 0.31
 // Rows of an operand that do not all start on a 32-byte sector (a pitch that is an odd multiple of 16 bytes)
 // reach shared memory more slowly: the K-blocks of a 128 x 128 tile take 0.265 us with one such operand and 0.385
-// with two, those of a single block on a pair 0.34 and 0.37, of two blocks 0.65 and 0.69 (256 x 3328 x 4096 with
+// with two, those of a single block on a pair 0.36 and 0.46, of two blocks 0.66 and 0.77 (256 x 3328 x 4096 with
 // small tiles: 18.1, 21.3 and 28.6 us). The pair kernels' time per K-block shrinks with the width of the block, see block_clocks(). At most half as
 // many tiles of two blocks as pairs left over are split into blocks.
+// The epilogue (Epilogue, below) comes on top. With one block the accumulators alternate and a wave takes the longer of
+// the products and the epilogue with what it delays; with two, the second block waits in tensor memory until the first
+// has been written, and the next tile with it. Measured (us), two blocks and one: 9450 x 5120 x 5120 with GELU 384 and
+// 344, with the derivative 415 and 329, with a residual 367 and 318, with nothing 311 and 318; 75600 x 15360 x 5120 with
+// the QKV epilogue 8514 and 7433; 16000 x 1280 x 640 with the derivative 70 and 52.
 // What the widths and the single block gave, against two blocks of 256 columns or the small tiles: 1000 x 5120 x
 // 5120 53.0 -> 41.8 us (two of 160), 512 x 5120 x 13824 81.6 -> 61.6 and 512 x 5120 x 5120 30.4 -> 25.8 (one of
 // 160), 4100 x 1536 x 4096 58.9 -> 47.2 (two of 192).
@@ -720,7 +725,25 @@ double block_clocks(int mb, int nb, int width)
 }
 
 // us per K-block, by how many of the two operands lie off the 32-byte sectors
-constexpr double kSmallBlock[3] = {0.225, 0.265, 0.385}, kOneBlock[3] = {0.30, 0.34, 0.37}, kTwoBlocks[3] = {0.61, 0.65, 0.69};
+constexpr double kSmallBlock[3] = {0.225, 0.265, 0.385}, kOneBlock[3] = {0.31, 0.36, 0.46}, kTwoBlocks[3] = {0.60, 0.66, 0.77};
+
+// us that the epilogue of a block of 256 columns takes, fitted to 320 - 1024 deep products of 2640 - 16000 rows. That of
+// nothing but a result is part of the start-and-end times.
+struct Epilogue {
+    double us;
+    static constexpr double kPlain = 2.8;
+    double beyond() const { return us - kPlain; }
+    // A narrow block's: pieces of 64 columns that are not whole, or do not lie on whole lines of 128 bytes.
+    double block(int width) const { return width == 256 ? us : width == 128 ? 0.8 * us : width > 128 ? 1.6 * us : us; }
+    double two_blocks(int width) const { return std::max(0.0, 2.0 * block(width) - 3.0); }
+    double small() const { return 0.62 * us; }
+};
+Epilogue epilogue_of(int act, bool pre, bool residual)
+{
+    const double acts[4] = {Epilogue::kPlain, 5.6, 7.0, 7.4};
+    return {acts[act] + (pre ? 0.9 : 0.0) + (residual ? 2.8 : 0.0)};
+}
+constexpr Epilogue kQkvEpilogue{8.0};
 
 int off_sectors(const void* a, int64_t lda, const void* b, int64_t ldb)
 {
@@ -728,49 +751,50 @@ int off_sectors(const void* a, int64_t lda, const void* b, int64_t ldb)
     return (off(a, lda) ? 1 : 0) + (off(b, ldb) ? 1 : 0);
 }
 
-Choice wide_choice(int64_t m, int64_t n, double kb, Shape shape, int width, int pairs, int off)
+Choice wide_choice(int64_t m, int64_t n, double kb, Shape shape, int width, int pairs, int off, Epilogue epi)
 {
     const int     mb = shape == Shape::kTall ? 2 : 1, nb = shape == Shape::kBroad ? 2 : 1;
     const int64_t tm = (m + 256 * mb - 1) / (256 * mb), tn = (n + width * nb - 1) / (width * nb), tiles = tm * tn;
     if (shape == Shape::kOne) {
+        const double products = kb * kOneBlock[off] / 512 * block_clocks(1, 1, width), waves = static_cast<double>((tiles + pairs - 1) / pairs);
         return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(tiles), static_cast<int>(tiles),
-                6.0 + kb * kOneBlock[off] / 512 * block_clocks(1, 1, width) * ((tiles + pairs - 1) / pairs), width};
+                6.0 + products + (waves - 1.0) * std::max(products, epi.block(width) + 0.45 * products) + epi.beyond(), width};
     }
     const int64_t left = tiles % pairs, full = 2 * left <= pairs ? tiles - left : tiles, items = full + 2 * (tiles - full);
+    const double  whole = static_cast<double>((full + pairs - 1) / pairs), halves = static_cast<double>((items - full + pairs - 1) / pairs);
     return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(full), static_cast<int>(items),
-            6.0 + kb * (kTwoBlocks[off] / 1024 * block_clocks(mb, nb, width) * ((full + pairs - 1) / pairs)
-                        + 1.05 * kOneBlock[off] / 512 * block_clocks(1, 1, width) * ((items - full + pairs - 1) / pairs)), width};
+            6.0 + kb * (kTwoBlocks[off] / 1024 * block_clocks(mb, nb, width) * whole + 1.05 * kOneBlock[off] / 512 * block_clocks(1, 1, width) * halves)
+                + epi.two_blocks(width) * whole + 0.5 * epi.block(width) * halves - Epilogue{Epilogue::kPlain}.two_blocks(256), width};
 }
 
 // `narrow`: the epilogue takes blocks of any width (the heads of the QKV projection need 128 columns at once).
-Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int flags, bool narrow, int off)
+Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int flags, bool narrow, int off, Epilogue epi)
 {
     const int64_t t128 = ((m + 127) / 128) * ((n + 127) / 128);
     const double  kb   = static_cast<double>((k + BK - 1) / BK);
-    const Choice  small{Shape::kSmall, static_cast<int>((m + 127) / 128), static_cast<int>((n + 127) / 128), 0,
-                       static_cast<int>(t128), 3.2 + kSmallBlock[off] * kb * ((t128 + sms - 1) / sms)};
+    const double  products = kSmallBlock[off] * kb, waves = static_cast<double>((t128 + sms - 1) / sms);
+    const Choice  small{Shape::kSmall, static_cast<int>((m + 127) / 128), static_cast<int>((n + 127) / 128), 0, static_cast<int>(t128),
+                       3.2 + products + (waves - 1.0) * std::max(products, epi.small() + 0.5 * products) + 0.62 * epi.beyond()};
     if (flags & FU_GEMM_SINGLE) {
         return small;
     }
-    const Choice tall = wide_choice(m, n, kb, Shape::kTall, 256, pairs, off), broad = wide_choice(m, n, kb, Shape::kBroad, 256, pairs, off);
+    const Choice tall = wide_choice(m, n, kb, Shape::kTall, 256, pairs, off, epi), broad = wide_choice(m, n, kb, Shape::kBroad, 256, pairs, off, epi);
     Choice       wide = tall.cost < broad.cost ? tall : broad;
     if (flags & FU_GEMM_PAIR) {
         return wide;
     }
-    if (narrow) {
-        Choice best = wide;
-        for (int width = 256; width >= 96; width -= 32) {
-            if ((flags & FU_GEMM_B_KN) && width % 128 != 0) {
-                continue;  // such a B comes in blocks of 64 columns, half of them for each CTA
-            }
-            for (const Shape shape : {Shape::kTall, Shape::kBroad, Shape::kOne}) {
-                const Choice c = wide_choice(m, n, kb, shape, width, pairs, off);
-                best           = c.cost < best.cost ? c : best;
-            }
+    Choice best = wide_choice(m, n, kb, Shape::kOne, 256, pairs, off, epi);
+    for (int width = narrow ? 224 : 0; width >= 96; width -= 32) {
+        if ((flags & FU_GEMM_B_KN) && width % 128 != 0) {
+            continue;  // such a B comes in blocks of 64 columns, half of them for each CTA
         }
-        if (best.cost < 0.96 * wide.cost) {  // whole blocks where it makes little difference: they take less power
-            wide = best;
+        for (const Shape shape : {Shape::kTall, Shape::kBroad, Shape::kOne}) {
+            const Choice c = wide_choice(m, n, kb, shape, width, pairs, off, epi);
+            best           = c.cost < best.cost ? c : best;
         }
+    }
+    if (best.cost < 0.96 * wide.cost) {  // two whole blocks where it makes little difference: they take less power
+        wide = best;
     }
     return small.cost < wide.cost ? small : wide;
 }
@@ -779,12 +803,12 @@ Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int fla
 // estimated to be faster than `best`. Measured (us): a wave of clusters takes 8.1 (two pairs) or 9.4 (four) and
 // 0.29 per K-block of a pair's share; behind another launch 1.5 of that are hidden. 2000 x 5120 x 5120 (80 tiles
 // on 74 pairs): 83.5 -> 79.5, 1000 x 5120 x 13824 (40 tiles: a wave of blocks and six more): 130 -> 115.
-Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, int pairs, int off)
+Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, int pairs, int off, Epilogue epi)
 {
     static fu::ClusterCapacity capacity;
     const int64_t              kb = (k + BK - 1) / BK;
     Choice                     chosen = best;
-    const Choice               broad  = wide_choice(m, n, static_cast<double>(kb), Shape::kBroad, 256, pairs, off);
+    const Choice               broad  = wide_choice(m, n, static_cast<double>(kb), Shape::kBroad, 256, pairs, off, epi);
     const int64_t              tiles = static_cast<int64_t>(broad.tiles_m) * broad.tiles_n, full = tiles / pairs * pairs;
     const int64_t              blocks = 2 * (tiles - full), single = blocks / pairs * pairs, rest = blocks - single;
     int                        dev = 0;
@@ -793,10 +817,12 @@ Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, in
     }
     double       limit = 0.96 * best.cost;
     const double before =
-        full + single > 0 ? 6.0 - 1.5 + kb * (kTwoBlocks[off] * (full / pairs) + 1.05 * kOneBlock[off] * (single / pairs)) : 0.0;
+        full + single > 0 ? 6.0 - 1.5 + kb * (kTwoBlocks[off] * (full / pairs) + 1.05 * kOneBlock[off] * (single / pairs))
+                                + epi.two_blocks(256) * (full / pairs) + 0.5 * epi.us * (single / pairs) - Epilogue{Epilogue::kPlain}.two_blocks(256)
+                          : 0.0;
     for (const int csize : {4, 8}) {
         const int64_t parts = csize / 2, share = (kb + parts - 1) / parts;
-        const double  wave  = (csize == 4 ? 8.1 : 9.4) + 0.97 * kOneBlock[off] * share;
+        const double  wave  = (csize == 4 ? 8.1 : 9.4) + 0.97 * kOneBlock[off] * share + 0.5 * epi.beyond();
         if ((kb + share - 1) / share != parts || before + wave >= limit) {
             continue;  // a pair would have nothing to do, or no gain beyond the estimate's error even in one wave
         }
@@ -822,7 +848,7 @@ Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, in
 // to be faster than `best`. The exchange takes 1.8, 2.4 and 2.8 us beyond the tile's own time (measured, for
 // two, four and eight CTAs). 64 x 2000 x 8000: 30.6 -> 13.3 us with four, 64 x 512 x 2048: 10.6 -> 7.0 with eight,
 // 512 x 1536 x 4096: 18.0 -> 13.2 with two; the 160 tiles of 512 x 5120 x 5120 stay as they are.
-int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k, int off)
+int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k, int off, Epilogue epi)
 {
     static fu::ClusterCapacity capacity;
     const int64_t              t128 = ((m + 127) / 128) * ((n + 127) / 128), kb = (k + BK - 1) / BK;
@@ -833,7 +859,7 @@ int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k, int off)
     }
     for (const int csize : {2, 4, 8}) {
         const int64_t share = (kb + csize - 1) / csize;
-        const double  once  = 3.2 + (csize == 2 ? 1.8 : csize == 4 ? 2.4 : 2.8) + kSmallBlock[off] * share;
+        const double  once  = 3.2 + (csize == 2 ? 1.8 : csize == 4 ? 2.4 : 2.8) + kSmallBlock[off] * share + 0.62 * epi.beyond() / csize;
         if ((kb + share - 1) / share != csize || once >= cost) {
             continue;  // a CTA would have nothing to do, or no gain even in one wave
         }
@@ -969,13 +995,14 @@ int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream
 {
     PlainArgs<ACT> a{};
     const int      off = off_sectors(g->a, g->lda, g->b, g->ldb);
+    const Epilogue epi = epilogue_of(g->act, g->c_pre != nullptr, g->residual != nullptr);
     int            csize = 1;
     if (g->ctas <= 0 && !(flags & (FU_GEMM_SINGLE | FU_GEMM_PAIR))) {
-        c     = choose_wide_split(c, g->m, g->n, g->k, pairs, off);
-        csize = choose_split(c, g->m, g->n, g->k, off);
+        c     = choose_wide_split(c, g->m, g->n, g->k, pairs, off, epi);
+        csize = choose_split(c, g->m, g->n, g->k, off, epi);
     }
     if (csize > 1) {
-        c = choose_shape(g->m, g->n, g->k, pairs, 1, FU_GEMM_SINGLE, false, off);
+        c = choose_shape(g->m, g->n, g->k, pairs, 1, FU_GEMM_SINGLE, false, off, epi);
     }
     const int      rc = fill_wide(a.core, c, g->a, g->b, g->m, g->n, g->k, g->lda, g->ldb, g->err, flags);
     if (rc != FU_OK) {
@@ -1042,7 +1069,8 @@ extern "C" int fu_gemm_bf16(const FuGemmArgs* g, void* stream_v)
     const bool   forced = pair_default && !(g->flags & FU_GEMM_SINGLE);
     const int    flags  = forced ? (g->flags | FU_GEMM_PAIR) : g->flags;
     const int    sms    = g->ctas > 0 ? std::min(g->ctas, device_sms()) : device_sms();
-    const Choice c      = choose_shape(g->m, g->n, g->k, pairs, sms, flags, true, off_sectors(g->a, g->lda, g->b, g->ldb));
+    const Choice c      = choose_shape(g->m, g->n, g->k, pairs, sms, flags, true, off_sectors(g->a, g->lda, g->b, g->ldb),
+                                      epilogue_of(g->act, g->c_pre != nullptr, g->residual != nullptr));
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     switch (g->act) {
     case 0: return launch_plain<0>(g, c, pairs, flags, stream);
@@ -1125,7 +1153,7 @@ extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream_v)
     }
     const int    sms   = q->ctas > 0 ? std::min(q->ctas, device_sms()) : device_sms();
     const int    flags = (q->flags & FU_QKV_W_KN) ? FU_GEMM_B_KN : 0;
-    const Choice c     = choose_shape(q->m, n, q->k, pairs, sms, flags, false, off_sectors(q->x, q->ldx, q->w, q->ldw));
+    const Choice c     = choose_shape(q->m, n, q->k, pairs, sms, flags, false, off_sectors(q->x, q->ldx, q->w, q->ldw), kQkvEpilogue);
     rc = fill_wide(a.core, c, q->x, q->w, q->m, n, q->k, q->ldx, q->ldw, q->err, flags);
     if (rc != FU_OK) {
         return rc;
@@ -1183,6 +1211,7 @@ extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream_v)
     switch (c.shape) {
     case Shape::kTall: return launch_pairs(qkv_wide_kernel<2, 1>, a, pairs, stream);
     case Shape::kBroad: return launch_pairs(qkv_wide_kernel<1, 2>, a, pairs, stream);
+    case Shape::kOne: return launch_pairs(qkv_wide_kernel<1, 1>, a, pairs, stream);
     default: return launch_small(qkv_small_kernel, a, q->ctas, stream);
     }
 }

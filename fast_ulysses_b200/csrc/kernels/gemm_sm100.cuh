@@ -916,6 +916,16 @@ __device__ __forceinline__ void stage_in(uint32_t stage, const __nv_bfloat16* sr
             v[i] = *reinterpret_cast<const uint4*>(p + i * ROWS * ld);
         }
     }
+    else if ((N - col0) % 8 == 0) {  // uniform: whole units or none
+        const __nv_bfloat16* p = src + static_cast<int64_t>(row0 + first) * ld + col;
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            v[i] = make_uint4(0u, 0u, 0u, 0u);
+            if (row0 + i * ROWS + first < M && col < N) {
+                v[i] = *reinterpret_cast<const uint4*>(p + i * ROWS * ld);
+            }
+        }
+    }
     else {
 #pragma unroll
         for (int i = 0; i < U; ++i) {
@@ -963,6 +973,16 @@ __device__ __forceinline__ void stage_out(uint32_t stage, __nv_bfloat16* dst, in
 #pragma unroll
         for (int i = 0; i < U; ++i) {
             ptx::st_v4(p + i * ROWS * ld, v[i]);
+        }
+        return;
+    }
+    if ((N - col0) % 8 == 0) {  // uniform: whole units or none
+        __nv_bfloat16* p = dst + static_cast<int64_t>(row0 + first) * ld + col;
+#pragma unroll
+        for (int i = 0; i < U; ++i) {
+            if (row0 + i * ROWS + first < M && col < N) {
+                ptx::st_v4(p + i * ROWS * ld, v[i]);
+            }
         }
         return;
     }
