@@ -738,10 +738,11 @@ struct Epilogue {
     double two_blocks(int width) const { return std::max(0.0, 2.0 * block(width) - 3.0); }
     double small() const { return 0.62 * us; }
 };
-Epilogue epilogue_of(int act, bool pre, bool residual)
+// Whether the pre-activation is saved (0.9 more) is left out: a forward pass has the same bits with gradients and without.
+Epilogue epilogue_of(int act, bool residual)
 {
     const double acts[4] = {Epilogue::kPlain, 5.6, 7.0, 7.4};
-    return {acts[act] + (pre ? 0.9 : 0.0) + (residual ? 2.8 : 0.0)};
+    return {acts[act] + (residual ? 2.8 : 0.0)};
 }
 constexpr Epilogue kQkvEpilogue{8.0};
 
@@ -995,7 +996,7 @@ int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream
 {
     PlainArgs<ACT> a{};
     const int      off = off_sectors(g->a, g->lda, g->b, g->ldb);
-    const Epilogue epi = epilogue_of(g->act, g->c_pre != nullptr, g->residual != nullptr);
+    const Epilogue epi = epilogue_of(g->act, g->residual != nullptr);
     int            csize = 1;
     if (g->ctas <= 0 && !(flags & (FU_GEMM_SINGLE | FU_GEMM_PAIR))) {
         c     = choose_wide_split(c, g->m, g->n, g->k, pairs, off, epi);
@@ -1070,7 +1071,7 @@ extern "C" int fu_gemm_bf16(const FuGemmArgs* g, void* stream_v)
     const int    flags  = forced ? (g->flags | FU_GEMM_PAIR) : g->flags;
     const int    sms    = g->ctas > 0 ? std::min(g->ctas, device_sms()) : device_sms();
     const Choice c      = choose_shape(g->m, g->n, g->k, pairs, sms, flags, true, off_sectors(g->a, g->lda, g->b, g->ldb),
-                                      epilogue_of(g->act, g->c_pre != nullptr, g->residual != nullptr));
+                                      epilogue_of(g->act, g->residual != nullptr));
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     switch (g->act) {
     case 0: return launch_plain<0>(g, c, pairs, flags, stream);
