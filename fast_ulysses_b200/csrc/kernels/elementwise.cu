@@ -189,6 +189,8 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(const NormRopeBwd
 __global__ void __launch_bounds__(256) layernorm_fwd_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, float* stats,
                                                             int64_t rows, int64_t cols, int64_t ldx, int64_t ldy, float eps)
 {
+    fu::ptx::grid_wait();
+    fu::ptx::grid_trigger();
     const int     lane = threadIdx.x & 31;
     const int64_t row  = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (row >= rows) {
@@ -235,6 +237,8 @@ __global__ void __launch_bounds__(256) layernorm_bwd_kernel(const __nv_bfloat16*
                                                             const float* stats, const __nv_bfloat16* add,
                                                             __nv_bfloat16* dx, int64_t rows, int64_t cols, int64_t ld)
 {
+    fu::ptx::grid_wait();
+    fu::ptx::grid_trigger();
     const int     lane = threadIdx.x & 31;
     const int64_t row  = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     if (row >= rows) {
@@ -302,6 +306,8 @@ template <bool kVec>
 __global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThreads)
     colsum_kernel(const __nv_bfloat16* x, __nv_bfloat16* out, int64_t rows, int64_t cols, int64_t ld)
 {
+    fu::ptx::grid_wait();
+    fu::ptx::grid_trigger();
     constexpr int kGroups = kSumThreads / 8;  // rows a CTA reads at once; eight lanes of 8 columns each per row
     constexpr int kAhead  = 4;
     __shared__ float part[kGroups][kSumCols + 4];
@@ -395,6 +401,7 @@ struct PullGrads {
 // of a full grid added its d(gamma) with atomics of its own.
 __global__ void __launch_bounds__(256, 2) pull_qkv_grads_kernel(const __grid_constant__ PullGrads p)
 {
+    fu::ptx::grid_wait();
     __shared__ uint32_t       ticket;
     __shared__ const uint8_t* from[3][MAX_HEADS];
     __shared__ uint32_t       pitch[MAX_HEADS];
@@ -641,6 +648,10 @@ extern "C" int fu_pull_qkv_grads(const FuPullGradsArgs* a, void* stream)
         return fu::fail(FU_E_ARG, "fu_pull_qkv_grads: %lld tokens x %d heads", (long long)a->m, a->heads);
     }
     const int grid = static_cast<int>(std::min<int64_t>(sms * (per_sm > 0 ? per_sm : 1), (warps + 7) / 8));
+    if (a->world == 1) {
+        FU_CUDA_OK(fu::launch_behind(pull_qkv_grads_kernel, dim3(static_cast<unsigned>(grid)), dim3(256), 0, static_cast<cudaStream_t>(stream), p));
+        return FU_OK;
+    }
     pull_qkv_grads_kernel<<<grid, 256, 0, static_cast<cudaStream_t>(stream)>>>(p);
     FU_CUDA_OK(cudaGetLastError());
     return FU_OK;
@@ -654,9 +665,8 @@ extern "C" int fu_layernorm_fwd(const void* x, void* y, float* stats, int64_t ro
         return fu::fail(FU_E_ARG, "fu_layernorm_fwd: needs 16-byte aligned rows of a multiple of 8 columns");
     }
     const unsigned blocks = static_cast<unsigned>((rows + 7) / 8);  // eight warps, one row each
-    layernorm_fwd_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), stats, rows, cols, ldx, ldy, eps);
-    FU_CUDA_OK(cudaGetLastError());
+    FU_CUDA_OK(fu::launch_behind(layernorm_fwd_kernel, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                 static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), stats, rows, cols, ldx, ldy, eps));
     return FU_OK;
 }
 
@@ -669,10 +679,9 @@ extern "C" int fu_layernorm_bwd_add(const void* dy, const void* x, const float* 
         return fu::fail(FU_E_ARG, "fu_layernorm_bwd_add: needs 16-byte aligned rows of a multiple of 8 columns");
     }
     const unsigned blocks = static_cast<unsigned>((rows + 7) / 8);
-    layernorm_bwd_kernel<<<blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(
-        static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
-        static_cast<const __nv_bfloat16*>(add), static_cast<__nv_bfloat16*>(dx), rows, cols, ld);
-    FU_CUDA_OK(cudaGetLastError());
+    FU_CUDA_OK(fu::launch_behind(layernorm_bwd_kernel, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                 static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
+                                 static_cast<const __nv_bfloat16*>(add), static_cast<__nv_bfloat16*>(dx), rows, cols, ld));
     return FU_OK;
 }
 
@@ -684,8 +693,7 @@ extern "C" int fu_colsum_bf16(const void* x, void* out, int64_t rows, int64_t co
     const bool     vec    = (ld % 8) == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     const dim3     grid(kSumCluster, static_cast<unsigned>((cols + kSumCols - 1) / kSumCols));
     auto           kernel = vec ? colsum_kernel<true> : colsum_kernel<false>;
-    kernel<<<grid, kSumThreads, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const __nv_bfloat16*>(x),
-                                                                        static_cast<__nv_bfloat16*>(out), rows, cols, ld);
-    FU_CUDA_OK(cudaGetLastError());
+    FU_CUDA_OK(fu::launch_behind(kernel, grid, dim3(kSumThreads), 0, static_cast<cudaStream_t>(stream), static_cast<const __nv_bfloat16*>(x),
+                                 static_cast<__nv_bfloat16*>(out), rows, cols, ld));
     return FU_OK;
 }

@@ -45,6 +45,8 @@ constexpr int kPreRows = 32;
 
 __global__ void __launch_bounds__(8 * kPreRows) fmha_bwd_pre_kernel(const PreParams p)
 {
+    ptx::grid_wait();
+    ptx::grid_trigger();
     const uint32_t blks = static_cast<uint32_t>(p.Sq_pad) / kPreRows;
     const int      h    = static_cast<int>(blockIdx.x % p.H);
     const uint32_t hb   = blockIdx.x / p.H;
@@ -93,6 +95,8 @@ __global__ void __launch_bounds__(8 * kPreRows) fmha_bwd_pre_kernel(const PrePar
 __global__ void fmha_bwd_post_kernel(const float* acc, __nv_bfloat16* dq, int64_t dq_row, int64_t dq_head,
                                      int64_t dq_batch, int B, int H, int Sq, float scale)
 {
+    ptx::grid_wait();
+    ptx::grid_trigger();
     const int64_t idx   = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;  // one per 8 elements
     const int64_t total = static_cast<int64_t>(B) * Sq * H * 16;
     if (idx >= total) {
@@ -166,8 +170,7 @@ extern "C" int fu_fmha_bwd(const FuFmhaArgs* a, void* stream_v)
     pre.Sq = a->seq_q;
     pre.Sq_pad = sq_pad;
     {
-        fmha_bwd_pre_kernel<<<static_cast<unsigned>(stats / kPreRows), 8 * kPreRows, 0, stream>>>(pre);
-        FU_CUDA_OK(cudaGetLastError());
+        FU_CUDA_OK(fu::launch_behind(fmha_bwd_pre_kernel, dim3(static_cast<unsigned>(stats / kPreRows)), dim3(8 * kPreRows), 0, stream, pre));
     }
     if (deterministic) {
         const int rc = fu_fmha_bwd_dkdv_launch(a, pre.lse2, pre.delta, sq_pad, stream_v);
@@ -178,10 +181,8 @@ extern "C" int fu_fmha_bwd(const FuFmhaArgs* a, void* stream_v)
         return rc;
     }
     const int64_t n = static_cast<int64_t>(a->batch) * a->seq_q * a->heads * 16;
-    fmha_bwd_post_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(
-        a->dq_acc, static_cast<__nv_bfloat16*>(a->dq), a->q_row, a->q_head, a->q_batch, a->batch, a->heads, a->seq_q,
-        a->scale);
-    FU_CUDA_OK(cudaGetLastError());
+    FU_CUDA_OK(fu::launch_behind(fmha_bwd_post_kernel, dim3(static_cast<unsigned>((n + 255) / 256)), dim3(256), 0, stream, a->dq_acc,
+                                 static_cast<__nv_bfloat16*>(a->dq), a->q_row, a->q_head, a->q_batch, a->batch, a->heads, a->seq_q, a->scale));
     return FU_OK;
 }
 

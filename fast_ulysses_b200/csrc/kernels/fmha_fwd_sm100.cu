@@ -333,7 +333,9 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
         ptx::tmem_relinquish();
     }
     ptx::tc_fence_before();
+    ptx::grid_wait();
     __syncthreads();
+    ptx::grid_trigger();  // with this CTA's tensor memory in hand
     ptx::tc_fence_after();
     const uint32_t tmem = ptx::uniform(tmem_holder);
     // The items of this CTA and the kv tiles of each: every gridDim.x-th item and all of its tiles; or
@@ -926,7 +928,7 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
         }
         int grid = a->ctas > 0 ? std::min(a->ctas, sms) : sms;
         grid     = std::max(1, std::min(grid, p.total_work));
-        kernel<<<grid, THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(p);
+        FU_CUDA_OK(fu::launch_behind(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), SMEM_BYTES, static_cast<cudaStream_t>(stream), p));
         FU_CUDA_OK(cudaGetLastError());
         return FU_OK;
     };

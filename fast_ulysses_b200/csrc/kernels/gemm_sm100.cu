@@ -947,27 +947,36 @@ int pairs_for(int ctas)
     return ctas > 0 ? std::max(1, std::min(pairs, ctas / 2)) : pairs;
 }
 
-template <class Kernel, class Args>
-int launch_pairs(Kernel kernel, const Args& a, int pairs, cudaStream_t stream)
+// `behind`: see launch_behind; not for kernels that other ranks wait for.
+template <class Args>
+cudaError_t launch(void (*kernel)(Args), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool behind, const Args& a)
+{
+    if (behind) {
+        return fu::launch_behind(kernel, grid, block, smem, stream, a);
+    }
+    kernel<<<grid, block, smem, stream>>>(a);
+    return cudaGetLastError();
+}
+
+template <class Args>
+int launch_pairs(void (*kernel)(Args), const Args& a, int pairs, cudaStream_t stream, bool behind = true)
 {
     const int rc = raise_smem_limit(kernel, WIDE_SMEM_BYTES);
     if (rc != FU_OK) {
         return rc;
     }
-    kernel<<<2 * std::max(1, std::min(pairs, a.core.items)), WIDE_THREADS, WIDE_SMEM_BYTES, stream>>>(a);
-    FU_CUDA_OK(cudaGetLastError());
+    FU_CUDA_OK(launch(kernel, dim3(static_cast<unsigned>(2 * std::max(1, std::min(pairs, a.core.items)))), dim3(WIDE_THREADS), WIDE_SMEM_BYTES, stream, behind, a));
     return FU_OK;
 }
 
-template <class Kernel, class Args>
-int launch_small(Kernel kernel, const Args& a, int ctas, cudaStream_t stream)
+template <class Args>
+int launch_small(void (*kernel)(Args), const Args& a, int ctas, cudaStream_t stream, bool behind = true)
 {
     const int rc = raise_smem_limit(kernel, SMALL_SMEM_BYTES);
     if (rc != FU_OK) {
         return rc;
     }
-    kernel<<<launch_grid(ctas, a.core.items), SMALL_THREADS, SMALL_SMEM_BYTES, stream>>>(a);
-    FU_CUDA_OK(cudaGetLastError());
+    FU_CUDA_OK(launch(kernel, dim3(static_cast<unsigned>(launch_grid(ctas, a.core.items))), dim3(SMALL_THREADS), SMALL_SMEM_BYTES, stream, behind, a));
     return FU_OK;
 }
 
@@ -1210,10 +1219,10 @@ extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream_v)
     }
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     switch (c.shape) {
-    case Shape::kTall: return launch_pairs(qkv_wide_kernel<2, 1>, a, pairs, stream);
-    case Shape::kBroad: return launch_pairs(qkv_wide_kernel<1, 2>, a, pairs, stream);
-    case Shape::kOne: return launch_pairs(qkv_wide_kernel<1, 1>, a, pairs, stream);
-    default: return launch_small(qkv_small_kernel, a, q->ctas, stream);
+    case Shape::kTall: return launch_pairs(qkv_wide_kernel<2, 1>, a, pairs, stream, q->world == 1);
+    case Shape::kBroad: return launch_pairs(qkv_wide_kernel<1, 2>, a, pairs, stream, q->world == 1);
+    case Shape::kOne: return launch_pairs(qkv_wide_kernel<1, 1>, a, pairs, stream, q->world == 1);
+    default: return launch_small(qkv_small_kernel, a, q->ctas, stream, q->world == 1);
     }
 }
 

@@ -382,7 +382,11 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
         ptx::tmem_relinquish_pair();
     }
     ptx::tc_fence_before();
+    ptx::grid_wait();
     __syncthreads();
+    if (!Epi::kPeers) {
+        ptx::grid_trigger();  // with this CTA's tensor memory in hand
+    }
     ptx::tc_fence_after();
     const uint32_t tmem_base = ptx::uniform(tmem_holder);
 
@@ -707,7 +711,11 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
         ptx::tmem_relinquish();
     }
     ptx::tc_fence_before();
+    ptx::grid_wait();
     __syncthreads();
+    if (!Epi::kPeers) {
+        ptx::grid_trigger();  // with this CTA's tensor memory in hand
+    }
     ptx::tc_fence_after();
     const uint32_t tmem_base = ptx::uniform(tmem_holder);
     const uint32_t leader = ptx::elect_one();

@@ -30,6 +30,27 @@ int raise_smem_limit(Kernel kernel, int bytes)
     return raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes);
 }
 
+// Launches a kernel that begins with ptx::grid_wait() so that it may be set up while the kernel before it in the stream
+// is still running: its CTAs come onto SMs as they become free and initialise their barriers, tensor memory and
+// descriptors there. Otherwise each launch waits for the last CTA before it to have left and then starts from
+// nothing, 1 - 3 us a kernel. Not for kernels that other ranks wait for, and not for clusters of more than two that
+// fill the device: taken up as SMs become free they leave SMs over that no whole cluster fits into.
+template <class... P, class... A>
+cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args)
+{
+    cudaLaunchConfig_t  cfg  = {};
+    cudaLaunchAttribute attr = {};
+    attr.id                  = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim              = grid;
+    cfg.blockDim             = block;
+    cfg.dynamicSmemBytes     = smem;
+    cfg.stream               = stream;
+    cfg.attrs                = &attr;
+    cfg.numAttrs             = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 }  // namespace fu
 
 #define FU_CUDA_OK(expr)                                                                                      \
