@@ -162,6 +162,8 @@ struct PlainEpi {
         for (int j = 0; j < 64; ++j) {
             v[j] = __uint_as_float(r[j]);
         }
+        // One copy of the code: with both halves unrolled, fetching it took the first unit of a launch that finds other
+        // kernels' code in the caches 24000 clocks instead of 11000 (256 x 512 x 256 with GELU: 20.5 -> 14.4 us).
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
             piece<64>(v, row0, col0 + h * 64, end, lane, stage);

@@ -254,10 +254,12 @@ __device__ __forceinline__ void load_unit(uint32_t taddr, uint32_t (&r)[128])
 // 1390 TFLOP/s on the feed-forward shapes, 9450 x 13824 x 5120 and its relatives (cuBLAS 1320 - 1430; the
 // 128 x 256 single-CTA tiles before this kernel 1120 - 1200).
 //
-// A block may be narrower, `width` = 32 .. 256 columns in steps of 32, and a pair may own a single block (MB =
-// NB = 1, whose accumulators alternate between the halves of tensor memory): both so that a problem of a few
-// waves fills the last one. A narrow or single block makes less of each byte in shared memory, see
-// block_clocks().
+// A block may be narrower, `width` = 32 .. 256 columns in steps of 32, so that a problem of a few waves fills the last
+// one, and a pair may own a single block (MB = NB = 1, whose accumulators alternate between the halves of tensor
+// memory), for the same reason and because it hides the whole epilogue: with two blocks the second waits in
+// tensor memory for the first one's arithmetic and stores, and the next tile behind it (9450 x 5120 x 5120 with GELU:
+// 384 us with two, 344 with one; with no epilogue 311 and 318). A narrow or single block makes less of each byte in
+// shared memory, see block_clocks().
 //
 // With two blocks there is no second accumulator buffer, so the blocks' order hides the epilogue instead: the first
 // kStages K-blocks of a tile are multiplied into block 0 and then into block 1, and so are the last
