@@ -57,6 +57,13 @@ def test_single_rank_batched_and_partial_tile():
     run_world([77], [6], 320, b=2)
 
 
+# sizes that run on pairs with one 256 x 256 block at a time: several waves, the last block half outside (odd
+# heads), a partial row block; one row beyond a block
+@pytest.mark.parametrize("seq,heads,hidden", [(4001, 13, 1536), (2817, 12, 1288)])
+def test_single_blocks_on_pairs(seq, heads, hidden):
+    run_world([seq], [heads], hidden, grid=(4, 26, 40))
+
+
 def test_three_ranks_uneven_heads():
     run_world([100, 60, 80], [3, 2, 3], 256)
 
