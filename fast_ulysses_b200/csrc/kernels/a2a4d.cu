@@ -910,6 +910,8 @@ __device__ __forceinline__ void vec_store(void* p, const Vec32& v)
 template <class Vec, int kThreads, int kUnroll, bool kFlat>
 __global__ void __launch_bounds__(kThreads) a2a4d_local_kernel(const __grid_constant__ LocalArgs a)
 {
+    grid_wait();
+    grid_trigger();
     if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
         *reinterpret_cast<volatile uint64_t*>(a.epoch) += 2;
     }
@@ -947,16 +949,14 @@ __global__ void __launch_bounds__(kThreads) a2a4d_local_kernel(const __grid_cons
 constexpr int64_t kLocalSmallBytes = 8 << 20;
 
 template <class Vec, bool kFlat>
-void launch_local_as(LocalArgs a, int64_t batches, int64_t bytes, cudaStream_t stream)
+cudaError_t launch_local_as(const LocalArgs& a, int64_t batches, int64_t bytes, cudaStream_t stream)
 {
     if (bytes <= kLocalSmallBytes) {
         const dim3 grid((a.n + 255) / 256, static_cast<unsigned>(batches));
-        a2a4d_local_kernel<Vec, 256, 1, kFlat><<<grid, 256, 0, stream>>>(a);
+        return fu::launch_behind(a2a4d_local_kernel<Vec, 256, 1, kFlat>, grid, dim3(256), 0, stream, a);
     }
-    else {
-        const dim3 grid((a.n + 2047) / 2048, static_cast<unsigned>(batches));
-        a2a4d_local_kernel<Vec, 512, 4, kFlat><<<grid, 512, 0, stream>>>(a);
-    }
+    const dim3 grid((a.n + 2047) / 2048, static_cast<unsigned>(batches));
+    return fu::launch_behind(a2a4d_local_kernel<Vec, 512, 4, kFlat>, grid, dim3(512), 0, stream, a);
 }
 
 // Runs the one route of a single-rank call, or returns 1 when the general kernel has to (a tensor
@@ -1001,12 +1001,11 @@ int launch_local(const FuRoute& in, const uint8_t* src, uint8_t* dst, FuCtrl* ow
     a.shift = 31 + s;
     const int64_t bytes = r.row_bytes * r.rows * r.batches;
     if (wide) {
-        flat ? launch_local_as<Vec32, true>(a, r.batches, bytes, stream) : launch_local_as<Vec32, false>(a, r.batches, bytes, stream);
+        FU_CUDA_OK((flat ? launch_local_as<Vec32, true>(a, r.batches, bytes, stream) : launch_local_as<Vec32, false>(a, r.batches, bytes, stream)));
     }
     else {
-        flat ? launch_local_as<uint4, true>(a, r.batches, bytes, stream) : launch_local_as<uint4, false>(a, r.batches, bytes, stream);
+        FU_CUDA_OK((flat ? launch_local_as<uint4, true>(a, r.batches, bytes, stream) : launch_local_as<uint4, false>(a, r.batches, bytes, stream)));
     }
-    FU_CUDA_OK(cudaGetLastError());
     return FU_OK;
 }
 

@@ -289,6 +289,8 @@ struct alignas(32) Bf16x16 {
 __global__ void __launch_bounds__(kFp8LocalThreads) fp8_round_trip_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
                                                                           int64_t rows)
 {
+    fu::ptx::grid_wait();
+    fu::ptx::grid_trigger();
     constexpr int kRows = kFp8LocalThreads / 8;  // rows per CTA and unroll step
     const int64_t row0 = static_cast<int64_t>(blockIdx.x) * (kRows * kFp8LocalUnroll) + (threadIdx.x >> 3);
     const int     part = threadIdx.x & 7;
@@ -396,9 +398,8 @@ extern "C" int fu_fp8_round_trip(const void* src, void* dst, int64_t rows, void*
         return fu::fail(FU_E_ARG, "fu_fp8_round_trip: %lld rows", (long long)rows);
     }
     if (ctas > 0) {
-        fp8_round_trip_kernel<<<static_cast<unsigned>(ctas), kFp8LocalThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-            static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), rows);
-        FU_CUDA_OK(cudaGetLastError());
+        FU_CUDA_OK(fu::launch_behind(fp8_round_trip_kernel, dim3(static_cast<unsigned>(ctas)), dim3(kFp8LocalThreads), 0, static_cast<cudaStream_t>(stream),
+                                     static_cast<const uint8_t*>(src), static_cast<uint8_t*>(dst), rows));
     }
     return FU_OK;
 }
