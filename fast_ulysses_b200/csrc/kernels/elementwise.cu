@@ -402,6 +402,9 @@ struct PullGrads {
 __global__ void __launch_bounds__(256, 2) pull_qkv_grads_kernel(const __grid_constant__ PullGrads p)
 {
     fu::ptx::grid_wait();
+    if (p.peers.world == 1) {
+        fu::ptx::grid_trigger();
+    }
     __shared__ uint32_t       ticket;
     __shared__ const uint8_t* from[3][MAX_HEADS];
     __shared__ uint32_t       pitch[MAX_HEADS];

@@ -59,6 +59,7 @@ struct PlainEpi {
     const __nv_bfloat16* aux;    // act 3: where the tanh-form GELU's derivative is evaluated
     __nv_bfloat16*       c_pre;  // optional second output: the value before the activation
 
+    __device__ bool alone() const { return true; }
     __device__ void open(int) {}
     __device__ void close(int) {}
 
@@ -242,6 +243,7 @@ struct QkvEpi {
     uint64_t         base_epoch;
 
     __device__ explicit QkvEpi(const QkvParams& params) : p(params), base_epoch(0) {}
+    __device__ bool alone() const { return p.peers.world == 1; }
 
     __device__ void open(int epi_tid)
     {

@@ -222,6 +222,7 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src, Aux aux
 // thread, the whole row of 128 fp32 in registers) and give the accumulator back to the MMA thread as
 // soon as the registers are loaded, before any arithmetic or store. Epi requirements:
 //   static constexpr bool kPeers          whether open() / close() run (kernels that touch peers)
+//   bool alone()                          no kernel of other ranks waits for this one
 //   void open(int epi_tid), close(int epi_tid)          all epilogue threads, once before / after the tiles
 //   void unit(uint32_t (&r)[128], int row0, int col0, int col_end, int lane, uint32_t stage)
 // Columns from `col_end` on are not the unit's. `stage` is the address of 4 KiB of shared memory of this warp's own (32 rows x 128 bytes).
@@ -386,7 +387,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
     ptx::tc_fence_before();
     ptx::grid_wait();
     __syncthreads();
-    if (!Epi::kPeers) {
+    if (epi.alone()) {
         ptx::grid_trigger();  // with this CTA's tensor memory in hand
     }
     ptx::tc_fence_after();
@@ -715,7 +716,7 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
     ptx::tc_fence_before();
     ptx::grid_wait();
     __syncthreads();
-    if (!Epi::kPeers) {
+    if (epi.alone()) {
         ptx::grid_trigger();  // with this CTA's tensor memory in hand
     }
     ptx::tc_fence_after();
