@@ -892,11 +892,11 @@ struct LocalArgs {
 struct alignas(32) Vec32 {
     uint32_t w[8];
 };
-__device__ __forceinline__ void vec_load(uint4& v, const void* p) { v = ld_nc_v4(p); }
+__device__ __forceinline__ void vec_load(uint4& v, const void* p) { v = ld_once_v4(p); }
 __device__ __forceinline__ void vec_store(void* p, const uint4& v) { st_v4(p, v); }
 __device__ __forceinline__ void vec_load(Vec32& v, const void* p)
 {
-    asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+    asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                  : "=r"(v.w[0]), "=r"(v.w[1]), "=r"(v.w[2]), "=r"(v.w[3]), "=r"(v.w[4]), "=r"(v.w[5]), "=r"(v.w[6]), "=r"(v.w[7])
                  : "l"(p));
 }

@@ -328,7 +328,7 @@ __global__ void __cluster_dims__(kSumCluster, 1, 1) __launch_bounds__(kSumThread
             v[u]            = make_uint4(0u, 0u, 0u, 0u);
             if (r < rows) {
                 if (kVec && c0 + 8 <= cols) {
-                    v[u] = fu::ptx::ld_nc_v4(x + r * ld + c0);
+                    v[u] = fu::ptx::ld_once_v4(x + r * ld + c0);
                 }
                 else {
                     __nv_bfloat16* e = reinterpret_cast<__nv_bfloat16*>(&v[u]);

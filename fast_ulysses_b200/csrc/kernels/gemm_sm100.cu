@@ -58,6 +58,7 @@ struct PlainEpi {
     int                  M, N, bias_bf16;
     const __nv_bfloat16* aux;    // act 3: where the tanh-form GELU's derivative is evaluated
     __nv_bfloat16*       c_pre;  // optional second output: the value before the activation
+    float                ahead[4];
 
     __device__ bool alone() const { return true; }
     __device__ void open(int) {}
@@ -73,45 +74,42 @@ struct PlainEpi {
         }
     }
 
-    // W columns of 32 rows, a row per thread; none from column N on
+    // The bias of the 128 columns from col0 on, four a lane, while their products are still being computed: the loads' latency
+    // behind the products cost a unit 0.7 us (256 x 512 x 256 with GELU 5.9 us so, 6.7 with read-only loads of all 64 columns by
+    // every thread, 10 % more with ordinary ones).
+    __device__ __forceinline__ void fetch(int col0, int lane)
+    {
+        if (bias) {
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                const int col = col0 + lane * 4 + k;
+                ahead[k]      = col >= N ? 0.0f : bias_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[col])
+                                                            : static_cast<const float*>(bias)[col];
+            }
+        }
+    }
+
+    // W columns of 32 rows, a row per thread; none from column N on. Lane `first` has fetched the bias of the first four.
+    // Each thread needs all of them: they go through the staging buffer.
     template <int W>
-    __device__ __forceinline__ void piece(float (&v)[W], int row0, int col0, int N, int lane, uint32_t stage) const
+    __device__ __forceinline__ void piece(float (&v)[W], int row0, int col0, int N, int lane, uint32_t stage, int first = 0) const
     {
         if (row0 >= M || col0 >= N) {
             return;  // warp-uniform
         }
         if (bias) {
-            const bool whole = col0 + W <= N && (reinterpret_cast<uintptr_t>(bias) & 15u) == 0;  // uniform
-            if (whole && !bias_bf16) {
-                const float4* b = reinterpret_cast<const float4*>(static_cast<const float*>(bias) + col0);
-#pragma unroll
-                for (int j = 0; j < W / 4; ++j) {
-                    const float4 f = __ldg(b + j);
-                    v[4 * j] += f.x, v[4 * j + 1] += f.y, v[4 * j + 2] += f.z, v[4 * j + 3] += f.w;
-                }
+            if (lane >= first && lane < first + W / 4) {
+                ptx::st_shared_v4(stage + (lane - first) * 16, make_uint4(__float_as_uint(ahead[0]), __float_as_uint(ahead[1]),
+                                                                          __float_as_uint(ahead[2]), __float_as_uint(ahead[3])));
             }
-            else if (whole) {
-                const uint4* b = reinterpret_cast<const uint4*>(static_cast<const __nv_bfloat16*>(bias) + col0);
+            __syncwarp();
 #pragma unroll
-                for (int j = 0; j < W / 8; ++j) {
-                    const uint4           q = __ldg(b + j);
-                    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&q);
-#pragma unroll
-                    for (int k = 0; k < 4; ++k) {
-                        const float2 f = __bfloat1622float2(h[k]);
-                        v[8 * j + 2 * k] += f.x, v[8 * j + 2 * k + 1] += f.y;
-                    }
-                }
+            for (int g = 0; g < W / 4; ++g) {
+                const uint4 q = ptx::ld_shared_v4(stage + g * 16);
+                v[4 * g] += __uint_as_float(q.x), v[4 * g + 1] += __uint_as_float(q.y);
+                v[4 * g + 2] += __uint_as_float(q.z), v[4 * g + 3] += __uint_as_float(q.w);
             }
-            else {
-#pragma unroll
-                for (int j = 0; j < W; ++j) {
-                    if (col0 + j < N) {
-                        v[j] += bias_bf16 ? __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[col0 + j])
-                                          : static_cast<const float*>(bias)[col0 + j];
-                    }
-                }
-            }
+            __syncwarp();
         }
         if (c_pre) {
             pack_row(v, stage, lane);
@@ -167,7 +165,7 @@ struct PlainEpi {
         // kernels' code in the caches 24000 clocks instead of 11000 (256 x 512 x 256 with GELU: 20.5 -> 14.4 us).
 #pragma unroll 1
         for (int h = 0; h < 2; ++h) {
-            piece<64>(v, row0, col0 + h * 64, end, lane, stage);
+            piece<64>(v, row0, col0 + h * 64, end, lane, stage, h * 16);
 #pragma unroll
             for (int j = 0; j < 64; ++j) {
                 v[j] = __uint_as_float(r[64 + j]);
@@ -244,6 +242,7 @@ struct QkvEpi {
 
     __device__ explicit QkvEpi(const QkvParams& params) : p(params), base_epoch(0) {}
     __device__ bool alone() const { return p.peers.world == 1; }
+    __device__ void fetch(int, int) {}
 
     __device__ void open(int epi_tid)
     {
@@ -288,7 +287,7 @@ struct QkvEpi {
     __device__ __forceinline__ float4 load4(const float* p) const
     {
         if (this->p.tables_aligned) {
-            return __ldg(reinterpret_cast<const float4*>(p));
+            return *reinterpret_cast<const float4*>(p);
         }
         return make_float4(p[0], p[1], p[2], p[3]);
     }

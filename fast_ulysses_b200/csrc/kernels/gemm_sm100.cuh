@@ -223,6 +223,7 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src, Aux aux
 // soon as the registers are loaded, before any arithmetic or store. Epi requirements:
 //   static constexpr bool kPeers          whether open() / close() run (kernels that touch peers)
 //   bool alone()                          no kernel of other ranks waits for this one
+//   void fetch(int col0, int lane)        before a unit's products are waited for: what can be read ahead
 //   void open(int epi_tid), close(int epi_tid)          all epilogue threads, once before / after the tiles
 //   void unit(uint32_t (&r)[128], int row0, int col0, int col_end, int lane, uint32_t stage)
 // Columns from `col_end` on are not the unit's. `stage` is the address of 4 KiB of shared memory of this warp's own (32 rows x 128 bytes).
@@ -571,14 +572,17 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
         }
         if constexpr (SPLIT) {
             const WideItem<MB, NB> item(core, w_0, 0);
-            bool                   ok = item.u0 != item.u1;  // an empty item only takes part in the barriers
+            const int              width = 256 / parts;
+            bool                   ok    = item.u0 != item.u1;  // an empty item only takes part in the barriers
+            if (ok) {
+                epi.fetch(item.col(item.u0) + part * width + cg * (width / 2), lane);
+            }
             if (ok && !ptx::mbar_wait(&tmem_full[item.u0], 0u)) {
                 flag_error(core.err, ERR_EPI_WAIT);
                 ok = false;
             }
             ptx::tc_fence_after();
             const uint32_t taddr = tmem_base + item.u0 * 256 + (static_cast<uint32_t>(quarter * 32) << 16);
-            const int      width = 256 / parts;
             const uint32_t slot  = base + quarter * 32768 + lane * 16;  // this warp's rows: [columns / 4][lane] of 16 bytes per pair
             ptx::cluster_sync();  // every pair's products are complete: its stages may be overwritten
 #pragma unroll 1
@@ -630,6 +634,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
             const WideItem<MB, NB> item(core, w, uses[0] + uses[1]);
             const int              cols = core.width / 2, col0 = cg * cols;  // a warp's share of a block
             for (int u = item.u0; u < item.u1; ++u) {
+                epi.fetch(item.col(u) + col0, lane);
                 if (!ptx::mbar_wait(&tmem_full[u], uses[u] & 1u)) {
                     flag_error(core.err, ERR_EPI_WAIT);
                     ok = false;
@@ -814,12 +819,13 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
         uint32_t tcount = 0;
         for (int t = t_0; t < tiles; t += t_inc, ++tcount) {
             const uint32_t acc = tcount & 1u;
-            const bool     ok  = ptx::mbar_wait(&tmem_full[acc], (tcount >> 1) & 1u);
+            int            mt, nt;
+            pair_tile_coords(core.tiles_m, core.tiles_n, 16, t, mt, nt);
+            epi.fetch(nt * 128 + (SPLIT ? crank * (128 / csize) : 0), lane);
+            const bool ok = ptx::mbar_wait(&tmem_full[acc], (tcount >> 1) & 1u);
             if (!ok) {
                 flag_error(core.err, ERR_EPI_WAIT);
             }
-            int mt, nt;
-            pair_tile_coords(core.tiles_m, core.tiles_n, 16, t, mt, nt);
             if constexpr (SPLIT) {  // one tile per cluster; also after a timeout: the other CTAs wait in its barriers
                 ptx::tc_fence_after();
                 const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);

@@ -286,8 +286,7 @@ struct alignas(32) Bf16x16 {
     uint32_t w[8];
 };
 
-__global__ void __launch_bounds__(kFp8LocalThreads) fp8_round_trip_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
-                                                                          int64_t rows)
+__global__ void __launch_bounds__(kFp8LocalThreads) fp8_round_trip_kernel(const uint8_t* src, uint8_t* dst, int64_t rows)
 {
     fu::ptx::grid_wait();
     fu::ptx::grid_trigger();
@@ -299,7 +298,7 @@ __global__ void __launch_bounds__(kFp8LocalThreads) fp8_round_trip_kernel(const 
     for (int u = 0; u < kFp8LocalUnroll; ++u) {
         const int64_t row = row0 + u * kRows;
         if (row < rows) {
-            asm volatile("ld.global.nc.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+            asm volatile("ld.global.L1::no_allocate.v8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
                          : "=r"(v[u].w[0]), "=r"(v[u].w[1]), "=r"(v[u].w[2]), "=r"(v[u].w[3]), "=r"(v[u].w[4]), "=r"(v[u].w[5]),
                            "=r"(v[u].w[6]), "=r"(v[u].w[7])
                          : "l"(src + row * 256 + part * 32));
