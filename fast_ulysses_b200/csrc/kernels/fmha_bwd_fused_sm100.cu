@@ -69,6 +69,7 @@ struct Params {
     int            B, H, Sq, Skv, Sq_pad;
     int            n_q, kv_blocks, total_work;
     int            first;  // split kernel: the item of cluster 0
+    int            overlap;  // the next kernel may come up beside this one
     float          scale, scale_log2;
     uint32_t*      err;
     uint64_t*      trace;
@@ -276,7 +277,9 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_bwd_fused_kernel(const __grid
     ptx::tc_fence_before();
     ptx::grid_wait();
     __syncthreads();
-    ptx::grid_trigger();  // with this CTA's tensor memory in hand
+    if (p.overlap) {
+        ptx::grid_trigger();  // with this CTA's tensor memory in hand
+    }
     ptx::tc_fence_after();
     const uint32_t tmem = ptx::uniform(bar.tmem_holder);
     const int      crank = SPLIT ? static_cast<int>(ptx::uniform(ptx::cluster_ctarank())) : 0;
@@ -683,6 +686,7 @@ int fu_fmha_bwd_fused_launch(const FuFmhaArgs* a, const float* lse2, const float
     p.scale      = a->scale;
     p.scale_log2 = a->scale * 1.4426950408889634f;
     p.err        = a->err;
+    p.overlap    = a->ctas <= 0;
     p.trace      = a->trace;
     int dev = 0, sms = 0;
     FU_CUDA_OK(cudaGetDevice(&dev));

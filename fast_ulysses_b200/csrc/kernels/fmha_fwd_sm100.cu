@@ -70,6 +70,7 @@ struct Params {
     int            B, H, Sq, Skv;
     int            q_blocks, total_work, n_kv;
     int            first;       // split kernel: the item of cluster 0
+    int            overlap;     // the next kernel may come up beside this one
     float          scale, scale_log2;
     uint32_t*      err;
     uint64_t*      trace;
@@ -335,7 +336,9 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_fwd_kernel(const __grid_const
     ptx::tc_fence_before();
     ptx::grid_wait();
     __syncthreads();
-    ptx::grid_trigger();  // with this CTA's tensor memory in hand
+    if (p.overlap) {
+        ptx::grid_trigger();  // with this CTA's tensor memory in hand
+    }
     ptx::tc_fence_after();
     const uint32_t tmem = ptx::uniform(tmem_holder);
     // The items of this CTA and the kv tiles of each: every gridDim.x-th item and all of its tiles; or
@@ -912,6 +915,7 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
     p.scale      = a->scale;
     p.scale_log2 = a->scale * 1.4426950408889634f;
     p.err        = a->err;
+    p.overlap    = a->ctas <= 0;
 
     int dev = 0, sms = 0;
     FU_CUDA_OK(cudaGetDevice(&dev));
@@ -928,7 +932,11 @@ extern "C" int fu_fmha_fwd(const FuFmhaArgs* a, void* stream)
         }
         int grid = a->ctas > 0 ? std::min(a->ctas, sms) : sms;
         grid     = std::max(1, std::min(grid, p.total_work));
-        FU_CUDA_OK(fu::launch_behind(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), SMEM_BYTES, static_cast<cudaStream_t>(stream), p));
+        if (p.overlap) {
+            FU_CUDA_OK(fu::launch_behind(kernel, dim3(static_cast<unsigned>(grid)), dim3(THREADS), SMEM_BYTES, static_cast<cudaStream_t>(stream), p));
+            return FU_OK;
+        }
+        kernel<<<grid, THREADS, SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(p);
         FU_CUDA_OK(cudaGetLastError());
         return FU_OK;
     };

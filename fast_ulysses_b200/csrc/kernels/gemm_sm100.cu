@@ -60,7 +60,6 @@ struct PlainEpi {
     __nv_bfloat16*       c_pre;  // optional second output: the value before the activation
     float                ahead[4];
 
-    __device__ bool alone() const { return true; }
     __device__ void open(int) {}
     __device__ void close(int) {}
 
@@ -241,7 +240,6 @@ struct QkvEpi {
     uint64_t         base_epoch;
 
     __device__ explicit QkvEpi(const QkvParams& params) : p(params), base_epoch(0) {}
-    __device__ bool alone() const { return p.peers.world == 1; }
     __device__ void fetch(int, int) {}
 
     __device__ void open(int epi_tid)
@@ -950,11 +948,10 @@ int pairs_for(int ctas)
     return ctas > 0 ? std::max(1, std::min(pairs, ctas / 2)) : pairs;
 }
 
-// `behind`: see launch_behind; not for kernels that other ranks wait for.
 template <class Args>
-cudaError_t launch(void (*kernel)(Args), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool behind, const Args& a)
+cudaError_t launch(void (*kernel)(Args), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, const Args& a)
 {
-    if (behind) {
+    if (a.core.overlap) {
         return fu::launch_behind(kernel, grid, block, smem, stream, a);
     }
     kernel<<<grid, block, smem, stream>>>(a);
@@ -962,24 +959,24 @@ cudaError_t launch(void (*kernel)(Args), dim3 grid, dim3 block, size_t smem, cud
 }
 
 template <class Args>
-int launch_pairs(void (*kernel)(Args), const Args& a, int pairs, cudaStream_t stream, bool behind = true)
+int launch_pairs(void (*kernel)(Args), const Args& a, int pairs, cudaStream_t stream)
 {
     const int rc = raise_smem_limit(kernel, WIDE_SMEM_BYTES);
     if (rc != FU_OK) {
         return rc;
     }
-    FU_CUDA_OK(launch(kernel, dim3(static_cast<unsigned>(2 * std::max(1, std::min(pairs, a.core.items)))), dim3(WIDE_THREADS), WIDE_SMEM_BYTES, stream, behind, a));
+    FU_CUDA_OK(launch(kernel, dim3(static_cast<unsigned>(2 * std::max(1, std::min(pairs, a.core.items)))), dim3(WIDE_THREADS), WIDE_SMEM_BYTES, stream, a));
     return FU_OK;
 }
 
 template <class Args>
-int launch_small(void (*kernel)(Args), const Args& a, int ctas, cudaStream_t stream, bool behind = true)
+int launch_small(void (*kernel)(Args), const Args& a, int ctas, cudaStream_t stream)
 {
     const int rc = raise_smem_limit(kernel, SMALL_SMEM_BYTES);
     if (rc != FU_OK) {
         return rc;
     }
-    FU_CUDA_OK(launch(kernel, dim3(static_cast<unsigned>(launch_grid(ctas, a.core.items))), dim3(SMALL_THREADS), SMALL_SMEM_BYTES, stream, behind, a));
+    FU_CUDA_OK(launch(kernel, dim3(static_cast<unsigned>(launch_grid(ctas, a.core.items))), dim3(SMALL_THREADS), SMALL_SMEM_BYTES, stream, a));
     return FU_OK;
 }
 
@@ -1021,6 +1018,7 @@ int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream
     if (rc != FU_OK) {
         return rc;
     }
+    a.core.overlap  = g->ctas <= 0;
     a.epi.c         = static_cast<__nv_bfloat16*>(g->c);
     a.epi.residual  = static_cast<const __nv_bfloat16*>(g->residual);
     a.epi.bias      = g->bias;
@@ -1220,12 +1218,13 @@ extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream_v)
     if (q->y_save && ((q->ld_y % 8) || (reinterpret_cast<uintptr_t>(q->y_save) & 15u))) {
         return fu::fail(FU_E_ARG, "fu_qkv_rope_scatter: y_save needs 16-byte aligned rows");
     }
+    a.core.overlap      = q->world == 1 && q->ctas <= 0;
     cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
     switch (c.shape) {
-    case Shape::kTall: return launch_pairs(qkv_wide_kernel<2, 1>, a, pairs, stream, q->world == 1);
-    case Shape::kBroad: return launch_pairs(qkv_wide_kernel<1, 2>, a, pairs, stream, q->world == 1);
-    case Shape::kOne: return launch_pairs(qkv_wide_kernel<1, 1>, a, pairs, stream, q->world == 1);
-    default: return launch_small(qkv_small_kernel, a, q->ctas, stream, q->world == 1);
+    case Shape::kTall: return launch_pairs(qkv_wide_kernel<2, 1>, a, pairs, stream);
+    case Shape::kBroad: return launch_pairs(qkv_wide_kernel<1, 2>, a, pairs, stream);
+    case Shape::kOne: return launch_pairs(qkv_wide_kernel<1, 1>, a, pairs, stream);
+    default: return launch_small(qkv_small_kernel, a, q->ctas, stream);
     }
 }
 

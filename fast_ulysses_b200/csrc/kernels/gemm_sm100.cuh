@@ -222,7 +222,6 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src, Aux aux
 // thread, the whole row of 128 fp32 in registers) and give the accumulator back to the MMA thread as
 // soon as the registers are loaded, before any arithmetic or store. Epi requirements:
 //   static constexpr bool kPeers          whether open() / close() run (kernels that touch peers)
-//   bool alone()                          no kernel of other ranks waits for this one
 //   void fetch(int col0, int lane)        before a unit's products are waited for: what can be read ahead
 //   void open(int epi_tid), close(int epi_tid)          all epilogue threads, once before / after the tiles
 //   void unit(uint32_t (&r)[128], int row0, int col0, int col_end, int lane, uint32_t stage)
@@ -302,6 +301,7 @@ struct WideCore {
     int         full, items;
     int         first;             // split kernel: the item of cluster 0
     int         a_mn, b_mn;
+    int         overlap;           // the next kernel may come up beside this one, see host_util.h: launch_behind
     uint32_t*   err;
 };
 
@@ -388,7 +388,7 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
     ptx::tc_fence_before();
     ptx::grid_wait();
     __syncthreads();
-    if (epi.alone()) {
+    if (core.overlap) {
         ptx::grid_trigger();  // with this CTA's tensor memory in hand
     }
     ptx::tc_fence_after();
@@ -721,7 +721,7 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
     ptx::tc_fence_before();
     ptx::grid_wait();
     __syncthreads();
-    if (epi.alone()) {
+    if (core.overlap) {
         ptx::grid_trigger();  // with this CTA's tensor memory in hand
     }
     ptx::tc_fence_after();

@@ -34,7 +34,9 @@ int raise_smem_limit(Kernel kernel, int bytes)
 // is still running: its CTAs come onto SMs as they become free and initialise their barriers, tensor memory and
 // descriptors there. Otherwise each launch waits for the last CTA before it to have left and then starts from
 // nothing, 1 - 3 us a kernel. Not for kernels that other ranks wait for, and not for clusters of more than two that
-// fill the device: taken up as SMs become free they leave SMs over that no whole cluster fits into.
+// fill the device: taken up as SMs become free they leave SMs over that no whole cluster fits into. Nor does a kernel whose grid
+// the caller has limited (`ctas`) start so or let the next one: the SMs that it leaves free are meant for another stream, and the
+// next kernel's CTAs would hold them until it ends.
 template <class... P, class... A>
 cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args)
 {
