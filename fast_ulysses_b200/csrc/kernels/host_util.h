@@ -59,6 +59,7 @@ cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
     do {                                                                                                      \
         cudaError_t fu_err__ = (expr);                                                                        \
         if (fu_err__ != cudaSuccess) {                                                                        \
+            (void)cudaGetLastError(); /* reported here: the next launch's own check must not find it again */ \
             return ::fu::fail(FU_E_CUDA, "%s failed: %s (%s:%d)", #expr, cudaGetErrorString(fu_err__),        \
                               __FILE__, __LINE__);                                                            \
         }                                                                                                     \

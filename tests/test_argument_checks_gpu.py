@@ -2,12 +2,15 @@
 operand on another device, or one that is shorter than what an epilogue reads, would otherwise be an address
 that the kernel may not touch."""
 
+import ctypes as C
+
 import pytest
 import torch
 
 import fast_ulysses_b200 as fu
 from fast_ulysses_b200.models.attention import UlyssesSelfAttention
-from fast_ulysses_b200.ops import attention, gemm, norm
+from fast_ulysses_b200.ops import _ckernels as ck
+from fast_ulysses_b200.ops import attention, fp8, gemm, norm
 
 pytestmark = pytest.mark.gpu
 
@@ -130,3 +133,16 @@ def test_gemm_refuses_an_operand_on_the_host(name):
     with pytest.raises(AssertionError):
         gemm.gemm_bf16(a, b.cpu())
     assert gemm.gemm_bf16(a, b, **{k: v.cuda() for k, v in extra.items()}).shape == (M, N)
+
+
+def test_a_launch_that_fails_is_reported_once():
+    """A grid beyond the device's limit is refused by the launch itself; the next call is not told of it again."""
+    x = torch.ones(1, 65536 * 64, device="cuda").bfloat16()  # column sums: a row of CTAs for every 64 columns
+    out = torch.empty(x.size(1), device="cuda", dtype=torch.bfloat16)
+    sums = ck.lib().fu_colsum_bf16
+    args = [C.c_void_p(out.data_ptr()), C.c_int64(1), C.c_int64(x.size(1)), C.c_int64(x.size(1)), C.c_void_p(torch.cuda.current_stream().cuda_stream)]
+    with pytest.raises(RuntimeError, match="launch refused"):
+        ck.check(sums(C.c_void_p(x.data_ptr()), *args))
+    v = bf16(64, 128)
+    back = fp8.dequantize(fp8.quantize(v))  # launched in the ordinary way
+    assert ((back - v).norm() / v.norm()).item() < 0.04  # three bits of mantissa: 2^-4 at most
