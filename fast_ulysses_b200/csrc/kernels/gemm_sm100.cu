@@ -18,6 +18,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
+#include <limits>
 
 namespace {
 
@@ -688,21 +689,28 @@ int pair_capacity()
 }
 
 // Which core and tile a problem gets, from its size alone: the one whose estimated time is lowest. The
-// estimate is a start-and-end time plus, per wave of CTAs, a time per 64-wide K-block, both measured
-// (us, SM clock 1.9 GHz, problems of 64 - 4100 rows and 256 - 13824 columns and K):
-//   128 x 128 tiles on single CTAs   3.2 + 0.225 per K-block and wave of 148
-//   two 256 x 256 blocks on pairs    6 + 0.60 per K-block and wave of 74, 0.33 for a wave of single blocks
-//   one 256 x 256 block on pairs     6 + 0.31
+// estimate is a start, per wave of CTAs a time per 64-wide K-block, and the epilogue. Fitted to 480 products of 64 - 20000
+// rows, 64 - 13824 columns and K, each timed in up to 24 shapes behind a launch of itself (us, SM clock 1.9 GHz), and checked on 240
+// others: the shape chosen takes 1.5 % more than the fastest one (geometric mean; 9 in 10 sizes less than 6 % more). With
+// the epilogue's time left out it was 5.4 %, with half of it for two blocks and launches of nothing but halves of tiles 4.4 %.
+//   128 x 128 tiles on single CTAs   2.0 + 0.223 per K-block and wave of 148
+//   two 256 x 256 blocks on pairs    2.6 + 0.622 per K-block and wave of 74, and the epilogue of both
+//   one 256 x 256 block on pairs     2.6 + 0.328
 // Rows of an operand that do not all start on a 32-byte sector (a pitch that is an odd multiple of 16 bytes)
-// reach shared memory more slowly: the K-blocks of a 128 x 128 tile take 0.265 us with one such operand and 0.385
-// with two, those of a single block on a pair 0.36 and 0.46, of two blocks 0.66 and 0.77 (256 x 3328 x 4096 with
-// small tiles: 18.1, 21.3 and 28.6 us). The pair kernels' time per K-block shrinks with the width of the block, see block_clocks(). At most half as
-// many tiles of two blocks as pairs left over are split into blocks.
-// The epilogue (Epilogue, below) comes on top. With one block the accumulators alternate and a wave takes the longer of
-// the products and the epilogue with what it delays; with two, the second block waits in tensor memory until the first
-// has been written, and the next tile with it. Measured (us), two blocks and one: 9450 x 5120 x 5120 with GELU 384 and
-// 344, with the derivative 415 and 329, with a residual 367 and 318, with nothing 311 and 318; 75600 x 15360 x 5120 with
-// the QKV epilogue 8514 and 7433; 16000 x 1280 x 640 with the derivative 70 and 52.
+// reach shared memory more slowly, see kSmallBlock and the next two (256 x 3328 x 4096 with small tiles and none, one or two such
+// operands: 18.1, 21.3 and 28.6 us). The pair kernels' time per K-block shrinks with the width of the block, see block_clocks(). At
+// most half as many tiles of two blocks as pairs left over are split into blocks.
+// With one block (and with small tiles) the accumulators alternate and a wave takes the longer of the products and the epilogue with
+// what it delays; with two, the second block waits in tensor memory until the first has been written, and the next tile with
+// it. Two blocks and one: 6729 x 7632 x 2592 with a residual 205 and 184 us, 14493 x 3408 x 3472 with erf GELU 270 (of 192
+// columns) and 246, 7478 x 10512 x 3248 with the derivative 412 and 375. Large products repeated for tenths of a second run at
+// the power limit, and there two blocks, which read less from shared memory, win where the estimates are close: 7800 x 5120 x 13824
+// with a residual 837 and 892 us, 7800 x 5120 x 5120 331 and 336, 7800 x 13824 x 5120 with GELU 854 and 860, with the derivative 912
+// and 911; with one operand off the sectors 13645 x 5672 -> 2336 with GELU and a residual, both products, 630 and 672, with three of
+// four 15717 x 6472 -> 3688 1320 and 1468. So beyond kLong (us) another shape has to be estimated 8 % faster than two whole
+// blocks, 12 % with an operand off the sectors.
+// A launch of nothing but halves of tiles of two blocks does what a launch of single blocks does, with a shorter ring: it is
+// left out (143 x 10928 x 12416 76 -> 65 us, 4105 x 288 x 9032 with erf GELU 50.5 -> 48).
 // What the widths and the single block gave, against two blocks of 256 columns or the small tiles: 1000 x 5120 x
 // 5120 53.0 -> 41.8 us (two of 160), 512 x 5120 x 13824 81.6 -> 61.6 and 512 x 5120 x 5120 30.4 -> 25.8 (one of
 // 160), 4100 x 1536 x 4096 58.9 -> 47.2 (two of 192).
@@ -726,26 +734,28 @@ double block_clocks(int mb, int nb, int width)
 }
 
 // us per K-block, by how many of the two operands lie off the 32-byte sectors
-constexpr double kSmallBlock[3] = {0.225, 0.265, 0.385}, kOneBlock[3] = {0.31, 0.36, 0.46}, kTwoBlocks[3] = {0.60, 0.66, 0.77};
+constexpr double kSmallBlock[3] = {0.223, 0.27, 0.38}, kOneBlock[3] = {0.328, 0.34, 0.42}, kTwoBlocks[3] = {0.622, 0.65, 0.73};
+constexpr double kSmallStart = 2.0, kPairStart = 2.6, kLong = 50.0;
 
-// us that the epilogue of a block of 256 columns takes, fitted to 320 - 1024 deep products of 2640 - 16000 rows. That of
-// nothing but a result is part of the start-and-end times.
+// us that the epilogue of a block of 256 columns and of a 128 x 128 tile takes
 struct Epilogue {
-    double us;
-    static constexpr double kPlain = 2.8;
-    double beyond() const { return us - kPlain; }
-    // A narrow block's: pieces of 64 columns that are not whole, or do not lie on whole lines of 128 bytes.
-    double block(int width) const { return width == 256 ? us : width == 128 ? 0.8 * us : width > 128 ? 1.6 * us : us; }
-    double two_blocks(int width) const { return std::max(0.0, 2.0 * block(width) - 3.0); }
-    double small() const { return 0.62 * us; }
+    double pair, small;
+    // A warp's share of a narrow block is half a unit, or more of it in pieces that are not whole.
+    double block(int width) const { return width > 128 ? pair : 0.59 * pair; }
 };
 // Whether the pre-activation is saved (0.9 more) is left out: a forward pass has the same bits with gradients and without.
 Epilogue epilogue_of(int act, bool residual)
 {
-    const double acts[4] = {Epilogue::kPlain, 5.6, 7.0, 7.4};
-    return {acts[act] + (residual ? 2.8 : 0.0)};
+    const double pair[4] = {2.4, 4.7, 7.3, 7.0}, small[4] = {1.4, 3.2, 6.4, 5.5};
+    return {pair[act] + (residual ? 1.7 : 0.0), small[act] + (residual ? 1.0 : 0.0)};
 }
-constexpr Epilogue kQkvEpilogue{8.0};
+constexpr Epilogue kQkvEpilogue{7.0, 4.0};  // fitted to 100 projections of 64 - 75600 rows, 1 - 40 heads: 0.9 % above the fastest shape
+
+// Waves of single blocks: an epilogue runs beside the next products and they delay it.
+double alternating(double products, double epilogue, int64_t waves)
+{
+    return waves < 1 ? 0.0 : products + (waves - 1) * std::max(products, epilogue + 0.46 * products) + epilogue;
+}
 
 int off_sectors(const void* a, int64_t lda, const void* b, int64_t ldb)
 {
@@ -757,16 +767,16 @@ Choice wide_choice(int64_t m, int64_t n, double kb, Shape shape, int width, int 
 {
     const int     mb = shape == Shape::kTall ? 2 : 1, nb = shape == Shape::kBroad ? 2 : 1;
     const int64_t tm = (m + 256 * mb - 1) / (256 * mb), tn = (n + width * nb - 1) / (width * nb), tiles = tm * tn;
+    const double  e = epi.block(width), block = kb * kOneBlock[off] / 512 * block_clocks(1, 1, width);
     if (shape == Shape::kOne) {
-        const double products = kb * kOneBlock[off] / 512 * block_clocks(1, 1, width), waves = static_cast<double>((tiles + pairs - 1) / pairs);
         return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(tiles), static_cast<int>(tiles),
-                6.0 + products + (waves - 1.0) * std::max(products, epi.block(width) + 0.45 * products) + epi.beyond(), width};
+                kPairStart + alternating(block, e, (tiles + pairs - 1) / pairs), width};
     }
     const int64_t left = tiles % pairs, full = 2 * left <= pairs ? tiles - left : tiles, items = full + 2 * (tiles - full);
-    const double  whole = static_cast<double>((full + pairs - 1) / pairs), halves = static_cast<double>((items - full + pairs - 1) / pairs);
+    const double  whole = static_cast<double>((full + pairs - 1) / pairs);
     return {shape, static_cast<int>(tm), static_cast<int>(tn), static_cast<int>(full), static_cast<int>(items),
-            6.0 + kb * (kTwoBlocks[off] / 1024 * block_clocks(mb, nb, width) * whole + 1.05 * kOneBlock[off] / 512 * block_clocks(1, 1, width) * halves)
-                + epi.two_blocks(width) * whole + 0.5 * epi.block(width) * halves - Epilogue{Epilogue::kPlain}.two_blocks(256), width};
+            kPairStart + whole * (kb * kTwoBlocks[off] / 1024 * block_clocks(mb, nb, width) + 2.0 * e)
+                + alternating(block, e, (items - full + pairs - 1) / pairs), width};
 }
 
 // `narrow`: the epilogue takes blocks of any width (the heads of the QKV projection need 128 columns at once).
@@ -776,34 +786,35 @@ Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int fla
     const double  kb   = static_cast<double>((k + BK - 1) / BK);
     const double  products = kSmallBlock[off] * kb, waves = static_cast<double>((t128 + sms - 1) / sms);
     const Choice  small{Shape::kSmall, static_cast<int>((m + 127) / 128), static_cast<int>((n + 127) / 128), 0, static_cast<int>(t128),
-                       3.2 + products + (waves - 1.0) * std::max(products, epi.small() + 0.5 * products) + 0.62 * epi.beyond()};
+                       kSmallStart + products + (waves - 1.0) * std::max(products + 0.35 * epi.small, epi.small) + epi.small};
     if (flags & FU_GEMM_SINGLE) {
         return small;
     }
     const Choice tall = wide_choice(m, n, kb, Shape::kTall, 256, pairs, off, epi), broad = wide_choice(m, n, kb, Shape::kBroad, 256, pairs, off, epi);
-    Choice       wide = tall.cost < broad.cost ? tall : broad;
     if (flags & FU_GEMM_PAIR) {
-        return wide;
+        return tall.cost < broad.cost ? tall : broad;
     }
-    Choice best = wide_choice(m, n, kb, Shape::kOne, 256, pairs, off, epi);
+    const auto cheaper = [](const Choice& a, const Choice& b) { return b.cost < a.cost && (b.shape == Shape::kOne || b.full > 0) ? b : a; };
+    Choice     two{}, best = wide_choice(m, n, kb, Shape::kOne, 256, pairs, off, epi);
+    two.cost = std::numeric_limits<double>::infinity();
+    two      = cheaper(cheaper(two, tall), broad);
     for (int width = narrow ? 224 : 0; width >= 96; width -= 32) {
         if ((flags & FU_GEMM_B_KN) && width % 128 != 0) {
             continue;  // such a B comes in blocks of 64 columns, half of them for each CTA
         }
         for (const Shape shape : {Shape::kTall, Shape::kBroad, Shape::kOne}) {
-            const Choice c = wide_choice(m, n, kb, shape, width, pairs, off, epi);
-            best           = c.cost < best.cost ? c : best;
+            best = cheaper(best, wide_choice(m, n, kb, shape, width, pairs, off, epi));
         }
     }
-    if (best.cost < 0.96 * wide.cost) {  // two whole blocks where it makes little difference: they take less power
-        wide = best;
+    if (best.cost >= (two.cost <= kLong ? 1.0 : off > 0 ? 0.88 : 0.92) * two.cost) {
+        best = two;
     }
-    return small.cost < wide.cost ? small : wide;
+    return small.cost < best.cost ? small : best;
 }
 
 // The broad tiles with what whole waves leave over shared by clusters (gemm_wide_split_kernel), when that is
-// estimated to be faster than `best`. Measured (us): a wave of clusters takes 8.1 (two pairs) or 9.4 (four) and
-// 0.29 per K-block of a pair's share; behind another launch 1.5 of that are hidden. 2000 x 5120 x 5120 (80 tiles
+// estimated to be faster than `best`. Fitted with the others (us): a wave of clusters takes 7.0 (two pairs) or 7.3 (four), 0.32
+// per K-block of a pair's share and 0.43 of an epilogue; behind another launch 1.5 of that are hidden. 2000 x 5120 x 5120 (80 tiles
 // on 74 pairs): 83.5 -> 79.5, 1000 x 5120 x 13824 (40 tiles: a wave of blocks and six more): 130 -> 115.
 Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, int pairs, int off, Epilogue epi)
 {
@@ -818,13 +829,12 @@ Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, in
         return best;
     }
     double       limit = 0.96 * best.cost;
-    const double before =
-        full + single > 0 ? 6.0 - 1.5 + kb * (kTwoBlocks[off] * (full / pairs) + 1.05 * kOneBlock[off] * (single / pairs))
-                                + epi.two_blocks(256) * (full / pairs) + 0.5 * epi.us * (single / pairs) - Epilogue{Epilogue::kPlain}.two_blocks(256)
-                          : 0.0;
+    const double before = full + single > 0 ? kPairStart - 1.5 + (kb * kTwoBlocks[off] + 2.0 * epi.pair) * (full / pairs)
+                                                  + alternating(kb * kOneBlock[off], epi.pair, single / pairs)
+                                            : 0.0;
     for (const int csize : {4, 8}) {
         const int64_t parts = csize / 2, share = (kb + parts - 1) / parts;
-        const double  wave  = (csize == 4 ? 8.1 : 9.4) + 0.97 * kOneBlock[off] * share + 0.5 * epi.beyond();
+        const double  wave  = (csize == 4 ? 7.0 : 7.3) + 0.97 * kOneBlock[off] * share + 0.43 * epi.pair;
         if ((kb + share - 1) / share != parts || before + wave >= limit) {
             continue;  // a pair would have nothing to do, or no gain beyond the estimate's error even in one wave
         }
@@ -847,7 +857,7 @@ Choice choose_wide_split(const Choice& best, int64_t m, int64_t n, int64_t k, in
 }
 
 // How many CTAs share the K-blocks of a 128 x 128 tile (1: none do), see run_small, when that is estimated
-// to be faster than `best`. The exchange takes 1.8, 2.4 and 2.8 us beyond the tile's own time (measured, for
+// to be faster than `best`. The exchange takes 2.9, 3.2 and 3.5 us beyond the tile's own time (fitted with the others, for
 // two, four and eight CTAs). 64 x 2000 x 8000: 30.6 -> 13.3 us with four, 64 x 512 x 2048: 10.6 -> 7.0 with eight,
 // 512 x 1536 x 4096: 18.0 -> 13.2 with two; the 160 tiles of 512 x 5120 x 5120 stay as they are.
 int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k, int off, Epilogue epi)
@@ -861,7 +871,7 @@ int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k, int off, E
     }
     for (const int csize : {2, 4, 8}) {
         const int64_t share = (kb + csize - 1) / csize;
-        const double  once  = 3.2 + (csize == 2 ? 1.8 : csize == 4 ? 2.4 : 2.8) + kSmallBlock[off] * share + 0.62 * epi.beyond() / csize;
+        const double  once  = kSmallStart + (csize == 2 ? 2.9 : csize == 4 ? 3.2 : 3.5) + kSmallBlock[off] * share + epi.small / csize;
         if ((kb + share - 1) / share != csize || once >= cost) {
             continue;  // a CTA would have nothing to do, or no gain even in one wave
         }

@@ -5,6 +5,7 @@ layouts; every epilogue on ragged columns. Oracle: the same contraction in fp32.
 import pytest
 import torch
 
+from _graph import kernel_names
 from fast_ulysses_b200.ops import gemm
 
 pytestmark = pytest.mark.gpu
@@ -133,6 +134,21 @@ def test_narrow_and_single_blocks(act, m, n, k):
         # the same products summed in fp32, perhaps in another order, then rounded to bf16 once
         whole = gemm.gemm_bf16(a, other, pair=True, **kw, **layout)
         assert rel_err(gemm.gemm_bf16(a, other, **kw, **layout), whole.float()) < 1e-3
+    gemm.check_errors()
+
+
+# few tiles of two blocks, all of which would be run block by block: the kernel for that, or small tiles, does
+@pytest.mark.parametrize("m,n,k,act,b_kn", [(1024, 2432, 512, 0, False), (1024, 2432, 512, 2, False),
+                                            (143, 10928, 12416, 0, True), (1216, 2528, 8112, 0, True), (4105, 288, 9032, 2, False)])
+def test_halves_of_tiles_are_single_blocks(m, n, k, act, b_kn):
+    torch.manual_seed(m + n + k)
+    a = torch.randn(m, k, device="cuda").bfloat16()
+    b = (torch.randn(*((k, n) if b_kn else (n, k)), device="cuda") * 0.05).bfloat16()
+    kw = dict(act=act, b_kn=b_kn)
+    names = kernel_names(lambda: gemm.gemm_bf16(a, b, **kw))
+    assert len(names) == 1 and any(kernel in names[0] for kernel in ("gemm_wide_kernelILi1ELi1E", "gemm_small_kernel", "gemm_split_kernel")), names
+    # the same products summed in fp32, perhaps in another order, then rounded to bf16 once
+    assert rel_err(gemm.gemm_bf16(a, b, **kw), gemm.gemm_bf16(a, b, pair=True, **kw).float()) < 1e-3
     gemm.check_errors()
 
 

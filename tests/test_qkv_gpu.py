@@ -5,6 +5,7 @@ after another). Oracle: fp32 matmul -> RMSNorm -> RoPE -> the permutation, in pl
 import pytest
 import torch
 
+from _graph import kernel_names
 from fast_ulysses_b200.ops import _ckernels as ck
 from fast_ulysses_b200.ops import gemm, qkv
 from fast_ulysses_b200.ops.rope import rope_table
@@ -12,7 +13,7 @@ from fast_ulysses_b200.ops.rope import rope_table
 pytestmark = pytest.mark.gpu
 
 
-def run_world(seq, head_splits, hidden, b=1, grid=(4, 6, 10)):
+def run_world(seq, head_splits, hidden, b=1, grid=(4, 6, 10), kernel=None):
     world = len(seq)
     heads = sum(head_splits)
     S = sum(seq)
@@ -28,11 +29,17 @@ def run_world(seq, head_splits, hidden, b=1, grid=(4, 6, 10)):
     for r in range(world):
         x = torch.randn(b * seq[r], hidden, device="cuda").bfloat16()
         rope = rope_table(torch.arange(s0, s0 + seq[r], device="cuda"), grid=grid)
-        qkv.qkv_rope_scatter_raw(
-            x, w, rope, gq, gk, heads=heads, s_local=seq[r], seq_off=s0, s_total=S, head_splits=head_splits, rank=r,
-            win_q=[t.data_ptr() for t in wins], win_k=[t.data_ptr() + region for t in wins],
-            win_v=[t.data_ptr() + 2 * region for t in wins], ctrl=[t.data_ptr() + 3 * region for t in wins],
-            win_bytes=region, flags=ck.FU_A2A_NO_HANDSHAKE)
+        def call():
+            qkv.qkv_rope_scatter_raw(
+                x, w, rope, gq, gk, heads=heads, s_local=seq[r], seq_off=s0, s_total=S, head_splits=head_splits, rank=r,
+                win_q=[t.data_ptr() for t in wins], win_k=[t.data_ptr() + region for t in wins],
+                win_v=[t.data_ptr() + 2 * region for t in wins], ctrl=[t.data_ptr() + 3 * region for t in wins],
+                win_bytes=region, flags=ck.FU_A2A_NO_HANDSHAKE)
+
+        call()
+        if kernel:
+            names = kernel_names(call)
+            assert len(names) == 1 and kernel in names[0], names
         refs.append(qkv.qkv_reference(x, w, rope, gq, gk, heads))
         xs.append(x)
         s0 += seq[r]
@@ -58,10 +65,10 @@ def test_single_rank_batched_and_partial_tile():
 
 
 # sizes that run on pairs with one 256 x 256 block at a time: several waves, the last block half outside (odd
-# heads), a partial row block; one row beyond a block
+# heads), a partial row block; one row beyond a block, operands off 32-byte sectors
 @pytest.mark.parametrize("seq,heads,hidden", [(4001, 13, 1536), (2817, 12, 1288)])
 def test_single_blocks_on_pairs(seq, heads, hidden):
-    run_world([seq], [heads], hidden, grid=(4, 26, 40))
+    run_world([seq], [heads], hidden, grid=(4, 26, 40), kernel="qkv_wide_kernelILi1ELi1E")
 
 
 def test_three_ranks_uneven_heads():
