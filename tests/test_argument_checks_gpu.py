@@ -2,10 +2,9 @@
 operand on another device, or one that is shorter than what an epilogue reads, would otherwise be an address
 that the kernel may not touch."""
 
-import ctypes as C
-
 import pytest
 import torch
+from cuda.bindings import driver
 
 import fast_ulysses_b200 as fu
 from fast_ulysses_b200.models.attention import UlyssesSelfAttention
@@ -136,13 +135,15 @@ def test_gemm_refuses_an_operand_on_the_host(name):
 
 
 def test_a_launch_that_fails_is_reported_once():
-    """A grid beyond the device's limit is refused by the launch itself; the next call is not told of it again."""
-    x = torch.ones(1, 65536 * 64, device="cuda").bfloat16()  # column sums: a row of CTAs for every 64 columns
-    out = torch.empty(x.size(1), device="cuda", dtype=torch.bfloat16)
-    sums = ck.lib().fu_colsum_bf16
-    args = [C.c_void_p(out.data_ptr()), C.c_int64(1), C.c_int64(x.size(1)), C.c_int64(x.size(1)), C.c_void_p(torch.cuda.current_stream().cuda_stream)]
-    with pytest.raises(RuntimeError, match="launch refused"):
-        ck.check(sums(C.c_void_p(x.data_ptr()), *args))
-    v = bf16(64, 128)
-    back = fp8.dequantize(fp8.quantize(v))  # launched in the ordinary way
-    assert ((back - v).norm() / v.norm()).item() < 0.04  # three bits of mantissa: 2^-4 at most
+    """A stream whose capture has been spoilt refuses the launch; the next call, on another one, is not told of it again."""
+    x, y = bf16(24, 128), bf16(24, 128)
+    stream = driver.cuStreamCreate(driver.CUstream_flags.CU_STREAM_NON_BLOCKING)[1]
+    driver.cuStreamBeginCapture(stream, driver.CUstreamCaptureMode.CU_STREAM_CAPTURE_MODE_RELAXED)
+    driver.cuStreamSynchronize(stream)  # not allowed while it is captured
+    rc = ck.lib().fu_layernorm_fwd(x.data_ptr(), y.data_ptr(), None, 24, 128, 128, 128, 1e-6, int(stream))
+    driver.cuStreamEndCapture(stream)
+    driver.cuStreamDestroy(stream)
+    with pytest.raises(RuntimeError, match="capture"):
+        ck.check(rc)
+    back = fp8.dequantize(fp8.quantize(x))  # launched in the ordinary way
+    assert ((back - x).norm() / x.norm()).item() < 0.04  # three bits of mantissa: 2^-4 at most

@@ -106,7 +106,7 @@ def test_fp8_exchange_of_a_single_rank_is_quantise_and_dequantise(group, rows):
     assert torch.equal(fp8.all_to_all_4d_fp8(group, x), fp8.dequantize(fp8.quantize(x)))
 
 
-@pytest.mark.parametrize("rows,cols,pitch", [(1, 8, 8), (3, 5, 5), (255, 64, 64), (256, 72, 80), (4097, 136, 136), (1025, 5120, 5120)])
+@pytest.mark.parametrize("rows,cols,pitch", [(1, 8, 8), (3, 5, 5), (255, 64, 64), (256, 72, 80), (4097, 136, 136), (1025, 5120, 5120), (1024, 1024, 1024), (1024, 1025, 1032)])
 def test_column_sums(rows, cols, pitch):
     x = torch.randn(rows, pitch, device="cuda").bfloat16()[:, :cols]
     out = torch.empty(cols, device="cuda", dtype=torch.bfloat16)
