@@ -4,8 +4,8 @@
 // its rows (A stored K x M, B stored K x N, "MN-major"): the weight gradient of a linear layer
 // contracts over the tokens and reads dY and X as they lie in memory, without a transposed copy.
 //
-//   run_wide    two 256 x 256 blocks per pair of CTAs: everything large enough to occupy the device
-//   run_small   128 x 128 tiles on single CTAs: everything else
+//   run_wide    one or two blocks of 256 rows and up to 256 columns per pair of CTAs: what is large enough to occupy the device
+//   run_small   128 x 128 tiles on single CTAs: what is not, and what is short enough
 //   run         128 x 256 tiles on single CTAs, A gathered from the peers by extra warps while the GEMM runs
 //
 // In each, warp 0 is the TMA producer (128B-swizzled operand tiles into a ring of shared-memory
@@ -258,13 +258,13 @@ __device__ __forceinline__ void load_unit(uint32_t taddr, uint32_t (&r)[128])
 // A block may be narrower, `width` = 32 .. 256 columns in steps of 32, so that a problem of a few waves fills the last
 // one, and a pair may own a single block (MB = NB = 1, whose accumulators alternate between the halves of tensor
 // memory), for the same reason and because it hides the whole epilogue: with two blocks the second waits in
-// tensor memory for the first one's arithmetic and stores, and the next tile behind it (9450 x 5120 x 5120 with GELU:
-// 384 us with two, 344 with one; with no epilogue 311 and 318). A narrow or single block makes less of each byte in
-// shared memory, see block_clocks().
+// tensor memory for the first one's arithmetic and stores, and the next tile behind it (6729 x 7632 x 2592 with a
+// residual: 205 us with two, 184 with one). A narrow or single block makes less of each byte in
+// shared memory, see block_clocks(); at the power limit that decides, see choose_shape().
 //
-// With two blocks there is no second accumulator buffer, so the blocks' order hides the epilogue instead: the first
-// kStages K-blocks of a tile are multiplied into block 0 and then into block 1, and so are the last
-// ones. Block 0 is finished (and read out) four stages before block 1, and the next tile can start in
+// With two blocks there is no second accumulator buffer, so the blocks' order hides what it can of the epilogue, the reads
+// of tensor memory: the first kStages K-blocks of a tile are multiplied into block 0 and then into block 1, and so are the
+// last ones. Block 0 is finished (and read out) four stages before block 1, and the next tile can start in
 // block 0 while block 1 is still being read out.
 constexpr int WIDE_STAGES      = 4;  // of 48 KiB; six of 32 KiB with one block per pair
 constexpr int WIDE_BLOCK_BYTES = 128 * BK * 2;  // 128 rows of one operand, one K-block

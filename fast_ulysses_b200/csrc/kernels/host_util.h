@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 #include <cstdarg>
 #include <cstdio>
+#include <utility>
 
 namespace fu {
 
@@ -30,13 +31,18 @@ int raise_smem_limit(Kernel kernel, int bytes)
     return raise_smem_limit(reinterpret_cast<const void*>(kernel), bytes);
 }
 
-// Launches a kernel that begins with ptx::grid_wait() so that it may be set up while the kernel before it in the stream
-// is still running: its CTAs come onto SMs as they become free and initialise their barriers, tensor memory and
-// descriptors there. Otherwise each launch waits for the last CTA before it to have left and then starts from
-// nothing, 1 - 3 us a kernel. Not for kernels that other ranks wait for, and not for clusters of more than two that
-// fill the device: taken up as SMs become free they leave SMs over that no whole cluster fits into. Nor does a kernel whose grid
-// the caller has limited (`ctas`) start so or let the next one: the SMs that it leaves free are meant for another stream, and the
-// next kernel's CTAs would hold them until it ends.
+// Launches a kernel whose threads all call ptx::grid_wait() before they touch global memory, so that it may be set up while
+// the kernel before it in the stream is still running: its CTAs come onto SMs as they become free and initialise their
+// barriers, tensor memory and descriptors there. Otherwise each launch waits for the last CTA before it to have left and
+// then starts from nothing, 1 - 3 us a kernel. Only kernels that trigger (ptx::grid_trigger) are overlapped: behind any other,
+// PyTorch's for instance, or behind a copy, this is an ordinary launch.
+//
+// Not for kernels that other ranks wait for, and not for clusters of more than two that fill the device: taken up as SMs
+// become free they leave SMs over that no whole cluster fits into, or crowd on the first ones. Nor does a kernel whose grid
+// the caller has limited (`ctas`) start so or let the next one: the SMs that it leaves free are meant for another stream, and
+// the next kernel's CTAs would hold them until it ends. Kernels without a limit are launched so on groups of any size: an
+// exchange that is queued on another stream meanwhile may find the next kernel's CTAs in the SMs that became free, and
+// waits for one kernel as it does when it comes just after its launch; none of these waits for a peer.
 template <class... P, class... A>
 cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A&&... args)
 {
@@ -50,7 +56,7 @@ cudaError_t launch_behind(void (*kernel)(P...), dim3 grid, dim3 block, size_t sm
     cfg.stream               = stream;
     cfg.attrs                = &attr;
     cfg.numAttrs             = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
 }
 
 }  // namespace fu

@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(256) a2a4d_fp8_kernel(const __grid_constant__ 
 // packed row is written and read again. Bound by HBM. Eight lanes share a row of 128 values, 16 values
 // (32 bytes in, 32 bytes out) each; two rows per thread, one short-lived CTA per 64 rows. The arithmetic
 // per value is that of the kernels above, in packed pairs.
-// Measured, 97 MB in and 97 MB out: 79 us through the window, 33 us here.
+// Measured, 97 MB in and 97 MB out: 79 us through the window, 33 us here and 30 behind a call of itself.
 constexpr int kFp8LocalThreads = 256;
 constexpr int kFp8LocalUnroll  = 2;
 

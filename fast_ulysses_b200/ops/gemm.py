@@ -43,6 +43,8 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, bias: torch.Tensor | None = N
     ``(k, m)`` and ``b`` as ``(k, n)``; the kernel reads it as it lies in memory (no transposed
     copy), which is what the weight gradient ``dY^T X`` of a linear layer wants.
 
+    ``ctas``: run on at most that many SMs and leave the others to kernels of other streams.
+
     ``pair``: run on pairs of CTAs (two 256 x 256 blocks each, one tcgen05 MMA over two SMs) or on
     single CTAs (128 x 128 tiles), with the same bits; ``None`` leaves the shape to the library, which may
     also share K between CTAs and so sum in another order."""
