@@ -20,9 +20,10 @@
 // Measured limits (S = 32768, 5 heads, SM clock counter): a 128x128x16 MMA takes 64 clocks when its
 // descriptors are ready (8 per product: 512), a tensor-memory load-and-wait about 200, and the fp32
 // reductions of all SMs together move 6.1 TB/s into L2 whatever their width (64 KiB per block: 3130
-// clocks). The dependent chain dP -> C2 -> dK, dQ -> drain -> dP sets the period, about 4050 clocks against
-// the 2560 of the products; with random operands the power limit lowers the clock below that (37888
-// tokens x 4 heads: 5.1 ms with zeros, 7.0 with random numbers). Tried and no faster: dK begun on the first
+// clocks). The dependent chain dP -> C2 -> dK, dQ -> drain -> dP sets the period, about 3700 clocks against
+// the 2560 of the products (4050 while the statistics were read one value at a time); with random operands the power limit
+// lowers the clock below that (37888 tokens x 4 heads, repeated for seconds: 4.84 ms with zeros and 6.7 with random numbers,
+// 5.12 and 6.94 before). Tried and no faster: dK begun on the first
 // half of dS, the products issued by three warps, paced issue, a share of the exponentials on the FMA pipe.
 // Warps: 0 = TMA producer, 1 = MMA issuer, 2..9 = two threads per kv row, 10..17 = dQ drain.
 #include "cluster_plan.h"
@@ -110,36 +111,58 @@ __device__ __forceinline__ void red_add(float* addr, float v)
     asm volatile("red.global.add.f32 [%0], %1;" ::"l"(addr), "f"(v) : "memory");
 }
 
-// 16 query columns of S^T -> 8 packed probability pairs
+// 16 query columns of S^T -> 8 packed probability pairs. All threads of a warp want the same statistics, and a shared-memory
+// load takes a turn of the memory that the products read their operands from whatever its width: four values each.
 template <int C>
-__device__ __forceinline__ void c1_chunk(const uint32_t (&r)[16], uint32_t (&pk)[32], const float* lse2, float c,
-                                         bool kv_ok)
+__device__ __forceinline__ void c1_chunk(const uint32_t (&r)[16], uint32_t (&pk)[32], const float* lse2, float c)
 {
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const float p0 = ptx::ex2(fmaf(__uint_as_float(r[2 * k]), c, -lse2[C * 16 + 2 * k]));
-        const float p1 = ptx::ex2(fmaf(__uint_as_float(r[2 * k + 1]), c, -lse2[C * 16 + 2 * k + 1]));
-        pk[C * 8 + k]  = kv_ok ? ptx::pack_bf16x2(p0, p1) : 0u;
+    for (int k = 0; k < 4; ++k) {
+        const float4 l = *reinterpret_cast<const float4*>(lse2 + C * 16 + 4 * k);
+        float        t0, t1, t2, t3;  // the exponents, negated
+        ptx::fma2(t0, t1, __uint_as_float(r[4 * k]), __uint_as_float(r[4 * k + 1]), -c, -c, l.x, l.y);
+        ptx::fma2(t2, t3, __uint_as_float(r[4 * k + 2]), __uint_as_float(r[4 * k + 3]), -c, -c, l.z, l.w);
+        pk[C * 8 + 2 * k]     = ptx::pack_bf16x2(ptx::ex2(-t0), ptx::ex2(-t1));
+        pk[C * 8 + 2 * k + 1] = ptx::pack_bf16x2(ptx::ex2(-t2), ptx::ex2(-t3));
     }
 }
 
-// 16 query columns of dP^T -> 8 packed dS pairs (without the softmax scale), stored over the first
-// columns this thread has already read and into the swizzled shared-memory row
+// Stores half H of a row's probabilities over the scores, which have been read; kv rows that do not exist have none.
+template <int H>
+__device__ __forceinline__ void store_p(uint32_t t_s, uint32_t (&pk)[32], bool tail, bool kv_ok)
+{
+    if (tail && !kv_ok) {
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+            pk[H * 16 + k] = 0u;
+        }
+    }
+    ptx::tmem_st_32x16(t_s + H * 16, reinterpret_cast<const uint32_t(&)[16]>(pk[H * 16]));
+}
+
+// 16 query columns of dP^T -> 8 packed dS pairs (without the softmax scale), into the swizzled shared-memory row and over the
+// first columns that this thread has already read, four at a time: with both stores behind all eight the registers that wait
+// for them cost 4 %.
 template <int C>
 __device__ __forceinline__ void c2_chunk(const uint32_t (&r)[16], const uint32_t (&pk)[32], const float* delta,
                                          uint32_t t_dp, uint8_t* ds_row, int row_in)
 {
-    // the difference in fp32 (it cancels), the product with the bf16 probabilities as a packed pair
-    uint32_t dd[8];
 #pragma unroll
-    for (int k = 0; k < 8; ++k) {
-        const float d0 = __uint_as_float(r[2 * k]) - delta[C * 16 + 2 * k];
-        const float d1 = __uint_as_float(r[2 * k + 1]) - delta[C * 16 + 2 * k + 1];
-        dd[k]          = ptx::mul_bf16x2(pk[C * 8 + k], ptx::pack_bf16x2(d0, d1));
+    for (int k = 0; k < 2; ++k) {
+        uint32_t dd[4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            // the difference in fp32 (it cancels), the product with the bf16 probabilities as a packed pair
+            const float4 l = *reinterpret_cast<const float4*>(delta + C * 16 + 8 * k + 4 * j);
+            float        d0, d1, d2, d3;
+            ptx::fma2(d0, d1, l.x, l.y, -1.0f, -1.0f, __uint_as_float(r[8 * k + 4 * j]), __uint_as_float(r[8 * k + 4 * j + 1]));
+            ptx::fma2(d2, d3, l.z, l.w, -1.0f, -1.0f, __uint_as_float(r[8 * k + 4 * j + 2]), __uint_as_float(r[8 * k + 4 * j + 3]));
+            dd[2 * j]     = ptx::mul_bf16x2(pk[C * 8 + 4 * k + 2 * j], ptx::pack_bf16x2(d0, d1));
+            dd[2 * j + 1] = ptx::mul_bf16x2(pk[C * 8 + 4 * k + 2 * j + 1], ptx::pack_bf16x2(d2, d3));
+        }
+        *reinterpret_cast<uint4*>(ds_row + (((2 * C + k) ^ (row_in & 7)) << 4)) = make_uint4(dd[0], dd[1], dd[2], dd[3]);
+        ptx::tmem_st_32x4(t_dp + C * 8 + k * 4, dd);
     }
-    ptx::tmem_st_32x8(t_dp + C * 8, dd);
-    *reinterpret_cast<uint4*>(ds_row + (((2 * C) ^ (row_in & 7)) << 4))     = make_uint4(dd[0], dd[1], dd[2], dd[3]);
-    *reinterpret_cast<uint4*>(ds_row + (((2 * C + 1) ^ (row_in & 7)) << 4)) = make_uint4(dd[4], dd[5], dd[6], dd[7]);
 }
 
 // 32 columns of one accumulator row, rounded
@@ -466,6 +489,7 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_bwd_fused_kernel(const __grid
             const int  b     = w / (p.kv_blocks * p.H);
             const int  kvr   = jb * BLK + row_in;
             const bool kv_ok = kvr < p.Skv;
+            const bool tail  = jb * BLK + quarter * 32 + 32 > p.Skv;  // some of this warp's rows do not exist
             for (int i = 0; i < n_q; ++i, ++it) {
                 const int    s     = it % STAGES;
                 const float* lse2  = reinterpret_cast<const float*>(sm + OFF_STATS + s * 1024) + c2 * 64;
@@ -486,16 +510,17 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_bwd_fused_kernel(const __grid
                     ptx::tmem_ld_32x16(t_s, ra);
                     ptx::tmem_ld_wait();
                     ptx::tmem_ld_32x16(t_s + 16, rb);
-                    c1_chunk<0>(ra, pk, lse2, c, kv_ok);
+                    c1_chunk<0>(ra, pk, lse2, c);
                     ptx::tmem_ld_wait();
                     ptx::tmem_ld_32x16(t_s + 32, ra);
-                    c1_chunk<1>(rb, pk, lse2, c, kv_ok);
+                    c1_chunk<1>(rb, pk, lse2, c);
                     ptx::tmem_ld_wait();
                     ptx::tmem_ld_32x16(t_s + 48, rb);
-                    c1_chunk<2>(ra, pk, lse2, c, kv_ok);
+                    store_p<0>(t_s, pk, tail, kv_ok);
+                    c1_chunk<2>(ra, pk, lse2, c);
                     ptx::tmem_ld_wait();
-                    c1_chunk<3>(rb, pk, lse2, c, kv_ok);
-                    ptx::tmem_st_32x32(t_s, pk);
+                    c1_chunk<3>(rb, pk, lse2, c);
+                    store_p<1>(t_s, pk, tail, kv_ok);
                 }
                 ptx::tmem_st_wait();
                 ptx::tc_fence_before();
@@ -571,7 +596,10 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_bwd_fused_kernel(const __grid
         // dQ_i^T sits in tensor memory with the head dimension on the lanes: lane d of a warp adds
         // its query columns into dq_acc[q][d], so that every warp-wide reduction covers 128
         // contiguous bytes of one query row. Warps 10..13 take query columns 0..63, warps 14..17
-        // columns 64..127. The columns are released as soon as they are in registers.
+        // columns 64..127. The columns are released as soon as they are in registers. What waits in the memory queue
+        // behind a burst of reductions is every other warp's loads, stores and products: the address arithmetic between them
+        // is what keeps them apart (37888 x 4 with zeros 4.92 ms then; with rows at constant offsets 6.35, four floats
+        // a reduction 6.81, spaced out by the clock 5.0 - 6.4).
         const int      quarter  = warp & 3;
         const int      qh       = (warp - 10) >> 2;
         const int      dcol     = quarter * 32 + lane;
