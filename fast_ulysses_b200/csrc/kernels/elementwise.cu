@@ -185,114 +185,252 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(const NormRopeBwd
 }
 
 // ---- LayerNorm without affine parameters ----------------------------------------------------------------
-// One warp per row, two passes over the row (the second is an L1/L2 hit): statistics in fp32.
+// A row is read once and stays in the registers of 1, 2, 4 or 8 warps, up to kRowUnits 16-byte units a lane, all of them on
+// their way at once; statistics in fp32. Bound by HBM. With one warp per row, which read it twice in a chain of short loops, forward
+// 75600 x 5120 (1.55 GB) 338 -> 260 us, 7800 x 5120 38 -> 30, 320 x 4096 4.8 -> 2.5. The backward of what L2 does not hold is walked
+// through twice by the same warps, with a third of the registers and three times the rows under way (its second pass finds the row
+// in L1): 75600 x 5120 (3.1 GB) 701 -> 474 us, in registers 561; 12000 x 1280 23.7 -> 23.0 and 24.7. What L2 holds is faster in
+// registers: 4000 x 2560 21.3 -> 13.1 and 15.0, 1500 x 5120 15.2 -> 10.1 and 11.1, and rows of one unit are: 100000 x 256 39.7 -> 38.2
+// and 44.7. Rows too long for the registers of eight warps are walked through twice: 2000 x 16384 54 -> 25 and 122 -> 51.
+constexpr int kRowUnits = 5;
+
+__device__ __forceinline__ float2 sum_of_warp(float2 v)
+{
+#pragma unroll
+    for (int off = 16; off > 0; off >>= 1) {
+        v.x += __shfl_xor_sync(0xffffffffu, v.x, off);
+        v.y += __shfl_xor_sync(0xffffffffu, v.y, off);
+    }
+    return v;
+}
+
+// The sums over the `warps` warps of a row, in their order. (All threads of the CTA.)
+__device__ __forceinline__ float2 sum_of_warps(float2 v, int warps)
+{
+    __shared__ float2 part[8];
+    v = sum_of_warp(v);
+    if (warps > 1) {
+        const int warp = threadIdx.x >> 5;
+        if ((threadIdx.x & 31) == 0) {
+            part[warp] = v;
+        }
+        __syncthreads();
+        const int first = warp & ~(warps - 1);
+        v               = part[first];
+        for (int w = 1; w < warps; ++w) {
+            v.x += part[first + w].x;
+            v.y += part[first + w].y;
+        }
+    }
+    return v;
+}
+
+// Where a thread works: its row and its first column of every `stride` columns.
+struct RowPlace {
+    int64_t row;
+    int     col, stride;
+    bool    leads;
+    __device__ __forceinline__ explicit RowPlace(int warps)
+        : row(static_cast<int64_t>(blockIdx.x) * (8 / warps) + (threadIdx.x >> 5) / warps), col((threadIdx.x & (32 * warps - 1)) * 8),
+          stride(256 * warps), leads(col == 0)
+    {
+    }
+};
+
+__device__ __forceinline__ void add_moments(const uint4& v, float2& sum)
+{
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(h[j]);
+        sum.x += f.x + f.y;
+        sum.y += f.x * f.x + f.y * f.y;
+    }
+}
+__device__ __forceinline__ uint4 normalised(const uint4& v, float mean, float rstd)
+{
+    const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+    uint32_t              o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 f = __bfloat1622float2(h[j]);
+        o[j]           = fu::ptx::pack_bf16x2((f.x - mean) * rstd, (f.y - mean) * rstd);
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+// UNITS: of a lane, 0 for rows of any length.
+template <int UNITS>
 __global__ void __launch_bounds__(256) layernorm_fwd_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, float* stats,
-                                                            int64_t rows, int64_t cols, int64_t ldx, int64_t ldy, float eps)
+                                                            int64_t rows, int64_t cols, int64_t ldx, int64_t ldy, float eps,
+                                                            int warps)
 {
     fu::ptx::grid_wait();
     fu::ptx::grid_trigger();
-    const int     lane = threadIdx.x & 31;
-    const int64_t row  = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (row >= rows) {
+    const RowPlace       at(warps);
+    const bool           here = at.row < rows;
+    const __nv_bfloat16* xr   = x + at.row * ldx;
+    __nv_bfloat16*       yr   = y + at.row * ldy;
+    uint4                v[UNITS > 0 ? UNITS : 1];
+    float2               sum = make_float2(0.0f, 0.0f);
+    if (UNITS > 0) {
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            const int c = at.col + u * at.stride;
+            v[u]        = here && c < cols ? fu::ptx::ld_once_v4(xr + c) : make_uint4(0u, 0u, 0u, 0u);
+        }
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            add_moments(v[u], sum);
+        }
+    }
+    else if (here) {
+        for (int64_t c = at.col; c < cols; c += at.stride) {
+            add_moments(fu::ptx::ld_v4(xr + c), sum);
+        }
+    }
+    sum              = sum_of_warps(sum, warps);
+    const float mean = sum.x / static_cast<float>(cols);
+    const float rstd = rsqrtf(fmaxf(sum.y / static_cast<float>(cols) - mean * mean, 0.f) + eps);
+    if (!here) {
         return;
     }
-    const __nv_bfloat16* xr = x + row * ldx;
-    float                s = 0.f, ss = 0.f;
-    for (int64_t c = lane * 8; c < cols; c += 256) {
-        const uint4           v = *reinterpret_cast<const uint4*>(xr + c);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
+    if (at.leads && stats) {
+        stats[2 * at.row]     = mean;
+        stats[2 * at.row + 1] = rstd;
+    }
+    if (UNITS > 0) {
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(h[j]);
-            s += f.x + f.y;
-            ss += f.x * f.x + f.y * f.y;
+        for (int u = 0; u < UNITS; ++u) {
+            const int c = at.col + u * at.stride;
+            if (c < cols) {
+                fu::ptx::st_v4(yr + c, normalised(v[u], mean, rstd));
+            }
         }
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, off);
-        ss += __shfl_xor_sync(0xffffffffu, ss, off);
-    }
-    const float mean = s / static_cast<float>(cols);
-    const float rstd = rsqrtf(fmaxf(ss / static_cast<float>(cols) - mean * mean, 0.f) + eps);
-    if (lane == 0 && stats) {
-        stats[2 * row]     = mean;
-        stats[2 * row + 1] = rstd;
-    }
-    __nv_bfloat16* yr = y + row * ldy;
-    for (int64_t c = lane * 8; c < cols; c += 256) {
-        const uint4           v = *reinterpret_cast<const uint4*>(xr + c);
-        const __nv_bfloat162* h = reinterpret_cast<const __nv_bfloat162*>(&v);
-        uint32_t              o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 f = __bfloat1622float2(h[j]);
-            o[j]           = fu::ptx::pack_bf16x2((f.x - mean) * rstd, (f.y - mean) * rstd);
+    else {
+        for (int64_t c = at.col; c < cols; c += at.stride) {
+            fu::ptx::st_v4(yr + c, normalised(fu::ptx::ld_v4(xr + c), mean, rstd));
         }
-        *reinterpret_cast<uint4*>(yr + c) = make_uint4(o[0], o[1], o[2], o[3]);
     }
 }
 
+__device__ __forceinline__ void add_products(const uint4& xv, const uint4& gv, float mean, float rstd, float2& sum)
+{
+    const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xv);
+    const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&gv);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 xf = __bfloat1622float2(xh[j]), gf = __bfloat1622float2(gh[j]);
+        sum.x += gf.x + gf.y;
+        sum.y += gf.x * (xf.x - mean) * rstd + gf.y * (xf.y - mean) * rstd;
+    }
+}
+// `mg`, `mgx`: the row's means of the gradient and of its product with the normalised value; `av` is added where `add` says so
+__device__ __forceinline__ uint4 norm_gradient(const uint4& xv, const uint4& gv, const uint4& av, bool add, float mean, float rstd, float mg,
+                                               float mgx)
+{
+    const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&av);
+    const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xv);
+    const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&gv);
+    uint32_t              o[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const float2 xf = __bfloat1622float2(xh[j]), gf = __bfloat1622float2(gh[j]);
+        float2       d  = make_float2(rstd * (gf.x - mg - (xf.x - mean) * rstd * mgx),
+                                      rstd * (gf.y - mg - (xf.y - mean) * rstd * mgx));
+        if (add) {
+            const float2 af = __bfloat1622float2(ah[j]);
+            d.x += af.x;
+            d.y += af.y;
+        }
+        o[j] = fu::ptx::pack_bf16x2(d.x, d.y);
+    }
+    return make_uint4(o[0], o[1], o[2], o[3]);
+}
+
+template <int UNITS>
 __global__ void __launch_bounds__(256) layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
                                                             const float* stats, const __nv_bfloat16* add,
-                                                            __nv_bfloat16* dx, int64_t rows, int64_t cols, int64_t ld)
+                                                            __nv_bfloat16* dx, int64_t rows, int64_t cols, int64_t ld, int warps)
 {
     fu::ptx::grid_wait();
     fu::ptx::grid_trigger();
-    const int     lane = threadIdx.x & 31;
-    const int64_t row  = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-    if (row >= rows) {
+    const RowPlace       at(warps);
+    const bool           here = at.row < rows;
+    const __nv_bfloat16 *xr = x + at.row * ld, *gr = dy + at.row * ld, *ar = add + at.row * ld;
+    __nv_bfloat16*       dr   = dx + at.row * ld;
+    const float          mean = here ? stats[2 * at.row] : 0.0f, rstd = here ? stats[2 * at.row + 1] : 0.0f;
+    const uint4          none = make_uint4(0u, 0u, 0u, 0u);
+    constexpr int        N    = UNITS > 0 ? UNITS : 1;
+    uint4                xv[N], gv[N];
+    float2               sum = make_float2(0.0f, 0.0f);
+    if (UNITS > 0) {
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            const int c = at.col + u * at.stride;
+            xv[u] = gv[u] = none;
+            if (here && c < cols) {
+                xv[u] = fu::ptx::ld_once_v4(xr + c);
+                gv[u] = fu::ptx::ld_once_v4(gr + c);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            add_products(xv[u], gv[u], mean, rstd, sum);  // a gradient of zero beyond the last column
+        }
+    }
+    else if (here) {
+        for (int64_t c = at.col; c < cols; c += at.stride) {
+            add_products(fu::ptx::ld_v4(xr + c), fu::ptx::ld_v4(gr + c), mean, rstd, sum);
+        }
+    }
+    sum            = sum_of_warps(sum, warps);
+    const float mg = sum.x / static_cast<float>(cols), mgx = sum.y / static_cast<float>(cols);
+    if (!here) {
         return;
     }
-    const float          mean = stats[2 * row], rstd = stats[2 * row + 1];
-    const __nv_bfloat16* xr = x + row * ld;
-    const __nv_bfloat16* gr = dy + row * ld;
-    float                sg = 0.f, sgx = 0.f;
-    for (int64_t c = lane * 8; c < cols; c += 256) {
-        const uint4           xv = *reinterpret_cast<const uint4*>(xr + c);
-        const uint4           gv = *reinterpret_cast<const uint4*>(gr + c);
-        const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xv);
-        const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&gv);
+    if (UNITS > 0) {
+        uint4 av[N];  // not earlier: its registers would cost rows under way
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 xf = __bfloat1622float2(xh[j]), gf = __bfloat1622float2(gh[j]);
-            sg += gf.x + gf.y;
-            sgx += gf.x * (xf.x - mean) * rstd + gf.y * (xf.y - mean) * rstd;
+        for (int u = 0; u < UNITS; ++u) {
+            const int c = at.col + u * at.stride;
+            av[u]       = add && c < cols ? fu::ptx::ld_once_v4(ar + c) : none;
         }
-    }
 #pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        sg += __shfl_xor_sync(0xffffffffu, sg, off);
-        sgx += __shfl_xor_sync(0xffffffffu, sgx, off);
-    }
-    const float mg = sg / static_cast<float>(cols), mgx = sgx / static_cast<float>(cols);
-    __nv_bfloat16* dr = dx + row * ld;
-    for (int64_t c = lane * 8; c < cols; c += 256) {
-        const uint4           xv = *reinterpret_cast<const uint4*>(xr + c);
-        const uint4           gv = *reinterpret_cast<const uint4*>(gr + c);
-        uint4                 av = make_uint4(0u, 0u, 0u, 0u);
-        if (add) {
-            av = *reinterpret_cast<const uint4*>(add + row * ld + c);
-        }
-        const __nv_bfloat162* ah = reinterpret_cast<const __nv_bfloat162*>(&av);
-        const __nv_bfloat162* xh = reinterpret_cast<const __nv_bfloat162*>(&xv);
-        const __nv_bfloat162* gh = reinterpret_cast<const __nv_bfloat162*>(&gv);
-        uint32_t              o[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const float2 xf = __bfloat1622float2(xh[j]), gf = __bfloat1622float2(gh[j]);
-            float2       d  = make_float2(rstd * (gf.x - mg - (xf.x - mean) * rstd * mgx),
-                                          rstd * (gf.y - mg - (xf.y - mean) * rstd * mgx));
-            if (add) {
-                const float2 af = __bfloat1622float2(ah[j]);
-                d.x += af.x;
-                d.y += af.y;
+        for (int u = 0; u < UNITS; ++u) {
+            const int c = at.col + u * at.stride;
+            if (c < cols) {
+                fu::ptx::st_v4(dr + c, norm_gradient(xv[u], gv[u], av[u], add != nullptr, mean, rstd, mg, mgx));
             }
-            o[j] = fu::ptx::pack_bf16x2(d.x, d.y);
         }
-        *reinterpret_cast<uint4*>(dr + c) = make_uint4(o[0], o[1], o[2], o[3]);
+    }
+    else {
+        for (int64_t c = at.col; c < cols; c += at.stride) {
+            const uint4 a = add ? fu::ptx::ld_v4(ar + c) : none;
+            fu::ptx::st_v4(dr + c, norm_gradient(fu::ptx::ld_v4(xr + c), fu::ptx::ld_v4(gr + c), a, add != nullptr, mean, rstd, mg, mgx));
+        }
     }
 }
+
+// Values of a matrix beyond which the backward's four (x, dy, the residual's gradient, dx) are more than L2 holds.
+constexpr int64_t kNormInL2 = 12ll << 20;
+
+// As few warps a row as its units allow, so that little rows need no meeting through shared memory.
+struct RowShape {
+    int      warps, units;  // units: 0 for rows that no eight warps hold
+    unsigned blocks;
+    RowShape(int64_t rows, int64_t cols)
+    {
+        const int64_t pieces = cols / 8;
+        for (warps = 1; warps < 8 && pieces > 32 * warps * kRowUnits;) {
+            warps *= 2;
+        }
+        const int64_t each = (pieces + 32 * warps - 1) / (32 * warps);
+        units              = each <= kRowUnits ? static_cast<int>(each) : 0;
+        blocks             = static_cast<unsigned>((rows + 8 / warps - 1) / (8 / warps));
+    }
+};
 
 // ---- column sums (bias gradients) --------------------------------------------------------------------------
 // A cluster of eight CTAs owns 64 columns and splits the rows; a warp reads four rows of 128 bytes per
@@ -667,9 +805,12 @@ extern "C" int fu_layernorm_fwd(const void* x, void* y, float* stats, int64_t ro
         || ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15u)) {
         return fu::fail(FU_E_ARG, "fu_layernorm_fwd: needs 16-byte aligned rows of a multiple of 8 columns");
     }
-    const unsigned blocks = static_cast<unsigned>((rows + 7) / 8);  // eight warps, one row each
-    FU_CUDA_OK(fu::launch_behind(layernorm_fwd_kernel, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
-                                 static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), stats, rows, cols, ldx, ldy, eps));
+    const RowShape shape(rows, cols);
+    decltype(&layernorm_fwd_kernel<0>) const kernels[kRowUnits + 1] = {layernorm_fwd_kernel<0>, layernorm_fwd_kernel<1>, layernorm_fwd_kernel<2>,
+                                                                       layernorm_fwd_kernel<3>, layernorm_fwd_kernel<4>, layernorm_fwd_kernel<5>};
+    FU_CUDA_OK(fu::launch_behind(kernels[shape.units], dim3(shape.blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                 static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), stats, rows, cols, ldx, ldy, eps,
+                                 shape.warps));
     return FU_OK;
 }
 
@@ -681,10 +822,15 @@ extern "C" int fu_layernorm_bwd_add(const void* dy, const void* x, const float* 
              | reinterpret_cast<uintptr_t>(add)) & 15u)) {
         return fu::fail(FU_E_ARG, "fu_layernorm_bwd_add: needs 16-byte aligned rows of a multiple of 8 columns");
     }
-    const unsigned blocks = static_cast<unsigned>((rows + 7) / 8);
-    FU_CUDA_OK(fu::launch_behind(layernorm_bwd_kernel, dim3(blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+    RowShape shape(rows, cols);
+    if (rows * cols > kNormInL2 && shape.units > 1) {
+        shape.units = 0;
+    }
+    decltype(&layernorm_bwd_kernel<0>) const kernels[kRowUnits + 1] = {layernorm_bwd_kernel<0>, layernorm_bwd_kernel<1>, layernorm_bwd_kernel<2>,
+                                                                       layernorm_bwd_kernel<3>, layernorm_bwd_kernel<4>, layernorm_bwd_kernel<5>};
+    FU_CUDA_OK(fu::launch_behind(kernels[shape.units], dim3(shape.blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
                                  static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
-                                 static_cast<const __nv_bfloat16*>(add), static_cast<__nv_bfloat16*>(dx), rows, cols, ld));
+                                 static_cast<const __nv_bfloat16*>(add), static_cast<__nv_bfloat16*>(dx), rows, cols, ld, shape.warps));
     return FU_OK;
 }
 

@@ -3,7 +3,7 @@
 import pytest
 import torch
 
-from fast_ulysses_b200.ops.norm import layer_norm
+from fast_ulysses_b200.ops.norm import layer_norm, layer_norm_fork
 
 pytestmark = pytest.mark.gpu
 
@@ -33,3 +33,21 @@ def test_layer_norm_reads_a_row_strided_view_in_place():
     y = layer_norm(x)
     want = torch.nn.functional.layer_norm(x.float(), (256,), eps=1e-6)
     assert rel_err(y, want) < 1e-2
+
+
+# one unit a lane to five with one warp a row, the last column beyond; the same with two, four and eight warps; rows that are
+# walked through; a matrix beyond L2; last CTAs with rows missing
+@pytest.mark.parametrize("rows, cols", [(1, 8), (9, 256), (7, 264), (17, 1280), (3, 1288), (5, 2560), (3, 2568), (7, 5120), (3, 5128), (2, 10240),
+                                        (3, 10248), (2, 20000), (2501, 5120), (9831, 1288)])
+def test_layer_norm_rows_of_every_form(rows, cols):
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x, g, r = (torch.randn(rows, cols, device="cuda", generator=gen).mul_(2).add_(0.5).bfloat16() for _ in range(3))
+    x.requires_grad_()
+    y, past = layer_norm_fork(x)
+    torch.autograd.backward((y, past), (g, r))
+    xr = x.detach().double().requires_grad_()
+    yr = torch.nn.functional.layer_norm(xr, (cols,), eps=1e-6)
+    torch.autograd.backward((yr, xr * 1), (g.double(), r.double()))
+    for got, want in ((y.detach(), yr.detach()), (x.grad, xr.grad)):
+        # one rounding to bf16 (2^-9 of the value) and fp32 sums of values of a few units
+        assert ((got.double() - want).abs() <= 2**-8 * want.abs() + 1e-4).all()
