@@ -693,6 +693,8 @@ int pair_capacity()
 // rows, 64 - 13824 columns and K, each timed in up to 24 shapes behind a launch of itself (us, SM clock 1.9 GHz), and checked on 240
 // others: the shape chosen takes 1.5 % more than the fastest one (geometric mean; 9 in 10 sizes less than 6 % more). With
 // the epilogue's time left out it was 5.4 %, with half of it for two blocks and launches of nothing but halves of tiles 4.4 %.
+// Since the producers look ahead, small tiles and narrow blocks on few SMs are faster than this says. Fitted again, 330 sizes took 0.6 %
+// less and 170 others 0.5, but of 1500 more, ten of 40 - 100 us, bound by L2 then, took 10 - 26 % more: left as it is.
 //   128 x 128 tiles on single CTAs   2.0 + 0.223 per K-block and wave of 148
 //   two 256 x 256 blocks on pairs    2.6 + 0.622 per K-block and wave of 74, and the epilogue of both
 //   one 256 x 256 block on pairs     2.6 + 0.328

@@ -9,7 +9,7 @@
 //   run         128 x 256 tiles on single CTAs, A gathered from the peers by extra warps while the GEMM runs
 //
 // In each, warp 0 is the TMA producer (128B-swizzled operand tiles into a ring of shared-memory
-// stages), warp 1 issues tcgen05.mma, and the other warps are the epilogue: they read the accumulator
+// stages; of one operand where run_wide has a warp for each), warp 1 issues tcgen05.mma, and the other warps are the epilogue: they read the accumulator
 // from tensor memory (each warp may touch one 32-lane quarter) and apply the epilogue functor. Tiles are
 // visited in bands of M-tiles so that a wave of CTAs shares operand tiles through L2. No TMA load is
 // multicast; every CTA fetches its own tiles. Kernels that write peers' memory from the epilogue run
@@ -270,7 +270,8 @@ constexpr int WIDE_STAGES      = 4;  // of 48 KiB; six of 32 KiB with one block 
 constexpr int WIDE_BLOCK_BYTES = 128 * BK * 2;  // 128 rows of one operand, one K-block
 constexpr int WIDE_STAGE_BYTES = 3 * WIDE_BLOCK_BYTES;
 constexpr int WIDE_EPI_WARPS   = 8;
-constexpr int WIDE_FIRST_EPI   = 4;  // warps 2 and 3 idle: they fill the first warpgroup, whose registers go to the others
+constexpr int WIDE_FIRST_EPI   = 4;  // warp 3 is idle: it fills the first warpgroup, whose registers go to the others
+constexpr int WIDE_B_WARP      = 2;  // the second operand's producer
 constexpr int WIDE_THREADS     = 32 * (WIDE_FIRST_EPI + WIDE_EPI_WARPS);
 constexpr int WIDE_REGS_LIGHT  = 88;   // 128 x 88 + 256 x 208 = the 384 x 168 of the launch
 constexpr int WIDE_REGS_EPI    = 208;  // a unit's 128 values, a row of loads in flight, addresses
@@ -398,9 +399,14 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
     ptx::setmaxnreg_dec<WIDE_REGS_LIGHT>();
     const uint32_t leader = ptx::elect_one();
     const uint32_t full_b = ptx::smem_addr(full), empty_b = ptx::smem_addr(empty);
-    if (warp == 0) {
-        uint32_t stage = 0, phase = 1;
-        bool     ok    = true;
+    // With one block, whose K-block's products may take no more than 192 clocks, each operand has a producer of its own, and both look
+    // at the next stage while they load this one: blocks of 128 and 96 columns 8 % faster on average, up to 30. Two blocks have
+    // 1024 clocks a K-block and lose 1 % so.
+    constexpr bool OPERAND_WARPS = MB * NB == 1;
+    if (warp == 0 || (OPERAND_WARPS && warp == WIDE_B_WARP)) {
+        const bool a_op = !OPERAND_WARPS || warp == 0, b_op = !OPERAND_WARPS || warp != 0;
+        uint32_t   stage = 0, phase = 1;
+        bool       ok = true, ready = false;
         // of an operand's 128 rows (or, stored the other way, two 64 x 64 blocks) B may need only a part
         const int      b_rows  = core.width / 2;
         const uint32_t b_bytes = core.b_mn ? (b_rows + 63) / 64 * 8192u : b_rows * 128u;
@@ -411,50 +417,55 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
             }
             const uint32_t bytes = (MB == 2 ? item.u1 - item.u0 : 1) * WIDE_BLOCK_BYTES + (NB == 2 ? item.u1 - item.u0 : 1) * b_bytes;
             for (int kb = 0; kb < kblocks; ++kb) {
-                if (!ptx::mbar_wait_warp(empty_b + stage * 8, phase)) {
+                if (!ready && !ptx::mbar_wait_warp(empty_b + stage * 8, phase)) {
                     ok = false;
                     break;
                 }
+                const uint32_t next = stage + 1 == STAGES ? 0 : stage + 1, next_phase = next == 0 ? phase ^ 1u : phase;
+                const uint32_t ahead = OPERAND_WARPS ? ptx::mbar_test(empty_b + next * 8, next_phase) : 0u;
                 const uint32_t sa = base + stage * STAGE_BYTES, sb = sa + MB * WIDE_BLOCK_BYTES, bar = full_b + stage * 8;
-                if (half == 0) {
-                    ptx::mbar_expect_tx_if(bar, 2 * bytes, leader);  // both CTAs' bytes
-                }
+                if (a_op) {
+                    if (half == 0) {
+                        ptx::mbar_expect_tx_if(bar, 2 * bytes, leader);  // both operands' bytes of both CTAs
+                    }
 #pragma unroll
-                for (int u = 0; u < MB; ++u) {
-                    if (MB == 2 && (u < item.u0 || u >= item.u1)) {
-                        continue;
-                    }
-                    const int      m  = item.m0 + u * 256 + half * 128;
-                    const uint32_t to = sa + u * WIDE_BLOCK_BYTES;
-                    if (!core.a_mn) {
-                        ptx::tma_load_2d_pair_if(to, &core.map_a, (kb_0 + kb) * BK, m, bar, leader);
-                    }
-                    else {  // 64 (k) x 64 (m) blocks of 8 KiB
-                        ptx::tma_load_2d_pair_if(to, &core.map_a, m, (kb_0 + kb) * BK, bar, leader);
-                        ptx::tma_load_2d_pair_if(to + 8192, &core.map_a, m + 64, (kb_0 + kb) * BK, bar, leader);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < NB; ++u) {
-                    if (NB == 2 && (u < item.u0 || u >= item.u1)) {
-                        continue;
-                    }
-                    const int      n  = item.col(u) + half * b_rows;
-                    const uint32_t to = sb + u * WIDE_BLOCK_BYTES;
-                    if (!core.b_mn) {
-                        ptx::tma_load_2d_pair_if(to, &core.map_b, (kb_0 + kb) * BK, n, bar, leader);
-                    }
-                    else {
-                        ptx::tma_load_2d_pair_if(to, &core.map_b, n, (kb_0 + kb) * BK, bar, leader);
-                        if (b_rows > 64) {
-                            ptx::tma_load_2d_pair_if(to + 8192, &core.map_b, n + 64, (kb_0 + kb) * BK, bar, leader);
+                    for (int u = 0; u < MB; ++u) {
+                        if (MB == 2 && (u < item.u0 || u >= item.u1)) {
+                            continue;
+                        }
+                        const int      m  = item.m0 + u * 256 + half * 128;
+                        const uint32_t to = sa + u * WIDE_BLOCK_BYTES;
+                        if (!core.a_mn) {
+                            ptx::tma_load_2d_pair_if(to, &core.map_a, (kb_0 + kb) * BK, m, bar, leader);
+                        }
+                        else {  // 64 (k) x 64 (m) blocks of 8 KiB
+                            ptx::tma_load_2d_pair_if(to, &core.map_a, m, (kb_0 + kb) * BK, bar, leader);
+                            ptx::tma_load_2d_pair_if(to + 8192, &core.map_a, m + 64, (kb_0 + kb) * BK, bar, leader);
                         }
                     }
                 }
-                if (++stage == STAGES) {
-                    stage = 0;
-                    phase ^= 1u;
+                if (b_op) {
+#pragma unroll
+                    for (int u = 0; u < NB; ++u) {
+                        if (NB == 2 && (u < item.u0 || u >= item.u1)) {
+                            continue;
+                        }
+                        const int      n  = item.col(u) + half * b_rows;
+                        const uint32_t to = sb + u * WIDE_BLOCK_BYTES;
+                        if (!core.b_mn) {
+                            ptx::tma_load_2d_pair_if(to, &core.map_b, (kb_0 + kb) * BK, n, bar, leader);
+                        }
+                        else {
+                            ptx::tma_load_2d_pair_if(to, &core.map_b, n, (kb_0 + kb) * BK, bar, leader);
+                            if (b_rows > 64) {
+                                ptx::tma_load_2d_pair_if(to + 8192, &core.map_b, n + 64, (kb_0 + kb) * BK, bar, leader);
+                            }
+                        }
+                    }
                 }
+                stage = next;
+                phase = next_phase;
+                ready = ptx::all_ready(ahead);
             }
         }
         if (!ok) {
@@ -730,16 +741,21 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
     const uint32_t full_b = ptx::smem_addr(full), empty_b = ptx::smem_addr(empty);
 
     if (warp == 0) {
+        // The next stage is looked at while this one's loads are issued: looked at only on coming to it, a K-block took the producer
+        // 390 clocks instead of 310, and the products take 256 (256 x 256 x 4096 15.5 -> 13.6 us, 120 x 5120 x 5120 14.8 -> 13.1). With a
+        // producer for each operand it is 270, but the seventh warp costs a launch 0.1 - 0.3 us: over 210 sizes nothing gained.
         uint32_t stage = 0, phase = 1;
-        bool     ok    = true;
+        bool     ok = true, ready = false;
         for (int t = t_0; t < tiles && ok; t += t_inc) {
             int mt, nt;
             pair_tile_coords(core.tiles_m, core.tiles_n, 16, t, mt, nt);
             for (int kb = kb_0; kb < kb_n; ++kb) {
-                if (!ptx::mbar_wait_warp(empty_b + stage * 8, phase)) {
+                if (!ready && !ptx::mbar_wait_warp(empty_b + stage * 8, phase)) {
                     ok = false;
                     break;
                 }
+                const uint32_t next = stage + 1 == SMALL_STAGES ? 0 : stage + 1, next_phase = next == 0 ? phase ^ 1u : phase;
+                const uint32_t ahead = ptx::mbar_test(empty_b + next * 8, next_phase);
                 const uint32_t sa = base + stage * SMALL_STAGE_BYTES, sb = sa + WIDE_BLOCK_BYTES, bar = full_b + stage * 8;
                 ptx::mbar_expect_tx_if(bar, SMALL_STAGE_BYTES, leader);
                 if (!core.a_mn) {
@@ -756,10 +772,9 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
                     ptx::tma_load_2d_if(sb, &core.map_b, nt * 128, kb * BK, bar, leader);
                     ptx::tma_load_2d_if(sb + 8192, &core.map_b, nt * 128 + 64, kb * BK, bar, leader);
                 }
-                if (++stage == SMALL_STAGES) {
-                    stage = 0;
-                    phase ^= 1u;
-                }
+                stage = next;
+                phase = next_phase;
+                ready = ptx::all_ready(ahead);
             }
         }
         if (!ok) {

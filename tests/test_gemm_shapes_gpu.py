@@ -174,3 +174,16 @@ def test_feed_forward_with_a_padded_hidden_layer(m, hidden, ffn):
     # the hidden layer and its gradient are rounded to bf16 on the way, and the results: 2^-9 each
     for got, want in zip((x, w1, b1, w2, b2), ref):
         assert rel_err(got.grad, want.grad) < 1e-2
+
+
+# K one block short of the ring of six, as long as it, one more, and twice round; a CTA's second tile begins where the first left the ring
+@pytest.mark.parametrize("k", [320, 384, 448, 768, 840])
+@pytest.mark.parametrize("a_km,b_kn", [(False, False), (False, True), (True, True)])
+def test_small_tiles_around_the_ring(k, a_km, b_kn):
+    m, n = 128 * 150, 136
+    gen = torch.Generator(device="cuda").manual_seed(k)
+    a, b = torch.randn(m, k, device="cuda", generator=gen).bfloat16(), torch.randn(n, k, device="cuda", generator=gen).bfloat16()
+    got = gemm.gemm_bf16(a.t().contiguous() if a_km else a, b.t().contiguous() if b_kn else b, a_km=a_km, b_kn=b_kn, pair=False)
+    gemm.check_errors()
+    assert rel_err(got, a.float() @ b.float().t()) < 4e-3  # bf16 rounding of the result, as above
+    assert torch.equal(got, gemm.gemm_bf16(a, b, pair=True))
