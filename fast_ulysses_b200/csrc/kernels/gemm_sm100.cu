@@ -153,6 +153,17 @@ struct PlainEpi {
         stage_out<W>(stage, c, ldc, row0, col0, M, N, lane);
     }
 
+    // Half a unit: a warp's share of a small tile.
+    __device__ __forceinline__ void unit(const uint32_t (&r)[64], int row0, int col0, int col_end, int lane, uint32_t stage) const
+    {
+        float v[64];
+#pragma unroll
+        for (int j = 0; j < 64; ++j) {
+            v[j] = __uint_as_float(r[j]);
+        }
+        piece<64>(v, row0, col0, min(N, col_end), lane, stage);
+    }
+
     __device__ __forceinline__ void unit(const uint32_t (&r)[128], int row0, int col0, int col_end, int lane, uint32_t stage) const
     {
         const int end = min(N, col_end);
@@ -195,17 +206,17 @@ __global__ void __launch_bounds__(WIDE_THREADS, 1) gemm_wide_split_kernel(const 
 }
 
 template <int ACT>
-__global__ void __launch_bounds__(SMALL_THREADS, 1) gemm_small_kernel(const __grid_constant__ PlainArgs<ACT> a)
+__global__ void __launch_bounds__(small_threads(64), 1) gemm_small_kernel(const __grid_constant__ PlainArgs<ACT> a)
 {
     PlainEpi<ACT> epi = a.epi;
-    run_small<false>(a.core, epi);
+    run_small<false, 64>(a.core, epi);
 }
 
 template <int ACT>
-__global__ void __launch_bounds__(SMALL_THREADS, 1) gemm_split_kernel(const __grid_constant__ PlainArgs<ACT> a)
+__global__ void __launch_bounds__(small_threads(128), 1) gemm_split_kernel(const __grid_constant__ PlainArgs<ACT> a)
 {
     PlainEpi<ACT> epi = a.epi;
-    run_small<true>(a.core, epi);
+    run_small<true, 128>(a.core, epi);
 }
 
 // ---- fused QKV epilogue: RMSNorm + 3D RoPE + scatter ---------------------------------------------------
@@ -409,10 +420,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(WIDE_THREADS, 1) qkv
     run_wide<MB, NB, false>(a.core, epi);
 }
 
-__global__ void __launch_bounds__(SMALL_THREADS, 1) qkv_small_kernel(const __grid_constant__ QkvArgs a)
+__global__ void __launch_bounds__(small_threads(128), 1) qkv_small_kernel(const __grid_constant__ QkvArgs a)
 {
-    QkvEpi<32 * SMALL_EPI_WARPS> epi(a.epi);
-    run_small<false>(a.core, epi);
+    QkvEpi<32 * small_epi_warps(128)> epi(a.epi);
+    run_small<false, 128>(a.core, epi);
 }
 
 // ---- fused mode-1 path: pull attention output from peers, feed the output projection -----------------
@@ -877,7 +888,7 @@ int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k, int off, E
         if ((kb + share - 1) / share != csize || once >= cost) {
             continue;  // a CTA would have nothing to do, or no gain even in one wave
         }
-        const int cap = capacity.of(gemm_split_kernel<0>, csize, dev, SMALL_THREADS, SMALL_SMEM_BYTES);
+        const int cap = capacity.of(gemm_split_kernel<0>, csize, dev, small_threads(128), small_smem_bytes(128));
         if (cap < 1) {
             continue;
         }
@@ -982,13 +993,13 @@ int launch_pairs(void (*kernel)(Args), const Args& a, int pairs, cudaStream_t st
 }
 
 template <class Args>
-int launch_small(void (*kernel)(Args), const Args& a, int ctas, cudaStream_t stream)
+int launch_small(void (*kernel)(Args), const Args& a, int cols, int ctas, cudaStream_t stream)
 {
-    const int rc = raise_smem_limit(kernel, SMALL_SMEM_BYTES);
+    const int rc = raise_smem_limit(kernel, small_smem_bytes(cols));
     if (rc != FU_OK) {
         return rc;
     }
-    FU_CUDA_OK(launch(kernel, dim3(static_cast<unsigned>(launch_grid(ctas, a.core.items))), dim3(SMALL_THREADS), SMALL_SMEM_BYTES, stream, a));
+    FU_CUDA_OK(launch(kernel, dim3(static_cast<unsigned>(launch_grid(ctas, a.core.items))), dim3(static_cast<unsigned>(small_threads(cols))), static_cast<size_t>(small_smem_bytes(cols)), stream, a));
     return FU_OK;
 }
 
@@ -1041,7 +1052,7 @@ int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream
     a.epi.aux       = static_cast<const __nv_bfloat16*>(g->aux);
     a.epi.c_pre     = static_cast<__nv_bfloat16*>(g->c_pre);
     if (csize > 1) {
-        return launch_clusters<ACT>(gemm_split_kernel<ACT>, a, a.core.items, csize, SMALL_THREADS, SMALL_SMEM_BYTES, stream);
+        return launch_clusters<ACT>(gemm_split_kernel<ACT>, a, a.core.items, csize, small_threads(128), small_smem_bytes(128), stream);
     }
     if (c.rest > 0) {
         a.core.first = c.items;
@@ -1053,7 +1064,7 @@ int launch_plain(const FuGemmArgs* g, Choice c, int pairs, int flags, cudaStream
     case Shape::kTall: return launch_pairs(gemm_wide_kernel<2, 1, ACT>, a, pairs, stream);
     case Shape::kBroad: return launch_pairs(gemm_wide_kernel<1, 2, ACT>, a, pairs, stream);
     case Shape::kOne: return launch_pairs(gemm_wide_kernel<1, 1, ACT>, a, pairs, stream);
-    default: return launch_small(gemm_small_kernel<ACT>, a, g->ctas, stream);
+    default: return launch_small(gemm_small_kernel<ACT>, a, 64, g->ctas, stream);
     }
 }
 
@@ -1236,7 +1247,7 @@ extern "C" int fu_qkv_rope_scatter(const FuQkvArgs* q, void* stream_v)
     case Shape::kTall: return launch_pairs(qkv_wide_kernel<2, 1>, a, pairs, stream);
     case Shape::kBroad: return launch_pairs(qkv_wide_kernel<1, 2>, a, pairs, stream);
     case Shape::kOne: return launch_pairs(qkv_wide_kernel<1, 1>, a, pairs, stream);
-    default: return launch_small(qkv_small_kernel, a, q->ctas, stream);
+    default: return launch_small(qkv_small_kernel, a, 128, q->ctas, stream);
     }
 }
 

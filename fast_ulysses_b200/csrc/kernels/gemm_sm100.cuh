@@ -228,10 +228,11 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src, Aux aux
 // Columns from `col_end` on are not the unit's. `stage` is the address of 4 KiB of shared memory of this warp's own (32 rows x 128 bytes).
 constexpr int UNIT_STAGE_BYTES = 32 * 128;
 
-__device__ __forceinline__ void load_unit(uint32_t taddr, uint32_t (&r)[128])
+template <int COLS>
+__device__ __forceinline__ void load_unit(uint32_t taddr, uint32_t (&r)[COLS])
 {
 #pragma unroll
-    for (int ch = 0; ch < 4; ++ch) {
+    for (int ch = 0; ch < COLS / 32; ++ch) {
         ptx::tmem_ld_32x32(taddr + ch * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[ch * 32]));
     }
     ptx::tmem_ld_wait();
@@ -689,13 +690,19 @@ __device__ __forceinline__ void run_wide(const WideCore& core, Epi& epi)
 // columns of the tile in the order of the CTAs, and each finishes and writes its columns.
 constexpr int SMALL_STAGES      = 6;
 constexpr int SMALL_STAGE_BYTES = 2 * WIDE_BLOCK_BYTES;
-constexpr int SMALL_EPI_WARPS   = 4;
-constexpr int SMALL_THREADS     = 32 * (2 + SMALL_EPI_WARPS);
-constexpr int SMALL_SMEM_BYTES  = SMALL_STAGES * SMALL_STAGE_BYTES + SMALL_EPI_WARPS * UNIT_STAGE_BYTES + 1024;
+// A warp of the epilogue takes 32 rows and `cols` columns of a tile. 64 where nothing speaks against it: a launch of one tile a CTA waits
+// for the whole epilogue. 78 products on single tiles 6 % faster than with 128, 68 x 13304 x 128 with the GELU's derivative 8.1 -> 6.2 us,
+// 2985 x 5360 x 480 with GELU 28.2 -> 22.6. 128 where a head is needed at once, and in clusters, whose CTAs have 64 columns or fewer
+// to finish and lose 0.2 us by the larger block.
+constexpr int small_epi_warps(int cols) { return 4 * 128 / cols; }
+constexpr int small_threads(int cols) { return 32 * (2 + small_epi_warps(cols)); }
+constexpr int small_smem_bytes(int cols) { return SMALL_STAGES * SMALL_STAGE_BYTES + small_epi_warps(cols) * UNIT_STAGE_BYTES + 1024; }
 
-template <bool SPLIT, class Epi>
+template <bool SPLIT, int COLS, class Epi>
 __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
 {
+    static_assert(!SPLIT || COLS == 128, "a warp finishes all of a CTA's columns of a shared tile");
+    constexpr int EPI_WARPS = small_epi_warps(COLS);
     extern __shared__ uint8_t smem_raw[];
     __shared__ uint64_t       full[SMALL_STAGES], empty[SMALL_STAGES], tmem_full[2], tmem_empty[2];
     __shared__ uint32_t       tmem_holder;
@@ -721,7 +728,7 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
         }
         for (int a = 0; a < 2; ++a) {
             ptx::mbar_init(&tmem_full[a], 1);
-            ptx::mbar_init(&tmem_empty[a], SMALL_EPI_WARPS);
+            ptx::mbar_init(&tmem_empty[a], EPI_WARPS);
         }
         ptx::mbar_fence_init();
     }
@@ -827,6 +834,7 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
     else {
         const int epi_warp = warp - 2;
         const int quarter  = warp & 3;
+        const int cg       = epi_warp >> 2;  // which COLS of the tile's columns
         const uint32_t stage = base + SMALL_STAGES * SMALL_STAGE_BYTES + epi_warp * UNIT_STAGE_BYTES;
         if (Epi::kPeers) {
             epi.open(threadIdx.x - 64);
@@ -836,7 +844,7 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
             const uint32_t acc = tcount & 1u;
             int            mt, nt;
             pair_tile_coords(core.tiles_m, core.tiles_n, 16, t, mt, nt);
-            epi.fetch(nt * 128 + (SPLIT ? crank * (128 / csize) : 0), lane);
+            epi.fetch(nt * 128 + (SPLIT ? crank * (128 / csize) : cg * COLS), lane);
             const bool ok = ptx::mbar_wait(&tmem_full[acc], (tcount >> 1) & 1u);
             if (!ok) {
                 flag_error(core.err, ERR_EPI_WAIT);
@@ -897,14 +905,14 @@ __device__ __forceinline__ void run_small(const WideCore& core, Epi& epi)
                 break;
             }
             ptx::tc_fence_after();
-            uint32_t r[128];
-            load_unit(tmem_base + acc * 128 + (static_cast<uint32_t>(quarter * 32) << 16), r);
+            uint32_t r[COLS];
+            load_unit(tmem_base + acc * 128 + cg * COLS + (static_cast<uint32_t>(quarter * 32) << 16), r);
             ptx::tc_fence_before();
             __syncwarp();
             if (lane == 0) {
                 ptx::mbar_arrive(&tmem_empty[acc]);
             }
-            epi.unit(r, mt * 128 + quarter * 32, nt * 128, nt * 128 + 128, lane, stage);
+            epi.unit(r, mt * 128 + quarter * 32, nt * 128 + cg * COLS, nt * 128 + (cg + 1) * COLS, lane, stage);
         }
         if (Epi::kPeers) {
             epi.close(threadIdx.x - 64);

@@ -187,3 +187,31 @@ def test_small_tiles_around_the_ring(k, a_km, b_kn):
     gemm.check_errors()
     assert rel_err(got, a.float() @ b.float().t()) < 4e-3  # bf16 rounding of the result, as above
     assert torch.equal(got, gemm.gemm_bf16(a, b, pair=True))
+
+
+# a tile's columns are shared by two epilogue warps of 64: the last tile ends inside the first one's, with it, inside the second one's
+@pytest.mark.parametrize("act", [0, 1, 2, 3])
+@pytest.mark.parametrize("n", [8, 56, 64, 72, 120, 128, 184, 200])
+def test_small_tiles_end_in_either_half(n, act):
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    m, k = 150, 136
+    a, b = torch.randn(m, k, device="cuda", generator=gen).bfloat16(), torch.randn(n, k, device="cuda", generator=gen).bfloat16()
+    bias = torch.randn(n, device="cuda", generator=gen)
+    res, aux = (torch.randn(m, n, device="cuda", generator=gen).bfloat16() for _ in range(2))
+    pitch, kw = n + 24, {}
+    if act == 3:
+        kw["aux"] = torch.empty(m, pitch, device="cuda", dtype=torch.bfloat16)[:, :n].copy_(aux)
+    buf, pre = (torch.full((m, pitch), 7.0, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+    residual = torch.empty(m, pitch, device="cuda", dtype=torch.bfloat16)[:, :n].copy_(res)
+    got = gemm.gemm_bf16(a, b, bias=bias, residual=residual, act=act, out=buf[:, :n], store_pre=pre[:, :n], pair=False, **kw)
+    gemm.check_errors()
+    assert (buf[:, n:] == 7.0).all() and (pre[:, n:] == 7.0).all()
+    y = a.double() @ b.double().t() + bias.double()
+    assert rel_err(pre[:, :n], y.float()) < 4e-3
+    if act == 3:
+        x = aux.double().requires_grad_()
+        torch.nn.functional.gelu(x, approximate="tanh").sum().backward()
+        y = y * x.grad
+    elif act:
+        y = torch.nn.functional.gelu(y, approximate="tanh" if act == 1 else "none")
+    assert rel_err(got, (y + res.double()).float()) < 4e-3  # bf16 rounding of the result, as above
