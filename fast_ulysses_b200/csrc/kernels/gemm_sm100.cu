@@ -748,21 +748,24 @@ double block_clocks(int mb, int nb, int width)
 
 // us per K-block, by how many of the two operands lie off the 32-byte sectors
 constexpr double kSmallBlock[3] = {0.223, 0.27, 0.38}, kOneBlock[3] = {0.328, 0.34, 0.42}, kTwoBlocks[3] = {0.622, 0.65, 0.73};
-constexpr double kSmallStart = 2.0, kPairStart = 2.6, kLong = 50.0;
+constexpr double kSmallStart = 2.0, kPairStart = 2.6, kLong = 50.0, kShortK = 16.0;
 
-// us that the epilogue of a block of 256 columns and of a 128 x 128 tile takes
+// us that the epilogue of a block of 256 columns takes, of a 128 x 128 tile with eight warps and with four, which share it in clusters.
+// The eight warps' figure stands up to kShortK blocks of K, where the epilogue decides: of 1500 products of 64 - 9000 rows the 54 with
+// GELU or SiLU whose shape it changes take up to 25 % less (6043 x 5432 x 384: 85.8 -> 63.7 us) and none more. Used for every K it took
+// products of 29 - 90 blocks, where small tiles read more of L2 than is counted here, 11 - 23 % longer (99 x 11456 x 4696: 31.5 -> 37.4).
 struct Epilogue {
-    double pair, small;
+    double pair, small, shared;
     // A warp's share of a narrow block is half a unit, or more of it in pieces that are not whole.
     double block(int width) const { return width > 128 ? pair : 0.59 * pair; }
 };
 // Whether the pre-activation is saved (0.9 more) is left out: a forward pass has the same bits with gradients and without.
 Epilogue epilogue_of(int act, bool residual)
 {
-    const double pair[4] = {2.4, 4.7, 7.3, 7.0}, small[4] = {1.4, 3.2, 6.4, 5.5};
-    return {pair[act] + (residual ? 1.7 : 0.0), small[act] + (residual ? 1.0 : 0.0)};
+    const double pair[4] = {2.4, 4.7, 7.3, 7.0}, small[4] = {1.4, 2.2, 4.4, 3.5}, shared[4] = {1.4, 3.2, 6.4, 5.5};
+    return {pair[act] + (residual ? 1.7 : 0.0), small[act] + (residual ? 1.0 : 0.0), shared[act] + (residual ? 1.0 : 0.0)};
 }
-constexpr Epilogue kQkvEpilogue{7.0, 4.0};  // fitted to 100 projections of 64 - 75600 rows, 1 - 40 heads: 0.9 % above the fastest shape
+constexpr Epilogue kQkvEpilogue{7.0, 4.0, 4.0};  // fitted to 100 projections of 64 - 75600 rows, 1 - 40 heads: 0.9 % above the fastest shape
 
 // Waves of single blocks: an epilogue runs beside the next products and they delay it.
 double alternating(double products, double epilogue, int64_t waves)
@@ -798,8 +801,9 @@ Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int fla
     const int64_t t128 = ((m + 127) / 128) * ((n + 127) / 128);
     const double  kb   = static_cast<double>((k + BK - 1) / BK);
     const double  products = kSmallBlock[off] * kb, waves = static_cast<double>((t128 + sms - 1) / sms);
+    const double  end = kb <= kShortK ? epi.small : epi.shared;
     const Choice  small{Shape::kSmall, static_cast<int>((m + 127) / 128), static_cast<int>((n + 127) / 128), 0, static_cast<int>(t128),
-                       kSmallStart + products + (waves - 1.0) * std::max(products + 0.35 * epi.small, epi.small) + epi.small};
+                       kSmallStart + products + (waves - 1.0) * std::max(products + 0.35 * end, end) + end};
     if (flags & FU_GEMM_SINGLE) {
         return small;
     }
@@ -884,7 +888,7 @@ int choose_split(const Choice& best, int64_t m, int64_t n, int64_t k, int off, E
     }
     for (const int csize : {2, 4, 8}) {
         const int64_t share = (kb + csize - 1) / csize;
-        const double  once  = kSmallStart + (csize == 2 ? 2.9 : csize == 4 ? 3.2 : 3.5) + kSmallBlock[off] * share + epi.small / csize;
+        const double  once  = kSmallStart + (csize == 2 ? 2.9 : csize == 4 ? 3.2 : 3.5) + kSmallBlock[off] * share + epi.shared / csize;
         if ((kb + share - 1) / share != csize || once >= cost) {
             continue;  // a CTA would have nothing to do, or no gain even in one wave
         }
