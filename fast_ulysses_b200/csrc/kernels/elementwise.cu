@@ -377,7 +377,9 @@ __global__ void __launch_bounds__(256) layernorm_bwd_kernel(const __nv_bfloat16*
         }
 #pragma unroll
         for (int u = 0; u < UNITS; ++u) {
-            add_products(xv[u], gv[u], mean, rstd, sum);  // a gradient of zero beyond the last column
+            // Beyond the last column, which only the last unit reaches, 0 x (0 - 0): against a mean that has overflowed it would be NaN.
+            const bool inside = u + 1 < UNITS || at.col + u * at.stride < cols;
+            add_products(xv[u], gv[u], inside ? mean : 0.0f, inside ? rstd : 0.0f, sum);
         }
     }
     else if (here) {

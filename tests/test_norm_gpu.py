@@ -51,3 +51,12 @@ def test_layer_norm_rows_of_every_form(rows, cols):
     for got, want in ((y.detach(), yr.detach()), (x.grad, xr.grad)):
         # one rounding to bf16 (2^-9 of the value) and fp32 sums of values of a few units
         assert ((got.double() - want).abs() <= 2**-8 * want.abs() + 1e-4).all()
+
+
+# a mean that has overflowed: -inf in every column, whether or not the row fills its lanes
+@pytest.mark.parametrize("cols", [256, 264, 1288, 5128, 10248])
+def test_layer_norm_backward_of_an_overflowed_mean(cols):
+    x = torch.full((3, cols), 3e38, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+    y = layer_norm(x)
+    y.backward(torch.ones_like(y))
+    assert (x.grad == float("-inf")).all()
