@@ -186,12 +186,14 @@ __global__ void __launch_bounds__(256) qk_norm_rope_bwd_kernel(const NormRopeBwd
 
 // ---- LayerNorm without affine parameters ----------------------------------------------------------------
 // A row is read once and stays in the registers of 1, 2, 4 or 8 warps, up to kRowUnits 16-byte units a lane, all of them on
-// their way at once; statistics in fp32. Bound by HBM. With one warp per row, which read it twice in a chain of short loops, forward
-// 75600 x 5120 (1.55 GB) 338 -> 260 us, 7800 x 5120 38 -> 30, 320 x 4096 4.8 -> 2.5. The backward of what L2 does not hold is walked
-// through twice by the same warps, with a third of the registers and three times the rows under way (its second pass finds the row
-// in L1): 75600 x 5120 (3.1 GB) 701 -> 474 us, in registers 561; 12000 x 1280 23.7 -> 23.0 and 24.7. What L2 holds is faster in
-// registers: 4000 x 2560 21.3 -> 13.1 and 15.0, 1500 x 5120 15.2 -> 10.1 and 11.1, and rows of one unit are: 100000 x 256 39.7 -> 38.2
-// and 44.7. Rows too long for the registers of eight warps are walked through twice: 2000 x 16384 54 -> 25 and 122 -> 51.
+// their way at once; statistics in fp32. Bound by HBM, and where L2 holds the matrix by what a CTA does before its first load: how many
+// warps a row has is known when the kernel is compiled. With the number passed to the kernel, its divisions and the addresses they hold
+// up took forward 75600 x 5120 (1.55 GB) from 230 us to 292, x 1536 from 70 to 87, 9450 x 1024 from 5.5 to 6.5; one warp for every row,
+// which read it twice in a chain of short loops, took 342, 73 and 6.1. The backward that adds a gradient to rows of a matrix that L2 does
+// not hold walks through them twice with the same warps and a third of the registers, so with three times the rows under way (its
+// second pass finds the row in L1): 75600 x 5120 (3.1 GB) 488 us, in registers 576, one warp for every row 720. Without a gradient to add
+// registers are faster (402 and 412, 574), and where L2 holds all of it (4000 x 2560 12.2 and 14.5, 20.9). Rows too long for the
+// registers of eight warps are walked through twice as well: 2000 x 16384 54 -> 25 and 122 -> 51.
 constexpr int kRowUnits = 5;
 
 __device__ __forceinline__ float2 sum_of_warp(float2 v)
@@ -204,20 +206,21 @@ __device__ __forceinline__ float2 sum_of_warp(float2 v)
     return v;
 }
 
-// The sums over the `warps` warps of a row, in their order. (All threads of the CTA.)
-__device__ __forceinline__ float2 sum_of_warps(float2 v, int warps)
+// The sums over the WARPS warps of a row, in their order. (All threads of the CTA.)
+template <int WARPS>
+__device__ __forceinline__ float2 sum_of_warps(float2 v)
 {
-    __shared__ float2 part[8];
     v = sum_of_warp(v);
-    if (warps > 1) {
-        const int warp = threadIdx.x >> 5;
+    if (WARPS > 1) {
+        __shared__ float2 part[8];
+        const int         warp = threadIdx.x >> 5, first = warp & ~(WARPS - 1);
         if ((threadIdx.x & 31) == 0) {
             part[warp] = v;
         }
         __syncthreads();
-        const int first = warp & ~(warps - 1);
-        v               = part[first];
-        for (int w = 1; w < warps; ++w) {
+        v = part[first];
+#pragma unroll
+        for (int w = 1; w < WARPS; ++w) {
             v.x += part[first + w].x;
             v.y += part[first + w].y;
         }
@@ -226,16 +229,32 @@ __device__ __forceinline__ float2 sum_of_warps(float2 v, int warps)
 }
 
 // Where a thread works: its row and its first column of every `stride` columns.
+template <int WARPS>
 struct RowPlace {
-    int64_t row;
-    int     col, stride;
-    bool    leads;
-    __device__ __forceinline__ explicit RowPlace(int warps)
-        : row(static_cast<int64_t>(blockIdx.x) * (8 / warps) + (threadIdx.x >> 5) / warps), col((threadIdx.x & (32 * warps - 1)) * 8),
-          stride(256 * warps), leads(col == 0)
+    static constexpr int stride = 256 * WARPS;
+    int64_t              row;
+    int                  col;
+    bool                 leads;
+    __device__ __forceinline__ RowPlace()
+        : row(static_cast<int64_t>(blockIdx.x) * (8 / WARPS) + (threadIdx.x >> 5) / WARPS), col((threadIdx.x & (32 * WARPS - 1)) * 8),
+          leads(col == 0)
     {
     }
 };
+
+// The loaded values, not what was made of them for the sums, wait for the row's sums. It costs their conversion a second time and pays
+// where the registers would keep a CTA away: backward without a gradient to add 75600 x 1024 91.1 -> 74.9 us, x 3584 345 -> 290.
+// With five units there is none to gain (75600 x 1280 98.9 -> 105.8), with three only for rows of several warps (x 3072 250 -> 238).
+__device__ __forceinline__ void keep_packed(uint4& v)
+{
+    asm volatile("" : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w));
+}
+constexpr bool keeps_packed(int warps, int units) { return units == 4 || (units == 3 && warps > 1); }
+
+__device__ __forceinline__ uint4 ld_unit(const __nv_bfloat16* p)
+{
+    return *reinterpret_cast<const uint4*>(p);
+}
 
 __device__ __forceinline__ void add_moments(const uint4& v, float2& sum)
 {
@@ -259,20 +278,20 @@ __device__ __forceinline__ uint4 normalised(const uint4& v, float mean, float rs
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// UNITS: of a lane, 0 for rows of any length.
-template <int UNITS>
-__global__ void __launch_bounds__(256) layernorm_fwd_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, float* stats,
-                                                            int64_t rows, int64_t cols, int64_t ldx, int64_t ldy, float eps,
-                                                            int warps)
+// UNITS: of a lane, 0 for rows of any length. The registers of three units with several warps, 45, are one too many for a sixth CTA
+// (75600 x 1288 65.8 -> 64.3 us, 9450 x 2568 16.6 -> 15.8).
+template <int WARPS, int UNITS>
+__global__ void __launch_bounds__(256, WARPS > 1 && UNITS == 3 ? 6 : 0)
+    layernorm_fwd_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, float* stats, int64_t rows, int64_t cols, int64_t ldx, int64_t ldy, float eps)
 {
     fu::ptx::grid_wait();
     fu::ptx::grid_trigger();
-    const RowPlace       at(warps);
-    const bool           here = at.row < rows;
-    const __nv_bfloat16* xr   = x + at.row * ldx;
-    __nv_bfloat16*       yr   = y + at.row * ldy;
-    uint4                v[UNITS > 0 ? UNITS : 1];
-    float2               sum = make_float2(0.0f, 0.0f);
+    const RowPlace<WARPS> at;
+    const bool            here = at.row < rows;
+    const __nv_bfloat16*  xr   = x + at.row * ldx;
+    __nv_bfloat16*        yr   = y + at.row * ldy;
+    uint4                 v[UNITS > 0 ? UNITS : 1];
+    float2                sum = make_float2(0.0f, 0.0f);
     if (UNITS > 0) {
 #pragma unroll
         for (int u = 0; u < UNITS; ++u) {
@@ -286,10 +305,10 @@ __global__ void __launch_bounds__(256) layernorm_fwd_kernel(const __nv_bfloat16*
     }
     else if (here) {
         for (int64_t c = at.col; c < cols; c += at.stride) {
-            add_moments(fu::ptx::ld_v4(xr + c), sum);
+            add_moments(ld_unit(xr + c), sum);
         }
     }
-    sum              = sum_of_warps(sum, warps);
+    sum              = sum_of_warps<WARPS>(sum);
     const float mean = sum.x / static_cast<float>(cols);
     const float rstd = rsqrtf(fmaxf(sum.y / static_cast<float>(cols) - mean * mean, 0.f) + eps);
     if (!here) {
@@ -310,7 +329,7 @@ __global__ void __launch_bounds__(256) layernorm_fwd_kernel(const __nv_bfloat16*
     }
     else {
         for (int64_t c = at.col; c < cols; c += at.stride) {
-            fu::ptx::st_v4(yr + c, normalised(fu::ptx::ld_v4(xr + c), mean, rstd));
+            fu::ptx::st_v4(yr + c, normalised(ld_unit(xr + c), mean, rstd));
         }
     }
 }
@@ -349,22 +368,22 @@ __device__ __forceinline__ uint4 norm_gradient(const uint4& xv, const uint4& gv,
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-template <int UNITS>
+template <int WARPS, int UNITS>
 __global__ void __launch_bounds__(256) layernorm_bwd_kernel(const __nv_bfloat16* dy, const __nv_bfloat16* x,
                                                             const float* stats, const __nv_bfloat16* add,
-                                                            __nv_bfloat16* dx, int64_t rows, int64_t cols, int64_t ld, int warps)
+                                                            __nv_bfloat16* dx, int64_t rows, int64_t cols, int64_t ld)
 {
     fu::ptx::grid_wait();
     fu::ptx::grid_trigger();
-    const RowPlace       at(warps);
-    const bool           here = at.row < rows;
-    const __nv_bfloat16 *xr = x + at.row * ld, *gr = dy + at.row * ld, *ar = add + at.row * ld;
-    __nv_bfloat16*       dr   = dx + at.row * ld;
-    const float          mean = here ? stats[2 * at.row] : 0.0f, rstd = here ? stats[2 * at.row + 1] : 0.0f;
-    const uint4          none = make_uint4(0u, 0u, 0u, 0u);
-    constexpr int        N    = UNITS > 0 ? UNITS : 1;
-    uint4                xv[N], gv[N];
-    float2               sum = make_float2(0.0f, 0.0f);
+    const RowPlace<WARPS> at;
+    const bool            here = at.row < rows;
+    const __nv_bfloat16 * xr = x + at.row * ld, *gr = dy + at.row * ld, *ar = add + at.row * ld;
+    __nv_bfloat16*        dr   = dx + at.row * ld;
+    const float           mean = here ? stats[2 * at.row] : 0.0f, rstd = here ? stats[2 * at.row + 1] : 0.0f;
+    const uint4           none = make_uint4(0u, 0u, 0u, 0u);
+    constexpr int         N    = UNITS > 0 ? UNITS : 1;
+    uint4                 xv[N], gv[N];
+    float2                sum = make_float2(0.0f, 0.0f);
     if (UNITS > 0) {
 #pragma unroll
         for (int u = 0; u < UNITS; ++u) {
@@ -384,10 +403,17 @@ __global__ void __launch_bounds__(256) layernorm_bwd_kernel(const __nv_bfloat16*
     }
     else if (here) {
         for (int64_t c = at.col; c < cols; c += at.stride) {
-            add_products(fu::ptx::ld_v4(xr + c), fu::ptx::ld_v4(gr + c), mean, rstd, sum);
+            add_products(ld_unit(xr + c), ld_unit(gr + c), mean, rstd, sum);
         }
     }
-    sum            = sum_of_warps(sum, warps);
+    sum            = sum_of_warps<WARPS>(sum);
+    if (keeps_packed(WARPS, UNITS)) {
+#pragma unroll
+        for (int u = 0; u < UNITS; ++u) {
+            keep_packed(xv[u]);
+            keep_packed(gv[u]);
+        }
+    }
     const float mg = sum.x / static_cast<float>(cols), mgx = sum.y / static_cast<float>(cols);
     if (!here) {
         return;
@@ -409,30 +435,45 @@ __global__ void __launch_bounds__(256) layernorm_bwd_kernel(const __nv_bfloat16*
     }
     else {
         for (int64_t c = at.col; c < cols; c += at.stride) {
-            const uint4 a = add ? fu::ptx::ld_v4(ar + c) : none;
-            fu::ptx::st_v4(dr + c, norm_gradient(fu::ptx::ld_v4(xr + c), fu::ptx::ld_v4(gr + c), a, add != nullptr, mean, rstd, mg, mgx));
+            const uint4 a = add ? ld_unit(ar + c) : none;
+            fu::ptx::st_v4(dr + c, norm_gradient(ld_unit(xr + c), ld_unit(gr + c), a, add != nullptr, mean, rstd, mg, mgx));
         }
     }
 }
 
-// Values of a matrix beyond which the backward's four (x, dy, the residual's gradient, dx) are more than L2 holds.
+// Values of a matrix beyond which the backward's four (x, dy, the gradient to add, dx) are more than L2 holds.
 constexpr int64_t kNormInL2 = 12ll << 20;
 
 // As few warps a row as its units allow, so that little rows need no meeting through shared memory.
 struct RowShape {
-    int      warps, units;  // units: 0 for rows that no eight warps hold
+    int      lg_warps, units;  // units: 0 for rows that no eight warps hold
     unsigned blocks;
     RowShape(int64_t rows, int64_t cols)
     {
         const int64_t pieces = cols / 8;
-        for (warps = 1; warps < 8 && pieces > 32 * warps * kRowUnits;) {
-            warps *= 2;
+        for (lg_warps = 0; lg_warps < 3 && pieces > (32 << lg_warps) * kRowUnits;) {
+            ++lg_warps;
         }
-        const int64_t each = (pieces + 32 * warps - 1) / (32 * warps);
-        units              = each <= kRowUnits ? static_cast<int>(each) : 0;
-        blocks             = static_cast<unsigned>((rows + 8 / warps - 1) / (8 / warps));
+        const int64_t lanes = 32 << lg_warps, each = (pieces + lanes - 1) / lanes, at_once = 8 >> lg_warps;
+        units               = each <= kRowUnits ? static_cast<int>(each) : 0;
+        blocks              = static_cast<unsigned>((rows + at_once - 1) / at_once);
     }
 };
+
+// By the number of warps and of units; rows of two warps or more have at least three units a lane.
+using NormForward  = decltype(&layernorm_fwd_kernel<8, 0>);
+using NormBackward = decltype(&layernorm_bwd_kernel<1, 0>);
+constexpr NormForward kNormForward[4][kRowUnits + 1] = {
+    {nullptr, layernorm_fwd_kernel<1, 1>, layernorm_fwd_kernel<1, 2>, layernorm_fwd_kernel<1, 3>, layernorm_fwd_kernel<1, 4>, layernorm_fwd_kernel<1, 5>},
+    {nullptr, nullptr, nullptr, layernorm_fwd_kernel<2, 3>, layernorm_fwd_kernel<2, 4>, layernorm_fwd_kernel<2, 5>},
+    {nullptr, nullptr, nullptr, layernorm_fwd_kernel<4, 3>, layernorm_fwd_kernel<4, 4>, layernorm_fwd_kernel<4, 5>},
+    {layernorm_fwd_kernel<8, 0>, nullptr, nullptr, layernorm_fwd_kernel<8, 3>, layernorm_fwd_kernel<8, 4>, layernorm_fwd_kernel<8, 5>}};
+constexpr NormBackward kNormBackward[4][kRowUnits + 1] = {
+    {layernorm_bwd_kernel<1, 0>, layernorm_bwd_kernel<1, 1>, layernorm_bwd_kernel<1, 2>, layernorm_bwd_kernel<1, 3>, layernorm_bwd_kernel<1, 4>,
+     layernorm_bwd_kernel<1, 5>},
+    {layernorm_bwd_kernel<2, 0>, nullptr, nullptr, layernorm_bwd_kernel<2, 3>, layernorm_bwd_kernel<2, 4>, layernorm_bwd_kernel<2, 5>},
+    {layernorm_bwd_kernel<4, 0>, nullptr, nullptr, layernorm_bwd_kernel<4, 3>, layernorm_bwd_kernel<4, 4>, layernorm_bwd_kernel<4, 5>},
+    {layernorm_bwd_kernel<8, 0>, nullptr, nullptr, layernorm_bwd_kernel<8, 3>, layernorm_bwd_kernel<8, 4>, layernorm_bwd_kernel<8, 5>}};
 
 // ---- column sums (bias gradients) --------------------------------------------------------------------------
 // A cluster of eight CTAs owns 64 columns and splits the rows; a warp reads four rows of 128 bytes per
@@ -808,11 +849,8 @@ extern "C" int fu_layernorm_fwd(const void* x, void* y, float* stats, int64_t ro
         return fu::fail(FU_E_ARG, "fu_layernorm_fwd: needs 16-byte aligned rows of a multiple of 8 columns");
     }
     const RowShape shape(rows, cols);
-    decltype(&layernorm_fwd_kernel<0>) const kernels[kRowUnits + 1] = {layernorm_fwd_kernel<0>, layernorm_fwd_kernel<1>, layernorm_fwd_kernel<2>,
-                                                                       layernorm_fwd_kernel<3>, layernorm_fwd_kernel<4>, layernorm_fwd_kernel<5>};
-    FU_CUDA_OK(fu::launch_behind(kernels[shape.units], dim3(shape.blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
-                                 static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), stats, rows, cols, ldx, ldy, eps,
-                                 shape.warps));
+    FU_CUDA_OK(fu::launch_behind(kNormForward[shape.lg_warps][shape.units], dim3(shape.blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+                                 static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), stats, rows, cols, ldx, ldy, eps));
     return FU_OK;
 }
 
@@ -825,14 +863,12 @@ extern "C" int fu_layernorm_bwd_add(const void* dy, const void* x, const float* 
         return fu::fail(FU_E_ARG, "fu_layernorm_bwd_add: needs 16-byte aligned rows of a multiple of 8 columns");
     }
     RowShape shape(rows, cols);
-    if (rows * cols > kNormInL2 && shape.units > 1) {
+    if (add && rows * cols > kNormInL2) {
         shape.units = 0;
     }
-    decltype(&layernorm_bwd_kernel<0>) const kernels[kRowUnits + 1] = {layernorm_bwd_kernel<0>, layernorm_bwd_kernel<1>, layernorm_bwd_kernel<2>,
-                                                                       layernorm_bwd_kernel<3>, layernorm_bwd_kernel<4>, layernorm_bwd_kernel<5>};
-    FU_CUDA_OK(fu::launch_behind(kernels[shape.units], dim3(shape.blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
+    FU_CUDA_OK(fu::launch_behind(kNormBackward[shape.lg_warps][shape.units], dim3(shape.blocks), dim3(256), 0, static_cast<cudaStream_t>(stream),
                                  static_cast<const __nv_bfloat16*>(dy), static_cast<const __nv_bfloat16*>(x), stats,
-                                 static_cast<const __nv_bfloat16*>(add), static_cast<__nv_bfloat16*>(dx), rows, cols, ld, shape.warps));
+                                 static_cast<const __nv_bfloat16*>(add), static_cast<__nv_bfloat16*>(dx), rows, cols, ld));
     return FU_OK;
 }
 
