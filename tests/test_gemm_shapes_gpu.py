@@ -152,6 +152,17 @@ def test_halves_of_tiles_are_single_blocks(m, n, k, act, b_kn):
     gemm.check_errors()
 
 
+# small tiles with the erf GELU: one K-block more than 16 is no reason for another kernel (pairs took a quarter longer there)
+@pytest.mark.parametrize("m,n", [(1914, 7104), (1086, 4224)])
+@pytest.mark.parametrize("k", [1024, 1040, 1088])
+def test_shape_around_sixteen_k_blocks(m, n, k):
+    torch.manual_seed(k)
+    a, b = torch.randn(m, k, device="cuda").bfloat16(), torch.randn(n, k, device="cuda").bfloat16()
+    names = kernel_names(lambda: gemm.gemm_bf16(a, b, act=2))
+    assert len(names) == 1 and "gemm_small_kernel" in names[0], names
+    gemm.check_errors()
+
+
 # a hidden layer whose rows are an odd multiple of 16 bytes is kept with a wider pitch; one that is not, as it is
 @pytest.mark.parametrize("m,hidden,ffn", [(1, 8, 8), (130, 72, 264), (300, 128, 256), (257, 264, 1032)])
 def test_feed_forward_with_a_padded_hidden_layer(m, hidden, ffn):
