@@ -702,8 +702,8 @@ int pair_capacity()
 // Which core and tile a problem gets, from its size alone: the one whose estimated time is lowest. The
 // estimate is a start, per wave of CTAs a time per 64-wide K-block, and the epilogue. Fitted to products of 64 - 20000 rows,
 // 64 - 13824 columns and K, each timed in up to 24 shapes behind a launch of itself (us, SM clock 1.9 GHz). On 450 others of up to 9000 rows
-// the shape chosen takes 1.3 % more than the fastest one (geometric mean; 9 in 10 sizes less than 4.6 % more, one 35 %), on 200 of
-// up to 75600 rows 1.5 % (5.4 %, 37 %). With the epilogue's time left out it was 5.4 % once, with half of it for two blocks and launches of
+// the shape chosen takes 0.9 % more than the fastest one (geometric mean; 9 in 10 sizes less than 2 % more, one 30 %), on 200 of
+// up to 75600 rows 1.3 % (5.3 %, 25 %). With the epilogue's time left out it was 5.4 % once, with half of it for two blocks and launches of
 // nothing but halves of tiles 4.4 %. Small tiles and narrow blocks on few SMs are faster than this says since the producers look ahead.
 // All constants fitted again took 0.5 % off most sizes, and put 10 - 26 % on ten of 1500, of 40 - 100 us, which L2 bounds then: left.
 //   128 x 128 tiles on single CTAs   2.0 + 0.223 per K-block and wave of 148
@@ -747,7 +747,7 @@ double block_clocks(int mb, int nb, int width)
 }
 
 // us per K-block, by how many of the two operands lie off the 32-byte sectors
-constexpr double kSmallBlock[3] = {0.223, 0.28, 0.38}, kOneBlock[3] = {0.328, 0.34, 0.42}, kTwoBlocks[3] = {0.622, 0.65, 0.73};
+constexpr double kSmallBlock[3] = {0.223, 0.27, 0.38}, kOneBlock[3] = {0.328, 0.34, 0.42}, kTwoBlocks[3] = {0.622, 0.65, 0.73};
 constexpr double kSmallStart = 2.0, kPairStart = 2.6, kLong = 50.0;
 
 // us that the epilogue of a block of 256 columns takes, of a 128 x 128 tile with eight warps and with four, which share it in clusters.
@@ -755,8 +755,9 @@ constexpr double kSmallStart = 2.0, kPairStart = 2.6, kLong = 50.0;
 // four warps' figures (6043 x 5432 x 384 with the GELU's derivative 85.8 -> 63.7 us). 112 of them take more than 50 us and were repeated until
 // the power limit held, and one takes more than 2 % longer: beyond kLong small tiles need no margin against two whole blocks. With
 // more K-blocks the tiles' reads from L2, which are not counted here, make the estimate less sure: a small tile has to be faster than
-// pairs by `doubt` of its time from 32 K-blocks on, in proportion from 16. Of 600 products beyond 16 K-blocks whose shape is another than
-// with the four warps' figures, 247 take 3 - 25 % less and 111 3 - 19 % more. The projection's figures are fitted without.
+// pairs by `doubt` of its time from 24 K-blocks on, twice that with an operand off the sectors, in proportion from 16. Of 600
+// products beyond 16 K-blocks whose shape is another than with the four warps' figures, 279 take 3 - 24 % less and 77 3 - 14 % more.
+// The projection's figures are fitted without.
 struct Epilogue {
     double pair, small, shared, doubt;
     // A warp's share of a narrow block is half a unit, or more of it in pieces that are not whole.
@@ -766,7 +767,7 @@ struct Epilogue {
 Epilogue epilogue_of(int act, bool residual)
 {
     const double pair[4] = {2.4, 4.7, 7.3, 7.0}, small[4] = {1.2, 2.2, 4.4, 3.5}, shared[4] = {1.4, 3.2, 6.4, 5.5};
-    return {pair[act] + (residual ? 1.7 : 0.0), small[act] + (residual ? 1.0 : 0.0), shared[act] + (residual ? 1.0 : 0.0), 0.05};
+    return {pair[act] + (residual ? 1.7 : 0.0), small[act] + (residual ? 1.0 : 0.0), shared[act] + (residual ? 1.0 : 0.0), 0.04};
 }
 constexpr Epilogue kQkvEpilogue{7.0, 4.0, 4.0, 0.0};  // fitted to 100 projections of 64 - 75600 rows, 1 - 40 heads: 0.9 % above the fastest shape
 
@@ -828,7 +829,8 @@ Choice choose_shape(int64_t m, int64_t n, int64_t k, int pairs, int sms, int fla
     if (best.cost >= (two.cost <= kLong ? 1.0 : off > 0 ? 0.88 : 0.92) * two.cost) {
         best = two;
     }
-    return small.cost * (1.0 + epi.doubt * std::min(1.0, std::max(0.0, kb - 16.0) / 16.0)) < best.cost ? small : best;
+    const double doubt = (off > 0 ? 2.0 : 1.0) * epi.doubt * std::min(1.0, std::max(0.0, kb - 16.0) / 8.0);
+    return small.cost * (1.0 + doubt) < best.cost ? small : best;
 }
 
 // The broad tiles with what whole waves leave over shared by clusters (gemm_wide_split_kernel), when that is
