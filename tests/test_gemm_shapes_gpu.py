@@ -152,6 +152,24 @@ def test_halves_of_tiles_are_single_blocks(m, n, k, act, b_kn):
     gemm.check_errors()
 
 
+# single blocks on pairs, whose operands have a producer each: many items to a pair, K one block short of the ring of six, as long,
+# longer by one, twice round and more with a part; then one item to a pair or two, of 160 to 256 columns. Both kinds of B.
+@pytest.mark.parametrize("m,n,k,b_kn,ctas", [(905, 936, 320, True, 4), (1348, 160, 384, False, 4), (928, 920, 384, True, 4), (1286, 160, 448, False, 4),
+                                             (922, 904, 448, True, 4), (1441, 400, 768, False, 4), (641, 1160, 768, True, 4),
+                                             (641, 528, 1032, False, 4), (1159, 656, 1032, True, 4), (388, 4744, 2696, False, 0),
+                                             (265, 6304, 2432, False, 0), (258, 7208, 3088, True, 0), (802, 2704, 1112, False, 0)])
+def test_single_blocks_with_a_producer_for_each_operand(m, n, k, b_kn, ctas):
+    gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+    a, b = torch.randn(m, k, device="cuda", generator=gen).bfloat16(), torch.randn(n, k, device="cuda", generator=gen).bfloat16()
+    other = b.t().contiguous() if b_kn else b
+    names = kernel_names(lambda: gemm.gemm_bf16(a, other, b_kn=b_kn, ctas=ctas))
+    assert len(names) == 1 and "gemm_wide_kernelILi1ELi1E" in names[0], names
+    got = gemm.gemm_bf16(a, other, b_kn=b_kn, ctas=ctas)
+    gemm.check_errors()
+    assert rel_err(got, a.float() @ b.float().t()) < 4e-3  # bf16 rounding of the result, as above
+    assert torch.equal(got, gemm.gemm_bf16(a, b, pair=False))
+
+
 # small tiles with the erf GELU: one K-block more than 16 is no reason for another kernel (pairs took a quarter longer there)
 @pytest.mark.parametrize("m,n", [(1914, 7104), (1086, 4224)])
 @pytest.mark.parametrize("k", [1024, 1040, 1088])

@@ -91,8 +91,9 @@ def _block(group, m, heads, ffn):
 
 
 PROGRAMS = {"forward": _forward, "exchange": _exchange, "sums": _sums, "block": _block}
-# one tile and several, single CTAs and pairs, attention of whole and of single query tiles
-SIZES = [(20, 1, 64), (140, 2, 520), (1100, 5, 2048), (4100, 12, 1536)]
+# one tile and several, single CTAs and pairs, attention of whole and of single query tiles; LayerNorm's rows of one, two, four and
+# eight warps, and a matrix whose backward walks through them
+SIZES = [(20, 1, 64), (140, 2, 520), (1100, 5, 2048), (4100, 12, 1536), (4000, 25, 512), (20, 41, 64)]
 
 
 def _prepared(name, size, group):

@@ -27,10 +27,10 @@ does not divide and an odd number of tiles, and checks in every reachable state 
 
 Negative controls: the same search with the producer's parity un-flipped, and with the accumulator
 barrier counting one warp too few, must each find a violation. `run_small` has the same structure on
-128 x 128 tiles.
+128 x 128 tiles; its producer also looks at the next stage's barrier while it loads this one and then need not wait for it.
 
 `fu::gemm::run_wide` (pairs of CTAs, two accumulator blocks or one) orders its work differently and is searched
-by itself: see `explore_wide`.
+by itself: see `explore_wide`. With one block its operands have a producer each, and both look at the next stage ahead of time.
 """
 
 import pytest
@@ -53,12 +53,13 @@ class Bar:
         return b[0] != parity
 
 
-def explore(stages=3, kblocks=2, tiles=3, warps=2, producer_flip=1, empty_count=None):
+def explore(stages=3, kblocks=2, tiles=3, warps=2, producer_flip=1, empty_count=None, look_flip=None):
+    """`look_flip`: the producer looks at the next stage's barrier while it fills this one (None: it does not)."""
     empty_count = warps if empty_count is None else empty_count
     total = tiles * kblocks
-    # state: producer it, mma (tile, kb, waiting_acc), epilogue per-warp tile index,
+    # state: producer it and whether it knows its stage to be free, mma (tile, kb, waiting_acc), epilogue per-warp tile index,
     #        barriers, stage contents, stage consumed marks, accumulator contents and drain marks
-    init = (0, (0, 0, True), tuple([0] * warps),
+    init = ((0, False), (0, 0, True), tuple([0] * warps),
             tuple(Bar.new(1) for _ in range(stages)), tuple(Bar.new(1) for _ in range(stages)),
             (Bar.new(1), Bar.new(1)), (Bar.new(empty_count), Bar.new(empty_count)),
             tuple([-1] * stages), tuple([True] * stages),  # stage holds item, stage has been read
@@ -66,7 +67,8 @@ def explore(stages=3, kblocks=2, tiles=3, warps=2, producer_flip=1, empty_count=
     seen, stack = {init}, [init]
     while stack:
         st = stack.pop()
-        p_it, (m_tile, m_kb, m_wait), e_tiles, full, empty, tfull, tempty, holds, read, acc, drained = st
+        prod, (m_tile, m_kb, m_wait), e_tiles, full, empty, tfull, tempty, holds, read, acc, drained = st
+        p_it, ready = prod
         done = p_it == total and m_tile == tiles and all(t == tiles for t in e_tiles)
         if done:
             continue
@@ -74,14 +76,17 @@ def explore(stages=3, kblocks=2, tiles=3, warps=2, producer_flip=1, empty_count=
         # ---- producer
         if p_it < total:
             s = p_it % stages
-            if Bar.passes(empty[s], ((p_it // stages) & 1) ^ producer_flip):
+            if ready or Bar.passes(empty[s], ((p_it // stages) & 1) ^ producer_flip):
                 if not read[s]:
                     return f"producer refills stage {s} (item {holds[s]}) before the MMA has read it"
                 h, r, f = list(holds), list(read), list(full)
                 h[s], r[s] = p_it, False
                 f[s] = Bar.arrive(f[s])
-                nxt_states.append((p_it + 1, (m_tile, m_kb, m_wait), e_tiles, tuple(f), empty, tfull, tempty,
-                                   tuple(h), tuple(r), acc, drained))
+                ahead = p_it + 1
+                free = look_flip is not None and Bar.passes(empty[ahead % stages], ((ahead // stages) & 1) ^ look_flip)
+                for seen_free in {free, False}:  # it may be looked at before the barrier says so
+                    nxt_states.append(((ahead, seen_free), (m_tile, m_kb, m_wait), e_tiles, tuple(f), empty, tfull, tempty,
+                                       tuple(h), tuple(r), acc, drained))
         # ---- MMA thread
         if m_tile < tiles:
             a = m_tile & 1
@@ -91,7 +96,7 @@ def explore(stages=3, kblocks=2, tiles=3, warps=2, producer_flip=1, empty_count=
                         return f"MMA starts tile {m_tile} in accumulator {a} before every epilogue warp has drained tile {acc[a][0]}"
                     ac = list(acc)
                     ac[a] = (m_tile, 0)
-                    nxt_states.append((p_it, (m_tile, 0, False), e_tiles, full, empty, tfull, tempty, holds, read,
+                    nxt_states.append((prod, (m_tile, 0, False), e_tiles, full, empty, tfull, tempty, holds, read,
                                        tuple(ac), drained))
             else:
                 it = m_tile * kblocks + m_kb
@@ -106,10 +111,10 @@ def explore(stages=3, kblocks=2, tiles=3, warps=2, producer_flip=1, empty_count=
                     if m_kb + 1 == kblocks:
                         tf[a] = Bar.arrive(tf[a])
                         dr[a] = (False,) * warps
-                        nxt_states.append((p_it, (m_tile + 1, 0, True), e_tiles, full, tuple(e), tuple(tf), tempty,
+                        nxt_states.append((prod, (m_tile + 1, 0, True), e_tiles, full, tuple(e), tuple(tf), tempty,
                                            holds, tuple(r), tuple(ac), tuple(dr)))
                     else:
-                        nxt_states.append((p_it, (m_tile, m_kb + 1, False), e_tiles, full, tuple(e), tfull, tempty,
+                        nxt_states.append((prod, (m_tile, m_kb + 1, False), e_tiles, full, tuple(e), tfull, tempty,
                                            holds, tuple(r), tuple(ac), drained))
         # ---- epilogue warps
         for w in range(warps):
@@ -126,7 +131,7 @@ def explore(stages=3, kblocks=2, tiles=3, warps=2, producer_flip=1, empty_count=
                 d = list(dr[a])
                 d[w] = True
                 dr[a] = tuple(d)
-                nxt_states.append((p_it, (m_tile, m_kb, m_wait), tuple(et), full, empty, tfull, tuple(te), holds, read,
+                nxt_states.append((prod, (m_tile, m_kb, m_wait), tuple(et), full, empty, tfull, tuple(te), holds, read,
                                    acc, tuple(dr)))
         if not nxt_states:
             return f"deadlock: producer at {p_it}, MMA at {(m_tile, m_kb)}, epilogue at {e_tiles}"
@@ -140,6 +145,12 @@ def explore(stages=3, kblocks=2, tiles=3, warps=2, producer_flip=1, empty_count=
 @pytest.mark.parametrize("stages,kblocks,tiles,warps", [(4, 3, 3, 2), (3, 2, 5, 2), (4, 1, 5, 2), (2, 5, 3, 4), (4, 6, 2, 4)])
 def test_pipeline_parities_hold_in_every_interleaving(stages, kblocks, tiles, warps):
     assert explore(stages, kblocks, tiles, warps) is None
+    assert explore(stages, kblocks, tiles, warps, look_flip=1) is None  # run_small
+
+
+def test_a_producer_looking_ahead_for_the_wrong_parity_is_found():
+    found = explore(3, 2, 3, 2, look_flip=0)
+    assert found is not None and "refills" in found
 
 
 def test_a_producer_waiting_for_the_wrong_parity_is_found():
@@ -194,21 +205,39 @@ def mma_program(items, stages, kblocks, release_early=False):
     return ops
 
 
-def explore_wide(items, stages=2, kblocks=3, warps=1, flip=1, empty_warps=None, release_early=False):
-    """Every interleaving of the two producers (a stage is full when both CTAs' loads have landed), the issuing warp
-    of the even CTA, whose commits reach both CTAs, and `warps` epilogue warps per CTA, which all arrive on the even
-    CTA's barrier when they have copied a block out. Returns what goes wrong, or None."""
+class Bytes:
+    """The mbarrier of a stage: phase parity, whether its bytes have been announced, parts of them that have landed. Parts may land
+    before the announcement; the phase completes with both."""
+
+    @staticmethod
+    def new():
+        return (0, 0, 0)
+
+    @staticmethod
+    def add(b, parts, announced, landed):
+        parity, a, n = b[0], b[1] + announced, b[2] + landed
+        assert a <= 1 and n <= parts, "more than a phase takes"
+        return (parity ^ 1, 0, 0) if a == 1 and n == parts else (parity, a, n)
+
+
+def explore_wide(items, stages=2, kblocks=3, warps=1, flip=1, empty_warps=None, release_early=False, operands=1, look_flip=1, announcers=1):
+    """Every interleaving of the producers (one per CTA, or with `operands` = 2 one for each of its operands, which look at the next
+    stage while they load this one; a stage is full when the even CTA's first producer has announced all bytes and they have
+    landed), the issuing warp of the even CTA, whose commits reach both CTAs, and `warps` epilogue warps per CTA, which all arrive
+    on the even CTA's barrier when they have copied a block out. Returns what goes wrong, or None."""
+    assert operands == 1 or all(u1 - u0 <= 1 for u0, u1 in items)  # in the kernel, where a pair has one block at a time
     loads = [(n, kb) for n, (u0, u1) in enumerate(items) if u0 != u1 for kb in range(kblocks)]
     blocks = [(n, u) for n, (u0, u1) in enumerate(items) for u in range(u0, u1)]
     ops = mma_program(items, stages, kblocks, release_early)
     total = 2 * warps
     empty_count = total if empty_warps is None else empty_warps
     reads_of = [items[n][1] - items[n][0] for n in range(len(items))]
-    # producers' positions, MMA program counter, positions of the epilogue warps;
-    # full (one barrier, on the even CTA), empty (one per CTA), tmem_full, tmem_empty; what each CTA's half of a stage
+    parts = 2 * operands  # of a stage, each loaded by a producer of its own
+    # producers' positions and what they know of the stage there; MMA program counter, positions of the epilogue warps;
+    # full (one barrier, on the even CTA), empty (one per CTA), tmem_full, tmem_empty; what each part of a stage
     # holds and how many blocks have read it; each accumulator's (item, K-blocks added) and who has still to drain it
-    init = ((0, 0), 0, (0,) * total, (Bar.new(2),) * stages, (Bar.new(1),) * stages, (Bar.new(1),) * 2, (Bar.new(empty_count),) * 2,
-            ((None, 0),) * (2 * stages), ((-1, 0),) * 2, (0,) * 2)
+    init = (((0, False),) * parts, 0, (0,) * total, (Bytes.new(),) * stages, (Bar.new(1),) * stages, (Bar.new(1),) * 2,
+            (Bar.new(empty_count),) * 2, ((None, 0),) * (parts * stages), ((-1, 0),) * 2, (0,) * 2)
     seen, stack = {init}, [init]
 
     def put(t, at, value):
@@ -217,15 +246,22 @@ def explore_wide(items, stages=2, kblocks=3, warps=1, flip=1, empty_warps=None, 
     while stack:
         prod, pc, epi, full, empty, tfull, tempty, held, acc, todo = stack.pop()
         nxt = []
-        for c in range(2):
-            if prod[c] < len(loads):
-                s, ph = prod[c] % stages, ((prod[c] // stages) & 1) ^ flip
-                if Bar.passes(empty[s], ph):  # the commit reaches both CTAs' barriers at once
-                    item, reads = held[2 * s + c]
+        for c in range(parts):
+            at, ready = prod[c]
+            if at < len(loads):
+                s, ph = at % stages, ((at // stages) & 1) ^ flip
+                if ready or Bar.passes(empty[s], ph):  # the commit reaches both CTAs' barriers at once
+                    item, reads = held[parts * s + c]
                     if item is not None and reads < reads_of[item[0]]:
-                        return f"CTA {c} refills stage {s} ({item}) after {reads} reads"
-                    nxt.append((put(prod, c, prod[c] + 1), pc, epi, put(full, s, Bar.arrive(full[s])), empty, tfull, tempty,
-                                put(held, 2 * s + c, (loads[prod[c]], 0)), acc, todo))
+                        return f"producer {c} refills stage {s} ({item}) after {reads} reads"
+                    free = operands == 2 and Bar.passes(empty[(at + 1) % stages], (((at + 1) // stages) & 1) ^ look_flip)
+                    try:
+                        landed = Bytes.add(full[s], parts, int(c < announcers), 1)
+                    except AssertionError as e:
+                        return f"stage {s}: {e}"
+                    for seen_free in {free, False}:  # it may be looked at before the barrier says so
+                        nxt.append((put(prod, c, (at + 1, seen_free)), pc, epi, put(full, s, landed), empty, tfull, tempty,
+                                    put(held, parts * s + c, (loads[at], 0)), acc, todo))
         if pc < len(ops):
             op = ops[pc]
             state = None
@@ -240,10 +276,10 @@ def explore_wide(items, stages=2, kblocks=3, warps=1, flip=1, empty_warps=None, 
             elif op[0] == "mma":
                 _, item, u, kb, s = op
                 new = held
-                for c in range(2):
-                    if held[2 * s + c][0] != (item, kb):
-                        return f"the MMA of {(item, u, kb)} finds {held[2 * s + c][0]} in stage {s} of CTA {c}"
-                    new = put(new, 2 * s + c, ((item, kb), held[2 * s + c][1] + 1))
+                for c in range(parts):
+                    if held[parts * s + c][0] != (item, kb):
+                        return f"the MMA of {(item, u, kb)} finds {held[parts * s + c][0]} in part {c} of stage {s}"
+                    new = put(new, parts * s + c, ((item, kb), held[parts * s + c][1] + 1))
                 if kb != 0 and acc[u] != (item, kb):
                     return f"the MMA of {(item, u, kb)} adds to {acc[u]}"
                 state = (prod, pc + 1, epi, full, empty, tfull, tempty, new, put(acc, u, (item, kb + 1)), todo)
@@ -263,7 +299,7 @@ def explore_wide(items, stages=2, kblocks=3, warps=1, flip=1, empty_warps=None, 
                         return f"epilogue warp {w} reads block {u} for item {item} and finds {acc[u]}"
                     nxt.append((prod, pc, put(epi, w, epi[w] + 1), full, empty, tfull, put(tempty, u, Bar.arrive(tempty[u])), held, acc,
                                 put(todo, u, todo[u] - 1)))
-        if not nxt and (pc < len(ops) or min(prod) < len(loads) or min(epi) < len(blocks)):
+        if not nxt and (pc < len(ops) or min(prod)[0] < len(loads) or min(epi) < len(blocks)):
             return f"deadlock: producers at {prod}, MMA at {ops[pc:pc + 1]}, epilogue at {epi}"
         for n in nxt:
             if n not in seen:
@@ -288,6 +324,19 @@ def test_two_blocks_of_a_pair_hold_in_every_interleaving(stages, kblocks, items)
 @pytest.mark.parametrize("stages,kblocks", [(2, 1), (2, 3), (3, 2), (3, 4)])
 def test_alternating_blocks_of_a_pair_hold_in_every_interleaving(stages, kblocks):
     assert explore_wide((FIRST, SECOND, FIRST, SECOND, FIRST), stages, kblocks) is None
+
+
+# the same with a producer for each operand: two announce nothing, and all may know from looking ahead that a stage is free
+@pytest.mark.parametrize("stages,kblocks,items", [(2, 1, (FIRST, SECOND, FIRST)), (2, 3, (FIRST, SECOND)), (3, 2, (FIRST, SECOND, FIRST)), (3, 4, (FIRST, OUTSIDE, SECOND))])
+def test_a_producer_for_each_operand_holds_in_every_interleaving(stages, kblocks, items):
+    assert explore_wide(items, stages, kblocks, operands=2) is None
+
+
+# looking for the wrong parity; both operands of the even CTA announced; none
+@pytest.mark.parametrize("fault,text", [(dict(look_flip=0), ("refills",)), (dict(announcers=2), ("more than a phase", "finds")), (dict(announcers=0), ("deadlock",))])
+def test_faults_of_the_operands_producers_are_found(fault, text):
+    found = explore_wide((FIRST, SECOND, FIRST), 2, 3, operands=2, **fault)
+    assert found is not None and any(t in found for t in text), found
 
 
 @pytest.mark.parametrize("fault,text", [(dict(flip=0), ("deadlock", "refills")), (dict(empty_warps=1), ("before every", "finds", "adds", "deadlock")),
