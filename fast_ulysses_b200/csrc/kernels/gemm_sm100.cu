@@ -76,7 +76,7 @@ struct PlainEpi {
 
     // The bias of the 128 columns from col0 on, four a lane, while their products are still being computed: the loads' latency
     // behind the products cost a unit 0.7 us (256 x 512 x 256 with GELU 5.9 us so, 6.7 with read-only loads of all 64 columns by
-    // every thread, 10 % more with ordinary ones).
+    // every thread, 10 % more with ordinary ones). A warp with 64 columns fetches 128 too: told not to, launches take 0.3 % longer.
     __device__ __forceinline__ void fetch(int col0, int lane)
     {
         if (bias) {

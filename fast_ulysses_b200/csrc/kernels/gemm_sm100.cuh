@@ -225,6 +225,7 @@ __device__ __forceinline__ void run(const Core& core, Epi& epi, Src src, Aux aux
 //   void fetch(int col0, int lane)        before a unit's products are waited for: what can be read ahead
 //   void open(int epi_tid), close(int epi_tid)          all epilogue threads, once before / after the tiles
 //   void unit(uint32_t (&r)[128], int row0, int col0, int col_end, int lane, uint32_t stage)
+//   void unit(uint32_t (&r)[64], ...)     the same of half as many columns, for run_small with 64 columns a warp
 // Columns from `col_end` on are not the unit's. `stage` is the address of 4 KiB of shared memory of this warp's own (32 rows x 128 bytes).
 constexpr int UNIT_STAGE_BYTES = 32 * 128;
 
