@@ -278,8 +278,8 @@ __device__ __forceinline__ uint4 normalised(const uint4& v, float mean, float rs
     return make_uint4(o[0], o[1], o[2], o[3]);
 }
 
-// UNITS: of a lane, 0 for rows of any length. The registers of three units with several warps, 45, are one too many for a sixth CTA
-// (75600 x 1288 65.8 -> 64.3 us, 9450 x 2568 16.6 -> 15.8).
+// UNITS: of a lane, 0 for rows of any length. Three units with several warps take 45 registers, which leaves room for five CTAs; with 40
+// there are six (75600 x 1288 65.8 -> 64.3 us, 9450 x 2568 16.6 -> 15.8).
 template <int WARPS, int UNITS>
 __global__ void __launch_bounds__(256, WARPS > 1 && UNITS == 3 ? 6 : 0)
     layernorm_fwd_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, float* stats, int64_t rows, int64_t cols, int64_t ldx, int64_t ldy, float eps)

@@ -21,9 +21,11 @@
 // descriptors are ready (8 per product: 512), a tensor-memory load-and-wait about 200, and the fp32
 // reductions of all SMs together move 6.1 TB/s into L2 whatever their width (64 KiB per block: 3130
 // clocks). The dependent chain dP -> C2 -> dK, dQ -> drain -> dP sets the period, about 3700 clocks against
-// the 2560 of the products (4050 while the statistics were read one value at a time); with random operands the power limit
-// lowers the clock below that (37888 tokens x 4 heads, repeated for seconds: 4.84 ms with zeros and 6.7 with random numbers,
-// 5.12 and 6.94 before). Tried and no faster: dK begun on the first
+// the 2560 of the products. With random operands the power limit lowers the clock below that. 37888 tokens x 4 heads: 4.83 ms with
+// zeros, with random numbers 5.91 in a launch by itself and 6.78 in launches repeated for seconds. With one thing as it was before (ms with
+// zeros; all of them 5.12, 6.09, 6.99 and a chain of 4050): statistics read one value at a time 5.14, dS stored eight registers at a time
+// 5.11, P in one piece 4.93, arithmetic that is not packed 4.85, the check for kv rows that do not exist in the inner loop 4.85.
+// Tried and no faster: dK begun on the first
 // half of dS, the products issued by three warps, paced issue, a share of the exponentials on the FMA pipe.
 // Warps: 0 = TMA producer, 1 = MMA issuer, 2..9 = two threads per kv row, 10..17 = dQ drain.
 #include "cluster_plan.h"
@@ -598,8 +600,8 @@ __global__ void __launch_bounds__(THREADS, 1) fmha_bwd_fused_kernel(const __grid
         // contiguous bytes of one query row. Warps 10..13 take query columns 0..63, warps 14..17
         // columns 64..127. The columns are released as soon as they are in registers. What waits in the memory queue
         // behind a burst of reductions is every other warp's loads, stores and products: the address arithmetic between them
-        // is what keeps them apart (37888 x 4 with zeros 4.92 ms then; with rows at constant offsets 6.35, four floats
-        // a reduction 6.81, spaced out by the clock 5.0 - 6.4).
+        // is what keeps them apart (37888 x 4 with zeros, beside 4.92 ms of the kernel of that time: rows at constant offsets 6.35, four
+        // floats a reduction 6.81, paced by the clock 5.0 - 5.3 in groups of two or four and 6.4 one by one, by nanosleep 5.56).
         const int      quarter  = warp & 3;
         const int      qh       = (warp - 10) >> 2;
         const int      dcol     = quarter * 32 + lane;
