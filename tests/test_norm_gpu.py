@@ -53,6 +53,24 @@ def test_layer_norm_rows_of_every_form(rows, cols):
         assert ((got.double() - want).abs() <= 2**-8 * want.abs() + 1e-4).all()
 
 
+# beyond L2: in registers without a gradient to add, with one walked through, rows of one unit too
+@pytest.mark.parametrize("rows, cols", [(50001, 256), (9831, 1288), (2501, 5120), (1301, 10240)])
+@pytest.mark.parametrize("fork", [False, True])
+def test_layer_norm_backward_beyond_l2(rows, cols, fork):
+    gen = torch.Generator(device="cuda").manual_seed(rows + cols)
+    x, g, r = (torch.randn(rows, cols, device="cuda", generator=gen).bfloat16() for _ in range(3))
+    x.requires_grad_()
+    if fork:
+        torch.autograd.backward(layer_norm_fork(x), (g, r))
+    else:
+        layer_norm(x).backward(g)
+    xr = x.detach().double().requires_grad_()
+    torch.nn.functional.layer_norm(xr, (cols,), eps=1e-6).backward(g.double())
+    want = xr.grad + r.double() if fork else xr.grad
+    # one rounding to bf16 (2^-9 of the value) and fp32 sums of values of a few units
+    assert ((x.grad.double() - want).abs() <= 2**-8 * want.abs() + 1e-4).all()
+
+
 # a mean that has overflowed: -inf in every column, whether or not the row fills its lanes
 @pytest.mark.parametrize("cols", [256, 264, 1288, 5128, 10248])
 def test_layer_norm_backward_of_an_overflowed_mean(cols):
